@@ -12,6 +12,7 @@
 #include "comm.h"
 #include "elementwise.h"
 #include "gemm.h"
+#include "gemm_half.h"
 #include "jacobi.h"
 #include "qr.h"
 #include "tridiag.h"
@@ -92,6 +93,35 @@ PYBIND11_MODULE(_C, m) {
 
   m.def("gemm_use_cta_pairs", [](bool on) { gemm_use_cta_pairs(on); },
         "Large plain GEMMs on CTA pairs (cta_group::2, default) or on single CTAs");
+
+  m.def("gemm_half",
+        [](uint64_t a_h, uint64_t a_l, int64_t lda, uint64_t a_scale, int64_t a_stride, uint64_t b_h, uint64_t b_l, int64_t ldb,
+           uint64_t b_scale, int64_t b_stride, int M, int N, int K, int mode, int symmetric, int tiles, float alpha, float beta,
+           uint64_t C, int64_t ldc, uint64_t Ch, uint64_t Cl, int64_t ldp, uint64_t Cscale, int64_t ldscale, uint64_t mom,
+           int64_t ldm, uint64_t var, int64_t ldv, float beta1, float beta2, float eps, float inv_bc1, float inv_sqrt_bc2,
+           uint64_t status, uint64_t stream) {
+          const HalfOperand a{ptr<const uint16_t>(a_h), ptr<const uint16_t>(a_l), lda, ptr<const float>(a_scale), a_stride};
+          const HalfOperand b{ptr<const uint16_t>(b_h), ptr<const uint16_t>(b_l), ldb, ptr<const float>(b_scale), b_stride};
+          HalfProblem p{};
+          p.M = M; p.N = N; p.K = K; p.mode = mode; p.symmetric = symmetric; p.tiles = tiles;
+          p.alpha = alpha; p.beta = beta; p.C = ptr<float>(C); p.ldc = ldc;
+          p.Ch = ptr<uint16_t>(Ch); p.Cl = ptr<uint16_t>(Cl); p.ldp = ldp; p.Cscale = ptr<float>(Cscale); p.ldscale = ldscale;
+          p.mom = ptr<float>(mom); p.ldm = ldm; p.var = ptr<float>(var); p.ldv = ldv;
+          p.beta1 = beta1; p.beta2 = beta2; p.eps = eps; p.inv_bc1 = inv_bc1; p.inv_sqrt_bc2 = inv_sqrt_bc2;
+          gemm_half(a, b, p, ptr<int>(status), stream_of(stream));
+        },
+        "acc[m,n] = sum_k Za[k,m] Zb[k,n] from scaled fp16 planes, with fused epilogue (gemm_half.h)");
+
+  m.def("half_planes",
+        [](uint64_t src, int source_type, int64_t s_i, int64_t s_j, int rows, int cols, uint64_t ph, uint64_t pl, int64_t pld,
+           uint64_t pscale, uint64_t plargest, uint64_t th, uint64_t tl, int64_t tld, uint64_t tscale, uint64_t tlargest,
+           uint64_t stream) {
+          half_planes(ptr<const void>(src), source_type, s_i, s_j, rows, cols,
+                      HalfTarget{ptr<uint16_t>(ph), ptr<uint16_t>(pl), pld, ptr<float>(pscale), ptr<uint32_t>(plargest)},
+                      HalfTarget{ptr<uint16_t>(th), ptr<uint16_t>(tl), tld, ptr<float>(tscale), ptr<uint32_t>(tlargest)},
+                      stream_of(stream));
+        },
+        "Scaled fp16 operand planes of a matrix in one or both orientations (gemm_half.h)");
 
   m.def("gemm_simt",
         [](uint64_t A, int64_t a_sk, int64_t a_sm, uint64_t B, int64_t b_sk, int64_t b_sn, uint64_t C, int64_t c_sm,

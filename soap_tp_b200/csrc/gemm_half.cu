@@ -1,0 +1,532 @@
+// C = op(A^T B) at fp32 accuracy from scaled fp16 planes (gemm_half.h) on 5th-generation tensor cores.
+//
+// acc[m, n] = sum_k Za[k, m] * Zb[k, n], both operands K-contiguous.  Each fp32 value is a pair of fp16 numbers times a
+// power of two, so a product is three fp16 MMAs, l*h + h*l + h*h (two, or one, where an operand comes from 16-bit values
+// and has no l), against one tf32 MMA (half the fp16 rate) and two bf16 ones of the mixed form in gemm_tf32x3.cu: 3/4 of
+// the tensor time, half the operand bytes, and a representation that is off by 2^-23 instead of 2^-20.
+//
+// Structure (192 KB of stages, one CTA per SM, 320 threads):
+//   warp 0, one lane : TMA producer - up to four boxes of 128 rows x 64 fp16 (128-byte swizzle) per stage
+//   warp 1, one lane : MMA issuer
+//   warps 2..9       : promotion and epilogue
+// PAIR: the two CTAs of a cluster share a 256 x 256 tile (cta_group::2, each stages its own 128 rows of A and half of the
+// rows of B, no multicast); otherwise one CTA computes 128 x 128.  TMA zero-fills rows and K beyond the operands.
+//
+// The tensor core adds into its accumulator with truncation, so the accumulator is drained every 128 of K into a
+// register-resident sum (round-to-nearest), multiplied by the scale of A's block of 128 on the way; B's scales are per
+// column and applied once, in the epilogue.  Within a chunk the small products come first.
+#include <cuda.h>
+#include <cuda_fp16.h>
+#include <cuda_runtime.h>
+
+#include <mutex>
+#include <stdexcept>
+#include <string>
+
+#include "gemm.h"
+#include "gemm_half.h"
+#include "launch_util.h"
+#include "ptx.cuh"
+
+namespace soapb200 {
+namespace {
+
+constexpr int kBM = 128;
+constexpr int kBK = 64;                          // one 128-byte swizzle row of fp16
+constexpr int kChunkBlocks = 2;                  // k-blocks per promotion: 128 of K
+static_assert(kBK * kChunkBlocks == kHalfScaleBlock, "one block of A's scales per promotion");
+constexpr int kBoxBytes = 128 * kBK * 2;
+constexpr int kStagePool = 12 * kBoxBytes;       // 3 stages of four boxes, 4 of three, 6 of two
+constexpr int kMaxStages = 6;
+constexpr int kEpiWarps = 8;
+constexpr int kThreads = 64 + 32 * kEpiWarps;
+constexpr int kSmemBytes = kStagePool + 1024 + 256;
+// Between A's factor and B's the sums are kept 2^-16 below scale: B's planes are 2^14 and more above scale where B is of
+// order one, and a large A must not overflow before B's factor brings the product back into range.
+constexpr float kDown = 1.0f / 65536.0f, kUp = 65536.0f;
+
+struct alignas(64) HalfMaps {
+  CUtensorMap a_h, a_l, b_h, b_l;
+};
+
+struct HalfArgs {
+  HalfProblem p;
+  const float* a_scale;
+  int64_t a_stride;
+  const float* b_scale;
+  int a_terms, b_terms;
+};
+
+constexpr int kUnroll = 4;       // columns per warp whose loads are in flight together
+constexpr int kRowsPerLane = 4;  // a column of the tile is 128 rows: rows lane, lane + 32, lane + 64, lane + 96
+
+// One column of the tile (four values per lane: rows 2 * lane, 2 * lane + 1, and those 64 further) as an operand of the next
+// product, with the scale of its own 128 rows.
+__device__ __forceinline__ void store_half_column(const HalfProblem& p, int m0, int n, int lane, const float (&v)[4]) {
+  uint32_t most = 0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) most = max(most, __float_as_uint(v[i]) & 0x7fffffffu);
+  const HalfScale s = half_scale(__reduce_max_sync(0xffffffffu, most));
+  if (lane == 0) p.Cscale[(m0 / kHalfScaleBlock) * p.ldscale + n] = s.inverse;
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int m = m0 + 64 * i + 2 * lane;
+    if (m < p.M) {       // pitches are multiples of 64: the second half of a last odd row lands in the padding
+      const float x0 = v[2 * i] * s.multiplier, x1 = v[2 * i + 1] * s.multiplier;
+      const __half2 h = __floats2half2_rn(x0, x1);
+      const float2 back = __half22float2(h);
+      *reinterpret_cast<__half2*>(p.Ch + m + static_cast<int64_t>(n) * p.ldp) = h;
+      *reinterpret_cast<__half2*>(p.Cl + m + static_cast<int64_t>(n) * p.ldp) = __floats2half2_rn(x0 - back.x, x1 - back.y);
+    }
+  }
+}
+
+// Epilogue over the staged tile: tile[n_local * PITCH + m_local] holds sums 2^-16 below scale, without B's scales.  Accesses
+// are four bytes per lane along M, so that no alignment of the outputs is needed, with kUnroll columns in flight.
+template <int BN, int MODE, int PITCH>
+__device__ __forceinline__ void half_epilogue(const HalfArgs& args, float* tile, int m0, int n0, int ew, int lane) {
+  const HalfProblem& p = args.p;
+  const int rows = min(kBM, p.M - m0), cols = min(BN, p.N - n0);
+  const float alpha = p.alpha * kUp;
+  if constexpr (MODE == kEpiRowMajor) {
+    float scale[BN / 32];
+#pragma unroll
+    for (int j = 0; j < BN / 32; ++j) scale[j] = (lane + 32 * j < cols) ? args.b_scale[n0 + lane + 32 * j] : 0.f;
+    for (int r = ew; r < rows; r += kEpiWarps) {
+      float* dst = p.C + static_cast<int64_t>(m0 + r) * p.ldc + n0;
+#pragma unroll
+      for (int j = 0; j < BN / 32; ++j) {
+        const int n = lane + 32 * j;
+        if (n < cols) dst[n] = alpha * (tile[n * PITCH + r] * scale[j]);
+      }
+    }
+  } else if constexpr (MODE == kEpiSplit) {
+    for (int nl = ew; nl < cols; nl += kEpiWarps) {
+      const float scale = args.b_scale[n0 + nl];
+      float v[4];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const float2 x = *reinterpret_cast<const float2*>(tile + nl * PITCH + 64 * i + 2 * lane);
+        v[2 * i] = alpha * (x.x * scale);
+        v[2 * i + 1] = alpha * (x.y * scale);
+      }
+      store_half_column(p, m0, n0 + nl, lane, v);
+    }
+  } else if constexpr (MODE == kEpiAdam) {
+    for (int base = ew * kUnroll; base < cols; base += kEpiWarps * kUnroll) {
+      float mo[kUnroll][kRowsPerLane], va[kUnroll][kRowsPerLane], scale[kUnroll];
+#pragma unroll
+      for (int u = 0; u < kUnroll; ++u) {
+        const int n = n0 + base + u;
+        const bool here = base + u < cols;
+        scale[u] = here ? args.b_scale[n] : 0.f;
+#pragma unroll
+        for (int i = 0; i < kRowsPerLane; ++i) {
+          const int r = lane + 32 * i;
+          const bool inside = here && r < rows;
+          mo[u][i] = inside ? p.mom[m0 + r + static_cast<int64_t>(n) * p.ldm] : 0.f;
+          va[u][i] = inside ? p.var[m0 + r + static_cast<int64_t>(n) * p.ldv] : 0.f;
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < kUnroll; ++u) {
+        if (base + u >= cols) break;
+        const int n = n0 + base + u;
+        float* column = tile + (base + u) * PITCH;
+#pragma unroll
+        for (int i = 0; i < kRowsPerLane; ++i) {
+          const int r = lane + 32 * i;
+          const float g = alpha * (column[r] * scale[u]);
+          const float m_new = fmaf(p.beta1, mo[u][i], (1.0f - p.beta1) * g);
+          const float v_new = fmaf(p.beta2, va[u][i], (1.0f - p.beta2) * g * g);
+          float update = 0.f;
+          if (r < rows) {
+            p.mom[m0 + r + static_cast<int64_t>(n) * p.ldm] = m_new;
+            p.var[m0 + r + static_cast<int64_t>(n) * p.ldv] = v_new;
+            update = (m_new * p.inv_bc1) / (sqrtf(v_new) * p.inv_sqrt_bc2 + p.eps);
+          }
+          column[r] = update;
+        }
+        __syncwarp();
+        float v[4];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const float2 x = *reinterpret_cast<const float2*>(column + 64 * i + 2 * lane);
+          v[2 * i] = x.x;
+          v[2 * i + 1] = x.y;
+        }
+        store_half_column(p, m0, n, lane, v);
+      }
+    }
+  } else {
+    // kEpiStore.  Symmetric: entries on and below the diagonal, whose final values go back into the tile for the mirror.
+    for (int base = ew * kUnroll; base < cols; base += kEpiWarps * kUnroll) {
+      float old[kUnroll][kRowsPerLane], scale[kUnroll];
+#pragma unroll
+      for (int u = 0; u < kUnroll; ++u) {
+        const int n = n0 + base + u;
+        const bool here = base + u < cols;
+        scale[u] = here ? args.b_scale[n] : 0.f;
+#pragma unroll
+        for (int i = 0; i < kRowsPerLane; ++i) {
+          const int r = lane + 32 * i;
+          const bool wanted = here && p.beta != 0.f && r < rows && (!p.symmetric || n <= m0 + r);
+          old[u][i] = wanted ? p.C[m0 + r + static_cast<int64_t>(n) * p.ldc] : 0.f;
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < kUnroll; ++u) {
+        const int n = n0 + base + u;
+        if (base + u >= cols) break;
+        float* column = tile + (base + u) * PITCH;
+#pragma unroll
+        for (int i = 0; i < kRowsPerLane; ++i) {
+          const int r = lane + 32 * i;
+          if (r < rows && (!p.symmetric || n <= m0 + r)) {
+            float v = alpha * (column[r] * scale[u]);
+            if (p.beta != 0.f) v = fmaf(p.beta, old[u][i], v);
+            p.C[m0 + r + static_cast<int64_t>(n) * p.ldc] = v;
+            if (p.symmetric) column[r] = v;
+          }
+        }
+      }
+    }
+    if (p.symmetric) {
+      // the mirror is written along its own rows: C[n, m] for the n < m of this tile, lanes along n
+      asm volatile("bar.sync 1, %0;" ::"r"(kEpiWarps * 32) : "memory");
+      for (int r = ew; r < rows; r += kEpiWarps) {
+        const int m = m0 + r;
+        const int limit = min(cols, m - n0);
+        float* dst = p.C + static_cast<int64_t>(m) * p.ldc + n0;
+        for (int n = lane; n < limit; n += 32) dst[n] = tile[n * PITCH + r];
+      }
+    }
+  }
+}
+
+template <bool PAIR, typename Epilogue>
+__device__ __forceinline__ void half_kernel_body(const HalfMaps& maps, const HalfArgs& args, int* status, Epilogue epilogue) {
+  constexpr int BN = PAIR ? 256 : 128;
+  constexpr int kCtas = PAIR ? 2 : 1;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + kStagePool);      // PAIR: used in the leader CTA only
+  uint64_t* empty_bar = full_bar + kMaxStages;      // each CTA its own: "my stage may be refilled"
+  uint64_t* acc_full = empty_bar + kMaxStages;      // [2] each CTA its own: tensor core -> epilogue
+  uint64_t* acc_empty = acc_full + 2;               // [2] PAIR: leader's only, epilogue warps of both CTAs -> tensor core
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const HalfProblem& prob = args.p;
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const uint32_t cta = PAIR ? cluster_cta_rank() : 0;
+
+  // Grouped raster: kGroup tile-rows share their B panels in L2 while they sweep the tile columns.
+  constexpr int kTileM = kCtas * kBM;
+  constexpr int kGroup = PAIR ? 8 : 16;
+  const int tiles_m = (prob.M + kTileM - 1) / kTileM;
+  const int tiles_n = (prob.N + BN - 1) / BN;
+  const int index = PAIR ? blockIdx.x >> 1 : blockIdx.x;
+  const int per_group = kGroup * tiles_n;
+  const int first_m = index / per_group * kGroup;
+  const int rows_in_group = min(kGroup, tiles_m - first_m);
+  const int tile_m0 = (first_m + index % per_group % rows_in_group) * kTileM;
+  const int m0 = tile_m0 + static_cast<int>(cta) * kBM;      // this CTA's rows of the result
+  const int n0 = index % per_group / rows_in_group * BN;
+  const int b_row0 = n0 + static_cast<int>(cta) * (BN / kCtas);
+  // symmetric products: tiles strictly above the diagonal are produced by mirroring (same decision in both CTAs)
+  if (prob.symmetric && n0 > min(tile_m0 + kTileM, prob.M) - 1) return;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kMaxStages; ++s) {
+      mbar_init(&full_bar[s], 1);
+      mbar_init(&empty_bar[s], 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&acc_full[b], 1);
+      mbar_init(&acc_empty[b], kCtas * kEpiWarps);
+    }
+    *abort_flag = 0;
+    mbar_fence_init();
+    tma_prefetch_descriptor(&maps.a_h);
+    tma_prefetch_descriptor(&maps.b_h);
+    if (args.a_terms == 2) tma_prefetch_descriptor(&maps.a_l);
+    if (args.b_terms == 2) tma_prefetch_descriptor(&maps.b_l);
+  }
+  if (warp == 1) {
+    if constexpr (PAIR) {
+      tmem_alloc_pair(tmem_slot, 2 * BN);
+      tmem_relinquish_pair();
+    } else {
+      tmem_alloc(tmem_slot, 2 * BN);
+      tmem_relinquish();
+    }
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  if constexpr (PAIR) cluster_sync_all();      // both CTAs' barriers exist before anything arrives on them remotely
+  tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;
+
+  const int k_blocks = (prob.K + kBK - 1) / kBK;
+  const int chunks = (k_blocks + kChunkBlocks - 1) / kChunkBlocks;
+  const int boxes = args.a_terms + args.b_terms;
+  const int stages = 12 / boxes;               // 3, 4 or 6 stages of four, three or two boxes
+  const int stage_bytes = boxes * kBoxBytes;
+  const int b_at = args.a_terms * kBoxBytes;   // a stage holds A's planes, then B's
+
+  if (warp == 0 && lane == 0) {
+    // ---------------- TMA producer (each CTA loads its own tiles; PAIR: the bytes are credited to the leader) ----------------
+    int s = 0;
+    uint32_t parity = 1;                       // of the previous round's release
+    for (int kb = 0; kb < k_blocks; ++kb) {
+      if (kb >= stages && !mbar_wait_bounded(&empty_bar[s], parity, abort_flag, status, kStatusSlotWaitTimeout)) break;
+      uint8_t* stage = smem + s * stage_bytes;
+      const int k0 = kb * kBK;
+      if constexpr (PAIR) {
+        if (cta == 0) mbar_expect_tx(&full_bar[s], 2 * stage_bytes);
+        const uint32_t bar = map_to_cta(smem_u32(&full_bar[s]), 0);
+        tma_load_2d_pair(stage, &maps.a_h, bar, k0, m0);
+        if (args.a_terms == 2) tma_load_2d_pair(stage + kBoxBytes, &maps.a_l, bar, k0, m0);
+        tma_load_2d_pair(stage + b_at, &maps.b_h, bar, k0, b_row0);
+        if (args.b_terms == 2) tma_load_2d_pair(stage + b_at + kBoxBytes, &maps.b_l, bar, k0, b_row0);
+      } else {
+        mbar_expect_tx(&full_bar[s], stage_bytes);
+        tma_load_2d(stage, &maps.a_h, &full_bar[s], k0, m0);
+        if (args.a_terms == 2) tma_load_2d(stage + kBoxBytes, &maps.a_l, &full_bar[s], k0, m0);
+        tma_load_2d(stage + b_at, &maps.b_h, &full_bar[s], k0, b_row0);
+        if (args.b_terms == 2) tma_load_2d(stage + b_at + kBoxBytes, &maps.b_l, &full_bar[s], k0, b_row0);
+      }
+      if (++s == stages) {
+        s = 0;
+        parity ^= 1;
+      }
+    }
+    if (*abort_flag) {
+      // give copies that are still in flight time to land before the CTA's shared memory is released
+      for (int i = 0; i < 1000; ++i) __nanosleep(1000);
+    }
+  } else if (warp == 1 && lane == 0 && cta == 0) {
+    // ---------------- MMA issuer (PAIR: leader CTA only) ----------------
+    constexpr uint32_t idesc = umma_idesc_fp16(kCtas * kBM, BN);
+    auto mma = [&](uint32_t acc, uint64_t a, uint64_t b, uint32_t accumulate) {
+      if constexpr (PAIR) umma_f16_ss_pair(acc, a, b, idesc, accumulate);
+      else umma_f16_ss(acc, a, b, idesc, accumulate);
+    };
+    auto commit = [&](uint64_t* bar) {
+      if constexpr (PAIR) umma_commit_pair(bar);
+      else umma_commit(bar);
+    };
+    bool ok = true;
+    int s = 0, kb = 0;
+    uint32_t parity = 0;
+    for (int c = 0; c < chunks && ok; ++c) {
+      const int buf = c & 1;
+      if (c >= 2) {
+        ok = mbar_wait_bounded(&acc_empty[buf], ((c >> 1) - 1) & 1, abort_flag, status, kStatusAccumWaitTimeout);
+        if (!ok) break;
+        tc_fence_after_sync();
+      }
+      const uint32_t acc = tmem_base + static_cast<uint32_t>(buf * BN);
+      const int kb_end = min(k_blocks, kb + kChunkBlocks);
+      uint32_t more = 0;                       // 0: the first product of the chunk overwrites the accumulator
+      for (; kb < kb_end; ++kb) {
+        ok = mbar_wait_bounded(&full_bar[s], parity, abort_flag, status, kStatusTmaWaitTimeout);
+        if (!ok) break;
+        tc_fence_after_sync();
+        const uint32_t stage = smem_u32(smem + s * stage_bytes);
+        const uint64_t a_h = umma_desc_kmajor<128>(stage);
+        const uint64_t b_h = umma_desc_kmajor<128>(stage + b_at);
+        constexpr uint64_t kLow = kBoxBytes >> 4, kStep = 32 >> 4;       // 16 fp16 = 32 bytes along the swizzle row
+        if (args.a_terms == 2) {
+#pragma unroll
+          for (int k = 0; k < kBK / 16; ++k, more = 1) mma(acc, a_h + kLow + k * kStep, b_h + k * kStep, more);     // l * h
+        }
+        if (args.b_terms == 2) {
+#pragma unroll
+          for (int k = 0; k < kBK / 16; ++k, more = 1) mma(acc, a_h + k * kStep, b_h + kLow + k * kStep, more);     // h * l
+        }
+#pragma unroll
+        for (int k = 0; k < kBK / 16; ++k, more = 1) mma(acc, a_h + k * kStep, b_h + k * kStep, more);              // h * h
+        commit(&empty_bar[s]);                 // the stage may be refilled once these products have read it
+        if (++s == stages) {
+          s = 0;
+          parity ^= 1;
+        }
+      }
+      if (ok) commit(&acc_full[buf]);
+    }
+  } else if (warp >= 2) {
+    // ---------------- promotion + epilogue (each CTA its own 128 rows) ----------------
+    const int ew = warp - 2;
+    const int quarter = warp & 3;              // TMEM lane quarter this warp may read
+    const int half = ew >> 2;                  // which half of the tile's columns
+    constexpr int kCols = BN / 2;
+    const int col0 = half * kCols;
+    const float* a_scale = args.a_scale + min(m0 + quarter * 32 + lane, prob.M - 1);     // this thread's row
+    const uint32_t drained = PAIR ? map_to_cta(smem_u32(&acc_empty[0]), 0) : 0;
+    float sum[kCols];
+#pragma unroll
+    for (int j = 0; j < kCols; ++j) sum[j] = 0.0f;
+    bool ok = true;
+    float scale = *a_scale * kDown;
+    for (int c = 0; c < chunks && ok; ++c) {
+      const int buf = c & 1;
+      // the next chunk's scale travels while this one is waited for
+      const float next = args.a_stride ? a_scale[min(c + 1, chunks - 1) * args.a_stride] * kDown : scale;
+      ok = mbar_wait_bounded(&acc_full[buf], (c >> 1) & 1, abort_flag, status, kStatusAccumWaitTimeout);
+      if (!ok) break;
+      tc_fence_after_sync();
+      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(buf * BN + col0);
+#pragma unroll
+      for (int cc = 0; cc < kCols; cc += 32) {
+        uint32_t raw[32];
+        tmem_ld_32x32(taddr + static_cast<uint32_t>(cc), raw);
+        tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 32; ++j) sum[cc + j] = fmaf(__uint_as_float(raw[j]), scale, sum[cc + j]);
+      }
+      scale = next;
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) {
+        if constexpr (PAIR) mbar_arrive_cluster(drained + static_cast<uint32_t>(buf * sizeof(uint64_t)));
+        else mbar_arrive(&acc_empty[buf]);
+      }
+    }
+    // The stages are idle once the last chunk has been drained: the sums are staged there and the epilogue runs as a
+    // compact rolled loop over the tile.
+    epilogue(reinterpret_cast<float*>(smem), sum, col0, quarter * 32 + lane, abort_flag, m0, n0, ew, lane);
+  }
+
+  tc_fence_before_sync();
+  __syncthreads();
+  if constexpr (PAIR) cluster_sync_all();      // nobody leaves while the other CTA may still touch its shared memory or TMEM
+  if (warp == 1) {
+    tc_fence_after_sync();
+    if constexpr (PAIR) tmem_dealloc_pair(tmem_base, 2 * BN);
+    else tmem_dealloc(tmem_base, 2 * BN);
+  }
+}
+
+// Column pitch of the staged tile in floats: odd where columns are read across (row-major and mirrored stores), even where
+// two neighbouring rows are read as one 8-byte word.
+template <int MODE>
+constexpr int kPitch = (MODE == kEpiSplit || MODE == kEpiAdam) ? kBM + 2 : kBM + 1;
+static_assert(256 * (kBM + 2) * 4 <= kStagePool, "the staged tile fits where the stages were");
+
+template <bool PAIR, int MODE>
+__device__ __forceinline__ void half_kernel_impl(const HalfMaps& maps, const HalfArgs& args, int* status) {
+  constexpr int BN = PAIR ? 256 : 128;
+  half_kernel_body<PAIR>(maps, args, status, [&](float* tile, float (&sum)[BN / 2], int col0, int row, volatile int* abort_flag,
+                                                 int m0, int n0, int ew, int lane) {
+#pragma unroll
+    for (int j = 0; j < BN / 2; ++j) tile[(col0 + j) * kPitch<MODE> + row] = sum[j];
+    asm volatile("bar.sync 1, %0;" ::"r"(kEpiWarps * 32) : "memory");
+    // read after the barrier, so that all warps of the CTA agree (the epilogue has a barrier of its own)
+    if (*abort_flag == 0 && m0 < args.p.M) half_epilogue<BN, MODE, kPitch<MODE>>(args, tile, m0, n0, ew, lane);
+  });
+}
+
+template <int MODE>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
+half_pair_kernel(const __grid_constant__ HalfMaps maps, const __grid_constant__ HalfArgs args, int* status) {
+  half_kernel_impl<true, MODE>(maps, args, status);
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(kThreads, 1)
+half_single_kernel(const __grid_constant__ HalfMaps maps, const __grid_constant__ HalfArgs args, int* status) {
+  half_kernel_impl<false, MODE>(maps, args, status);
+}
+
+// ---------------------------------------------------------------------------------------------
+using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+EncodeTiledFn encode_tiled_fn() {
+  static EncodeTiledFn fn = nullptr;
+  static std::once_flag once;
+  std::call_once(once, [] {
+    void* ptr = nullptr;
+    cudaDriverEntryPointQueryResult query;
+    cudaError_t err = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &query);
+    if (err != cudaSuccess || query != cudaDriverEntryPointSuccess || ptr == nullptr)
+      throw std::runtime_error("cuTensorMapEncodeTiled is not available from the CUDA driver");
+    fn = reinterpret_cast<EncodeTiledFn>(ptr);
+  });
+  return fn;
+}
+
+// K-contiguous fp16 plane [rows][K] with row pitch ld: boxes of 64 elements x 128 rows.
+CUtensorMap make_map(const uint16_t* base, int64_t K, int64_t rows, int64_t ld) {
+  if ((reinterpret_cast<uintptr_t>(base) & 15) != 0 || ld % 64 != 0 || ld < K)
+    throw std::invalid_argument("gemm_half: planes need 16-byte alignment and a pitch that is a multiple of 64 covering K");
+  CUtensorMap map;
+  cuuint64_t dims[2] = {static_cast<cuuint64_t>(K), static_cast<cuuint64_t>(rows)};
+  cuuint64_t strides[1] = {static_cast<cuuint64_t>(ld) * 2};
+  cuuint32_t box[2] = {kBK, 128};
+  cuuint32_t elem[2] = {1, 1};
+  CUresult res = encode_tiled_fn()(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<uint16_t*>(base), dims, strides, box,
+                                   elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (res != CUDA_SUCCESS) throw std::runtime_error("gemm_half: cuTensorMapEncodeTiled failed with code " + std::to_string(res));
+  return map;
+}
+
+template <int MODE>
+void launch(bool pairs, const HalfMaps& maps, const HalfArgs& args, int* status, cudaStream_t stream) {
+  const HalfProblem& p = args.p;
+  if (pairs) {
+    static PerDeviceOnce configured;
+    allow_dynamic_smem(reinterpret_cast<const void*>(half_pair_kernel<MODE>), kSmemBytes, configured, "gemm_half");
+    const int tiles = ((p.M + 2 * kBM - 1) / (2 * kBM)) * ((p.N + 255) / 256);
+    half_pair_kernel<MODE><<<2 * tiles, kThreads, kSmemBytes, stream>>>(maps, args, status);
+  } else {
+    static PerDeviceOnce configured;
+    allow_dynamic_smem(reinterpret_cast<const void*>(half_single_kernel<MODE>), kSmemBytes, configured, "gemm_half");
+    const int tiles = ((p.M + kBM - 1) / kBM) * ((p.N + 127) / 128);
+    half_single_kernel<MODE><<<tiles, kThreads, kSmemBytes, stream>>>(maps, args, status);
+  }
+  const cudaError_t err = cudaGetLastError();
+  if (err != cudaSuccess) throw std::runtime_error(std::string("gemm_half launch: ") + cudaGetErrorString(err));
+}
+
+}  // namespace
+
+void gemm_half(const HalfOperand& a, const HalfOperand& b, const HalfProblem& prob, int* status, cudaStream_t stream) {
+  if (prob.M <= 0 || prob.N <= 0) return;
+  if (prob.K <= 0) throw std::invalid_argument("gemm_half needs K >= 1");
+  if (b.scale_stride != 0) throw std::invalid_argument("gemm_half: the second operand has one scale per column");
+  if (prob.symmetric && (prob.mode != kEpiStore || prob.M != prob.N))
+    throw std::invalid_argument("gemm_half: symmetric results are square and stored plainly");
+  const bool to_planes = prob.mode == kEpiSplit || prob.mode == kEpiAdam;
+  if (to_planes && (!prob.Ch || !prob.Cl || !prob.Cscale || prob.ldp % 64 != 0 || prob.ldp < prob.M ||
+                    (reinterpret_cast<uintptr_t>(prob.Ch) & 15) != 0 || (reinterpret_cast<uintptr_t>(prob.Cl) & 15) != 0))
+    throw std::invalid_argument("gemm_half: output planes need 16-byte alignment and a pitch that is a multiple of 64");
+  HalfMaps maps;
+  maps.a_h = make_map(a.h, prob.K, prob.M, a.ld);
+  maps.a_l = a.l ? make_map(a.l, prob.K, prob.M, a.ld) : maps.a_h;
+  maps.b_h = make_map(b.h, prob.K, prob.N, b.ld);
+  maps.b_l = b.l ? make_map(b.l, prob.K, prob.N, b.ld) : maps.b_h;
+  const HalfArgs args{prob, a.scale, a.scale_stride, b.scale, a.l ? 2 : 1, b.l ? 2 : 1};
+  // A pair's 256 x 256 tile takes about 1.5 times as long as a CTA's 128 x 128 one (it loads half as much per product): pairs
+  // unless single CTAs get by with so few waves that they finish earlier.  Pairs against singles, measured: 1024^3 32 and
+  // 24 us, 2048^3 50 and 69, 4096^3 333 and 410; symmetric 1024 39 and 28, 2048 54 and 44, 4096 186 and 255.
+  auto tiles_of = [&](int64_t side) {
+    const int64_t m = (prob.M + side - 1) / side, n = (prob.N + side - 1) / side;
+    return prob.symmetric ? m * (m + 1) / 2 : m * n;
+  };
+  const bool pairs = prob.tiles ? prob.tiles == 2 : 3 * ((tiles_of(256) + 73) / 74) <= 2 * ((tiles_of(128) + 147) / 148);
+  switch (prob.mode) {
+    case kEpiStore: launch<kEpiStore>(pairs, maps, args, status, stream); return;
+    case kEpiSplit: launch<kEpiSplit>(pairs, maps, args, status, stream); return;
+    case kEpiAdam: launch<kEpiAdam>(pairs, maps, args, status, stream); return;
+    case kEpiRowMajor: launch<kEpiRowMajor>(pairs, maps, args, status, stream); return;
+    default: throw std::invalid_argument("gemm_half: unknown epilogue mode");
+  }
+}
+
+}  // namespace soapb200

@@ -1,0 +1,75 @@
+// Host-side interface of the fp16-pair GEMM (gemm_half.cu) and of the kernels that make its operands (half_planes.cu).
+#pragma once
+#include <cstdint>
+#include <cuda_runtime.h>
+
+namespace soapb200 {
+
+// A K x cols operand as scaled fp16 planes: element (k, c) is
+//   scale[(k / 128) * scale_stride + c] * (h[k + c * ld] + l[k + c * ld]),
+// scales being powers of two that bring the largest magnitude of the vector (scale_stride == 0: the whole K-vector c;
+// else: its 128-element block) into [2^14, 2^15).  h = rn_fp16(x), l = rn_fp16(x - h) are off by 2^-23 of an element or by
+// 2^-39 of the largest one of its vector or block (fp16's smallest step), whichever is more: the latter is far under the
+// rounding of an fp32 sum that the largest one is part of.  l is null where h alone is exact in that sense (bf16 values).
+struct HalfOperand {
+  const uint16_t* h;
+  const uint16_t* l;
+  int64_t ld;              // multiple of 64
+  const float* scale;
+  int64_t scale_stride;    // 0 for the second operand of a product, whose scales are applied after the sum over K
+};
+
+constexpr int kHalfScaleBlock = 128;
+
+struct HalfProblem {
+  int M, N, K;
+  int mode;                // kEpiStore, kEpiSplit, kEpiAdam or kEpiRowMajor (gemm.h)
+  int symmetric;           // A == B: tiles on and below the diagonal, mirrored (kEpiStore)
+  int tiles;               // 0: chosen by size; 1: single CTAs (128 x 128); 2: CTA pairs (256 x 256)
+  float alpha, beta;
+  float* C;
+  int64_t ldc;
+  // kEpiSplit, kEpiAdam: the result as an operand of depth M with one scale per 128 rows and column
+  uint16_t* Ch;
+  uint16_t* Cl;
+  int64_t ldp;
+  float* Cscale;
+  int64_t ldscale;
+  float* mom;
+  float* var;
+  int64_t ldm, ldv;
+  float beta1, beta2, eps, inv_bc1, inv_sqrt_bc2;
+};
+
+void gemm_half(const HalfOperand& a, const HalfOperand& b, const HalfProblem& prob, int* status, cudaStream_t stream);
+
+// Where one orientation of a matrix goes as scaled fp16 planes (h == null: not wanted).  `scale` has one entry per vector,
+// `largest` is scratch of the same length.
+struct HalfTarget {
+  uint16_t* h;
+  uint16_t* l;             // null: one term
+  int64_t ld;
+  float* scale;
+  uint32_t* largest;
+};
+
+// The operand `plain` (depth rows, vectors = columns) and / or `turned` (depth cols, vectors = rows) of src[i*s_i + j*s_j],
+// i < rows, j < cols; source_type 0: fp32, 1: bf16.
+void half_planes(const void* src, int source_type, int64_t s_i, int64_t s_j, int rows, int cols, const HalfTarget& plain,
+                 const HalfTarget& turned, cudaStream_t stream);
+
+// Scale of a vector or block from the bit pattern of its largest magnitude (clamped so that both factors are normal):
+// x * multiplier is what the planes hold, `inverse` undoes it.  Infinities and NaN pass through with a factor of one.
+struct HalfScale {
+  float multiplier, inverse;
+};
+#ifdef __CUDACC__
+__device__ __forceinline__ HalfScale half_scale(uint32_t largest_bits) {
+  const uint32_t exponent = largest_bits >> 23;
+  if (exponent == 255u) return HalfScale{1.0f, 1.0f};
+  const uint32_t up = exponent < 15u ? 253u : 268u - exponent;      // biased exponent of 2^(14 - floor(log2 largest))
+  return HalfScale{__uint_as_float(up << 23), __uint_as_float((254u - up) << 23)};
+}
+#endif
+
+}  // namespace soapb200

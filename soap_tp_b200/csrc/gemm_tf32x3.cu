@@ -551,9 +551,9 @@ gemm_tf32x3_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant_
 #pragma unroll
           for (int k = 0; k < kBK / 16; ++k) {
             const uint64_t adv = static_cast<uint64_t>(k * 32 >> 4);
-            umma_bf16_ss(tmem_acc, a_hl + kLb + adv, b_hl + adv, idesc16, first ? 0u : 1u);      // lo * hi
+            umma_f16_ss(tmem_acc, a_hl + kLb + adv, b_hl + adv, idesc16, first ? 0u : 1u);      // lo * hi
             first = 0;
-            umma_bf16_ss(tmem_acc, a_hl + adv, b_hl + kLb + adv, idesc16, 1);                    // hi * lo
+            umma_f16_ss(tmem_acc, a_hl + adv, b_hl + kLb + adv, idesc16, 1);                    // hi * lo
           }
           if (!tf32_first) {
 #pragma unroll
@@ -786,9 +786,9 @@ gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ 
 #pragma unroll
           for (int k = 0; k < kBK / 16; ++k) {
             const uint64_t adv = static_cast<uint64_t>(k * 32 >> 4);
-            umma_bf16_ss_pair(tmem_acc, a_2 + kLb + adv, b_2 + adv, idesc16, first ? 0u : 1u);     // lo * hi
+            umma_f16_ss_pair(tmem_acc, a_2 + kLb + adv, b_2 + adv, idesc16, first ? 0u : 1u);     // lo * hi
             first = 0;
-            umma_bf16_ss_pair(tmem_acc, a_2 + adv, b_2 + kLb + adv, idesc16, 1);                   // hi * lo
+            umma_f16_ss_pair(tmem_acc, a_2 + adv, b_2 + kLb + adv, idesc16, 1);                   // hi * lo
           }
           if (!tf32_first) {
 #pragma unroll

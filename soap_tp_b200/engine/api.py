@@ -73,15 +73,15 @@ def rotate(matrix, Q_left, Q_right, global_shape, block_size, grid, direction) -
 def gram_update(G_local, preconditioner, beta, block_size, grid, shard_dim, side) -> Tensor:
     if _world() == 1:
         rows, cols = G_local.shape
-        g32 = G_local if G_local.dtype == torch.float32 else G_local.float()
         size = rows if side == "left" else cols
         from ..layout import validate_2d_block_cyclic_buffer
 
         validate_2d_block_cyclic_buffer(f"{side}_preconditioner", preconditioner, (size, size), block_size, grid, 0)
-        planes = k.split_planes(g32, transpose=(side == "left"),
-                                out=local.workspace_planes("GT" if side == "left" else "X",
-                                                           cols if side == "left" else rows, size, g32.device))
-        k.gemm(planes, planes, out=preconditioner[:size, :size], alpha=1.0 - beta, beta=beta, symmetric=True)
+        if side == "left":
+            _, planes = local.gradient_planes(G_local, turned="GT")
+        else:
+            planes, _ = local.gradient_planes(G_local, plain="X")
+        local.product(planes, planes, out=preconditioner[:size, :size], alpha=1.0 - beta, beta=beta, symmetric=True)
         return preconditioner
     return _distributed().gram_update(G_local, preconditioner, beta, block_size, grid, shard_dim, side)
 

@@ -196,6 +196,10 @@ class Planes:
     def mixed(self) -> bool:
         return self.hl is not None
 
+    @property
+    def device(self):
+        return self.hi.device
+
     @staticmethod
     def empty(depth: int, cols: int, device, mixed: bool = False) -> "Planes":
         ld = max(4, round_up(depth, 4))
@@ -243,6 +247,114 @@ class Planes:
         """The represented K x cols matrix (for tests; to bf16 accuracy of the low part for mixed planes)."""
         low = self.halves()[1] if self.mixed else self.lo[: self.cols, : self.depth]
         return (self.hi[: self.cols, : self.depth] + low).T
+
+
+HALF_SCALE_BLOCK = 128      # rows of a result that share one scale per column when it becomes the next operand
+
+
+@dataclass
+class HalfPlanes:
+    """Operand of a single-GPU product as scaled fp16 planes of a K x cols matrix (``csrc/gemm_half.h``).
+
+    ``x = scale * (h + l)`` with ``h``, ``l`` fp16 (22 to 24 bits of x) and ``scale`` a power of two per K-vector
+    (``blocked=False``: what ``half_planes`` makes, usable on either side of a product) or per K-vector and block of 128
+    (``blocked=True``: what a product's epilogue writes, usable as the first operand).  ``l`` is absent where the matrix
+    comes from bf16 values, which ``h`` holds by itself.
+    """
+
+    h: Tensor
+    l: Optional[Tensor]
+    scale: Tensor               # (cols,) or (blocks, cols)
+    depth: int
+    cols: int
+    ld: int
+    blocked: bool
+    largest: Optional[Tensor] = None      # scratch of ``half_planes``: the largest magnitude of every vector
+
+    @staticmethod
+    def empty(depth: int, cols: int, device, *, blocked: bool = False, terms: int = 2) -> "HalfPlanes":
+        ld = round_up(max(1, depth), 64)
+        planes = torch.empty((terms, max(1, cols), ld), dtype=torch.float16, device=device)
+        blocks = -(-max(1, depth) // HALF_SCALE_BLOCK) if blocked else 1
+        scale = torch.empty((blocks, max(1, cols)), dtype=torch.float32, device=device)
+        largest = None if blocked else torch.empty(max(1, cols), dtype=torch.int32, device=device)
+        return HalfPlanes(planes[0], planes[1] if terms == 2 else None, scale, depth, cols, ld, blocked, largest)
+
+    @property
+    def terms(self) -> int:
+        return 1 if self.l is None else 2
+
+    @property
+    def device(self):
+        return self.h.device
+
+    def dense(self) -> Tensor:
+        """The represented K x cols matrix in fp64 (tests)."""
+        total = self.h[: self.cols, : self.depth].double()
+        if self.l is not None:
+            total = total + self.l[: self.cols, : self.depth].double()
+        scale = self.scale.double()[:, : self.cols]
+        if self.blocked:
+            scale = scale.repeat_interleave(HALF_SCALE_BLOCK, dim=0)[: self.depth]
+        return total.T * scale
+
+    def _target(self) -> tuple:
+        return (self.h.data_ptr(), 0 if self.l is None else self.l.data_ptr(), self.ld, self.scale.data_ptr(),
+                self.largest.data_ptr())
+
+    def _operand(self) -> tuple:
+        return (self.h.data_ptr(), 0 if self.l is None else self.l.data_ptr(), self.ld, self.scale.data_ptr(),
+                self.scale.shape[1] if self.blocked else 0)
+
+
+_NO_TARGET = (0, 0, 64, 0, 0)
+
+
+def half_planes(source: Tensor, plain: Optional[HalfPlanes] = None, turned: Optional[HalfPlanes] = None) -> None:
+    """Write a 2-D tensor (any strides; fp32 or bf16) as scaled fp16 planes: ``plain`` is the operand ``source`` itself,
+    ``turned`` its transpose.  One-term planes take bf16 sources only."""
+    rows, cols = source.shape
+    if source.dtype not in (torch.float32, torch.bfloat16):
+        source = source.float()
+    for planes, shape in ((plain, (rows, cols)), (turned, (cols, rows))):
+        if planes is not None:
+            assert (planes.depth, planes.cols) == shape and not planes.blocked
+            assert planes.terms == 2 or source.dtype == torch.bfloat16
+    _C.half_planes(source.data_ptr(), int(source.dtype == torch.bfloat16), source.stride(0), source.stride(1), rows, cols,
+                   *(plain._target() if plain is not None else _NO_TARGET),
+                   *(turned._target() if turned is not None else _NO_TARGET), _stream())
+    _count("largest_kernel")
+    _count("half_planes_kernel")
+
+
+def gemm_half(a: HalfPlanes, b: HalfPlanes, *, mode: int = EPI_STORE, out: Optional[Tensor] = None,
+              out_planes: Optional[HalfPlanes] = None, alpha: float = 1.0, beta: float = 0.0, symmetric: bool = False,
+              momentum: Optional[Tensor] = None, variance: Optional[Tensor] = None, adam: Optional[dict] = None,
+              tiles: int = 0) -> None:
+    """``acc[m, n] = sum_k a[k, m] * b[k, n]`` on scaled fp16 planes, then the fused epilogue; arguments as :func:`gemm`.
+    ``tiles``: 1 single CTAs, 2 CTA pairs, 0 by size."""
+    assert a.depth == b.depth, (a.depth, b.depth)
+    M, N, K = a.cols, b.cols, a.depth
+    if M == 0 or N == 0:
+        return
+    c = ldc = mom = ldm = var = ldv = 0
+    target = (0, 0, 64, 0, 0)
+    moments = (0.0, 0.0, 0.0, 0.0, 0.0)
+    if out is not None:
+        c = out.data_ptr()
+        ldc = (out.stride(0) if M > 1 else max(1, N)) if mode == EPI_ROW_MAJOR else _ld(out)
+        assert (out.stride(1) == 1 or N == 1) if mode == EPI_ROW_MAJOR else (out.stride(0) == 1 or M == 1)
+    if out_planes is not None:
+        assert out_planes.blocked and out_planes.depth == M and out_planes.cols == N
+        target = out_planes._operand()
+    if mode == EPI_ADAM:
+        mom, ldm, var, ldv = momentum.data_ptr(), _ld(momentum), variance.data_ptr(), _ld(variance)
+        moments = (adam["beta1"], adam["beta2"], adam["eps"], 1.0 / adam["bias_correction1"],
+                   1.0 / math.sqrt(adam["bias_correction2"]))
+    _C.gemm_half(*a._operand(), *b._operand(), M, N, K, mode, int(symmetric), tiles, alpha, beta, c, ldc, *target, mom, ldm,
+                 var, ldv, *moments, status_word(a.device).data_ptr(), _stream())
+    mark_written(out, momentum, variance)
+    _count("gemm_half_kernel")
 
 
 SPLIT_ROUND_NEAREST = os.environ.get("SOAP_TP_SPLIT_NEAREST", "1") == "1"

@@ -3,16 +3,17 @@
 With one rank the packed block-cyclic buffers ARE the dense column-major matrices, so the whole
 step is a chain of this package's kernels on one stream:
 
-    split G (both orientations)                                   split_planes_kernel x2
-    T   = X^T Q_L                (planes)                          gemm_tf32x3 / split epilogue
-    Y   = T^T Q_R, Adam(Y) -> U  (planes), m, v updated in place   gemm_tf32x3 / Adam epilogue
-    T2  = U^T Q_L^T              (planes)                          gemm_tf32x3 / split epilogue
-    out = T2^T Q_R^T             (row-major shard)                 gemm_tf32x3 / row-major epilogue
-    L   = b L + (1-b) G G^T,  R = b R + (1-b) G^T G                gemm_tf32x3 / EMA epilogue, lower tiles + mirror
+    split G (both orientations)                                   largest_kernel, half_planes_kernel
+    T   = X^T Q_L                (planes)                          gemm_half / split epilogue
+    Y   = T^T Q_R, Adam(Y) -> U  (planes), m, v updated in place   gemm_half / Adam epilogue
+    T2  = U^T Q_L^T              (planes)                          gemm_half / split epilogue
+    out = T2^T Q_R^T             (row-major shard)                 gemm_half / row-major epilogue
+    L   = b L + (1-b) G G^T,  R = b R + (1-b) G^T G                gemm_half / EMA epilogue, lower tiles + mirror
 
 Every product is brought to the kernel's single form ``acc = Za^T Zb`` with K-contiguous operands
-by keeping each basis in both orientations as hi/lo planes; the planes are rebuilt only when the
-basis tensor changes (refresh, initialisation, or a user writing into ``state``).
+by keeping each basis in both orientations as operand planes; the planes are rebuilt only when the
+basis tensor changes (refresh, initialisation, or a user writing into ``state``).  The planes are scaled fp16 pairs
+(``kernels.HalfPlanes``); with ``SOAP_TP_MIXED_CORRECTIONS=0`` they are tf32 pairs and every product is three tf32 MMAs.
 """
 from __future__ import annotations
 
@@ -33,11 +34,12 @@ from . import factor
 class BasisPlanes:
     """Both orientations of one orthogonal basis as operand planes, tied to a tensor version."""
 
-    def __init__(self) -> None:
+    def __init__(self, half: bool = True) -> None:
+        self.half = half                  # scaled fp16 planes; else tf32 planes with bf16 corrections
         self.key: Optional[tuple] = None
-        self.owner = None                           # weak reference to the tensor object the planes were made from
-        self.plain: Optional[k.Planes] = None       # operand Q   (depth = rows of Q)
-        self.transposed: Optional[k.Planes] = None  # operand Q^T (depth = cols of Q)
+        self.owner = None                 # weak reference to the tensor object the planes were made from
+        self.plain = None                 # operand Q   (depth = rows of Q)
+        self.transposed = None            # operand Q^T (depth = cols of Q)
 
     def refresh(self, Q: Tensor, size: int) -> None:
         key = (Q.data_ptr(), Q._version, size)
@@ -46,10 +48,11 @@ class BasisPlanes:
         if key == self.key and self.owner is not None and self.owner() is Q:
             return
         view = Q[:size, :size]
-        if self.plain is not None and (self.plain.depth != size or self.plain.hi.device != Q.device):
-            self.plain = self.transposed = None   # the address was recycled by a tensor of another size
-        self.plain = k.split_planes(view, out=self.plain, mixed=k.MIXED_CORRECTIONS)
-        self.transposed = k.split_planes(view, transpose=True, out=self.transposed, mixed=k.MIXED_CORRECTIONS)
+        if self.plain is None or self.plain.depth != size or self.plain.device != Q.device:
+            # (an address that was recycled by a tensor of another size starts over)
+            make = _operand if self.half else _tf32_operand
+            self.plain, self.transposed = make(size, size, Q.device), make(size, size, Q.device)
+        split(view, self.plain, self.transposed)
         self.key = (Q.data_ptr(), Q._version, size)
         self.owner = weakref.ref(Q)
 
@@ -100,14 +103,41 @@ def context_for(state: MutableMapping[str, Any]) -> ParameterContext:
 CLASSIC_TAGS = {"P", "Qtmp"}      # operands of the power iteration, which feeds the QR: always 3xTF32
 
 
-def workspace_planes(tag: str, depth: int, cols: int, device) -> k.Planes:
-    """Scratch operand planes shared by every parameter of the same shape on ``device``.  The operands of the
-    optimizer-step products are mixed planes (``kernels.Planes``) unless that is switched off."""
-    mixed = k.MIXED_CORRECTIONS and tag not in CLASSIC_TAGS
-    key = (tag, depth, cols, str(device), mixed)
+def _operand(depth: int, cols: int, device, *, blocked: bool = False, terms: int = 2):
+    """Uninitialised operand planes for the products of the optimizer step."""
+    if k.MIXED_CORRECTIONS:
+        return k.HalfPlanes.empty(depth, cols, device, blocked=blocked, terms=terms)
+    return k.Planes.empty(depth, cols, device)
+
+
+def _tf32_operand(depth: int, cols: int, device) -> k.Planes:
+    return k.Planes.empty(depth, cols, device, mixed=k.MIXED_CORRECTIONS)
+
+
+def split(source: Tensor, plain=None, turned=None) -> None:
+    """Write a matrix as operand planes: ``plain`` is the operand ``source`` itself, ``turned`` its transpose."""
+    if isinstance(plain if plain is not None else turned, k.HalfPlanes):
+        k.half_planes(source, plain, turned)
+        return
+    if plain is not None:
+        k.split_planes(source, out=plain)
+    if turned is not None:
+        k.split_planes(source, transpose=True, out=turned)
+
+
+def product(a, b, **epilogue) -> None:
+    """``a^T b`` with a fused epilogue, by the kernel that the operands' form belongs to."""
+    (k.gemm_half if isinstance(a, k.HalfPlanes) else k.gemm)(a, b, **epilogue)
+
+
+def workspace_planes(tag: str, depth: int, cols: int, device, *, blocked: bool = False, terms: int = 2):
+    """Scratch operand planes shared by every parameter of the same shape on ``device``.  ``blocked``: written by a
+    product's epilogue; ``terms=1``: written from bf16 values."""
+    key = (tag, depth, cols, str(device), terms)
     planes = _WORKSPACES.get(key)
     if planes is None:
-        planes = k.Planes.empty(depth, cols, device, mixed=mixed)
+        planes = (k.Planes.empty(depth, cols, device) if tag in CLASSIC_TAGS
+                  else _operand(depth, cols, device, blocked=blocked, terms=terms))
         _WORKSPACES[key] = planes
     return planes
 
@@ -126,28 +156,54 @@ def release_workspaces() -> None:
     _CONTEXTS.clear()
 
 
-def _gradient_planes(gradient: Tensor, rows: int, cols: int) -> Tuple[k.Planes, k.Planes]:
-    """Planes of G (depth = rows) and of G^T (depth = cols) from the row-major gradient."""
-    g32 = gradient.detach()
-    if g32.dtype != torch.float32:
-        g32 = g32.float()
-    device = g32.device
-    xp = k.split_planes(g32, out=workspace_planes("X", rows, cols, device))
-    gtp = k.split_planes(g32, transpose=True, out=workspace_planes("GT", cols, rows, device))
+def gradient_planes(gradient: Tensor, *, plain: Optional[str] = None, turned: Optional[str] = None) -> tuple:
+    """Planes of G (depth = rows) and of G^T (depth = columns) in the workspaces of these names; one term for bf16."""
+    g = gradient.detach()
+    if g.dtype != torch.bfloat16 or not k.MIXED_CORRECTIONS:
+        g = g.float()
+    terms = 1 if g.dtype == torch.bfloat16 else 2
+    rows, cols = g.shape
+    xp = workspace_planes(plain, rows, cols, g.device, terms=terms) if plain else None
+    gtp = workspace_planes(turned, cols, rows, g.device, terms=terms) if turned else None
+    split(g, xp, gtp)
     return xp, gtp
 
 
-def rotate_planes(source: k.Planes, first: k.Planes, second: k.Planes, rows: int, cols: int, device, *, tag: str,
-                  **final) -> None:
+def tf32_workspace(tag: str, depth: int, cols: int, device) -> k.Planes:
+    """Scratch planes of the tf32 form with bf16 corrections (``kernels.Planes``, mixed)."""
+    key = ("tf32", tag, depth, cols, str(device))
+    planes = _WORKSPACES.get(key)
+    if planes is None:
+        planes = _WORKSPACES[key] = _tf32_operand(depth, cols, device)
+    return planes
+
+
+def tf32_planes(matrix: Tensor, tag: str, *, transpose: bool = False) -> k.Planes:
+    depth, cols = matrix.shape[::-1] if transpose else matrix.shape
+    return k.split_planes(matrix, transpose=transpose, out=tf32_workspace(tag, depth, cols, matrix.device))
+
+
+def rotate_planes(source, first, second, rows: int, cols: int, device, *, tag: str, **final) -> None:
     """``final epilogue( (source^T first)^T second )`` -- two chained GEMMs through scratch planes."""
-    middle = workspace_planes(tag, source.cols, first.cols, device)
-    k.gemm(source, first, mode=k.EPI_SPLIT, out_planes=middle)
-    k.gemm(middle, second, **final)
+    middle = workspace_planes(tag, source.cols, first.cols, device, blocked=True)
+    product(source, first, mode=k.EPI_SPLIT, out_planes=middle)
+    product(middle, second, **final)
 
 
-def gram_updates(xp: k.Planes, gtp: k.Planes, state, beta: float, rows: int, cols: int) -> None:
-    k.gemm(gtp, gtp, out=state["left_preconditioner"][:rows, :rows], alpha=1.0 - beta, beta=beta, symmetric=True)
-    k.gemm(xp, xp, out=state["right_preconditioner"][:cols, :cols], alpha=1.0 - beta, beta=beta, symmetric=True)
+def gram_updates(xp, gtp, state, beta: float, rows: int, cols: int) -> None:
+    product(gtp, gtp, out=state["left_preconditioner"][:rows, :rows], alpha=1.0 - beta, beta=beta, symmetric=True)
+    product(xp, xp, out=state["right_preconditioner"][:cols, :cols], alpha=1.0 - beta, beta=beta, symmetric=True)
+
+
+def gram_updates_for_bases(gradient: Tensor, state, beta: float, rows: int, cols: int) -> None:
+    """The averages of a step that derives bases from them (the first one, and those with a refresh), on tf32 planes like
+    everything else that is factored.
+
+    A factorisation decides signs by rounding (the last pivot's by its last bit), so the averages that go into one keep, bit
+    for bit, the products they have always been formed with: the same gradient and state give the same bases, not the same
+    ones up to signs."""
+    g = gradient.detach().float()
+    gram_updates(tf32_planes(g, "G"), tf32_planes(g, "GT", transpose=True), state, beta, rows, cols)
 
 
 def soap_step(
@@ -165,10 +221,8 @@ def soap_step(
 ) -> Tensor:
     rows, cols = global_shape
     device = gradient.device
-    with TIMER.stage("split_gradient", device):
-        xp, gtp = _gradient_planes(gradient.reshape(rows, cols), rows, cols)
     if initializing:
-        gram_updates(xp, gtp, state, beta, rows, cols)
+        gram_updates_for_bases(gradient.reshape(rows, cols), state, beta, rows, cols)
         for side, size in (("left", rows), ("right", cols)):
             values = torch.empty(size, dtype=torch.float32, device=device)
             factor.symmetric_eigenbasis(
@@ -180,13 +234,16 @@ def soap_step(
         return torch.zeros((rows, cols), dtype=torch.float32, device=device)
 
     step = int(state["step"]) + 1
+    refreshing = step % interval == 0
+    with TIMER.stage("split_gradient", device):
+        xp, gtp = gradient_planes(gradient.reshape(rows, cols), plain="X", turned=None if refreshing else "GT")
     ctx = context_for(state)
     ctx.left.refresh(state["left_basis"], rows)
     ctx.right.refresh(state["right_basis"], cols)
     bias2 = 1.0 - beta2**step
     adam = dict(beta1=beta1, beta2=beta2, eps=eps / math.sqrt(bias2),
                 bias_correction1=1.0 - beta1**step, bias_correction2=bias2)
-    up = workspace_planes("U", rows, cols, device)
+    up = workspace_planes("U", rows, cols, device, blocked=True)
     with TIMER.stage("rotate_forward+adam", device):
         rotate_planes(xp, ctx.left.plain, ctx.right.plain, rows, cols, device, tag="T",
                       mode=k.EPI_ADAM, out_planes=up, momentum=state["momentum"][:rows, :cols],
@@ -196,8 +253,11 @@ def soap_step(
         rotate_planes(up, ctx.left.transposed, ctx.right.transposed, rows, cols, device, tag="T",
                       mode=k.EPI_ROW_MAJOR, out=update)
     with TIMER.stage("gram", device):
-        gram_updates(xp, gtp, state, beta, rows, cols)
-    if step % interval == 0:
+        if refreshing:
+            gram_updates_for_bases(gradient.reshape(rows, cols), state, beta, rows, cols)
+        else:
+            gram_updates(xp, gtp, state, beta, rows, cols)
+    if refreshing:
         with TIMER.stage("refresh", device):
             refresh(state, global_shape)
     state["step"] = step
@@ -251,8 +311,9 @@ def prepare_refresh(rows: int, cols: int, device) -> None:
     else:
         qr_driver._workspace(rows, device, 0), qr_driver._workspace(cols, device, 1)
     workspace_matrix("perm", rows, cols, device)
-    for tag, depth, width in (("X", rows, cols), ("U", rows, cols), ("T", cols, rows)):
-        workspace_planes(tag, depth, width, device)
+    workspace_planes("X", rows, cols, device)
+    for tag, depth, width in (("U", rows, cols), ("T", cols, rows)):
+        workspace_planes(tag, depth, width, device, blocked=True)
     warm_refresh_kernels(device, sizes={rows, cols})
 
 
@@ -263,7 +324,8 @@ def rotate(matrix: Tensor, Q_left: Tensor, Q_right: Tensor, global_shape, direct
     left.refresh(Q_left, rows)
     right.refresh(Q_right, cols)
     view = matrix[:rows, :cols]
-    source = k.split_planes(view, out=workspace_planes("X", rows, cols, device))
+    source = workspace_planes("X", rows, cols, device)
+    split(view, source)
     if direction == "forward":
         rotate_planes(source, left.plain, right.plain, rows, cols, device, tag="T", mode=k.EPI_STORE, out=view)
     else:
@@ -306,8 +368,9 @@ def refresh(state: MutableMapping[str, Any], global_shape) -> Tuple[Tensor, Tens
     ctx.right.refresh(state["right_basis"], cols)
     # momentum out of the old bases: Q_L M Q_R^T, kept as planes for the way back
     with TIMER.stage("refresh.momentum_out", device):
-        mp = k.split_planes(momentum[:rows, :cols], out=workspace_planes("X", rows, cols, device))
-        parameter_space = workspace_planes("U", rows, cols, device)
+        mp = workspace_planes("X", rows, cols, device)
+        split(momentum[:rows, :cols], mp)
+        parameter_space = workspace_planes("U", rows, cols, device, blocked=True)
         rotate_planes(mp, ctx.left.transposed, ctx.right.transposed, rows, cols, device, tag="T",
                       mode=k.EPI_SPLIT, out_planes=parameter_space)
     with TIMER.stage("refresh.power_iteration", device):

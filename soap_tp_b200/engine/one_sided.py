@@ -35,27 +35,31 @@ def step(gradient: Tensor, state: MutableMapping[str, Any], *, beta: float, beta
     """One update for the row shard ``gradient`` (``rows_local x h``); returns the fp32 update of that shape."""
     rows, h = gradient.shape
     device = gradient.device
-    g32 = gradient.detach()
-    if g32.dtype != torch.float32:
-        g32 = g32.float()
     world = dist.get_world_size() if dist.is_initialized() else 1
-    gp = k.split_planes(g32, out=local.workspace_planes("os_G", rows, h, device))              # operand G   (K = rows)
-    gtp = k.split_planes(g32, transpose=True, out=local.workspace_planes("os_GT", h, rows, device))  # operand G^T (K = h)
+    initializing = "right_basis" not in state
+    # The products of the update itself stay on tf32 planes: a 16-bit parameter turns a difference in their last bits into
+    # whole steps of its own rounding.
+    g32 = gradient.detach().float()
+    gtp = None if initializing else local.tf32_planes(g32, "os_GT", transpose=True)                  # operand G^T (K = h)
 
-    def gram_update() -> None:
+    def gram_update(for_basis: bool) -> None:
         fresh = local.workspace_matrix("os_gram", h, h, device)
-        k.gemm(gp, gp, out=fresh, symmetric=True)                      # G_r^T G_r
+        if for_basis:
+            gp = local.tf32_planes(g32, "os_G")                                     # operand G (K = rows)
+        else:
+            gp, _ = local.gradient_planes(gradient, plain="os_G")
+        local.product(gp, gp, out=fresh, symmetric=True)                           # G_r^T G_r
         if world > 1:
             dist.all_reduce(fresh.T)               # the contiguous view of the column-major buffer (same layout on every rank)
         state["right_preconditioner"].mul_(beta).add_(fresh, alpha=1.0 - beta)
 
-    if "right_basis" not in state:
+    if initializing:
         state["right_preconditioner"] = torch.zeros((h, h), dtype=torch.float32, device=device).T
         state["right_basis"] = torch.zeros((h, h), dtype=torch.float32, device=device).T
         state["right_work"] = torch.zeros((h, h), dtype=torch.float32, device=device).T
         state["momentum"] = torch.zeros((rows, h), dtype=torch.float32, device=device).T       # stored transposed: h x rows
         state["variance"] = torch.zeros((rows, h), dtype=torch.float32, device=device).T
-        gram_update()
+        gram_update(for_basis=True)
         factor.symmetric_eigenbasis(state["right_preconditioner"], state["right_basis"], state["right_work"],
                                     torch.empty(h, dtype=torch.float32, device=device), implementation)
         state["step"] = 0
@@ -64,21 +68,22 @@ def step(gradient: Tensor, state: MutableMapping[str, Any], *, beta: float, beta
     count = int(state["step"]) + 1
     basis = _PLANES.get(state["right_basis"].data_ptr())
     if basis is None:
-        basis = _PLANES[state["right_basis"].data_ptr()] = local.BasisPlanes()
+        basis = _PLANES[state["right_basis"].data_ptr()] = local.BasisPlanes(half=False)
     basis.refresh(state["right_basis"], h)
     bias2 = 1.0 - beta2**count
     adam = dict(beta1=beta1, beta2=beta2, eps=eps / math.sqrt(bias2), bias_correction1=1.0 - beta1**count,
                 bias_correction2=bias2)
-    ut = local.workspace_planes("os_UT", h, rows, device)
+    ut = local.tf32_workspace("os_UT", h, rows, device)
     # Y^T = Q^T G^T with Adam in the epilogue: momentum, variance and U^T are h x rows_local, column-major
     k.gemm(basis.plain, gtp, mode=k.EPI_ADAM, out_planes=ut, momentum=state["momentum"], variance=state["variance"], adam=adam)
     update = torch.empty((rows, h), dtype=torch.float32, device=device)
     k.gemm(basis.transposed, ut, out=update.T)                          # (U Q^T)^T = Q U^T, i.e. the row-major update
-    gram_update()
-    if count % interval == 0:
+    refreshing = count % interval == 0
+    gram_update(for_basis=refreshing)
+    if refreshing:
         # momentum leaves the old basis, M' = (M Q_old^T) Q_new, in the transposed storage: M'^T = Q_new^T Q_old M^T
-        mt = k.split_planes(state["momentum"], out=local.workspace_planes("os_MT", h, rows, device))
-        middle = local.workspace_planes("os_mid", h, rows, device)
+        mt = local.tf32_planes(state["momentum"], "os_MT")
+        middle = local.tf32_workspace("os_mid", h, rows, device)
         k.gemm(basis.transposed, mt, mode=k.EPI_SPLIT, out_planes=middle)                       # Q_old M^T
         order = local.power_iteration_qr(state["right_preconditioner"], state["right_basis"], state["right_work"], h)
         scratch = local.workspace_matrix("os_perm", h, rows, device)
