@@ -8,6 +8,9 @@
 #include <pybind11/stl.h>
 
 #include <cstdint>
+#include <stdexcept>
+#include <tuple>
+#include <vector>
 
 #include "comm.h"
 #include "elementwise.h"
@@ -122,6 +125,44 @@ PYBIND11_MODULE(_C, m) {
                       stream_of(stream));
         },
         "Scaled fp16 operand planes of a matrix in one or both orientations (gemm_half.h)");
+
+  // Integers in the order of SteadyStep (planes and operands as five each: h, l, pitch, scale, then scratch of the largest
+  // magnitudes or the stride of the scales), then the status word and the stream.
+  m.def("steady_step", [](const std::vector<int64_t>& v, double beta, float beta1, float beta2, float eps, float inv_bc1,
+                          float inv_sqrt_bc2) {
+    if (v.size() != 57) throw std::invalid_argument("steady_step: 57 integers expected");
+    size_t at = 0;
+    auto next = [&] { return v[at++]; };
+    auto address = [&] { return reinterpret_cast<void*>(static_cast<uintptr_t>(v[at++])); };
+    auto target = [&] {
+      HalfTarget t{};
+      t.h = static_cast<uint16_t*>(address()); t.l = static_cast<uint16_t*>(address()); t.ld = next();
+      t.scale = static_cast<float*>(address()); t.largest = static_cast<uint32_t*>(address());
+      return t;
+    };
+    auto operand = [&] {
+      HalfOperand o{};
+      o.h = static_cast<uint16_t*>(address()); o.l = static_cast<uint16_t*>(address()); o.ld = next();
+      o.scale = static_cast<float*>(address()); o.scale_stride = next();
+      return o;
+    };
+    SteadyStep s{};
+    s.gradient = address(); s.gradient_type = static_cast<int>(next()); s.s_i = next(); s.s_j = next();
+    s.rows = static_cast<int>(next()); s.cols = static_cast<int>(next());
+    s.x = target(); s.xt = target();
+    s.left = operand(); s.left_turned = operand(); s.right = operand(); s.right_turned = operand();
+    s.middle = operand(); s.update = operand();
+    s.momentum = static_cast<float*>(address()); s.ldm = next();
+    s.variance = static_cast<float*>(address()); s.ldv = next();
+    s.out = static_cast<float*>(address());
+    s.left_gram = static_cast<float*>(address()); s.ld_left = next();
+    s.right_gram = static_cast<float*>(address()); s.ld_right = next();
+    int* status = static_cast<int*>(address());
+    cudaStream_t stream = static_cast<cudaStream_t>(address());
+    s.beta = beta; s.beta1 = beta1; s.beta2 = beta2; s.eps = eps; s.inv_bc1 = inv_bc1; s.inv_sqrt_bc2 = inv_sqrt_bc2;
+    py::gil_scoped_release release;
+    steady_step(s, status, stream);
+  }, "The launches of one ordinary single-GPU step (gemm_half.h, SteadyStep)");
 
   m.def("gemm_simt",
         [](uint64_t A, int64_t a_sk, int64_t a_sm, uint64_t B, int64_t b_sk, int64_t b_sn, uint64_t C, int64_t c_sm,

@@ -58,6 +58,29 @@ struct HalfTarget {
 void half_planes(const void* src, int source_type, int64_t s_i, int64_t s_j, int rows, int cols, const HalfTarget& plain,
                  const HalfTarget& turned, cudaStream_t stream);
 
+// One ordinary step of a rows x cols parameter (steady_step.cpp): every operand, result and scalar of its launches.
+struct SteadyStep {
+  const void* gradient;
+  int gradient_type;
+  int64_t s_i, s_j;
+  int rows, cols;
+  HalfTarget x, xt;                                          // planes of G (depth rows) and G^T (depth cols), written
+  HalfOperand left, left_turned, right, right_turned;        // planes of Q_L, Q_L^T, Q_R, Q_R^T
+  HalfOperand middle, update;                                // scratch planes cols x rows and rows x cols, scales per block
+  float* momentum;
+  int64_t ldm;
+  float* variance;
+  int64_t ldv;
+  float* out;                                                // rows x cols, row-major
+  float* left_gram;
+  int64_t ld_left;
+  float* right_gram;
+  int64_t ld_right;
+  double beta;
+  float beta1, beta2, eps, inv_bc1, inv_sqrt_bc2;
+};
+void steady_step(const SteadyStep& s, int* status, cudaStream_t stream);
+
 // Scale of a vector or block from the bit pattern of its largest magnitude (clamped so that both factors are normal):
 // x * multiplier is what the planes hold, `inverse` undoes it.  Infinities and NaN pass through with a factor of one.
 struct HalfScale {

@@ -98,6 +98,7 @@ class _StatusMonitor:
         self.events = [torch.cuda.Event(), torch.cuda.Event()] if on_device else None
         if on_device:
             self.host = self.host.pin_memory()
+        self.words = (self.host[0:1], self.host[1:2])
         self.pending = [False, False]
         self.turn = 0
 
@@ -115,7 +116,7 @@ class _StatusMonitor:
                 word.zero_()
                 self.pending = [False, False]
                 _raise_for(self.index, code)
-        self.host[self.turn:self.turn + 1].copy_(word[:1], non_blocking=True)
+        self.words[self.turn].copy_(word[:1], non_blocking=True)
         if self.events is not None:
             self.events[self.turn].record()
         self.pending[self.turn] = True
@@ -298,11 +299,11 @@ class HalfPlanes:
             scale = scale.repeat_interleave(HALF_SCALE_BLOCK, dim=0)[: self.depth]
         return total.T * scale
 
-    def _target(self) -> tuple:
+    def target(self) -> tuple:
         return (self.h.data_ptr(), 0 if self.l is None else self.l.data_ptr(), self.ld, self.scale.data_ptr(),
                 self.largest.data_ptr())
 
-    def _operand(self) -> tuple:
+    def operand(self) -> tuple:
         return (self.h.data_ptr(), 0 if self.l is None else self.l.data_ptr(), self.ld, self.scale.data_ptr(),
                 self.scale.shape[1] if self.blocked else 0)
 
@@ -321,8 +322,8 @@ def half_planes(source: Tensor, plain: Optional[HalfPlanes] = None, turned: Opti
             assert (planes.depth, planes.cols) == shape and not planes.blocked
             assert planes.terms == 2 or source.dtype == torch.bfloat16
     _C.half_planes(source.data_ptr(), int(source.dtype == torch.bfloat16), source.stride(0), source.stride(1), rows, cols,
-                   *(plain._target() if plain is not None else _NO_TARGET),
-                   *(turned._target() if turned is not None else _NO_TARGET), _stream())
+                   *(plain.target() if plain is not None else _NO_TARGET),
+                   *(turned.target() if turned is not None else _NO_TARGET), _stream())
     _count("largest_kernel")
     _count("half_planes_kernel")
 
@@ -346,12 +347,12 @@ def gemm_half(a: HalfPlanes, b: HalfPlanes, *, mode: int = EPI_STORE, out: Optio
         assert (out.stride(1) == 1 or N == 1) if mode == EPI_ROW_MAJOR else (out.stride(0) == 1 or M == 1)
     if out_planes is not None:
         assert out_planes.blocked and out_planes.depth == M and out_planes.cols == N
-        target = out_planes._operand()
+        target = out_planes.operand()
     if mode == EPI_ADAM:
         mom, ldm, var, ldv = momentum.data_ptr(), _ld(momentum), variance.data_ptr(), _ld(variance)
         moments = (adam["beta1"], adam["beta2"], adam["eps"], 1.0 / adam["bias_correction1"],
                    1.0 / math.sqrt(adam["bias_correction2"]))
-    _C.gemm_half(*a._operand(), *b._operand(), M, N, K, mode, int(symmetric), tiles, alpha, beta, c, ldc, *target, mom, ldm,
+    _C.gemm_half(*a.operand(), *b.operand(), M, N, K, mode, int(symmetric), tiles, alpha, beta, c, ldc, *target, mom, ldm,
                  var, ldv, *moments, status_word(a.device).data_ptr(), _stream())
     mark_written(out, momentum, variance)
     _count("gemm_half_kernel")

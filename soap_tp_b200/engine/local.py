@@ -30,6 +30,8 @@ from ..profiling import GLOBAL_STAGE_TIMER as TIMER
 from . import kernels as k
 from . import factor
 
+_C = k._C
+
 
 class BasisPlanes:
     """Both orientations of one orthogonal basis as operand planes, tied to a tensor version."""
@@ -40,6 +42,7 @@ class BasisPlanes:
         self.owner = None                 # weak reference to the tensor object the planes were made from
         self.plain = None                 # operand Q   (depth = rows of Q)
         self.transposed = None            # operand Q^T (depth = cols of Q)
+        self.addresses: tuple = ()        # both as the native step takes them
 
     def refresh(self, Q: Tensor, size: int) -> None:
         key = (Q.data_ptr(), Q._version, size)
@@ -52,6 +55,8 @@ class BasisPlanes:
             # (an address that was recycled by a tensor of another size starts over)
             make = _operand if self.half else _tf32_operand
             self.plain, self.transposed = make(size, size, Q.device), make(size, size, Q.device)
+            if isinstance(self.plain, k.HalfPlanes):
+                self.addresses = self.plain.operand() + self.transposed.operand()
         split(view, self.plain, self.transposed)
         self.key = (Q.data_ptr(), Q._version, size)
         self.owner = weakref.ref(Q)
@@ -206,6 +211,48 @@ def gram_updates_for_bases(gradient: Tensor, state, beta: float, rows: int, cols
     gram_updates(tf32_planes(g, "G"), tf32_planes(g, "GT", transpose=True), state, beta, rows, cols)
 
 
+def _step_workspace(rows: int, cols: int, device, terms: int) -> tuple:
+    """Scratch planes of an ordinary step as the native step takes them (shared by parameters of one shape)."""
+    key = ("step", rows, cols, str(device), terms)
+    entry = _WORKSPACES.get(key)
+    if entry is None:
+        xp, gtp = (workspace_planes(tag, *size, device, terms=terms) for tag, size in (("X", (rows, cols)), ("GT", (cols, rows))))
+        middle, update = (workspace_planes(tag, *size, device, blocked=True)
+                          for tag, size in (("T", (cols, rows)), ("U", (rows, cols))))
+        entry = _WORKSPACES[key] = (xp.target() + gtp.target(), middle.operand() + update.operand())
+    return entry
+
+
+def _native_step(gradient: Tensor, state, step: int, rows: int, cols: int, *, beta, beta1, beta2, eps) -> Tensor:
+    """A step without a refresh, its eight launches issued by one native call."""
+    g = gradient.detach().reshape(rows, cols)
+    if g.dtype != torch.float32 and g.dtype != torch.bfloat16:
+        g = g.float()
+    half = g.dtype == torch.bfloat16
+    ctx = context_for(state)
+    ctx.left.refresh(state["left_basis"], rows)
+    ctx.right.refresh(state["right_basis"], cols)
+    bias2 = 1.0 - beta2**step
+    momentum, variance = state["momentum"], state["variance"]
+    left, right = state["left_preconditioner"], state["right_preconditioner"]
+    assert (left.stride(0) == 1 or rows == 1) and (right.stride(0) == 1 or cols == 1)
+    planes, scratch = _step_workspace(rows, cols, g.device, 1 if half else 2)
+    update = torch.empty((rows, cols), dtype=torch.float32, device=g.device)
+    _C.steady_step((g.data_ptr(), int(half), g.stride(0), g.stride(1), rows, cols, *planes, *ctx.left.addresses,
+                    *ctx.right.addresses, *scratch, momentum.data_ptr(), k._ld(momentum), variance.data_ptr(), k._ld(variance),
+                    update.data_ptr(), left.data_ptr(), k._ld(left), right.data_ptr(), k._ld(right),
+                    k.status_word(g.device).data_ptr(), k._stream()),
+                   beta, beta1, beta2, eps / math.sqrt(bias2), 1.0 / (1.0 - beta1**step), 1.0 / math.sqrt(bias2))
+    torch.autograd.graph.increment_version((momentum, variance, left, right))
+    for name, count in _STEP_LAUNCHES:
+        k.LAUNCH_COUNTS[name] = k.LAUNCH_COUNTS.get(name, 0) + count
+    state["step"] = step
+    return update
+
+
+_STEP_LAUNCHES = (("largest_kernel", 1), ("half_planes_kernel", 1), ("gemm_half_kernel", 6))
+
+
 def soap_step(
     gradient: Tensor,
     state: MutableMapping[str, Any],
@@ -235,6 +282,8 @@ def soap_step(
 
     step = int(state["step"]) + 1
     refreshing = step % interval == 0
+    if not refreshing and k.MIXED_CORRECTIONS and not TIMER.enabled and rows and cols:
+        return _native_step(gradient, state, step, rows, cols, beta=beta, beta1=beta1, beta2=beta2, eps=eps)
     with TIMER.stage("split_gradient", device):
         xp, gtp = gradient_planes(gradient.reshape(rows, cols), plain="X", turned=None if refreshing else "GT")
     ctx = context_for(state)
