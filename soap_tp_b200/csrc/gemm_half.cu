@@ -236,7 +236,10 @@ __device__ __forceinline__ void half_kernel_body(const HalfMaps& maps, const Hal
   const int n0 = index % per_group / rows_in_group * BN;
   const int b_row0 = n0 + static_cast<int>(cta) * (BN / kCtas);
   // symmetric products: tiles strictly above the diagonal are produced by mirroring (same decision in both CTAs)
-  if (prob.symmetric && n0 > min(tile_m0 + kTileM, prob.M) - 1) return;
+  if (prob.symmetric && n0 > min(tile_m0 + kTileM, prob.M) - 1) {
+    wait_for_predecessor();      // (no part of this grid ends before its predecessor has)
+    return;
+  }
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kMaxStages; ++s) {
@@ -268,6 +271,8 @@ __device__ __forceinline__ void half_kernel_body(const HalfMaps& maps, const Hal
   if constexpr (PAIR) cluster_sync_all();      // both CTAs' barriers exist before anything arrives on them remotely
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  wait_for_predecessor();
+  let_successor_start();
 
   const int k_blocks = (prob.K + kBK - 1) / kBK;
   const int chunks = (k_blocks + kChunkBlocks - 1) / kChunkBlocks;
@@ -479,18 +484,18 @@ CUtensorMap make_map(const uint16_t* base, int64_t K, int64_t rows, int64_t ld) 
 template <int MODE>
 void launch(bool pairs, const HalfMaps& maps, const HalfArgs& args, int* status, cudaStream_t stream) {
   const HalfProblem& p = args.p;
+  cudaError_t err;
   if (pairs) {
     static PerDeviceOnce configured;
     allow_dynamic_smem(reinterpret_cast<const void*>(half_pair_kernel<MODE>), kSmemBytes, configured, "gemm_half");
     const int tiles = ((p.M + 2 * kBM - 1) / (2 * kBM)) * ((p.N + 255) / 256);
-    half_pair_kernel<MODE><<<2 * tiles, kThreads, kSmemBytes, stream>>>(maps, args, status);
+    err = launch_dependent(half_pair_kernel<MODE>, dim3(2 * tiles), dim3(kThreads), kSmemBytes, stream, maps, args, status);
   } else {
     static PerDeviceOnce configured;
     allow_dynamic_smem(reinterpret_cast<const void*>(half_single_kernel<MODE>), kSmemBytes, configured, "gemm_half");
     const int tiles = ((p.M + kBM - 1) / kBM) * ((p.N + 127) / 128);
-    half_single_kernel<MODE><<<tiles, kThreads, kSmemBytes, stream>>>(maps, args, status);
+    err = launch_dependent(half_single_kernel<MODE>, dim3(tiles), dim3(kThreads), kSmemBytes, stream, maps, args, status);
   }
-  const cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) throw std::runtime_error(std::string("gemm_half launch: ") + cudaGetErrorString(err));
 }
 

@@ -10,6 +10,7 @@
 #include <string>
 
 #include "gemm_half.h"
+#include "launch_util.h"
 
 namespace soapb200 {
 namespace {
@@ -61,6 +62,8 @@ __global__ void __launch_bounds__(kThreads) largest_kernel(const T* __restrict__
   __shared__ uint32_t fast_max[8][kTile];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int fast0 = blockIdx.x * kTile;
+  wait_for_predecessor();
+  let_successor_start();
   uint32_t mine0 = 0, mine1 = 0;
   for (int t = 0; t < strip; ++t) {
     const int slow0 = (blockIdx.y * strip + t) * kTile;
@@ -105,6 +108,8 @@ __global__ void __launch_bounds__(kThreads) half_planes_kernel(const T* __restri
   __shared__ float up_along[kTile], up_across[kTile];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int fast0 = blockIdx.x * kTile, slow0 = blockIdx.y * kTile;
+  wait_for_predecessor();
+  let_successor_start();
   if (threadIdx.x < kTile) {
     const int slow = slow0 + threadIdx.x;
     if (along.h && slow < n_slow) {
@@ -154,11 +159,12 @@ void launch(const T* src, int64_t s_fast, int64_t s_slow, int n_fast, int n_slow
   strip = strip < 1 ? 1 : (strip > 16 ? 16 : strip);
   const dim3 strips(tiles_fast, (tiles_slow + strip - 1) / strip), tiles(tiles_fast, tiles_slow);
   if (strips.y > 65535 || tiles.y > 65535) throw std::invalid_argument("half_planes: matrix too long");
-  largest_kernel<T><<<strips, kThreads, 0, stream>>>(src, s_fast, s_slow, n_fast, n_slow, strip, pairs,
-                                                     across.h ? across.largest : nullptr, along.h ? along.largest : nullptr);
-  check(cudaGetLastError(), "largest_kernel");
-  half_planes_kernel<T><<<tiles, kThreads, 0, stream>>>(src, s_fast, s_slow, n_fast, n_slow, pairs, along, across);
-  check(cudaGetLastError(), "half_planes_kernel");
+  check(launch_dependent(largest_kernel<T>, strips, dim3(kThreads), 0, stream, src, s_fast, s_slow, n_fast, n_slow, strip, pairs,
+                         across.h ? across.largest : nullptr, along.h ? along.largest : nullptr),
+        "largest_kernel");
+  check(launch_dependent(half_planes_kernel<T>, tiles, dim3(kThreads), 0, stream, src, s_fast, s_slow, n_fast, n_slow, pairs,
+                         along, across),
+        "half_planes_kernel");
 }
 
 }  // namespace

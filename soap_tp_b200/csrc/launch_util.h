@@ -26,4 +26,31 @@ inline void allow_dynamic_smem(const void* kernel, size_t bytes, PerDeviceOnce& 
   if (tracked) once.done[device] = true;
 }
 
+// Launch that may begin before the kernel ahead of it in the stream has ended (programmatic dependent launch): what a kernel
+// does before `wait_for_predecessor` -- barriers, TMEM, descriptor prefetch -- overlaps the tail of the one before, and the
+// gap between two launches closes (a step of eight dependent launches: 118 -> 106 us at 256 x 512, 193 -> 181 us at
+// 1000 x 1501).  Everything that touches global memory comes after that wait, which lasts until the
+// predecessor has ended and its writes are visible.
+template <typename... Parameters, typename... Arguments>
+cudaError_t launch_dependent(void (*kernel)(Parameters...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                             Arguments&&... arguments) {
+  cudaLaunchAttribute overlap{};
+  overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  overlap.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t config{};
+  config.gridDim = grid;
+  config.blockDim = block;
+  config.dynamicSmemBytes = smem;
+  config.stream = stream;
+  config.attrs = &overlap;
+  config.numAttrs = 1;
+  return cudaLaunchKernelEx(&config, kernel, static_cast<Parameters>(arguments)...);
+}
+
+#ifdef __CUDACC__
+__device__ __forceinline__ void wait_for_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// From here on the next kernel's CTAs may take the SMs that this one leaves free.
+__device__ __forceinline__ void let_successor_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+#endif
+
 }  // namespace soapb200
