@@ -127,10 +127,11 @@ PYBIND11_MODULE(_C, m) {
         "Scaled fp16 operand planes of a matrix in one or both orientations (gemm_half.h)");
 
   // Integers in the order of SteadyStep (planes and operands as five each: h, l, pitch, scale, then scratch of the largest
-  // magnitudes or the stride of the scales), then the status word and the stream.
+  // magnitudes or the stride of the scales), then the status word, the stream and the
+  // stream of the rotations.
   m.def("steady_step", [](const std::vector<int64_t>& v, double beta, float beta1, float beta2, float eps, float inv_bc1,
                           float inv_sqrt_bc2) {
-    if (v.size() != 57) throw std::invalid_argument("steady_step: 57 integers expected");
+    if (v.size() != 58) throw std::invalid_argument("steady_step: 58 integers expected");
     size_t at = 0;
     auto next = [&] { return v[at++]; };
     auto address = [&] { return reinterpret_cast<void*>(static_cast<uintptr_t>(v[at++])); };
@@ -159,6 +160,7 @@ PYBIND11_MODULE(_C, m) {
     s.right_gram = static_cast<float*>(address()); s.ld_right = next();
     int* status = static_cast<int*>(address());
     cudaStream_t stream = static_cast<cudaStream_t>(address());
+    s.chain = static_cast<cudaStream_t>(address());
     s.beta = beta; s.beta1 = beta1; s.beta2 = beta2; s.eps = eps; s.inv_bc1 = inv_bc1; s.inv_sqrt_bc2 = inv_sqrt_bc2;
     py::gil_scoped_release release;
     steady_step(s, status, stream);

@@ -78,6 +78,7 @@ struct SteadyStep {
   int64_t ld_right;
   double beta;
   float beta1, beta2, eps, inv_bc1, inv_sqrt_bc2;
+  cudaStream_t chain;                                        // the rotations run here, the rest on the step's own stream
 };
 void steady_step(const SteadyStep& s, int* status, cudaStream_t stream);
 

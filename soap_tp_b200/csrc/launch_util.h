@@ -26,6 +26,23 @@ inline void allow_dynamic_smem(const void* kernel, size_t bytes, PerDeviceOnce& 
   if (tracked) once.done[device] = true;
 }
 
+// An event for ordering streams, given back when the scope ends (work that waits for it keeps what it needs).
+class ScopedEvent {
+ public:
+  ScopedEvent() { check(cudaEventCreateWithFlags(&event_, cudaEventDisableTiming)); }
+  ~ScopedEvent() { cudaEventDestroy(event_); }
+  ScopedEvent(const ScopedEvent&) = delete;
+  ScopedEvent& operator=(const ScopedEvent&) = delete;
+  void record(cudaStream_t stream) { check(cudaEventRecord(event_, stream)); }
+  void hold(cudaStream_t stream) { check(cudaStreamWaitEvent(stream, event_, 0)); }
+
+ private:
+  static void check(cudaError_t err) {
+    if (err != cudaSuccess) throw std::runtime_error(std::string("event: ") + cudaGetErrorString(err));
+  }
+  cudaEvent_t event_ = nullptr;
+};
+
 // Launch that may begin before the kernel ahead of it in the stream has ended (programmatic dependent launch): what a kernel
 // does before `wait_for_predecessor` -- barriers, TMEM, descriptor prefetch -- overlaps the tail of the one before, and the
 // gap between two launches closes (a step of eight dependent launches: 118 -> 106 us at 256 x 512, 193 -> 181 us at

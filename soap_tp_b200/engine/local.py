@@ -223,6 +223,17 @@ def _step_workspace(rows: int, cols: int, device, terms: int) -> tuple:
     return entry
 
 
+_CHAIN_STREAMS: Dict[torch.device, "torch.cuda.Stream"] = {}
+
+
+def _chain_stream(device) -> int:
+    """The high-priority stream of the rotations (forked from and joined to the step's own stream within every step)."""
+    stream = _CHAIN_STREAMS.get(device)
+    if stream is None:
+        stream = _CHAIN_STREAMS[device] = torch.cuda.Stream(device=device, priority=-1)
+    return stream.cuda_stream
+
+
 def _native_step(gradient: Tensor, state, step: int, rows: int, cols: int, *, beta, beta1, beta2, eps) -> Tensor:
     """A step without a refresh, its eight launches issued by one native call."""
     g = gradient.detach().reshape(rows, cols)
@@ -241,7 +252,7 @@ def _native_step(gradient: Tensor, state, step: int, rows: int, cols: int, *, be
     _C.steady_step((g.data_ptr(), int(half), g.stride(0), g.stride(1), rows, cols, *planes, *ctx.left.addresses,
                     *ctx.right.addresses, *scratch, momentum.data_ptr(), k._ld(momentum), variance.data_ptr(), k._ld(variance),
                     update.data_ptr(), left.data_ptr(), k._ld(left), right.data_ptr(), k._ld(right),
-                    k.status_word(g.device).data_ptr(), k._stream()),
+                    k.status_word(g.device).data_ptr(), k._stream(), _chain_stream(g.device)),
                    beta, beta1, beta2, eps / math.sqrt(bias2), 1.0 / (1.0 - beta1**step), 1.0 / math.sqrt(bias2))
     torch.autograd.graph.increment_version((momentum, variance, left, right))
     for name, count in _STEP_LAUNCHES:
