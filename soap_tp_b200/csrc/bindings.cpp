@@ -181,14 +181,26 @@ PYBIND11_MODULE(_C, m) {
                       beta1, beta2, eps, inv_bc1, inv_sqrt_bc2, stream_of(stream));
         });
 
+  // One orientation of an fp32 matrix: (i, j) of the operand at src[i * s_i + j * s_j].
   m.def("split_planes",
         [](uint64_t src, int64_t s_i, int64_t s_j, uint64_t hi, uint64_t lo, int64_t ldo, int rows, int cols,
            float scale, int nearest, uint64_t stream, uint64_t hl, int64_t ld16) {
-          split_planes(ptr<const float>(src), s_i, s_j, ptr<float>(hi), ptr<float>(lo), ldo, rows, cols, scale, nearest,
-                       stream_of(stream), ptr<uint16_t>(hl), ld16);
+          split_planes(ptr<const void>(src), 0, s_i, s_j, rows, cols,
+                       SplitTarget{ptr<float>(hi), ptr<float>(lo), ldo, ptr<uint16_t>(hl), ld16}, SplitTarget{}, scale, nearest,
+                       stream_of(stream));
         },
         py::arg("src"), py::arg("s_i"), py::arg("s_j"), py::arg("hi"), py::arg("lo"), py::arg("ldo"), py::arg("rows"),
         py::arg("cols"), py::arg("scale"), py::arg("nearest"), py::arg("stream"), py::arg("hl") = 0, py::arg("ld16") = 0);
+  // One or both orientations (hi, lo, pitch, interleaved plane, its pitch each) of an fp32 or bf16 matrix.
+  m.def("split_planes_both",
+        [](uint64_t src, int source_type, int64_t s_i, int64_t s_j, int rows, int cols, uint64_t phi, uint64_t plo, int64_t pld,
+           uint64_t phl, int64_t pld16, uint64_t thi, uint64_t tlo, int64_t tld, uint64_t thl, int64_t tld16, int nearest,
+           uint64_t stream) {
+          split_planes(ptr<const void>(src), source_type, s_i, s_j, rows, cols,
+                       SplitTarget{ptr<float>(phi), ptr<float>(plo), pld, ptr<uint16_t>(phl), pld16},
+                       SplitTarget{ptr<float>(thi), ptr<float>(tlo), tld, ptr<uint16_t>(thl), tld16}, 1.0f, nearest,
+                       stream_of(stream));
+        });
 
   m.def("column_dot",
         [](uint64_t a, int64_t lda, uint64_t b, int64_t ldb, uint64_t out, int rows, int cols, uint64_t stream) {

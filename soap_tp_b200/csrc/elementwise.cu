@@ -8,6 +8,7 @@
 #include "elementwise.h"
 #include "gemm.h"
 #include "launch_util.h"
+#include "tile_sweep.cuh"
 
 namespace soapb200 {
 namespace {
@@ -68,47 +69,62 @@ __global__ void adam_flat4_kernel(const float4* __restrict__ g, float4* __restri
 }
 
 // ---- operand split --------------------------------------------------------------------------
-// out(i, j) = src[i*s_i + j*s_j] for i < rows, j < cols, written as hi/lo planes with i contiguous
-// (pitch ldo).  A 32x33 shared tile makes both the read and the write coalesced whichever of s_i,
-// s_j is the unit stride, so the same kernel splits in place-order and transposes.
+// Bound by memory: the source is read once for both orientations, 64 x 64 tiles turned in shared memory, 8-byte accesses
+// along the source's unit stride and along each plane's depth.  32 x 32 tiles with 4-byte accesses took 231 us an orientation
+// of an 8192 x 8192 matrix (3.5 TB/s); a one-sided step of 32064 x 2048 bf16 went from 3233 to 3054 us with this kernel.
 __device__ __forceinline__ uint16_t bf16_bits(float v) {
   const __nv_bfloat16 b = __float2bfloat16_rn(v);
   return *reinterpret_cast<const uint16_t*>(&b);
 }
 
-// With `hl` (interleaved bf16 plane, pitch ld16, see gemm.h) the low part is written there as bf16(x) and
-// bf16(x - hi) instead of `lo`: the operand format of the GEMM's mixed-precision corrections.
-__global__ void __launch_bounds__(256) split_planes_kernel(const float* __restrict__ src, int64_t s_i, int64_t s_j,
-                                                           float* __restrict__ hi, float* __restrict__ lo, int64_t ldo,
-                                                           int rows, int cols, float scale, int nearest,
-                                                           uint16_t* __restrict__ hl, int64_t ld16) {
-  __shared__ float tile[32][33];
-  const int i0 = blockIdx.x * 32, j0 = blockIdx.y * 32;
-  const int tx = threadIdx.x % 32, ty = threadIdx.x / 32;  // 32 x 8
-  const bool read_i_fast = (s_i <= s_j);
-  for (int t = ty; t < 32; t += 8) {
-    const int i = read_i_fast ? i0 + tx : i0 + t;
-    const int j = read_i_fast ? j0 + t : j0 + tx;
-    float val = 0.f;
-    if (i < rows && j < cols) val = src[i * s_i + j * s_j];
-    if (read_i_fast) tile[t][tx] = val; else tile[tx][t] = val;  // tile[j - j0][i - i0]
+// Elements i, i + 1 of column j of an operand of depth n; nothing past the depth is written (the planes may be a window).
+__device__ __forceinline__ void write_split(const SplitTarget& to, bool pairs, int64_t i, int64_t j, int n, float x0, float x1,
+                                            int nearest) {
+  const float h0 = tf32_hi(x0, nearest), h1 = tf32_hi(x1, nearest);
+  const int64_t at = i + j * to.ldo, at16 = to.hl ? bf16_plane_index(i) + j * to.ld16 : 0;
+  if (pairs && i + 1 < n) {
+    *reinterpret_cast<float2*>(to.hi + at) = make_float2(h0, h1);
+    if (to.hl) {
+      *reinterpret_cast<__nv_bfloat162*>(to.hl + at16) = __floats2bfloat162_rn(x0, x1);
+      *reinterpret_cast<__nv_bfloat162*>(to.hl + at16 + 32) = __floats2bfloat162_rn(x0 - h0, x1 - h1);
+    } else {
+      *reinterpret_cast<float2*>(to.lo + at) = make_float2(x0 - h0, x1 - h1);
+    }
+    return;
   }
-  __syncthreads();
-  for (int t = ty; t < 32; t += 8) {
-    const int i = i0 + tx, j = j0 + t;
-    if (i < rows && j < cols) {
-      const float x = tile[t][tx] * scale;
-      const float h = tf32_hi(x, nearest);
-      hi[i + j * ldo] = h;
-      if (hl != nullptr) {
-        const int64_t at = bf16_plane_index(i) + j * ld16;
-        hl[at] = bf16_bits(x);
-        hl[at + 32] = bf16_bits(x - h);
-      } else {
-        lo[i + j * ldo] = x - h;
-      }
+  for (int e = 0; e < 2 && i + e < n; ++e) {
+    const float x = e ? x1 : x0, h = e ? h1 : h0;
+    to.hi[at + e] = h;
+    if (to.hl) {         // i is even, so that i and i + 1 are neighbours in the interleaved plane too
+      to.hl[at16 + e] = bf16_bits(x);
+      to.hl[at16 + e + 32] = bf16_bits(x - h);
+    } else {
+      to.lo[at + e] = x - h;
     }
   }
+}
+
+// `along`: depth runs along the source's fast axis; `across`: along its slow axis.
+template <typename T>
+__global__ void __launch_bounds__(sweep::kThreads) split_planes_kernel(const T* __restrict__ src, int64_t s_fast, int64_t s_slow,
+                                                                      int n_fast, int n_slow, bool pairs, const SplitTarget along,
+                                                                      bool along_pairs, const SplitTarget across, bool across_pairs,
+                                                                      float scale, int nearest) {
+  constexpr int kTile = sweep::kTile;
+  __shared__ float tile[kTile][kTile + 1];           // [slow][fast]
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int fast0 = blockIdx.x * kTile, slow0 = blockIdx.y * kTile;
+  sweep::sweep_tile(src, s_fast, s_slow, fast0, slow0, n_fast, n_slow, pairs, [&](int fast, int slow, float x0, float x1) {
+    tile[slow][fast] = x0 * scale;
+    tile[slow][fast + 1] = x1 * scale;
+  });
+  __syncthreads();
+  if (along.hi && fast0 + 2 * lane < n_fast)
+    for (int s = warp; s < kTile && slow0 + s < n_slow; s += 8)
+      write_split(along, along_pairs, fast0 + 2 * lane, slow0 + s, n_fast, tile[s][2 * lane], tile[s][2 * lane + 1], nearest);
+  if (across.hi && slow0 + 2 * lane < n_slow)
+    for (int f = warp; f < kTile && fast0 + f < n_fast; f += 8)
+      write_split(across, across_pairs, slow0 + 2 * lane, fast0 + f, n_slow, tile[2 * lane][f], tile[2 * lane + 1][f], nearest);
 }
 
 // ---- column dots: out[j] = sum_i a[i, j] * b[i, j] -----------------------------------------
@@ -214,12 +230,35 @@ void adam_update(const float* g, int64_t ldg, float* m, int64_t ldm, float* v, i
   check_launch("adam_kernel");
 }
 
-void split_planes(const float* src, int64_t s_i, int64_t s_j, float* hi, float* lo, int64_t ldo, int rows, int cols,
-                  float scale, int nearest, cudaStream_t stream, uint16_t* hl, int64_t ld16) {
-  if (rows <= 0 || cols <= 0) return;
-  dim3 grid((rows + 31) / 32, (cols + 31) / 32);
-  split_planes_kernel<<<grid, 256, 0, stream>>>(src, s_i, s_j, hi, lo, ldo, rows, cols, scale, nearest, hl, ld16);
+namespace {
+bool writes_pairs(const SplitTarget& t) {
+  return (reinterpret_cast<uintptr_t>(t.hi) & 7) == 0 && t.ldo % 2 == 0 &&
+         (t.hl ? (reinterpret_cast<uintptr_t>(t.hl) & 3) == 0 && t.ld16 % 2 == 0 : (reinterpret_cast<uintptr_t>(t.lo) & 7) == 0);
+}
+
+template <typename T>
+void launch_split(const T* src, int64_t s_fast, int64_t s_slow, int n_fast, int n_slow, const SplitTarget& along,
+                  const SplitTarget& across, float scale, int nearest, cudaStream_t stream) {
+  const dim3 grid((n_fast + sweep::kTile - 1) / sweep::kTile, (n_slow + sweep::kTile - 1) / sweep::kTile);
+  if (grid.y > 65535) throw std::invalid_argument("split_planes: matrix too long");
+  split_planes_kernel<T><<<grid, sweep::kThreads, 0, stream>>>(src, s_fast, s_slow, n_fast, n_slow,
+                                                               sweep::reads_pairs(src, s_fast, s_slow, n_slow), along,
+                                                               writes_pairs(along), across, writes_pairs(across), scale, nearest);
   check_launch("split_planes_kernel");
+}
+}  // namespace
+
+void split_planes(const void* src, int source_type, int64_t s_i, int64_t s_j, int rows, int cols, const SplitTarget& plain,
+                  const SplitTarget& turned, float scale, int nearest, cudaStream_t stream) {
+  if (rows <= 0 || cols <= 0 || (!plain.hi && !turned.hi)) return;
+  const bool rows_fast = cols == 1 || (rows > 1 && s_i <= s_j);       // the axis with the smaller stride is swept by the lanes
+  auto go = [&](auto* typed) {
+    if (rows_fast) launch_split(typed, s_i, s_j, rows, cols, plain, turned, scale, nearest, stream);
+    else launch_split(typed, s_j, s_i, cols, rows, turned, plain, scale, nearest, stream);
+  };
+  if (source_type == 0) go(static_cast<const float*>(src));
+  else if (source_type == 1) go(static_cast<const __nv_bfloat16*>(src));
+  else throw std::invalid_argument("split_planes: unknown source type");
 }
 
 void column_dot(const float* a, int64_t lda, const float* b, int64_t ldb, float* out, int rows, int cols,

@@ -11,10 +11,20 @@ void adam_update(const float* g, int64_t ldg, float* m, int64_t ldm, float* v, i
                  int rows, int cols, float beta1, float beta2, float eps, float inv_bc1, float inv_sqrt_bc2,
                  cudaStream_t stream);
 
-// hi/lo planes of out(i, j) = scale * src[i*s_i + j*s_j]; planes are column-major with pitch ldo.  With `hl` (the
-// interleaved bf16 plane of gemm.h, pitch ld16 elements) the low part goes there and `lo` is not written.
-void split_planes(const float* src, int64_t s_i, int64_t s_j, float* hi, float* lo, int64_t ldo, int rows, int cols,
-                  float scale, int nearest, cudaStream_t stream, uint16_t* hl = nullptr, int64_t ld16 = 0);
+// Where one orientation of a matrix goes as operand planes (hi == null: not wanted): column-major with pitch ldo; with `hl`
+// (the interleaved bf16 plane of gemm.h, pitch ld16 elements) the low part goes there and `lo` is not written.
+struct SplitTarget {
+  float* hi = nullptr;
+  float* lo = nullptr;
+  int64_t ldo = 0;
+  uint16_t* hl = nullptr;
+  int64_t ld16 = 0;
+};
+
+// Operand planes of scale * src[i*s_i + j*s_j], i < rows, j < cols: `plain` the matrix itself (depth rows), `turned` its
+// transpose (depth cols).  source_type 0: fp32, 1: bf16.
+void split_planes(const void* src, int source_type, int64_t s_i, int64_t s_j, int rows, int cols, const SplitTarget& plain,
+                  const SplitTarget& turned, float scale, int nearest, cudaStream_t stream);
 
 // out[j] = sum_i a[i, j] * b[i, j] for column-major a, b (deterministic tree reduction per column).
 void column_dot(const float* a, int64_t lda, const float* b, int64_t ldb, float* out, int rows, int cols,

@@ -384,6 +384,24 @@ def split_planes(source: Tensor, *, transpose: bool = False, out: Optional[Plane
     return out
 
 
+def split_planes_both(source: Tensor, plain: Optional[Planes] = None, turned: Optional[Planes] = None) -> None:
+    """Operand planes of a 2-D fp32 or bf16 tensor (any strides) and of its transpose in one pass over it."""
+    if source.dtype not in (torch.float32, torch.bfloat16):
+        source = source.float()
+    rows, cols = source.shape
+    arguments = []
+    for planes, shape in ((plain, (rows, cols)), (turned, (cols, rows))):
+        if planes is None:
+            arguments += (0, 0, 0, 0, 0)
+            continue
+        assert (planes.depth, planes.cols) == shape
+        low = planes.low_pointers()
+        arguments += (planes.hi.data_ptr(), low["lo"], planes.ld, low["hl"], low["ld16"])
+    _C.split_planes_both(source.data_ptr(), int(source.dtype == torch.bfloat16), source.stride(0), source.stride(1), rows, cols,
+                         *arguments, int(SPLIT_ROUND_NEAREST), _stream())
+    _count("split_planes_kernel")
+
+
 def gemm(
     a: Planes,
     b: Planes,

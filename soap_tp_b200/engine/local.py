@@ -124,10 +124,7 @@ def split(source: Tensor, plain=None, turned=None) -> None:
     if isinstance(plain if plain is not None else turned, k.HalfPlanes):
         k.half_planes(source, plain, turned)
         return
-    if plain is not None:
-        k.split_planes(source, out=plain)
-    if turned is not None:
-        k.split_planes(source, transpose=True, out=turned)
+    k.split_planes_both(source, plain, turned)
 
 
 def product(a, b, **epilogue) -> None:
@@ -164,7 +161,7 @@ def release_workspaces() -> None:
 def gradient_planes(gradient: Tensor, *, plain: Optional[str] = None, turned: Optional[str] = None) -> tuple:
     """Planes of G (depth = rows) and of G^T (depth = columns) in the workspaces of these names; one term for bf16."""
     g = gradient.detach()
-    if g.dtype != torch.bfloat16 or not k.MIXED_CORRECTIONS:
+    if g.dtype != torch.bfloat16:
         g = g.float()
     terms = 1 if g.dtype == torch.bfloat16 else 2
     rows, cols = g.shape
@@ -181,11 +178,6 @@ def tf32_workspace(tag: str, depth: int, cols: int, device) -> k.Planes:
     if planes is None:
         planes = _WORKSPACES[key] = _tf32_operand(depth, cols, device)
     return planes
-
-
-def tf32_planes(matrix: Tensor, tag: str, *, transpose: bool = False) -> k.Planes:
-    depth, cols = matrix.shape[::-1] if transpose else matrix.shape
-    return k.split_planes(matrix, transpose=transpose, out=tf32_workspace(tag, depth, cols, matrix.device))
 
 
 def rotate_planes(source, first, second, rows: int, cols: int, device, *, tag: str, **final) -> None:
@@ -207,8 +199,9 @@ def gram_updates_for_bases(gradient: Tensor, state, beta: float, rows: int, cols
     A factorisation decides signs by rounding (the last pivot's by its last bit), so the averages that go into one keep, bit
     for bit, the products they have always been formed with: the same gradient and state give the same bases, not the same
     ones up to signs."""
-    g = gradient.detach().float()
-    gram_updates(tf32_planes(g, "G"), tf32_planes(g, "GT", transpose=True), state, beta, rows, cols)
+    gp, gtp = tf32_workspace("G", rows, cols, gradient.device), tf32_workspace("GT", cols, rows, gradient.device)
+    split(gradient.detach(), gp, gtp)
+    gram_updates(gp, gtp, state, beta, rows, cols)
 
 
 def _step_workspace(rows: int, cols: int, device, terms: int) -> tuple:

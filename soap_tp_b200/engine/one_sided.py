@@ -39,13 +39,15 @@ def step(gradient: Tensor, state: MutableMapping[str, Any], *, beta: float, beta
     initializing = "right_basis" not in state
     # The products of the update itself stay on tf32 planes: a 16-bit parameter turns a difference in their last bits into
     # whole steps of its own rounding.
-    g32 = gradient.detach().float()
-    gtp = None if initializing else local.tf32_planes(g32, "os_GT", transpose=True)                  # operand G^T (K = h)
+    gtp = None if initializing else local.tf32_workspace("os_GT", h, rows, device)         # operand G^T (K = h)
+    if gtp is not None:
+        local.split(gradient.detach(), turned=gtp)
 
     def gram_update(for_basis: bool) -> None:
         fresh = local.workspace_matrix("os_gram", h, h, device)
         if for_basis:
-            gp = local.tf32_planes(g32, "os_G")                                     # operand G (K = rows)
+            gp = local.tf32_workspace("os_G", rows, h, device)                      # operand G (K = rows)
+            local.split(gradient.detach(), gp)
         else:
             gp, _ = local.gradient_planes(gradient, plain="os_G")
         local.product(gp, gp, out=fresh, symmetric=True)                           # G_r^T G_r
@@ -82,7 +84,8 @@ def step(gradient: Tensor, state: MutableMapping[str, Any], *, beta: float, beta
     gram_update(for_basis=refreshing)
     if refreshing:
         # momentum leaves the old basis, M' = (M Q_old^T) Q_new, in the transposed storage: M'^T = Q_new^T Q_old M^T
-        mt = local.tf32_planes(state["momentum"], "os_MT")
+        mt = local.tf32_workspace("os_MT", h, rows, device)
+        local.split(state["momentum"], mt)
         middle = local.tf32_workspace("os_mid", h, rows, device)
         k.gemm(basis.transposed, mt, mode=k.EPI_SPLIT, out_planes=middle)                       # Q_old M^T
         order = local.power_iteration_qr(state["right_preconditioner"], state["right_basis"], state["right_work"], h)
