@@ -202,6 +202,16 @@ PYBIND11_MODULE(_C, m) {
                        stream_of(stream));
         });
 
+  m.def("apply_update", [](uint64_t p, int type, uint64_t update, int64_t n, float keep, float lr, uint64_t stream) {
+    apply_update(ptr<void>(p), type, ptr<const float>(update), n, keep, lr, stream_of(stream));
+  });
+  m.def("adamw_update", [](uint64_t p, int type, uint64_t gradient, uint64_t mo, uint64_t v, int64_t n, float beta1_rest,
+                           float beta2, float beta2_rest, float bias1, float bias2, float eps, float keep, float lr,
+                           uint64_t stream) {
+    adamw_update(ptr<void>(p), type, ptr<const void>(gradient), ptr<float>(mo), ptr<float>(v), n, beta1_rest, beta2, beta2_rest,
+                 bias1, bias2, eps, keep, lr, stream_of(stream));
+  });
+
   m.def("column_dot",
         [](uint64_t a, int64_t lda, uint64_t b, int64_t ldb, uint64_t out, int rows, int cols, uint64_t stream) {
           column_dot(ptr<const float>(a), lda, ptr<const float>(b), ldb, ptr<float>(out), rows, cols, stream_of(stream));

@@ -2,6 +2,7 @@
 // transposing), column dot products for the eigenvalue estimates, and index-mapped gathers.
 #include <stdexcept>
 #include <string>
+#include <type_traits>
 
 #include <cuda_bf16.h>
 
@@ -65,6 +66,62 @@ __global__ void adam_flat4_kernel(const float4* __restrict__ g, float4* __restri
     m[i] = mo;
     v[i] = va;
     u[i] = out;
+  }
+}
+
+// ---- parameter updates ---------------------------------------------------------------------------
+// Bound by memory (p read and written, the update read: 12 bytes an element for fp32, 8 for bf16) or, for the vectors of a
+// model, by the launch: one instead of the two to thirteen that the same arithmetic takes as tensor operations (optimizer step
+// over a layer of hidden size 512: 1101 -> 947 us; one-sided step of 32064 x 2048 bf16: 3054 -> 2980 us).
+__device__ __forceinline__ float to_float(float x) { return x; }
+__device__ __forceinline__ float to_float(__nv_bfloat16 x) { return __bfloat162float(x); }
+template <typename T>
+__device__ __forceinline__ T round_to(float x);
+template <>
+__device__ __forceinline__ float round_to<float>(float x) { return x; }
+template <>
+__device__ __forceinline__ __nv_bfloat16 round_to<__nv_bfloat16>(float x) { return __float2bfloat16_rn(x); }
+
+// Each operation rounds to the parameter's type, as separate tensor operations do.
+template <typename T>
+__device__ __forceinline__ T updated(T p, float update, float keep, float lr) {
+  const T kept = keep == 1.0f ? p : round_to<T>(__fmul_rn(to_float(p), keep));
+  return round_to<T>(fmaf(-lr, to_float(round_to<T>(update)), to_float(kept)));
+}
+
+// 16 bytes of update per thread and step where everything is aligned (`quads`); the rest one by one.
+template <typename T>
+__global__ void __launch_bounds__(256) apply_update_kernel(T* __restrict__ p, const float* __restrict__ update, int64_t n,
+                                                          int64_t quads, float keep, float lr) {
+  struct alignas(4 * sizeof(T)) Four {
+    T x[4];
+  };
+  const int64_t first = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
+  for (int64_t i = first; i < quads; i += stride) {
+    Four mine = reinterpret_cast<Four*>(p)[i];
+    const float4 u = reinterpret_cast<const float4*>(update)[i];
+    mine.x[0] = updated(mine.x[0], u.x, keep, lr);
+    mine.x[1] = updated(mine.x[1], u.y, keep, lr);
+    mine.x[2] = updated(mine.x[2], u.z, keep, lr);
+    mine.x[3] = updated(mine.x[3], u.w, keep, lr);
+    reinterpret_cast<Four*>(p)[i] = mine;
+  }
+  for (int64_t i = 4 * quads + first; i < n; i += stride) p[i] = updated(p[i], update[i], keep, lr);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) adamw_kernel(T* __restrict__ p, const T* __restrict__ gradient, float* __restrict__ m,
+                                                   float* __restrict__ v, int64_t n, float beta1_rest, float beta2,
+                                                   float beta2_rest, float bias1, float bias2, float eps, float keep, float lr) {
+  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
+       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    const float g = to_float(gradient[i]);
+    const float mo = fmaf(beta1_rest, g - m[i], m[i]);
+    const float va = fmaf(beta2_rest * g, g, __fmul_rn(beta2, v[i]));
+    m[i] = mo;
+    v[i] = va;
+    p[i] = updated(p[i], (mo / bias1) / (sqrtf(va / bias2) + eps), keep, lr);
   }
 }
 
@@ -228,6 +285,33 @@ void adam_update(const float* g, int64_t ldg, float* m, int64_t ldm, float* v, i
   adam_kernel<<<grid_for(static_cast<int64_t>(rows) * cols, 256), 256, 0, stream>>>(
       g, ldg, m, ldm, v, ldv, u, ldu, rows, cols, beta1, beta2, eps, inv_bc1, inv_sqrt_bc2);
   check_launch("adam_kernel");
+}
+
+void apply_update(void* p, int type, const float* update, int64_t n, float keep, float lr, cudaStream_t stream) {
+  if (n <= 0) return;
+  auto go = [&](auto* typed) {
+    const bool aligned = reinterpret_cast<uintptr_t>(typed) % (4 * sizeof(*typed)) == 0 && (reinterpret_cast<uintptr_t>(update) & 15) == 0;
+    const int64_t quads = aligned ? n / 4 : 0;
+    apply_update_kernel<<<grid_for(aligned ? (n + 3) / 4 : n, 256), 256, 0, stream>>>(typed, update, n, quads, keep, lr);
+    check_launch("apply_update_kernel");
+  };
+  if (type == 0) go(static_cast<float*>(p));
+  else if (type == 1) go(static_cast<__nv_bfloat16*>(p));
+  else throw std::invalid_argument("apply_update: unknown parameter type");
+}
+
+void adamw_update(void* p, int type, const void* gradient, float* m, float* v, int64_t n, float beta1_rest, float beta2,
+                  float beta2_rest, float bias1, float bias2, float eps, float keep, float lr, cudaStream_t stream) {
+  if (n <= 0) return;
+  auto go = [&](auto* typed) {
+    using T = std::remove_pointer_t<decltype(typed)>;
+    adamw_kernel<T><<<grid_for(n, 256), 256, 0, stream>>>(typed, static_cast<const T*>(gradient), m, v, n, beta1_rest, beta2,
+                                                          beta2_rest, bias1, bias2, eps, keep, lr);
+    check_launch("adamw_kernel");
+  };
+  if (type == 0) go(static_cast<float*>(p));
+  else if (type == 1) go(static_cast<__nv_bfloat16*>(p));
+  else throw std::invalid_argument("adamw_update: unknown parameter type");
 }
 
 namespace {

@@ -550,6 +550,37 @@ def adam_update(gradient: Tensor, momentum: Tensor, variance: Tensor, beta1: flo
     return update
 
 
+_PARAMETER_TYPES = {torch.float32: 0, torch.bfloat16: 1}
+
+
+def apply_update(p: Tensor, update: Tensor, keep: float, lr: float) -> bool:
+    """``p.mul_(keep); p.add_(update.to(p.dtype), alpha=-lr)`` in one pass, value for value; ``False`` (and nothing done) for
+    tensors that the kernel does not take."""
+    kind = _PARAMETER_TYPES.get(p.dtype)
+    if (kind is None or update.dtype != torch.float32 or not p.is_contiguous() or not update.is_contiguous()
+            or p.shape != update.shape or p.device != update.device):
+        return False
+    _C.apply_update(p.data_ptr(), kind, update.data_ptr(), p.numel(), keep, lr, _stream())
+    mark_written(p)
+    _count("apply_update_kernel")
+    return True
+
+
+def adamw_update(p: Tensor, gradient: Tensor, exp_avg: Tensor, exp_avg_sq: Tensor, beta1: float, beta2: float, bias1: float,
+                 bias2: float, eps: float, keep: float, lr: float) -> bool:
+    """One AdamW step of a parameter in one pass; ``False`` for tensors that the kernel does not take."""
+    kind = _PARAMETER_TYPES.get(p.dtype)
+    moments = (exp_avg, exp_avg_sq)
+    if (kind is None or gradient.dtype != p.dtype or any(t.dtype != torch.float32 for t in moments)
+            or any(t.shape != p.shape or t.device != p.device or not t.is_contiguous() for t in (p, gradient) + moments)):
+        return False
+    _C.adamw_update(p.data_ptr(), kind, gradient.data_ptr(), exp_avg.data_ptr(), exp_avg_sq.data_ptr(), p.numel(), 1.0 - beta1,
+                    beta2, 1.0 - beta2, bias1, bias2, eps, keep, lr, _stream())
+    mark_written(p, exp_avg, exp_avg_sq)
+    _count("adamw_kernel")
+    return True
+
+
 def column_dot(a: Tensor, b: Tensor, rows: int, cols: int, out: Optional[Tensor] = None) -> Tensor:
     if out is None:
         out = torch.empty(cols, dtype=torch.float32, device=a.device)

@@ -35,6 +35,18 @@ from .layout import allocate_2d_block_cyclic, most_square_grid
 from .step import soap_step, state_shapes
 
 
+def _apply(p: Tensor, update: Tensor, lr: float, weight_decay: float) -> None:
+    """Decoupled weight decay, then the update."""
+    if p.is_cuda:
+        from .engine import kernels
+
+        if kernels.apply_update(p, update, 1.0 - lr * weight_decay, lr):
+            return
+    if weight_decay != 0.0:
+        p.mul_(1.0 - lr * weight_decay)
+    p.add_(update.to(p.dtype), alpha=-lr)
+
+
 class SoapTP(torch.optim.Optimizer):
     def __init__(
         self,
@@ -125,9 +137,7 @@ class SoapTP(torch.optim.Optimizer):
                         interval=group["precondition_frequency"], implementation=group["basis_implementation"])
                     if not rows_sharded:
                         update = update.T
-                    if wd != 0.0:
-                        p.mul_(1.0 - lr * wd)
-                    p.add_(update.to(p.dtype), alpha=-lr)
+                    _apply(p, update, lr, wd)
                     continue
                 if plan["replicated"] and world > 1:
                     gradient = gradient.chunk(world, dim=plan["shard_dim"])[rank].contiguous()
@@ -142,9 +152,7 @@ class SoapTP(torch.optim.Optimizer):
                     parts = [torch.empty_like(update) for _ in range(world)]
                     dist.all_gather(parts, update.contiguous())
                     update = torch.cat(parts, dim=plan["shard_dim"])
-                if wd != 0.0:
-                    p.mul_(1.0 - lr * wd)
-                p.add_(update.to(p.dtype), alpha=-lr)
+                _apply(p, update, lr, wd)
         return loss
 
     def _adamw(self, p: Tensor, group: dict) -> None:
@@ -155,6 +163,13 @@ class SoapTP(torch.optim.Optimizer):
             state["exp_avg_sq"] = torch.zeros_like(p, dtype=torch.float32)
         state["step"] += 1
         beta1, beta2 = group["adamw_betas"]
+        if p.is_cuda:
+            from .engine import kernels
+
+            if kernels.adamw_update(p, p.grad, state["exp_avg"], state["exp_avg_sq"], beta1, beta2, 1.0 - beta1 ** state["step"],
+                                    1.0 - beta2 ** state["step"], group["eps"], 1.0 - group["lr"] * group["weight_decay"],
+                                    group["lr"]):
+                return
         grad = p.grad.float()
         state["exp_avg"].lerp_(grad, 1.0 - beta1)
         state["exp_avg_sq"].mul_(beta2).addcmul_(grad, grad, value=1.0 - beta2)

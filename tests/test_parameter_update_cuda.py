@@ -1,0 +1,58 @@
+"""Parameter updates in one pass against the tensor operations that they stand for."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [(1,), (7,), (512,), (3, 5), (64, 130), (1025, 33)]
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("decay", [0.0, 0.01])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_apply_is_value_for_value_the_tensor_operations(shape, dtype, decay, offset):
+    from soap_tp_b200.engine import kernels as k
+
+    g = torch.Generator().manual_seed(sum(shape))
+    count = int(torch.tensor(shape).prod())
+    values = (torch.randn(count + offset, generator=g) * 0.02).to(dtype).cuda()
+    p = values[offset:].view(shape)
+    update = torch.randn(count + offset, generator=g).cuda()[offset:].view(shape)
+    expected = p.clone()
+    if decay:
+        expected.mul_(1.0 - 3e-3 * decay)
+    expected.add_(update.to(dtype), alpha=-3e-3)
+    version = p._version
+    assert k.apply_update(p, update, 1.0 - 3e-3 * decay, 3e-3)
+    assert torch.equal(p, expected) and p._version > version
+
+
+def test_apply_leaves_other_tensors_to_the_caller():
+    from soap_tp_b200.engine import kernels as k
+
+    p = torch.ones(4, 6, device="cuda")
+    assert not k.apply_update(p.double(), torch.ones(4, 6, device="cuda"), 1.0, 0.1)
+    assert not k.apply_update(p, torch.ones(6, 4, device="cuda").T, 1.0, 0.1)
+    assert not k.apply_update(p[:, ::2], torch.ones(4, 3, device="cuda"), 1.0, 0.1)
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_adamw_matches_fp64(shape, dtype):
+    """A few fp32 roundings in each of m, v and the update; bf16 parameters round once or twice more (2^-8 each)."""
+    from soap_tp_b200.engine import kernels as k
+
+    g = torch.Generator().manual_seed(1)
+    p = (torch.randn(shape, generator=g) * 0.02).to(dtype).cuda()
+    grad = torch.randn(shape, generator=g).to(dtype).cuda()
+    m, v = torch.randn(shape, generator=g).cuda() * 0.1, torch.rand(shape, generator=g).cuda() + 0.1
+    em = 0.9 * m.double() + 0.1 * grad.double()
+    ev = 0.95 * v.double() + 0.05 * grad.double() ** 2
+    bias1, bias2, keep, lr = 1 - 0.9**3, 1 - 0.95**3, 1 - 3e-5, 3e-3
+    ep = p.double() * keep - lr * (em / bias1) / ((ev / bias2).sqrt() + 1e-8)
+    assert k.adamw_update(p, grad, m, v, 0.9, 0.95, bias1, bias2, 1e-8, keep, lr)
+    torch.testing.assert_close(m.double(), em, rtol=1e-6, atol=1e-7)
+    torch.testing.assert_close(v.double(), ev, rtol=1e-6, atol=1e-7)
+    bound = dict(rtol=2e-6, atol=1e-8) if dtype == torch.float32 else dict(rtol=2.0**-7, atol=lr * 2.0**-6)
+    torch.testing.assert_close(p.double(), ep, **bound)
