@@ -115,6 +115,7 @@ def main(argv=None) -> int:
     parser.add_argument("--pairs", action="store_true", help="panel: the two-columns-per-exchange kernel")
     parser.add_argument("--rows-per-cta", type=int, default=256, choices=(128, 256), help="panel --pairs: CTA height")
     parser.add_argument("--mixed", action="store_true", help="gemm: operands as mixed planes (bf16 correction products)")
+    parser.add_argument("--half", action="store_true", help="gemm: operands as scaled fp16 pairs")
     parser.add_argument("--trace", action="store_true",
                         help="panel: print clock64 stamps of one column step (needs a library built with SOAP_QR_TRACE=1)")
     args = parser.parse_args(argv)
@@ -128,7 +129,21 @@ def main(argv=None) -> int:
     device = torch.device("cuda", torch.cuda.current_device())
     generator = torch.Generator(device=device).manual_seed(0)
     rand = lambda *shape: torch.randn(*shape, generator=generator, device=device)
-    if args.case == "gemm":
+    if args.case == "gemm" and args.half:
+        a, b, target = (k.HalfPlanes.empty(n, n, device, blocked=blocked) for blocked in (False, False, True))
+        k.half_planes(rand(n, n), a)
+        k.half_planes(rand(n, n), b)
+        out, momentum, variance = (torch.zeros(n, n, device=device).T for _ in range(3))
+        adam = dict(beta1=0.95, beta2=0.95, eps=1e-8, bias_correction1=0.5, bias_correction2=0.5)
+        fn = {"store": lambda: k.gemm_half(a, b, out=out),
+              "ema": lambda: k.gemm_half(a, a, out=out, alpha=0.05, beta=0.95, symmetric=True),
+              "split": lambda: k.gemm_half(a, b, mode=k.EPI_SPLIT, out_planes=target),
+              "adam": lambda: k.gemm_half(a, b, mode=k.EPI_ADAM, out_planes=target, momentum=momentum, variance=variance,
+                                          adam=adam)}[args.mode]
+        us = timed(fn, args.repeats)
+        print(f"gemm_half {args.mode} {n}^3: {us:.1f} us/launch, {2 * n**3 / us / 1e6:.1f} TFLOP/s fp32-equivalent "
+              f"({6 * n**3 / us / 1e6:.1f} TFLOP/s of fp16 MMAs)")
+    elif args.case == "gemm":
         a, b = k.split_planes(rand(n, n), mixed=args.mixed), k.split_planes(rand(n, n), mixed=args.mixed)
         out = torch.zeros(n, n, device=device).T
         if args.mode == "store":
