@@ -154,8 +154,9 @@ def round_up(value: int, multiple: int) -> int:
 
 
 # SOAP_TP_MIXED_CORRECTIONS=0 keeps every product on three tf32 MMAs per k-step.  By default the products of the
-# optimizer step (rotations, Gram EMAs, momentum transport) take their two correction terms as bf16 MMAs, see
-# ``Planes``; the factorisations (QR, eigensolvers, power iteration) always use the full 3xTF32 form.
+# single-GPU step run on scaled fp16 pairs (``HalfPlanes``), those of the multi-GPU engine and of the one-sided step take their
+# two correction terms as bf16 MMAs (``Planes``, mixed form); the factorisations (QR, eigensolvers, power iteration) always use
+# the full 3xTF32 form.
 MIXED_CORRECTIONS = os.environ.get("SOAP_TP_MIXED_CORRECTIONS", "1") != "0"
 
 
