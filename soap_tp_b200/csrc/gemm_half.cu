@@ -12,7 +12,7 @@
 // PAIR: the two CTAs of a cluster share a 256 x 256 tile (cta_group::2, each stages its own 128 rows of A and half of the
 // rows of B, no multicast); otherwise one CTA computes 128 x 128.  TMA zero-fills rows and K beyond the operands.
 //
-// The tensor core adds into its accumulator with truncation, so the accumulator is drained every 128 of K into a
+// The tensor core adds into its accumulator with truncation, so the accumulator is drained every 128 or 64 of K into a
 // register-resident sum (round-to-nearest), multiplied by the scale of A's block of 128 on the way; B's scales are per
 // column and applied once, in the epilogue.  Within a chunk the small products come first.
 #include <cuda.h>
@@ -33,7 +33,11 @@ namespace {
 
 constexpr int kBM = 128;
 constexpr int kBK = 64;                          // one 128-byte swizzle row of fp16
-constexpr int kChunkBlocks = 2;                  // k-blocks per promotion: 128 of K
+// k-blocks per promotion: 128 of K, one block of A's scales; 64 of K for symmetric products, whose diagonal is a sum of squares:
+// there the truncated additions all err to one side.  Against fp64 at K = 8192, bf16 operands: 1.8e-7 with 64, 2.1e-7 with 128,
+// 2.0e-7 in the mixed form that drains every 64 (averages of 43 fp32 gradients of 8192^2: 6.8e-7 with 128 against 4.8e-7).
+// The price is a drain per 4 to 12 MMAs: a symmetric one-term product of 4096 takes 220 us instead of 133.
+constexpr int kChunkBlocks = 2, kShortChunkBlocks = 1;
 static_assert(kBK * kChunkBlocks == kHalfScaleBlock, "one block of A's scales per promotion");
 constexpr int kBoxBytes = 128 * kBK * 2;
 constexpr int kStagePool = 12 * kBoxBytes;       // 3 stages of four boxes, 4 of three, 6 of two
@@ -55,6 +59,7 @@ struct HalfArgs {
   int64_t a_stride;
   const float* b_scale;
   int a_terms, b_terms;
+  int chunk_blocks;        // k-blocks per promotion; kChunkBlocks where A's scales are per block
 };
 
 constexpr int kUnroll = 4;       // columns per warp whose loads are in flight together
@@ -275,7 +280,7 @@ __device__ __forceinline__ void half_kernel_body(const HalfMaps& maps, const Hal
   let_successor_start();
 
   const int k_blocks = (prob.K + kBK - 1) / kBK;
-  const int chunks = (k_blocks + kChunkBlocks - 1) / kChunkBlocks;
+  const int chunks = (k_blocks + args.chunk_blocks - 1) / args.chunk_blocks;
   const int boxes = args.a_terms + args.b_terms;
   const int stages = 12 / boxes;               // 3, 4 or 6 stages of four, three or two boxes
   const int stage_bytes = boxes * kBoxBytes;
@@ -334,7 +339,7 @@ __device__ __forceinline__ void half_kernel_body(const HalfMaps& maps, const Hal
         tc_fence_after_sync();
       }
       const uint32_t acc = tmem_base + static_cast<uint32_t>(buf * BN);
-      const int kb_end = min(k_blocks, kb + kChunkBlocks);
+      const int kb_end = min(k_blocks, kb + args.chunk_blocks);
       uint32_t more = 0;                       // 0: the first product of the chunk overwrites the accumulator
       for (; kb < kb_end; ++kb) {
         ok = mbar_wait_bounded(&full_bar[s], parity, abort_flag, status, kStatusTmaWaitTimeout);
@@ -516,7 +521,9 @@ void gemm_half(const HalfOperand& a, const HalfOperand& b, const HalfProblem& pr
   maps.a_l = a.l ? make_map(a.l, prob.K, prob.M, a.ld) : maps.a_h;
   maps.b_h = make_map(b.h, prob.K, prob.N, b.ld);
   maps.b_l = b.l ? make_map(b.l, prob.K, prob.N, b.ld) : maps.b_h;
-  const HalfArgs args{prob, a.scale, a.scale_stride, b.scale, a.l ? 2 : 1, b.l ? 2 : 1};
+  const bool short_chunks = prob.symmetric && a.scale_stride == 0;
+  const HalfArgs args{prob, a.scale, a.scale_stride, b.scale, a.l ? 2 : 1, b.l ? 2 : 1,
+                      short_chunks ? kShortChunkBlocks : kChunkBlocks};
   // A pair's 256 x 256 tile takes about 1.5 times as long as a CTA's 128 x 128 one (it loads half as much per product): pairs
   // unless single CTAs get by with so few waves that they finish earlier.  Pairs against singles, measured: 1024^3 32 and
   // 24 us, 2048^3 50 and 69, 4096^3 333 and 410; symmetric 1024 39 and 28, 2048 54 and 44, 4096 186 and 255.

@@ -165,3 +165,25 @@ def test_no_further_from_fp64_than_the_tf32_forms():
         errors["half"] = _rel(out, expected)
         print(errors)
         assert errors["half"] < 1.05 * min(errors.values())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("symmetric", [False, True])
+def test_sums_of_squares_are_no_further_from_fp64_than_in_the_mixed_form(dtype, symmetric):
+    """On the diagonal of a Gram product every truncated addition errs to the same side; the mixed form is what these products
+    ran on before."""
+    from soap_tp_b200.engine import kernels as k
+
+    g = torch.Generator(device="cuda").manual_seed(4)
+    a = torch.randn(8192, 768, generator=g, device="cuda").to(dtype)
+    b = a if symmetric else torch.randn(8192, 768, generator=g, device="cuda").to(dtype)
+    expected = (a.double().T @ b.double()).cpu()
+    mixed, half = (torch.empty(768, 768, device="cuda").T for _ in range(2))
+    am, bm = (k.split_planes(t.float(), mixed=True) for t in (a, b))
+    k.gemm(am, bm, out=mixed)
+    ap = _planes(a)
+    k.gemm_half(ap, ap if symmetric else _planes(b), out=half, symmetric=symmetric)
+    k.check_status()
+    errors = _rel(half, expected), _rel(mixed, expected)
+    print(errors)
+    assert errors[0] < 1.05 * errors[1]
