@@ -439,7 +439,7 @@ def run(args: argparse.Namespace) -> int:
             "higher_is_better": False,
             "scaling": "strong",
             "vs_baseline": None,
-            "dtype": "fp32 state; 3xTF32 tcgen05 products (fp32-class accuracy)" if args.impl == "ours" else "fp32",
+            "dtype": "fp32 state; tcgen05 products of fp16 pairs or 3xTF32, fp32 sums (fp32-class accuracy)" if args.impl == "ours" else "fp32",
             "data": "synthetic: gradients i.i.d. N(0,1)*1e-2 seeded per step; random-init state from the first gradient",
             "config": {
                 "model": f"one {size}x{size} fp32 parameter (SOAP-TP state: L, R, Q_L, Q_R, momentum, variance)",

@@ -526,7 +526,8 @@ void gemm_half(const HalfOperand& a, const HalfOperand& b, const HalfProblem& pr
                       short_chunks ? kShortChunkBlocks : kChunkBlocks};
   // A pair's 256 x 256 tile takes about 1.5 times as long as a CTA's 128 x 128 one (it loads half as much per product): pairs
   // unless single CTAs get by with so few waves that they finish earlier.  Pairs against singles, measured: 1024^3 32 and
-  // 24 us, 2048^3 50 and 69, 4096^3 333 and 410; symmetric 1024 39 and 28, 2048 54 and 44, 4096 186 and 255.
+  // 24 us, 2048^3 50 and 69, 4096^3 333 and 410; symmetric, then drained every 128 of K, 1024 39 and 28, 2048 54 and 44, 4096 186 and
+  // 255 (drained every 64, one term: 220 and 241).
   auto tiles_of = [&](int64_t side) {
     const int64_t m = (prob.M + side - 1) / side, n = (prob.N + side - 1) / side;
     return prob.symmetric ? m * (m + 1) / 2 : m * n;
