@@ -552,14 +552,24 @@ def adam_update(gradient: Tensor, momentum: Tensor, variance: Tensor, beta1: flo
 
 
 _PARAMETER_TYPES = {torch.float32: 0, torch.bfloat16: 1}
+_PLAIN_TENSORS = (Tensor, torch.nn.Parameter)
+
+
+def _addressable(*tensors: Tensor) -> bool:
+    """Whether a flat kernel of the current stream may work on these tensors through their addresses: plain, dense tensors
+    (a subclass may have no storage behind its address, or a meaning of its own) of one shape on the current device."""
+    first = tensors[0]
+    return (all(type(t) in _PLAIN_TENSORS for t in tensors)
+            and first.device.type == "cuda" and first.device.index == torch.cuda.current_device()
+            and all(t.device == first.device and t.shape == first.shape and t.layout == torch.strided and t.is_contiguous()
+                    and not t.is_neg() for t in tensors))
 
 
 def apply_update(p: Tensor, update: Tensor, keep: float, lr: float) -> bool:
     """``p.mul_(keep); p.add_(update.to(p.dtype), alpha=-lr)`` in one pass, value for value; ``False`` (and nothing done) for
     tensors that the kernel does not take."""
     kind = _PARAMETER_TYPES.get(p.dtype)
-    if (kind is None or update.dtype != torch.float32 or not p.is_contiguous() or not update.is_contiguous()
-            or p.shape != update.shape or p.device != update.device):
+    if kind is None or update.dtype != torch.float32 or not _addressable(p, update):
         return False
     _C.apply_update(p.data_ptr(), kind, update.data_ptr(), p.numel(), keep, lr, _stream())
     mark_written(p)
@@ -571,9 +581,8 @@ def adamw_update(p: Tensor, gradient: Tensor, exp_avg: Tensor, exp_avg_sq: Tenso
                  bias2: float, eps: float, keep: float, lr: float) -> bool:
     """One AdamW step of a parameter in one pass; ``False`` for tensors that the kernel does not take."""
     kind = _PARAMETER_TYPES.get(p.dtype)
-    moments = (exp_avg, exp_avg_sq)
-    if (kind is None or gradient.dtype != p.dtype or any(t.dtype != torch.float32 for t in moments)
-            or any(t.shape != p.shape or t.device != p.device or not t.is_contiguous() for t in (p, gradient) + moments)):
+    if (kind is None or gradient.dtype != p.dtype or exp_avg.dtype != torch.float32 or exp_avg_sq.dtype != torch.float32
+            or not _addressable(p, gradient, exp_avg, exp_avg_sq)):
         return False
     _C.adamw_update(p.data_ptr(), kind, gradient.data_ptr(), exp_avg.data_ptr(), exp_avg_sq.data_ptr(), p.numel(), 1.0 - beta1,
                     beta2, 1.0 - beta2, bias1, bias2, eps, keep, lr, _stream())
