@@ -117,7 +117,8 @@ __global__ void __launch_bounds__(256) adamw_kernel(T* __restrict__ p, const T* 
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const float g = to_float(gradient[i]);
-    const float mo = fmaf(beta1_rest, g - m[i], m[i]);
+    // from the nearer end, as lerp does: with a small beta1 an old average far above the gradient must not swallow it
+    const float mo = beta1_rest < 0.5f ? fmaf(beta1_rest, g - m[i], m[i]) : fmaf(-(g - m[i]), 1.0f - beta1_rest, g);
     const float va = fmaf(beta2_rest * g, g, __fmul_rn(beta2, v[i]));
     m[i] = mo;
     v[i] = va;

@@ -56,3 +56,19 @@ def test_adamw_matches_fp64(shape, dtype):
     torch.testing.assert_close(v.double(), ev, rtol=1e-6, atol=1e-7)
     bound = dict(rtol=2e-6, atol=1e-8) if dtype == torch.float32 else dict(rtol=2.0**-7, atol=lr * 2.0**-6)
     torch.testing.assert_close(p.double(), ep, **bound)
+
+
+@pytest.mark.parametrize("beta1", [0.0, 0.3, 0.5, 0.9])
+def test_adamw_average_is_lerp_for_every_beta(beta1):
+    """Also where the old average is far above the gradient: beta1 = 0 leaves the gradient itself."""
+    from soap_tp_b200.engine import kernels as k
+
+    g = torch.Generator().manual_seed(2)
+    grad = torch.randn(1000, generator=g).cuda()
+    m = (torch.randn(1000, generator=g) * torch.logspace(-3, 9, 1000)).cuda()
+    p, v = torch.zeros(1000, device="cuda"), torch.ones(1000, device="cuda")
+    expected = m.clone().lerp_(grad, 1.0 - beta1)
+    assert k.adamw_update(p, grad, m, v, beta1, 0.95, 1.0, 1.0, 1e-8, 1.0, 0.1)
+    assert torch.equal(m, expected)
+    if beta1 == 0.0:
+        assert torch.equal(m, grad)
