@@ -77,10 +77,14 @@ def gram_update(G_local, preconditioner, beta, block_size, grid, shard_dim, side
         from ..layout import validate_2d_block_cyclic_buffer
 
         validate_2d_block_cyclic_buffer(f"{side}_preconditioner", preconditioner, (size, size), block_size, grid, 0)
-        if side == "left":
-            _, planes = local.gradient_planes(G_local, turned="GT")
+        # on the planes of an average that bases are derived from: the op cannot know whether its result will be factored, and
+        # a step composed from the ops takes the same averages as the engine's
+        turned = side == "left"
+        planes = local.tf32_workspace("GT" if turned else "G", cols if turned else rows, size, G_local.device)
+        if turned:
+            local.split(G_local.detach(), turned=planes)
         else:
-            planes, _ = local.gradient_planes(G_local, plain="X")
+            local.split(G_local.detach(), planes)
         local.product(planes, planes, out=preconditioner[:size, :size], alpha=1.0 - beta, beta=beta, symmetric=True)
         return preconditioner
     return _distributed().gram_update(G_local, preconditioner, beta, block_size, grid, shard_dim, side)
