@@ -12,9 +12,9 @@
 // PAIR: the two CTAs of a cluster share a 256 x 256 tile (cta_group::2, each stages its own 128 rows of A and half of the
 // rows of B, no multicast); otherwise one CTA computes 128 x 128.  TMA zero-fills rows and K beyond the operands.
 //
-// The tensor core adds into its accumulator with truncation, so the accumulator is drained every 128 or 64 of K into a
-// register-resident sum (round-to-nearest), multiplied by the scale of A's block of 128 on the way; B's scales are per
-// column and applied once, in the epilogue.  Within a chunk the small products come first.
+// The tensor core adds into its accumulator with truncation, so the accumulator is drained every 64 of K (one k-block) into
+// a register-resident sum (round-to-nearest), multiplied by the scale of A's block of 128 on the way; B's scales are per
+// column and applied once, in the epilogue.  Within a k-block the small products come first.
 #include <cuda.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -33,12 +33,12 @@ namespace {
 
 constexpr int kBM = 128;
 constexpr int kBK = 64;                          // one 128-byte swizzle row of fp16
-// k-blocks per promotion: 128 of K, one block of A's scales; 64 of K for symmetric products, whose diagonal is a sum of squares:
-// there the truncated additions all err to one side.  Against fp64 at K = 8192, bf16 operands: 1.8e-7 with 64, 2.1e-7 with 128,
-// 2.0e-7 in the mixed form that drains every 64 (averages of 43 fp32 gradients of 8192^2: 6.8e-7 with 128 against 4.8e-7).
-// The price is a drain per 4 to 12 MMAs: a symmetric one-term product of 4096 takes 220 us instead of 133.
-constexpr int kChunkBlocks = 2, kShortChunkBlocks = 1;
-static_assert(kBK * kChunkBlocks == kHalfScaleBlock, "one block of A's scales per promotion");
+// One k-block per promotion, 64 of K, as the mixed form drains.  Truncated additions of a one-sided sum (a diagonal of
+// squares, a rotation along a leading singular vector) all err to one side, and small products that meet a main sum are
+// truncated at its size.  Relative error of products of positive operands, drained every 64 / every 128 / mixed form: two
+// terms 2.7e-7 / 6.6e-7 / 4.6e-7 at K = 8192 and 2.1e-7 / 6.6e-7 / 4.5e-7 at K = 128, one term against two 2.1e-7 / 3.7e-7 /
+// 3.1e-7 and 1.3e-7 / 3.6e-7 / 2.7e-7.  The price: two terms 4096^3 351 us instead of 319, one term against two 293 instead of 247.
+constexpr int kScaleBlocks = kHalfScaleBlock / kBK;      // k-blocks that share one of A's scales
 constexpr int kBoxBytes = 128 * kBK * 2;
 constexpr int kStagePool = 12 * kBoxBytes;       // 3 stages of four boxes, 4 of three, 6 of two
 constexpr int kMaxStages = 6;
@@ -59,7 +59,6 @@ struct HalfArgs {
   int64_t a_stride;
   const float* b_scale;
   int a_terms, b_terms;
-  int chunk_blocks;        // k-blocks per promotion; kChunkBlocks where A's scales are per block
 };
 
 constexpr int kUnroll = 4;       // columns per warp whose loads are in flight together
@@ -280,7 +279,6 @@ __device__ __forceinline__ void half_kernel_body(const HalfMaps& maps, const Hal
   let_successor_start();
 
   const int k_blocks = (prob.K + kBK - 1) / kBK;
-  const int chunks = (k_blocks + args.chunk_blocks - 1) / args.chunk_blocks;
   const int boxes = args.a_terms + args.b_terms;
   const int stages = 12 / boxes;               // 3, 4 or 6 stages of four, three or two boxes
   const int stage_bytes = boxes * kBoxBytes;
@@ -329,43 +327,40 @@ __device__ __forceinline__ void half_kernel_body(const HalfMaps& maps, const Hal
       else umma_commit(bar);
     };
     bool ok = true;
-    int s = 0, kb = 0;
+    int s = 0;
     uint32_t parity = 0;
-    for (int c = 0; c < chunks && ok; ++c) {
-      const int buf = c & 1;
-      if (c >= 2) {
-        ok = mbar_wait_bounded(&acc_empty[buf], ((c >> 1) - 1) & 1, abort_flag, status, kStatusAccumWaitTimeout);
+    for (int kb = 0; kb < k_blocks; ++kb) {
+      const int buf = kb & 1;
+      if (kb >= 2) {
+        ok = mbar_wait_bounded(&acc_empty[buf], ((kb >> 1) - 1) & 1, abort_flag, status, kStatusAccumWaitTimeout);
         if (!ok) break;
         tc_fence_after_sync();
       }
+      ok = mbar_wait_bounded(&full_bar[s], parity, abort_flag, status, kStatusTmaWaitTimeout);
+      if (!ok) break;
+      tc_fence_after_sync();
       const uint32_t acc = tmem_base + static_cast<uint32_t>(buf * BN);
-      const int kb_end = min(k_blocks, kb + args.chunk_blocks);
-      uint32_t more = 0;                       // 0: the first product of the chunk overwrites the accumulator
-      for (; kb < kb_end; ++kb) {
-        ok = mbar_wait_bounded(&full_bar[s], parity, abort_flag, status, kStatusTmaWaitTimeout);
-        if (!ok) break;
-        tc_fence_after_sync();
-        const uint32_t stage = smem_u32(smem + s * stage_bytes);
-        const uint64_t a_h = umma_desc_kmajor<128>(stage);
-        const uint64_t b_h = umma_desc_kmajor<128>(stage + b_at);
-        constexpr uint64_t kLow = kBoxBytes >> 4, kStep = 32 >> 4;       // 16 fp16 = 32 bytes along the swizzle row
-        if (args.a_terms == 2) {
+      const uint32_t stage = smem_u32(smem + s * stage_bytes);
+      const uint64_t a_h = umma_desc_kmajor<128>(stage);
+      const uint64_t b_h = umma_desc_kmajor<128>(stage + b_at);
+      constexpr uint64_t kLow = kBoxBytes >> 4, kStep = 32 >> 4;         // 16 fp16 = 32 bytes along the swizzle row
+      uint32_t more = 0;                       // 0: the first product of the k-block overwrites the accumulator
+      if (args.a_terms == 2) {
 #pragma unroll
-          for (int k = 0; k < kBK / 16; ++k, more = 1) mma(acc, a_h + kLow + k * kStep, b_h + k * kStep, more);     // l * h
-        }
-        if (args.b_terms == 2) {
-#pragma unroll
-          for (int k = 0; k < kBK / 16; ++k, more = 1) mma(acc, a_h + k * kStep, b_h + kLow + k * kStep, more);     // h * l
-        }
-#pragma unroll
-        for (int k = 0; k < kBK / 16; ++k, more = 1) mma(acc, a_h + k * kStep, b_h + k * kStep, more);              // h * h
-        commit(&empty_bar[s]);                 // the stage may be refilled once these products have read it
-        if (++s == stages) {
-          s = 0;
-          parity ^= 1;
-        }
+        for (int k = 0; k < kBK / 16; ++k, more = 1) mma(acc, a_h + kLow + k * kStep, b_h + k * kStep, more);     // l * h
       }
-      if (ok) commit(&acc_full[buf]);
+      if (args.b_terms == 2) {
+#pragma unroll
+        for (int k = 0; k < kBK / 16; ++k, more = 1) mma(acc, a_h + k * kStep, b_h + kLow + k * kStep, more);     // h * l
+      }
+#pragma unroll
+      for (int k = 0; k < kBK / 16; ++k, more = 1) mma(acc, a_h + k * kStep, b_h + k * kStep, more);              // h * h
+      commit(&empty_bar[s]);                   // the stage may be refilled once these products have read it
+      commit(&acc_full[buf]);
+      if (++s == stages) {
+        s = 0;
+        parity ^= 1;
+      }
     }
   } else if (warp >= 2) {
     // ---------------- promotion + epilogue (each CTA its own 128 rows) ----------------
@@ -379,14 +374,12 @@ __device__ __forceinline__ void half_kernel_body(const HalfMaps& maps, const Hal
     float sum[kCols];
 #pragma unroll
     for (int j = 0; j < kCols; ++j) sum[j] = 0.0f;
-    bool ok = true;
     float scale = *a_scale * kDown;
-    for (int c = 0; c < chunks && ok; ++c) {
-      const int buf = c & 1;
-      // the next chunk's scale travels while this one is waited for
-      const float next = args.a_stride ? a_scale[min(c + 1, chunks - 1) * args.a_stride] * kDown : scale;
-      ok = mbar_wait_bounded(&acc_full[buf], (c >> 1) & 1, abort_flag, status, kStatusAccumWaitTimeout);
-      if (!ok) break;
+    for (int kb = 0; kb < k_blocks; ++kb) {
+      const int buf = kb & 1;
+      // the next k-block's scale travels while this one is waited for
+      const float next = args.a_stride ? a_scale[min(kb + 1, k_blocks - 1) / kScaleBlocks * args.a_stride] * kDown : scale;
+      if (!mbar_wait_bounded(&acc_full[buf], (kb >> 1) & 1, abort_flag, status, kStatusAccumWaitTimeout)) break;
       tc_fence_after_sync();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(buf * BN + col0);
 #pragma unroll
@@ -405,7 +398,7 @@ __device__ __forceinline__ void half_kernel_body(const HalfMaps& maps, const Hal
         else mbar_arrive(&acc_empty[buf]);
       }
     }
-    // The stages are idle once the last chunk has been drained: the sums are staged there and the epilogue runs as a
+    // The stages are idle once the last k-block has been drained: the sums are staged there and the epilogue runs as a
     // compact rolled loop over the tile.
     epilogue(reinterpret_cast<float*>(smem), sum, col0, quarter * 32 + lane, abort_flag, m0, n0, ew, lane);
   }
@@ -521,9 +514,7 @@ void gemm_half(const HalfOperand& a, const HalfOperand& b, const HalfProblem& pr
   maps.a_l = a.l ? make_map(a.l, prob.K, prob.M, a.ld) : maps.a_h;
   maps.b_h = make_map(b.h, prob.K, prob.N, b.ld);
   maps.b_l = b.l ? make_map(b.l, prob.K, prob.N, b.ld) : maps.b_h;
-  const bool short_chunks = prob.symmetric && a.scale_stride == 0;
-  const HalfArgs args{prob, a.scale, a.scale_stride, b.scale, a.l ? 2 : 1, b.l ? 2 : 1,
-                      short_chunks ? kShortChunkBlocks : kChunkBlocks};
+  const HalfArgs args{prob, a.scale, a.scale_stride, b.scale, a.l ? 2 : 1, b.l ? 2 : 1};
   // A pair's 256 x 256 tile takes about 1.5 times as long as a CTA's 128 x 128 one (it loads half as much per product): pairs
   // unless single CTAs get by with so few waves that they finish earlier.  Pairs against singles, measured: 1024^3 32 and
   // 24 us, 2048^3 50 and 69, 4096^3 333 and 410; symmetric, then drained every 128 of K, 1024 39 and 28, 2048 54 and 44, 4096 186 and

@@ -164,8 +164,11 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t smem_addr, uint32_t rank
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(mapped) : "r"(smem_addr), "r"(rank));
   return mapped;
 }
+// Arrival on an mbarrier of either CTA of the cluster.  It hands over tensor memory that this thread's warp has read (ordered
+// by tcgen05.wait::ld and tcgen05.fence::before_thread_sync), no generic memory, so it is not a cluster-scope release: that
+// one waits for all earlier writes of the SM, and cost 80 of 434 us where a 4096^3 product drains its accumulator every 64 of K.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 // Tiled 2-D load into this CTA's shared memory whose completion bytes are credited to the mbarrier at `bar_cluster_addr`
 // (a shared::cluster address: the leader CTA's barrier).  No multicast: every CTA loads its own tile.

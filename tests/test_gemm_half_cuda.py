@@ -4,7 +4,7 @@ import torch
 
 pytestmark = pytest.mark.gpu
 
-# Both operands carry at least 22 bits and the sums are rounded to nearest in fp32 every 128 of K, so a product is as far from
+# Both operands carry at least 22 bits and the sums are rounded to nearest in fp32 every 64 of K, so a product is as far from
 # fp64 as an fp32 one: the bound of the tf32 kernels' tests.
 BOUND = 2e-6
 
@@ -187,3 +187,53 @@ def test_sums_of_squares_are_no_further_from_fp64_than_in_the_mixed_form(dtype, 
     errors = _rel(half, expected), _rel(mixed, expected)
     print(errors)
     assert errors[0] < 1.05 * errors[1]
+
+
+@pytest.mark.parametrize("depth", [128, 1000, 8192])
+@pytest.mark.parametrize("terms", [(2, 2), (1, 2), (2, 1), (1, 1)])
+@pytest.mark.parametrize("kind", ["positive", "itself"])
+@pytest.mark.parametrize("tiles", [1, 2])
+def test_one_sided_sums_are_no_further_from_fp64_than_in_the_mixed_form(depth, terms, kind, tiles):
+    """Plain products whose terms do not cancel, as in a rotation along a leading singular vector: every truncated addition errs
+    to the same side.  The whole result where all entries are such sums, the diagonal where the second operand is the first."""
+    from soap_tp_b200.engine import kernels as k
+
+    g = torch.Generator(device="cuda").manual_seed(depth)
+    a, b = (torch.randn(depth, 384, generator=g, device="cuda") for _ in range(2))
+    if kind == "itself":
+        b = a
+    else:
+        a, b = a.abs(), b.abs()
+    a, b = (t.bfloat16() if count == 1 else t for t, count in zip((a, b), terms))
+    expected = (a.double().T @ b.double()).cpu()
+    mixed, half = (torch.empty(384, 384, device="cuda").T for _ in range(2))
+    k.gemm(*(k.split_planes(t.float(), mixed=True) for t in (a, b)), out=mixed)
+    k.gemm_half(_planes(a), _planes(b), out=half, tiles=tiles)
+    k.check_status()
+    if kind == "itself":
+        mixed, half, expected = mixed.diagonal(), half.diagonal(), expected.diagonal()
+    assert _rel(half, expected) < 1.05 * _rel(mixed, expected)
+
+
+@pytest.mark.parametrize("size", [130, 1024])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_one_sided_chains_are_no_further_from_fp64_than_in_the_mixed_form(size, dtype):
+    """Two products in a row, the first one's result as scaled planes: positive operands, and a rotation of a matrix into its own
+    singular vectors."""
+    from soap_tp_b200.engine import kernels as k
+
+    g = torch.Generator(device="cuda").manual_seed(size)
+    x, q, w = (torch.rand(size, size, generator=g, device="cuda") + 0.1 for _ in range(3))
+    left, _, right = torch.linalg.svd((x - 0.6).double())
+    for source, first, second in ((x, q, w), (x - 0.6, left.float(), right.T.float())):
+        source = source.to(dtype)
+        expected = ((source.double().T @ first.double()).T @ second.double()).cpu()
+        middle = k.Planes.empty(size, size, "cuda", mixed=True)
+        mixed, half = (torch.empty(size, size, device="cuda").T for _ in range(2))
+        k.gemm(k.split_planes(source.float(), mixed=True), k.split_planes(first, mixed=True), mode=k.EPI_SPLIT, out_planes=middle)
+        k.gemm(middle, k.split_planes(second, mixed=True), out=mixed)
+        middle = k.HalfPlanes.empty(size, size, "cuda", blocked=True)
+        k.gemm_half(_planes(source), _planes(first), mode=k.EPI_SPLIT, out_planes=middle)
+        k.gemm_half(middle, _planes(second), out=half)
+        k.check_status()
+        assert _rel(half, expected) < 1.05 * _rel(mixed, expected)
