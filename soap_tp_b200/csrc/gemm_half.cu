@@ -49,6 +49,17 @@ constexpr int kSmemBytes = kStagePool + 1024 + 256;
 // order one, and a large A must not overflow before B's factor brings the product back into range.
 constexpr float kDown = 1.0f / 65536.0f, kUp = 65536.0f;
 
+// What brings a column's sums back to scale: kUp and the column's scale in an order that rounds once.  A scale below one takes
+// kUp in (together exact); above one it comes after kUp (both only enlarge a sum that is below the product).  Sums are about
+// half as large as A's elements times their number, so bits are lost below 2^-124 only, where fp32 operands lose them too,
+// and what overflows is A above 2^128 over that number.
+struct ColumnFactor {
+  float first, second;
+  __device__ __forceinline__ explicit ColumnFactor(float scale = 0.f)
+      : first(scale < 1.f ? scale * kUp : kUp), second(scale < 1.f ? 1.f : scale) {}
+  __device__ __forceinline__ float operator()(float sum) const { return (sum * first) * second; }
+};
+
 struct alignas(64) HalfMaps {
   CUtensorMap a_h, a_l, b_h, b_l;
 };
@@ -91,28 +102,28 @@ template <int BN, int MODE, int PITCH>
 __device__ __forceinline__ void half_epilogue(const HalfArgs& args, float* tile, int m0, int n0, int ew, int lane) {
   const HalfProblem& p = args.p;
   const int rows = min(kBM, p.M - m0), cols = min(BN, p.N - n0);
-  const float alpha = p.alpha * kUp;
+  const float alpha = p.alpha;
   if constexpr (MODE == kEpiRowMajor) {
-    float scale[BN / 32];
+    ColumnFactor scaled[BN / 32];
 #pragma unroll
-    for (int j = 0; j < BN / 32; ++j) scale[j] = (lane + 32 * j < cols) ? args.b_scale[n0 + lane + 32 * j] : 0.f;
+    for (int j = 0; j < BN / 32; ++j) scaled[j] = ColumnFactor((lane + 32 * j < cols) ? args.b_scale[n0 + lane + 32 * j] : 0.f);
     for (int r = ew; r < rows; r += kEpiWarps) {
       float* dst = p.C + static_cast<int64_t>(m0 + r) * p.ldc + n0;
 #pragma unroll
       for (int j = 0; j < BN / 32; ++j) {
         const int n = lane + 32 * j;
-        if (n < cols) dst[n] = alpha * (tile[n * PITCH + r] * scale[j]);
+        if (n < cols) dst[n] = alpha * scaled[j](tile[n * PITCH + r]);
       }
     }
   } else if constexpr (MODE == kEpiSplit) {
     for (int nl = ew; nl < cols; nl += kEpiWarps) {
-      const float scale = args.b_scale[n0 + nl];
+      const ColumnFactor scaled(args.b_scale[n0 + nl]);
       float v[4];
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
         const float2 x = *reinterpret_cast<const float2*>(tile + nl * PITCH + 64 * i + 2 * lane);
-        v[2 * i] = alpha * (x.x * scale);
-        v[2 * i + 1] = alpha * (x.y * scale);
+        v[2 * i] = alpha * scaled(x.x);
+        v[2 * i + 1] = alpha * scaled(x.y);
       }
       store_half_column(p, m0, n0 + nl, lane, v);
     }
@@ -137,10 +148,11 @@ __device__ __forceinline__ void half_epilogue(const HalfArgs& args, float* tile,
         if (base + u >= cols) break;
         const int n = n0 + base + u;
         float* column = tile + (base + u) * PITCH;
+        const ColumnFactor scaled(scale[u]);
 #pragma unroll
         for (int i = 0; i < kRowsPerLane; ++i) {
           const int r = lane + 32 * i;
-          const float g = alpha * (column[r] * scale[u]);
+          const float g = alpha * scaled(column[r]);
           const float m_new = fmaf(p.beta1, mo[u][i], (1.0f - p.beta1) * g);
           const float v_new = fmaf(p.beta2, va[u][i], (1.0f - p.beta2) * g * g);
           float update = 0.f;
@@ -183,11 +195,12 @@ __device__ __forceinline__ void half_epilogue(const HalfArgs& args, float* tile,
         const int n = n0 + base + u;
         if (base + u >= cols) break;
         float* column = tile + (base + u) * PITCH;
+        const ColumnFactor scaled(scale[u]);
 #pragma unroll
         for (int i = 0; i < kRowsPerLane; ++i) {
           const int r = lane + 32 * i;
           if (r < rows && (!p.symmetric || n <= m0 + r)) {
-            float v = alpha * (column[r] * scale[u]);
+            float v = alpha * scaled(column[r]);
             if (p.beta != 0.f) v = fmaf(p.beta, old[u][i], v);
             p.C[m0 + r + static_cast<int64_t>(n) * p.ldc] = v;
             if (p.symmetric) column[r] = v;

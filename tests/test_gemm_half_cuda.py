@@ -237,3 +237,41 @@ def test_one_sided_chains_are_no_further_from_fp64_than_in_the_mixed_form(size, 
         k.gemm_half(middle, _planes(second), out=half)
         k.check_status()
         assert _rel(half, expected) < 1.05 * _rel(mixed, expected)
+
+
+@pytest.mark.parametrize("sizes", [(-60, -60), (-62, -50), (-110, 0), (-75, 25), (25, -75), (60, 58), (100, 20), (20, 100)])
+@pytest.mark.parametrize("mode", ["store", "split", "row", "average"])
+def test_operands_near_the_limits_of_fp32(sizes, mode):
+    """Powers of two on either operand change no bit of a product as long as the result is a normal number."""
+    from soap_tp_b200.engine import kernels as k
+
+    g = torch.Generator().manual_seed(6)
+    a, b = torch.randn(100, 140, generator=g), torch.randn(100, 150, generator=g)
+    plain, scaled = [], []
+    for results, (down_a, down_b) in ((plain, (0, 0)), (scaled, sizes)):
+        ap, bp = _planes((a * 2.0**down_a).cuda()), _planes((b * 2.0**down_b).cuda())
+        if mode == "split":
+            out = k.HalfPlanes.empty(140, 150, "cuda", blocked=True)
+            k.gemm_half(ap, bp, mode=k.EPI_SPLIT, out_planes=out)
+            results.append(out.dense())
+        elif mode == "row":
+            out = torch.empty(140, 150, device="cuda")
+            k.gemm_half(ap, bp, mode=k.EPI_ROW_MAJOR, out=out)
+            results.append(out.double())
+        elif mode == "store":
+            out = torch.empty(150, 140, device="cuda").T
+            k.gemm_half(ap, bp, out=out)
+            results.append(out.double())
+        else:
+            out = torch.empty(140, 140, device="cuda").T
+            k.gemm_half(ap, ap, out=out, symmetric=True)
+            results.append(out.double())
+    k.check_status()
+    exponent = 2 * sizes[0] if mode == "average" else sum(sizes)
+    if not -124 < exponent < 120:
+        pytest.skip("the result is not a normal number")
+    assert _rel(plain[0], (a.double().T @ (a if mode == "average" else b).double())) < BOUND
+    expected = plain[0] * 2.0**exponent
+    # entries of a product that fall below the smallest normal number round there
+    assert bool((scaled[0] - expected).abs().max() <= 2.0**-148)
+    assert _rel(scaled[0], expected.cpu()) < 1e-6
