@@ -9,6 +9,7 @@
 #include "elementwise.h"
 #include "gemm.h"
 #include "launch_util.h"
+#include "split_write.cuh"
 #include "tile_sweep.cuh"
 
 namespace soapb200 {
@@ -17,15 +18,6 @@ namespace {
 inline void check_launch(const char* what) {
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) throw std::runtime_error(std::string(what) + ": " + cudaGetErrorString(err));
-}
-
-__device__ __forceinline__ float tf32_hi(float x, int nearest) {
-  if (nearest) {
-    uint32_t r;
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
-    return __uint_as_float(r);
-  }
-  return __uint_as_float(__float_as_uint(x) & 0xFFFFE000u);
 }
 
 // ---- Adam ---------------------------------------------------------------------------------
@@ -130,38 +122,6 @@ __global__ void __launch_bounds__(256) adamw_kernel(T* __restrict__ p, const T* 
 // Bound by memory: the source is read once for both orientations, 64 x 64 tiles turned in shared memory, 8-byte accesses
 // along the source's unit stride and along each plane's depth.  32 x 32 tiles with 4-byte accesses took 231 us an orientation
 // of an 8192 x 8192 matrix (3.5 TB/s); a one-sided step of 32064 x 2048 bf16 went from 3233 to 3054 us with this kernel.
-__device__ __forceinline__ uint16_t bf16_bits(float v) {
-  const __nv_bfloat16 b = __float2bfloat16_rn(v);
-  return *reinterpret_cast<const uint16_t*>(&b);
-}
-
-// Elements i, i + 1 of column j of an operand of depth n; nothing past the depth is written (the planes may be a window).
-__device__ __forceinline__ void write_split(const SplitTarget& to, bool pairs, int64_t i, int64_t j, int n, float x0, float x1,
-                                            int nearest) {
-  const float h0 = tf32_hi(x0, nearest), h1 = tf32_hi(x1, nearest);
-  const int64_t at = i + j * to.ldo, at16 = to.hl ? bf16_plane_index(i) + j * to.ld16 : 0;
-  if (pairs && i + 1 < n) {
-    *reinterpret_cast<float2*>(to.hi + at) = make_float2(h0, h1);
-    if (to.hl) {
-      *reinterpret_cast<__nv_bfloat162*>(to.hl + at16) = __floats2bfloat162_rn(x0, x1);
-      *reinterpret_cast<__nv_bfloat162*>(to.hl + at16 + 32) = __floats2bfloat162_rn(x0 - h0, x1 - h1);
-    } else {
-      *reinterpret_cast<float2*>(to.lo + at) = make_float2(x0 - h0, x1 - h1);
-    }
-    return;
-  }
-  for (int e = 0; e < 2 && i + e < n; ++e) {
-    const float x = e ? x1 : x0, h = e ? h1 : h0;
-    to.hi[at + e] = h;
-    if (to.hl) {         // i is even, so that i and i + 1 are neighbours in the interleaved plane too
-      to.hl[at16 + e] = bf16_bits(x);
-      to.hl[at16 + e + 32] = bf16_bits(x - h);
-    } else {
-      to.lo[at + e] = x - h;
-    }
-  }
-}
-
 // `along`: depth runs along the source's fast axis; `across`: along its slow axis.
 template <typename T>
 __global__ void __launch_bounds__(sweep::kThreads) split_planes_kernel(const T* __restrict__ src, int64_t s_fast, int64_t s_slow,
@@ -316,11 +276,6 @@ void adamw_update(void* p, int type, const void* gradient, float* m, float* v, i
 }
 
 namespace {
-bool writes_pairs(const SplitTarget& t) {
-  return (reinterpret_cast<uintptr_t>(t.hi) & 7) == 0 && t.ldo % 2 == 0 &&
-         (t.hl ? (reinterpret_cast<uintptr_t>(t.hl) & 3) == 0 && t.ld16 % 2 == 0 : (reinterpret_cast<uintptr_t>(t.lo) & 7) == 0);
-}
-
 template <typename T>
 void launch_split(const T* src, int64_t s_fast, int64_t s_slow, int n_fast, int n_slow, const SplitTarget& along,
                   const SplitTarget& across, float scale, int nearest, cudaStream_t stream) {

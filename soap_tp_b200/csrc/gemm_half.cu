@@ -19,7 +19,6 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
-#include <mutex>
 #include <stdexcept>
 #include <string>
 
@@ -27,6 +26,7 @@
 #include "gemm_half.h"
 #include "launch_util.h"
 #include "ptx.cuh"
+#include "tensor_map.h"
 
 namespace soapb200 {
 namespace {
@@ -458,38 +458,10 @@ half_single_kernel(const __grid_constant__ HalfMaps maps, const __grid_constant_
 }
 
 // ---------------------------------------------------------------------------------------------
-using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_tiled_fn() {
-  static EncodeTiledFn fn = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    void* ptr = nullptr;
-    cudaDriverEntryPointQueryResult query;
-    cudaError_t err = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &query);
-    if (err != cudaSuccess || query != cudaDriverEntryPointSuccess || ptr == nullptr)
-      throw std::runtime_error("cuTensorMapEncodeTiled is not available from the CUDA driver");
-    fn = reinterpret_cast<EncodeTiledFn>(ptr);
-  });
-  return fn;
-}
-
 // K-contiguous fp16 plane [rows][K] with row pitch ld: boxes of 64 elements x 128 rows.
 CUtensorMap make_map(const uint16_t* base, int64_t K, int64_t rows, int64_t ld) {
-  if ((reinterpret_cast<uintptr_t>(base) & 15) != 0 || ld % 64 != 0 || ld < K)
-    throw std::invalid_argument("gemm_half: planes need 16-byte alignment and a pitch that is a multiple of 64 covering K");
-  CUtensorMap map;
-  cuuint64_t dims[2] = {static_cast<cuuint64_t>(K), static_cast<cuuint64_t>(rows)};
-  cuuint64_t strides[1] = {static_cast<cuuint64_t>(ld) * 2};
-  cuuint32_t box[2] = {kBK, 128};
-  cuuint32_t elem[2] = {1, 1};
-  CUresult res = encode_tiled_fn()(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<uint16_t*>(base), dims, strides, box,
-                                   elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (res != CUDA_SUCCESS) throw std::runtime_error("gemm_half: cuTensorMapEncodeTiled failed with code " + std::to_string(res));
-  return map;
+  if (ld % 64 != 0 || ld < K) throw std::invalid_argument("gemm_half: planes need a pitch that is a multiple of 64 covering K");
+  return encode_k_major(CU_TENSOR_MAP_DATA_TYPE_FLOAT16, base, K, rows, 2 * ld, kBK, 128, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
 template <int MODE>

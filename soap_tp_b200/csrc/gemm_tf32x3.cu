@@ -25,7 +25,6 @@
 
 #include <cstdio>
 #include <map>
-#include <mutex>
 #include <stdexcept>
 #include <string>
 #include <tuple>
@@ -33,6 +32,7 @@
 #include "gemm.h"
 #include "launch_util.h"
 #include "ptx.cuh"
+#include "tensor_map.h"
 
 namespace soapb200 {
 
@@ -862,58 +862,17 @@ gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ 
 }
 
 // ---------------------------------------------------------------------------------------------
-// Host side: tensor maps (driver entry point fetched at run time, so no link-time libcuda) and launch.
-using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+// Host side: tensor maps and launch.
 
-EncodeTiledFn encode_tiled_fn() {
-  static EncodeTiledFn fn = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    void* ptr = nullptr;
-    cudaDriverEntryPointQueryResult query;
-    cudaError_t err = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &query);
-    if (err != cudaSuccess || query != cudaDriverEntryPointSuccess || ptr == nullptr)
-      throw std::runtime_error("cuTensorMapEncodeTiled is not available from the CUDA driver");
-    fn = reinterpret_cast<EncodeTiledFn>(ptr);
-  });
-  return fn;
-}
-
-// K-contiguous fp32 matrix [rows][K] with row pitch ld (floats); box = 32 floats x box_rows rows.
+// K-contiguous fp32 matrix [rows][K] with row pitch ld (floats); box = one k-block x box_rows rows.
 CUtensorMap make_operand_map(const float* base, int64_t K, int64_t rows, int64_t ld, int box_rows) {
-  if ((reinterpret_cast<uintptr_t>(base) & 15) != 0) throw std::invalid_argument("operand plane must be 16-byte aligned");
-  if ((ld * 4) % 16 != 0) throw std::invalid_argument("operand plane pitch must be a multiple of 4 floats");
-  CUtensorMap map;
-  cuuint64_t dims[2] = {static_cast<cuuint64_t>(K), static_cast<cuuint64_t>(rows)};
-  cuuint64_t strides[1] = {static_cast<cuuint64_t>(ld) * 4};
-  cuuint32_t box[2] = {static_cast<cuuint32_t>(kBK), static_cast<cuuint32_t>(box_rows)};
-  cuuint32_t elem[2] = {1, 1};
-  CUresult res = encode_tiled_fn()(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(base), dims, strides, box,
-                                   elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                                   kRowBytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
-                                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (res != CUDA_SUCCESS) throw std::runtime_error("cuTensorMapEncodeTiled failed with code " + std::to_string(res));
-  return map;
+  return encode_k_major(CU_TENSOR_MAP_DATA_TYPE_FLOAT32, base, K, rows, 4 * ld, kBK, box_rows,
+                        kRowBytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B);
 }
 
-// Interleaved bf16 plane of a K-contiguous operand: [rows][64 * ceil(K / 32)] elements with row pitch ld
-// (elements); box = 64 elements (128 bytes: hb and lb of one 32-element k-block) x box_rows rows.
+// Interleaved bf16 plane; box = hb and lb of one k-block x box_rows rows.
 CUtensorMap make_bf16_map(const uint16_t* base, int64_t K, int64_t rows, int64_t ld, int box_rows) {
-  if ((reinterpret_cast<uintptr_t>(base) & 15) != 0) throw std::invalid_argument("bf16 operand plane must be 16-byte aligned");
-  const int64_t extent = 64 * ((K + 31) / 32);
-  if (ld % 64 != 0 || ld < extent) throw std::invalid_argument("bf16 operand plane pitch must be a multiple of 64 elements covering K");
-  CUtensorMap map;
-  cuuint64_t dims[2] = {static_cast<cuuint64_t>(extent), static_cast<cuuint64_t>(rows)};
-  cuuint64_t strides[1] = {static_cast<cuuint64_t>(ld) * 2};
-  cuuint32_t box[2] = {static_cast<cuuint32_t>(2 * kBK), static_cast<cuuint32_t>(box_rows)};
-  cuuint32_t elem[2] = {1, 1};
-  CUresult res = encode_tiled_fn()(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<uint16_t*>(base), dims, strides, box,
-                                   elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (res != CUDA_SUCCESS) throw std::runtime_error("cuTensorMapEncodeTiled (bf16) failed with code " + std::to_string(res));
-  return map;
+  return encode_interleaved(base, K, rows, ld, 2 * kBK, box_rows);
 }
 
 template <int BN, int MODE, bool MIXED>
