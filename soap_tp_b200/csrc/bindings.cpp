@@ -29,7 +29,79 @@ T* ptr(uint64_t address) {
   return reinterpret_cast<T*>(static_cast<uintptr_t>(address));
 }
 cudaStream_t stream_of(uint64_t handle) { return reinterpret_cast<cudaStream_t>(static_cast<uintptr_t>(handle)); }
+
+// A flat list of integers (addresses, pitches, sizes) read in order: a call with one list costs the interpreter a third of one
+// with as many arguments.
+class Arguments {
+ public:
+  explicit Arguments(const std::vector<int64_t>& values) : values_(values) {}
+  int64_t next() {
+    if (at_ >= values_.size()) throw std::invalid_argument("too few integers for this call");
+    return values_[at_++];
+  }
+  template <typename T>
+  T* pointer() { return ptr<T>(static_cast<uint64_t>(next())); }
+  cudaStream_t stream() { return stream_of(static_cast<uint64_t>(next())); }
+  // scaled fp16 planes: h, l, pitch, scale, then scratch of the largest magnitudes or the stride of the scales
+  HalfTarget target() {
+    HalfTarget t{};
+    t.h = pointer<uint16_t>(); t.l = pointer<uint16_t>(); t.ld = next(); t.scale = pointer<float>(); t.largest = pointer<uint32_t>();
+    return t;
+  }
+  HalfOperand operand() {
+    HalfOperand o{};
+    o.h = pointer<uint16_t>(); o.l = pointer<uint16_t>(); o.ld = next(); o.scale = pointer<float>(); o.scale_stride = next();
+    return o;
+  }
+  // the mixed form: tf32 values, pitch, interleaved bf16 plane, pitch
+  SplitTarget mixed() {
+    SplitTarget t{};
+    t.hi = pointer<float>(); t.ldo = next(); t.hl = pointer<uint16_t>(); t.ld16 = next();
+    return t;
+  }
+  void matrix_and_bases(Rotation& r) {
+    r.source = pointer<void>(); r.source_type = static_cast<int>(next()); r.s_i = next(); r.s_j = next();
+    r.rows = static_cast<int>(next()); r.cols = static_cast<int>(next());
+    auto basis = [&](HalfOperand& plain, HalfOperand& turned, WideBasis& source, int size) {
+      plain = operand(); turned = operand();
+      source.src = pointer<float>(); source.s_i = next(); source.s_j = next(); source.size = size;
+      plain.mixed = source.plain; turned.mixed = source.turned;
+    };
+    basis(r.left, r.left_turned, r.guard.bases[0], r.rows);
+    basis(r.right, r.right_turned, r.guard.bases[1], r.cols);
+  }
+  void finish() const {
+    if (at_ != values_.size()) throw std::invalid_argument("too many integers for this call");
+  }
+
+ private:
+  const std::vector<int64_t>& values_;
+  size_t at_ = 0;
+};
 }  // namespace
+
+// The scratch of rotations of one shape, handed over once: planes, the decision on the range, and the mixed form of everything.
+struct RotationScratch {
+  Rotation rotation{};       // without the matrix and its bases
+  HalfOperand update{};
+
+  explicit RotationScratch(const std::vector<int64_t>& values) {
+    Arguments in(values);
+    Rotation& r = rotation;
+    r.x = in.target(); r.xt = in.target();
+    r.middle = in.operand();
+    r.guard.wide = in.pointer<int>(); r.guard.nearest = static_cast<int>(in.next());
+    r.guard.mixed = in.mixed();
+    r.middle.mixed = in.mixed();
+    for (WideBasis& basis : r.guard.bases) {
+      basis.plain = in.mixed();
+      basis.turned = in.mixed();
+    }
+    update = in.operand();
+    update.mixed = in.mixed();
+    in.finish();
+  }
+};
 
 PYBIND11_MODULE(_C, m) {
   m.doc() = "sm_100a kernels of soap_tp_b200";
@@ -122,49 +194,53 @@ PYBIND11_MODULE(_C, m) {
           half_planes(ptr<const void>(src), source_type, s_i, s_j, rows, cols,
                       HalfTarget{ptr<uint16_t>(ph), ptr<uint16_t>(pl), pld, ptr<float>(pscale), ptr<uint32_t>(plargest)},
                       HalfTarget{ptr<uint16_t>(th), ptr<uint16_t>(tl), tld, ptr<float>(tscale), ptr<uint32_t>(tlargest)},
-                      stream_of(stream));
+                      RangeGuard{}, stream_of(stream));
         },
         "Scaled fp16 operand planes of a matrix in one or both orientations (gemm_half.h)");
 
-  // Integers in the order of SteadyStep (planes and operands as five each: h, l, pitch, scale, then scratch of the largest
-  // magnitudes or the stride of the scales), then the status word, the stream and the
-  // stream of the rotations.
-  m.def("steady_step", [](const std::vector<int64_t>& v, double beta, float beta1, float beta2, float eps, float inv_bc1,
-                          float inv_sqrt_bc2) {
-    if (v.size() != 58) throw std::invalid_argument("steady_step: 58 integers expected");
-    size_t at = 0;
-    auto next = [&] { return v[at++]; };
-    auto address = [&] { return reinterpret_cast<void*>(static_cast<uintptr_t>(v[at++])); };
-    auto target = [&] {
-      HalfTarget t{};
-      t.h = static_cast<uint16_t*>(address()); t.l = static_cast<uint16_t*>(address()); t.ld = next();
-      t.scale = static_cast<float*>(address()); t.largest = static_cast<uint32_t*>(address());
-      return t;
-    };
-    auto operand = [&] {
-      HalfOperand o{};
-      o.h = static_cast<uint16_t*>(address()); o.l = static_cast<uint16_t*>(address()); o.ld = next();
-      o.scale = static_cast<float*>(address()); o.scale_stride = next();
-      return o;
-    };
+  py::class_<RotationScratch>(m, "RotationScratch", "Scratch planes of rotations of one shape, as addresses (see Arguments)")
+      .def(py::init<const std::vector<int64_t>&>());
+  // Integers: the matrix and its bases (Arguments), the moments, results and phases in the order of SteadyStep, then the status
+  // word, the stream and the stream of the rotations.
+  m.def("steady_step", [](const RotationScratch& scratch, const std::vector<int64_t>& v, double beta, float beta1, float beta2,
+                          float eps, float inv_bc1, float inv_sqrt_bc2) {
+    Arguments in(v);
     SteadyStep s{};
-    s.gradient = address(); s.gradient_type = static_cast<int>(next()); s.s_i = next(); s.s_j = next();
-    s.rows = static_cast<int>(next()); s.cols = static_cast<int>(next());
-    s.x = target(); s.xt = target();
-    s.left = operand(); s.left_turned = operand(); s.right = operand(); s.right_turned = operand();
-    s.middle = operand(); s.update = operand();
-    s.momentum = static_cast<float*>(address()); s.ldm = next();
-    s.variance = static_cast<float*>(address()); s.ldv = next();
-    s.out = static_cast<float*>(address());
-    s.left_gram = static_cast<float*>(address()); s.ld_left = next();
-    s.right_gram = static_cast<float*>(address()); s.ld_right = next();
-    int* status = static_cast<int*>(address());
-    cudaStream_t stream = static_cast<cudaStream_t>(address());
-    s.chain = static_cast<cudaStream_t>(address());
+    s.rotation = scratch.rotation;
+    s.update = scratch.update;
+    in.matrix_and_bases(s.rotation);
+    s.momentum = in.pointer<float>(); s.ldm = in.next();
+    s.variance = in.pointer<float>(); s.ldv = in.next();
+    s.out = in.pointer<float>();
+    s.left_gram = in.pointer<float>(); s.ld_left = in.next();
+    s.right_gram = in.pointer<float>(); s.ld_right = in.next();
+    s.phases = static_cast<int>(in.next());
+    int* status = in.pointer<int>();
+    cudaStream_t stream = in.stream();
+    s.chain = in.stream();
+    in.finish();
     s.beta = beta; s.beta1 = beta1; s.beta2 = beta2; s.eps = eps; s.inv_bc1 = inv_bc1; s.inv_sqrt_bc2 = inv_sqrt_bc2;
     py::gil_scoped_release release;
     steady_step(s, status, stream);
-  }, "The launches of one ordinary single-GPU step (gemm_half.h, SteadyStep)");
+  }, "The launches of one ordinary single-GPU step, or some of its phases (gemm_half.h, SteadyStep)");
+  m.attr("STEP_PLANES") = kStepPlanes;
+  m.attr("STEP_FORWARD") = kStepForward;
+  m.attr("STEP_BACKWARD") = kStepBackward;
+  m.attr("STEP_AVERAGES") = kStepAverages;
+  // Integers: the matrix and its bases, then direction, result, its pitch, the status word and the stream.
+  m.def("rotate_half", [](const RotationScratch& scratch, const std::vector<int64_t>& v) {
+    Arguments in(v);
+    Rotation r = scratch.rotation;
+    in.matrix_and_bases(r);
+    const bool turned = in.next() != 0;
+    float* out = in.pointer<float>();
+    const int64_t ldc = in.next();
+    int* status = in.pointer<int>();
+    cudaStream_t stream = in.stream();
+    in.finish();
+    py::gil_scoped_release release;
+    rotate_half(r, turned, out, ldc, status, stream);
+  }, "A matrix rotated by two bases on scaled fp16 planes, or on their mixed form where its range asks for it (gemm_half.h)");
 
   m.def("gemm_simt",
         [](uint64_t A, int64_t a_sk, int64_t a_sm, uint64_t B, int64_t b_sk, int64_t b_sn, uint64_t C, int64_t c_sm,

@@ -15,17 +15,24 @@
 // The tensor core adds into its accumulator with truncation, so the accumulator is drained every 64 of K (one k-block) into
 // a register-resident sum (round-to-nearest), multiplied by the scale of A's block of 128 on the way; B's scales are per
 // column and applied once, in the epilogue.  Within a k-block the small products come first.
+//
+// Where the device word `wide` is set (RangeGuard: rows or columns that fp16 pairs do not hold) the same kernel runs the
+// mixed form: four boxes of the same size, 32 of K each, tf32 and bf16 MMAs in gemm_tf32x3.cu's order, two k-blocks per drain,
+// and bit for bit its results.  One launch serves both, so that nobody waits for the decision on the host.
 #include <cuda.h>
+#include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
 #include <stdexcept>
 #include <string>
+#include <type_traits>
 
 #include "gemm.h"
 #include "gemm_half.h"
 #include "launch_util.h"
 #include "ptx.cuh"
+#include "split_write.cuh"
 #include "tensor_map.h"
 
 namespace soapb200 {
@@ -39,6 +46,8 @@ constexpr int kBK = 64;                          // one 128-byte swizzle row of 
 // terms 2.7e-7 / 6.6e-7 / 4.6e-7 at K = 8192 and 2.1e-7 / 6.6e-7 / 4.5e-7 at K = 128, one term against two 2.1e-7 / 3.7e-7 /
 // 3.1e-7 and 1.3e-7 / 3.6e-7 / 2.7e-7.  The price: two terms 4096^3 351 us instead of 319, one term against two 293 instead of 247.
 constexpr int kScaleBlocks = kHalfScaleBlock / kBK;      // k-blocks that share one of A's scales
+constexpr int kMixedBK = 32;                     // one 128-byte swizzle row of fp32, or of the interleaved bf16 plane
+constexpr int kMixedDrain = 2;                   // its k-blocks per promotion
 constexpr int kBoxBytes = 128 * kBK * 2;
 constexpr int kStagePool = 12 * kBoxBytes;       // 3 stages of four boxes, 4 of three, 6 of two
 constexpr int kMaxStages = 6;
@@ -62,6 +71,7 @@ struct ColumnFactor {
 
 struct alignas(64) HalfMaps {
   CUtensorMap a_h, a_l, b_h, b_l;
+  CUtensorMap mixed[4];                          // A's tf32 values and corrections, B's: read where `wide` says so
 };
 
 struct HalfArgs {
@@ -71,6 +81,25 @@ struct HalfArgs {
   const float* b_scale;
   int a_terms, b_terms;
 };
+
+// One CTA's way along K: k-blocks, stages, and drains of the accumulator.
+struct KLoop {
+  int blocks, drains, a_terms, b_terms, stages, stage_bytes, b_at;
+  template <bool MIXED>
+  __device__ __forceinline__ static KLoop over(const HalfArgs& args) {
+    KLoop l;
+    l.blocks = (args.p.K + (MIXED ? kMixedBK : kBK) - 1) / (MIXED ? kMixedBK : kBK);
+    l.drains = MIXED ? (l.blocks + kMixedDrain - 1) / kMixedDrain : l.blocks;
+    l.a_terms = MIXED ? 2 : args.a_terms;
+    l.b_terms = MIXED ? 2 : args.b_terms;
+    const int boxes = l.a_terms + l.b_terms;
+    l.stages = 12 / boxes;                     // 3, 4 or 6 stages of four, three or two boxes
+    l.stage_bytes = boxes * kBoxBytes;
+    l.b_at = l.a_terms * kBoxBytes;            // a stage holds A's planes, then B's
+    return l;
+  }
+};
+static_assert(kMixedBK * kMixedDrain == kBK, "both forms drain as often");
 
 constexpr int kUnroll = 4;       // columns per warp whose loads are in flight together
 constexpr int kRowsPerLane = 4;  // a column of the tile is 128 rows: rows lane, lane + 32, lane + 64, lane + 96
@@ -96,17 +125,33 @@ __device__ __forceinline__ void store_half_column(const HalfProblem& p, int m0, 
   }
 }
 
-// Epilogue over the staged tile: tile[n_local * PITCH + m_local] holds sums 2^-16 below scale, without B's scales.  Accesses
-// are four bytes per lane along M, so that no alignment of the outputs is needed, with kUnroll columns in flight.
+// The same column as an operand in the mixed form.
+__device__ __forceinline__ void store_mixed_column(const HalfProblem& p, int m0, int n, int lane, const float (&v)[4]) {
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int m = m0 + 64 * i + 2 * lane;
+    if (m < p.M) write_split(p.mixed, true, m, n, p.M, v[2 * i], v[2 * i + 1], 1);
+  }
+}
+
+__device__ __forceinline__ void store_column(const HalfProblem& p, bool wide, int m0, int n, int lane, const float (&v)[4]) {
+  if (wide) store_mixed_column(p, m0, n, lane, v);
+  else store_half_column(p, m0, n, lane, v);
+}
+
+// Epilogue over the staged tile: tile[n_local * PITCH + m_local] holds sums 2^-16 below scale, without B's scales (`wide`: the
+// sums themselves).  Accesses are four bytes per lane along M, so that no alignment of the outputs is needed, with kUnroll
+// columns in flight.
 template <int BN, int MODE, int PITCH>
-__device__ __forceinline__ void half_epilogue(const HalfArgs& args, float* tile, int m0, int n0, int ew, int lane) {
+__device__ __forceinline__ void half_epilogue(const HalfArgs& args, bool wide, float* tile, int m0, int n0, int ew, int lane) {
   const HalfProblem& p = args.p;
+  auto column_scale = [&](int n) { return wide ? kDown : args.b_scale[n]; };      // kDown undoes kUp: a factor of one
   const int rows = min(kBM, p.M - m0), cols = min(BN, p.N - n0);
   const float alpha = p.alpha;
   if constexpr (MODE == kEpiRowMajor) {
     ColumnFactor scaled[BN / 32];
 #pragma unroll
-    for (int j = 0; j < BN / 32; ++j) scaled[j] = ColumnFactor((lane + 32 * j < cols) ? args.b_scale[n0 + lane + 32 * j] : 0.f);
+    for (int j = 0; j < BN / 32; ++j) scaled[j] = ColumnFactor((lane + 32 * j < cols) ? column_scale(n0 + lane + 32 * j) : 0.f);
     for (int r = ew; r < rows; r += kEpiWarps) {
       float* dst = p.C + static_cast<int64_t>(m0 + r) * p.ldc + n0;
 #pragma unroll
@@ -117,7 +162,7 @@ __device__ __forceinline__ void half_epilogue(const HalfArgs& args, float* tile,
     }
   } else if constexpr (MODE == kEpiSplit) {
     for (int nl = ew; nl < cols; nl += kEpiWarps) {
-      const ColumnFactor scaled(args.b_scale[n0 + nl]);
+      const ColumnFactor scaled(column_scale(n0 + nl));
       float v[4];
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
@@ -125,7 +170,7 @@ __device__ __forceinline__ void half_epilogue(const HalfArgs& args, float* tile,
         v[2 * i] = alpha * scaled(x.x);
         v[2 * i + 1] = alpha * scaled(x.y);
       }
-      store_half_column(p, m0, n0 + nl, lane, v);
+      store_column(p, wide, m0, n0 + nl, lane, v);
     }
   } else if constexpr (MODE == kEpiAdam) {
     for (int base = ew * kUnroll; base < cols; base += kEpiWarps * kUnroll) {
@@ -134,7 +179,7 @@ __device__ __forceinline__ void half_epilogue(const HalfArgs& args, float* tile,
       for (int u = 0; u < kUnroll; ++u) {
         const int n = n0 + base + u;
         const bool here = base + u < cols;
-        scale[u] = here ? args.b_scale[n] : 0.f;
+        scale[u] = here ? column_scale(n) : 0.f;
 #pragma unroll
         for (int i = 0; i < kRowsPerLane; ++i) {
           const int r = lane + 32 * i;
@@ -171,7 +216,7 @@ __device__ __forceinline__ void half_epilogue(const HalfArgs& args, float* tile,
           v[2 * i] = x.x;
           v[2 * i + 1] = x.y;
         }
-        store_half_column(p, m0, n, lane, v);
+        store_column(p, wide, m0, n, lane, v);
       }
     }
   } else {
@@ -182,7 +227,7 @@ __device__ __forceinline__ void half_epilogue(const HalfArgs& args, float* tile,
       for (int u = 0; u < kUnroll; ++u) {
         const int n = n0 + base + u;
         const bool here = base + u < cols;
-        scale[u] = here ? args.b_scale[n] : 0.f;
+        scale[u] = here ? column_scale(n) : 0.f;
 #pragma unroll
         for (int i = 0; i < kRowsPerLane; ++i) {
           const int r = lane + 32 * i;
@@ -288,38 +333,45 @@ __device__ __forceinline__ void half_kernel_body(const HalfMaps& maps, const Hal
   if constexpr (PAIR) cluster_sync_all();      // both CTAs' barriers exist before anything arrives on them remotely
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  // The same in every CTA.  Where the decision is older than the kernel ahead -- which waited for the one that made it before
+  // it let this one start -- it is read while that one still runs.
+  auto decision = [&] { return prob.wide && *static_cast<const volatile int*>(prob.wide); };
+  bool wide = prob.settled && decision();
   wait_for_predecessor();
   let_successor_start();
+  if (!prob.settled) wide = decision();
 
-  const int k_blocks = (prob.K + kBK - 1) / kBK;
-  const int boxes = args.a_terms + args.b_terms;
-  const int stages = 12 / boxes;               // 3, 4 or 6 stages of four, three or two boxes
-  const int stage_bytes = boxes * kBoxBytes;
-  const int b_at = args.a_terms * kBoxBytes;   // a stage holds A's planes, then B's
 
-  if (warp == 0 && lane == 0) {
+  // The roles, for either form.
+  auto produce = [&](auto mixed) {
     // ---------------- TMA producer (each CTA loads its own tiles; PAIR: the bytes are credited to the leader) ----------------
+    constexpr bool kMixed = decltype(mixed)::value;
+    const KLoop loop = KLoop::over<kMixed>(args);
+    const CUtensorMap* a_first = kMixed ? &maps.mixed[0] : &maps.a_h;
+    const CUtensorMap* a_second = kMixed ? &maps.mixed[1] : &maps.a_l;
+    const CUtensorMap* b_first = kMixed ? &maps.mixed[2] : &maps.b_h;
+    const CUtensorMap* b_second = kMixed ? &maps.mixed[3] : &maps.b_l;
     int s = 0;
     uint32_t parity = 1;                       // of the previous round's release
-    for (int kb = 0; kb < k_blocks; ++kb) {
-      if (kb >= stages && !mbar_wait_bounded(&empty_bar[s], parity, abort_flag, status, kStatusSlotWaitTimeout)) break;
-      uint8_t* stage = smem + s * stage_bytes;
-      const int k0 = kb * kBK;
+    for (int kb = 0; kb < loop.blocks; ++kb) {
+      if (kb >= loop.stages && !mbar_wait_bounded(&empty_bar[s], parity, abort_flag, status, kStatusSlotWaitTimeout)) break;
+      uint8_t* stage = smem + s * loop.stage_bytes;
+      const int k0 = kb * (kMixed ? kMixedBK : kBK), k1 = kb * kBK;        // the interleaved plane has 64 elements per 32 of K
       if constexpr (PAIR) {
-        if (cta == 0) mbar_expect_tx(&full_bar[s], 2 * stage_bytes);
+        if (cta == 0) mbar_expect_tx(&full_bar[s], 2 * loop.stage_bytes);
         const uint32_t bar = map_to_cta(smem_u32(&full_bar[s]), 0);
-        tma_load_2d_pair(stage, &maps.a_h, bar, k0, m0);
-        if (args.a_terms == 2) tma_load_2d_pair(stage + kBoxBytes, &maps.a_l, bar, k0, m0);
-        tma_load_2d_pair(stage + b_at, &maps.b_h, bar, k0, b_row0);
-        if (args.b_terms == 2) tma_load_2d_pair(stage + b_at + kBoxBytes, &maps.b_l, bar, k0, b_row0);
+        tma_load_2d_pair(stage, a_first, bar, k0, m0);
+        if (loop.a_terms == 2) tma_load_2d_pair(stage + kBoxBytes, a_second, bar, k1, m0);
+        tma_load_2d_pair(stage + loop.b_at, b_first, bar, k0, b_row0);
+        if (loop.b_terms == 2) tma_load_2d_pair(stage + loop.b_at + kBoxBytes, b_second, bar, k1, b_row0);
       } else {
-        mbar_expect_tx(&full_bar[s], stage_bytes);
-        tma_load_2d(stage, &maps.a_h, &full_bar[s], k0, m0);
-        if (args.a_terms == 2) tma_load_2d(stage + kBoxBytes, &maps.a_l, &full_bar[s], k0, m0);
-        tma_load_2d(stage + b_at, &maps.b_h, &full_bar[s], k0, b_row0);
-        if (args.b_terms == 2) tma_load_2d(stage + b_at + kBoxBytes, &maps.b_l, &full_bar[s], k0, b_row0);
+        mbar_expect_tx(&full_bar[s], loop.stage_bytes);
+        tma_load_2d(stage, a_first, &full_bar[s], k0, m0);
+        if (loop.a_terms == 2) tma_load_2d(stage + kBoxBytes, a_second, &full_bar[s], k1, m0);
+        tma_load_2d(stage + loop.b_at, b_first, &full_bar[s], k0, b_row0);
+        if (loop.b_terms == 2) tma_load_2d(stage + loop.b_at + kBoxBytes, b_second, &full_bar[s], k1, b_row0);
       }
-      if (++s == stages) {
+      if (++s == loop.stages) {
         s = 0;
         parity ^= 1;
       }
@@ -328,53 +380,94 @@ __device__ __forceinline__ void half_kernel_body(const HalfMaps& maps, const Hal
       // give copies that are still in flight time to land before the CTA's shared memory is released
       for (int i = 0; i < 1000; ++i) __nanosleep(1000);
     }
-  } else if (warp == 1 && lane == 0 && cta == 0) {
+  };
+
+  auto issue = [&](auto mixed) {
     // ---------------- MMA issuer (PAIR: leader CTA only) ----------------
-    constexpr uint32_t idesc = umma_idesc_fp16(kCtas * kBM, BN);
-    auto mma = [&](uint32_t acc, uint64_t a, uint64_t b, uint32_t accumulate) {
-      if constexpr (PAIR) umma_f16_ss_pair(acc, a, b, idesc, accumulate);
-      else umma_f16_ss(acc, a, b, idesc, accumulate);
+    constexpr bool kMixed = decltype(mixed)::value;
+    const KLoop loop = KLoop::over<kMixed>(args);
+    constexpr uint32_t idesc16 = kMixed ? umma_idesc_bf16(kCtas * kBM, BN) : umma_idesc_fp16(kCtas * kBM, BN);
+    constexpr uint32_t idesc32 = umma_idesc_tf32(kCtas * kBM, BN);
+    auto mma16 = [&](uint32_t acc, uint64_t a, uint64_t b, uint32_t accumulate) {
+      if constexpr (PAIR) umma_f16_ss_pair(acc, a, b, idesc16, accumulate);
+      else umma_f16_ss(acc, a, b, idesc16, accumulate);
+    };
+    auto mma32 = [&](uint32_t acc, uint64_t a, uint64_t b, uint32_t accumulate) {
+      if constexpr (PAIR) umma_tf32_ss_pair(acc, a, b, idesc32, accumulate);
+      else umma_tf32_ss(acc, a, b, idesc32, accumulate);
     };
     auto commit = [&](uint64_t* bar) {
       if constexpr (PAIR) umma_commit_pair(bar);
       else umma_commit(bar);
     };
     bool ok = true;
-    int s = 0;
+    int s = 0, kb = 0;
     uint32_t parity = 0;
-    for (int kb = 0; kb < k_blocks; ++kb) {
-      const int buf = kb & 1;
-      if (kb >= 2) {
-        ok = mbar_wait_bounded(&acc_empty[buf], ((kb >> 1) - 1) & 1, abort_flag, status, kStatusAccumWaitTimeout);
+    for (int d = 0; d < loop.drains; ++d) {
+      const int buf = d & 1;
+      if (d >= 2) {
+        ok = mbar_wait_bounded(&acc_empty[buf], ((d >> 1) - 1) & 1, abort_flag, status, kStatusAccumWaitTimeout);
         if (!ok) break;
         tc_fence_after_sync();
       }
-      ok = mbar_wait_bounded(&full_bar[s], parity, abort_flag, status, kStatusTmaWaitTimeout);
-      if (!ok) break;
-      tc_fence_after_sync();
       const uint32_t acc = tmem_base + static_cast<uint32_t>(buf * BN);
-      const uint32_t stage = smem_u32(smem + s * stage_bytes);
-      const uint64_t a_h = umma_desc_kmajor<128>(stage);
-      const uint64_t b_h = umma_desc_kmajor<128>(stage + b_at);
-      constexpr uint64_t kLow = kBoxBytes >> 4, kStep = 32 >> 4;         // 16 fp16 = 32 bytes along the swizzle row
-      uint32_t more = 0;                       // 0: the first product of the k-block overwrites the accumulator
-      if (args.a_terms == 2) {
+      uint32_t more = 0;                       // 0: the first product since the last drain overwrites the accumulator
 #pragma unroll
-        for (int k = 0; k < kBK / 16; ++k, more = 1) mma(acc, a_h + kLow + k * kStep, b_h + k * kStep, more);     // l * h
+      for (int i = 0; i < (kMixed ? kMixedDrain : 1); ++i, ++kb) {
+        if (kMixed && kb == loop.blocks) break;
+        ok = mbar_wait_bounded(&full_bar[s], parity, abort_flag, status, kStatusTmaWaitTimeout);
+        if (!ok) break;
+        tc_fence_after_sync();
+        const uint32_t stage = smem_u32(smem + s * loop.stage_bytes);
+        const uint64_t a_0 = umma_desc_kmajor<128>(stage);
+        const uint64_t b_0 = umma_desc_kmajor<128>(stage + loop.b_at);
+        constexpr uint64_t kSecond = kBoxBytes >> 4, kStep = 32 >> 4;      // 16 fp16 or 8 fp32 = 32 bytes along the swizzle row
+        if constexpr (kMixed) {
+          constexpr uint64_t kLb = 64 >> 4;    // lb follows hb in a row of the interleaved plane
+          const bool main_first = kb & 1;      // one change of the MMAs' kind per k-block
+          if (main_first) {
+#pragma unroll
+            for (int k = 0; k < kMixedBK / 8; ++k, more = 1) mma32(acc, a_0 + k * kStep, b_0 + k * kStep, more);
+          }
+#pragma unroll
+          for (int k = 0; k < kMixedBK / 16; ++k, more = 1) {
+            const uint64_t a_1 = a_0 + kSecond + k * kStep, b_1 = b_0 + kSecond + k * kStep;
+            mma16(acc, a_1 + kLb, b_1, more);                                                                          // lb * hb
+            mma16(acc, a_1, b_1 + kLb, 1);                                                                             // hb * lb
+          }
+          if (!main_first) {
+#pragma unroll
+            for (int k = 0; k < kMixedBK / 8; ++k) mma32(acc, a_0 + k * kStep, b_0 + k * kStep, 1);
+          }
+        } else {
+          if (loop.a_terms == 2) {
+#pragma unroll
+            for (int k = 0; k < kBK / 16; ++k, more = 1) mma16(acc, a_0 + kSecond + k * kStep, b_0 + k * kStep, more);  // l * h
+          }
+          if (loop.b_terms == 2) {
+#pragma unroll
+            for (int k = 0; k < kBK / 16; ++k, more = 1) mma16(acc, a_0 + k * kStep, b_0 + kSecond + k * kStep, more);  // h * l
+          }
+#pragma unroll
+          for (int k = 0; k < kBK / 16; ++k, more = 1) mma16(acc, a_0 + k * kStep, b_0 + k * kStep, more);              // h * h
+        }
+        commit(&empty_bar[s]);                 // the stage may be refilled once these products have read it
+        if (++s == loop.stages) {
+          s = 0;
+          parity ^= 1;
+        }
       }
-      if (args.b_terms == 2) {
-#pragma unroll
-        for (int k = 0; k < kBK / 16; ++k, more = 1) mma(acc, a_h + k * kStep, b_h + kLow + k * kStep, more);     // h * l
-      }
-#pragma unroll
-      for (int k = 0; k < kBK / 16; ++k, more = 1) mma(acc, a_h + k * kStep, b_h + k * kStep, more);              // h * h
-      commit(&empty_bar[s]);                   // the stage may be refilled once these products have read it
+      if (!ok) break;
       commit(&acc_full[buf]);
-      if (++s == stages) {
-        s = 0;
-        parity ^= 1;
-      }
     }
+  };
+
+  if (warp == 0 && lane == 0) {
+    if (wide) produce(std::true_type{});
+    else produce(std::false_type{});
+  } else if (warp == 1 && lane == 0 && cta == 0) {
+    if (wide) issue(std::true_type{});
+    else issue(std::false_type{});
   } else if (warp >= 2) {
     // ---------------- promotion + epilogue (each CTA its own 128 rows) ----------------
     const int ew = warp - 2;
@@ -387,12 +480,14 @@ __device__ __forceinline__ void half_kernel_body(const HalfMaps& maps, const Hal
     float sum[kCols];
 #pragma unroll
     for (int j = 0; j < kCols; ++j) sum[j] = 0.0f;
-    float scale = *a_scale * kDown;
-    for (int kb = 0; kb < k_blocks; ++kb) {
-      const int buf = kb & 1;
+    const int64_t a_stride = wide ? 0 : args.a_stride;
+    const int drains = (prob.K + kBK - 1) / kBK;         // of either form
+    float scale = wide ? 1.0f : *a_scale * kDown;
+    for (int d = 0; d < drains; ++d) {
+      const int buf = d & 1;
       // the next k-block's scale travels while this one is waited for
-      const float next = args.a_stride ? a_scale[min(kb + 1, k_blocks - 1) / kScaleBlocks * args.a_stride] * kDown : scale;
-      if (!mbar_wait_bounded(&acc_full[buf], (kb >> 1) & 1, abort_flag, status, kStatusAccumWaitTimeout)) break;
+      const float next = a_stride ? a_scale[min(d + 1, drains - 1) / kScaleBlocks * a_stride] * kDown : scale;
+      if (!mbar_wait_bounded(&acc_full[buf], (d >> 1) & 1, abort_flag, status, kStatusAccumWaitTimeout)) break;
       tc_fence_after_sync();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(buf * BN + col0);
 #pragma unroll
@@ -411,9 +506,9 @@ __device__ __forceinline__ void half_kernel_body(const HalfMaps& maps, const Hal
         else mbar_arrive(&acc_empty[buf]);
       }
     }
-    // The stages are idle once the last k-block has been drained: the sums are staged there and the epilogue runs as a
+    // The stages are idle once the accumulator has been drained for the last time: the sums are staged there and the epilogue runs as a
     // compact rolled loop over the tile.
-    epilogue(reinterpret_cast<float*>(smem), sum, col0, quarter * 32 + lane, abort_flag, m0, n0, ew, lane);
+    epilogue(reinterpret_cast<float*>(smem), wide, sum, col0, quarter * 32 + lane, abort_flag, m0, n0, ew, lane);
   }
 
   tc_fence_before_sync();
@@ -435,13 +530,13 @@ static_assert(256 * (kBM + 2) * 4 <= kStagePool, "the staged tile fits where the
 template <bool PAIR, int MODE>
 __device__ __forceinline__ void half_kernel_impl(const HalfMaps& maps, const HalfArgs& args, int* status) {
   constexpr int BN = PAIR ? 256 : 128;
-  half_kernel_body<PAIR>(maps, args, status, [&](float* tile, float (&sum)[BN / 2], int col0, int row, volatile int* abort_flag,
+  half_kernel_body<PAIR>(maps, args, status, [&](float* tile, bool wide, float (&sum)[BN / 2], int col0, int row, volatile int* abort_flag,
                                                  int m0, int n0, int ew, int lane) {
 #pragma unroll
     for (int j = 0; j < BN / 2; ++j) tile[(col0 + j) * kPitch<MODE> + row] = sum[j];
     asm volatile("bar.sync 1, %0;" ::"r"(kEpiWarps * 32) : "memory");
     // read after the barrier, so that all warps of the CTA agree (the epilogue has a barrier of its own)
-    if (*abort_flag == 0 && m0 < args.p.M) half_epilogue<BN, MODE, kPitch<MODE>>(args, tile, m0, n0, ew, lane);
+    if (*abort_flag == 0 && m0 < args.p.M) half_epilogue<BN, MODE, kPitch<MODE>>(args, wide, tile, m0, n0, ew, lane);
   });
 }
 
@@ -462,6 +557,11 @@ half_single_kernel(const __grid_constant__ HalfMaps maps, const __grid_constant_
 CUtensorMap make_map(const uint16_t* base, int64_t K, int64_t rows, int64_t ld) {
   if (ld % 64 != 0 || ld < K) throw std::invalid_argument("gemm_half: planes need a pitch that is a multiple of 64 covering K");
   return encode_k_major(CU_TENSOR_MAP_DATA_TYPE_FLOAT16, base, K, rows, 2 * ld, kBK, 128, CU_TENSOR_MAP_SWIZZLE_128B);
+}
+
+void make_mixed_maps(CUtensorMap* to, const SplitTarget& planes, int64_t K, int64_t rows) {
+  to[0] = encode_k_major(CU_TENSOR_MAP_DATA_TYPE_FLOAT32, planes.hi, K, rows, 4 * planes.ldo, kMixedBK, 128, CU_TENSOR_MAP_SWIZZLE_128B);
+  to[1] = encode_interleaved(planes.hl, K, rows, planes.ld16, 2 * kMixedBK, 128);
 }
 
 template <int MODE>
@@ -494,11 +594,21 @@ void gemm_half(const HalfOperand& a, const HalfOperand& b, const HalfProblem& pr
   if (to_planes && (!prob.Ch || !prob.Cl || !prob.Cscale || prob.ldp % 64 != 0 || prob.ldp < prob.M ||
                     (reinterpret_cast<uintptr_t>(prob.Ch) & 15) != 0 || (reinterpret_cast<uintptr_t>(prob.Cl) & 15) != 0))
     throw std::invalid_argument("gemm_half: output planes need 16-byte alignment and a pitch that is a multiple of 64");
+  if (prob.wide) {
+    if (!a.mixed.hl || !b.mixed.hl) throw std::invalid_argument("gemm_half: a decided product needs both operands' mixed form");
+    if (to_planes && (!prob.mixed.hi || !prob.mixed.hl || prob.mixed.ldo < prob.M || prob.mixed.ld16 < bf16_plane_index(prob.M - 1) + 33 ||
+                      !writes_pairs(prob.mixed)))
+      throw std::invalid_argument("gemm_half: mixed output planes need 8-byte alignment and an even pitch");
+  }
   HalfMaps maps;
   maps.a_h = make_map(a.h, prob.K, prob.M, a.ld);
   maps.a_l = a.l ? make_map(a.l, prob.K, prob.M, a.ld) : maps.a_h;
   maps.b_h = make_map(b.h, prob.K, prob.N, b.ld);
   maps.b_l = b.l ? make_map(b.l, prob.K, prob.N, b.ld) : maps.b_h;
+  if (prob.wide) {
+    make_mixed_maps(maps.mixed, a.mixed, prob.K, prob.M);
+    make_mixed_maps(maps.mixed + 2, b.mixed, prob.K, prob.N);
+  }
   const HalfArgs args{prob, a.scale, a.scale_stride, b.scale, a.l ? 2 : 1, b.l ? 2 : 1};
   // A pair's 256 x 256 tile takes about 1.5 times as long as a CTA's 128 x 128 one (it loads half as much per product): pairs
   // unless single CTAs get by with so few waves that they finish earlier.  Pairs against singles, measured: 1024^3 32 and

@@ -3,20 +3,28 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "elementwise.h"
+
 namespace soapb200 {
 
 // A K x cols operand as scaled fp16 planes: element (k, c) is
 //   scale[(k / 128) * scale_stride + c] * (h[k + c * ld] + l[k + c * ld]),
 // scales being powers of two that bring the largest magnitude of the vector (scale_stride == 0: the whole K-vector c;
 // else: its 128-element block) into [2^14, 2^15).  h = rn_fp16(x), l = rn_fp16(x - h) are off by 2^-23 of an element or by
-// 2^-39 of the largest one of its vector or block (fp16's smallest step), whichever is more: the latter is far under the
-// rounding of an fp32 sum that the largest one is part of.  l is null where h alone is exact in that sense (bf16 values).
+// 2^-39 of the largest one of its vector or block (fp16's smallest step), whichever is more.  l is null for bf16 values,
+// which h holds by itself down to 2^-32 of the largest one.
+//
+// The second kind of error is hidden by the rounding of an fp32 sum that the largest element is part of -- unless the other
+// operand is nearly zero there, as the eigenvectors of a graded matrix are: a coordinate of a rotated gradient that only the
+// small rows or columns feed would come out with fewer bits than from the mixed form (gemm.h, 2^-20 of each element), and
+// Adam divides it by its own size.  So a rotation decides on the device (RangeGuard) which form its products take.
 struct HalfOperand {
   const uint16_t* h;
   const uint16_t* l;
   int64_t ld;              // multiple of 64
   const float* scale;
   int64_t scale_stride;    // 0 for the second operand of a product, whose scales are applied after the sum over K
+  SplitTarget mixed{};     // the same operand in the mixed form, read where HalfProblem::wide says so
 };
 
 constexpr int kHalfScaleBlock = 128;
@@ -39,12 +47,17 @@ struct HalfProblem {
   float* var;
   int64_t ldm, ldv;
   float beta1, beta2, eps, inv_bc1, inv_sqrt_bc2;
+  // Device word (null: never): where it is set the product runs on the operands' mixed form -- tf32 and two bf16 corrections,
+  // drained every 64 of K like gemm_tf32x3 -- and kEpiSplit, kEpiAdam write the mixed form, here.
+  const int* wide;
+  int settled;             // the word was written before the kernel ahead of this one in the stream began
+  SplitTarget mixed;
 };
 
 void gemm_half(const HalfOperand& a, const HalfOperand& b, const HalfProblem& prob, int* status, cudaStream_t stream);
 
 // Where one orientation of a matrix goes as scaled fp16 planes (h == null: not wanted).  `scale` has one entry per vector,
-// `largest` is scratch of the same length.
+// `largest` is scratch of the same length (needed without planes too where a RangeGuard looks at it).
 struct HalfTarget {
   uint16_t* h;
   uint16_t* l;             // null: one term
@@ -53,20 +66,54 @@ struct HalfTarget {
   uint32_t* largest;
 };
 
+// A basis that is kept as fp16 planes, and where its mixed form goes on demand.
+struct WideBasis {
+  const float* src;        // element (i, j) at src[i * s_i + j * s_j], i, j < size
+  int64_t s_i, s_j;
+  int size;
+  SplitTarget plain, turned;
+};
+
+// Decides whether scaled fp16 pairs hold a matrix that is to be rotated.  They do unless a row's or a column's largest
+// magnitude lies more than kRangeOrders binary orders under the matrix's (all zeros included: what meets such a row is what a
+// basis nearly misses), or the matrix has infinities or NaN.
+//
+// Why the rows and columns of the matrix: Y = Q_L^T G Q_R passes through T = G^T Q_L, whose row j is as long as column j of G.
+// The floor of 2^-39 of the largest puts an error of 2^-39 |G|max on a column of Y, whose fp32 rounding is at least 2^-24 of
+// the shortest column of G; likewise for rows.  Within 2^12 of each other the floor is 2^-27 of every row and column, and 2^-20,
+// what the mixed form keeps, where one entry stands against rows of 16384.
+constexpr int kRangeOrders = 12;
+struct RangeGuard {
+  int* wide;               // device word: set to 1 (too wide) or 0; null: no decision
+  SplitTarget mixed;       // `plain` in the mixed form, written where it is set
+  WideBasis bases[2];      // likewise
+  int nearest;             // rounding of tf32 values, as split_planes
+};
+
 // The operand `plain` (depth rows, vectors = columns) and / or `turned` (depth cols, vectors = rows) of src[i*s_i + j*s_j],
 // i < rows, j < cols; source_type 0: fp32, 1: bf16.
 void half_planes(const void* src, int source_type, int64_t s_i, int64_t s_j, int rows, int cols, const HalfTarget& plain,
-                 const HalfTarget& turned, cudaStream_t stream);
+                 const HalfTarget& turned, const RangeGuard& guard, cudaStream_t stream);
 
-// One ordinary step of a rows x cols parameter (steady_step.cpp): every operand, result and scalar of its launches.
-struct SteadyStep {
-  const void* gradient;
-  int gradient_type;
+// A matrix to be rotated by two bases (steady_step.cpp).
+struct Rotation {
+  const void* source;
+  int source_type;
   int64_t s_i, s_j;
   int rows, cols;
   HalfTarget x, xt;                                          // planes of G (depth rows) and G^T (depth cols), written
   HalfOperand left, left_turned, right, right_turned;        // planes of Q_L, Q_L^T, Q_R, Q_R^T
-  HalfOperand middle, update;                                // scratch planes cols x rows and rows x cols, scales per block
+  HalfOperand middle;                                        // scratch planes cols x rows, scales per block
+  RangeGuard guard;
+};
+
+// out = Q_L^T G Q_R, or Q_L G Q_R^T (`turned`), column-major rows x cols; may overwrite the source.
+void rotate_half(const Rotation& r, bool turned, float* out, int64_t ldc, int* status, cudaStream_t stream);
+
+// One ordinary step of a rows x cols parameter: every operand, result and scalar of its launches.
+struct SteadyStep {
+  Rotation rotation;                                         // of the gradient
+  HalfOperand update;                                        // scratch planes rows x cols, scales per block
   float* momentum;
   int64_t ldm;
   float* variance;
@@ -78,8 +125,10 @@ struct SteadyStep {
   int64_t ld_right;
   double beta;
   float beta1, beta2, eps, inv_bc1, inv_sqrt_bc2;
-  cudaStream_t chain;                                        // the rotations run here, the rest on the step's own stream
+  int phases;                                                // kStep*
+  cudaStream_t chain;                                        // the rotations run here, the averages on the step's own stream
 };
+constexpr int kStepPlanes = 1, kStepForward = 2, kStepBackward = 4, kStepAverages = 8;
 void steady_step(const SteadyStep& s, int* status, cudaStream_t stream);
 
 // Scale of a vector or block from the bit pattern of its largest magnitude (clamped so that both factors are normal):

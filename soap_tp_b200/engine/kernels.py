@@ -238,6 +238,10 @@ class Planes:
             return dict(lo=0, hl=self.hl.data_ptr(), ld16=self.ld16)
         return dict(lo=self.lo.data_ptr(), hl=0, ld16=0)
 
+    def mixed_target(self) -> tuple:
+        """Mixed planes as the native rotation takes them."""
+        return (self.hi.data_ptr(), self.ld, self.hl.data_ptr(), self.ld16)
+
     def halves(self):
         """(hb, lb) of mixed planes as ``cols x depth`` fp32 tensors (tests)."""
         groups = self.hl[: max(1, self.cols)].view(max(1, self.cols), -1, 2, 32).float()
@@ -258,10 +262,11 @@ HALF_SCALE_BLOCK = 128      # rows of a result that share one scale per column w
 class HalfPlanes:
     """Operand of a single-GPU product as scaled fp16 planes of a K x cols matrix (``csrc/gemm_half.h``).
 
-    ``x = scale * (h + l)`` with ``h``, ``l`` fp16 (22 to 24 bits of x) and ``scale`` a power of two per K-vector
-    (``blocked=False``: what ``half_planes`` makes, usable on either side of a product) or per K-vector and block of 128
-    (``blocked=True``: what a product's epilogue writes, usable as the first operand).  ``l`` is absent where the matrix
-    comes from bf16 values, which ``h`` holds by itself.
+    ``x = scale * (h + l)`` with ``h``, ``l`` fp16 (22 to 24 bits of x, or to 2^-39 of the largest element that shares the
+    scale) and ``scale`` a power of two per K-vector (``blocked=False``: what ``half_planes`` makes, usable on either side of
+    a product) or per K-vector and block of 128 (``blocked=True``: what a product's epilogue writes, usable as the first
+    operand).  ``l`` is absent where the matrix comes from bf16 values, which ``h`` holds by itself down to 2^-32 of the
+    largest.  Rotations (``rotate_half``, ``steady_step``) decide on the device whether that is enough.
     """
 
     h: Tensor
@@ -551,6 +556,20 @@ def adam_update(gradient: Tensor, momentum: Tensor, variance: Tensor, beta1: flo
     return update
 
 
+def strided_source(matrix: Tensor) -> tuple:
+    """A 2-D fp32 or bf16 tensor as the native rotation takes it."""
+    return (matrix.data_ptr(), int(matrix.dtype == torch.bfloat16), matrix.stride(0), matrix.stride(1), *matrix.shape)
+
+
+def rotate_half(scratch, matrix_and_bases: tuple, turned: bool, out: Tensor) -> None:
+    """``out <- Q_L^T G Q_R`` (``turned``: ``Q_L G Q_R^T``), ``out`` column-major."""
+    assert out.stride(0) == 1 or out.shape[0] == 1
+    _C.rotate_half(scratch, matrix_and_bases + (int(turned), out.data_ptr(), _ld(out), status_word(out.device).data_ptr(), _stream()))
+    mark_written(out)
+    for name in ("largest_kernel", "half_planes_kernel", "gemm_half_kernel", "gemm_half_kernel"):
+        _count(name)
+
+
 _PARAMETER_TYPES = {torch.float32: 0, torch.bfloat16: 1}
 _PLAIN_TENSORS = (Tensor, torch.nn.Parameter)
 
@@ -558,11 +577,12 @@ _PLAIN_TENSORS = (Tensor, torch.nn.Parameter)
 def _addressable(*tensors: Tensor) -> bool:
     """Whether a flat kernel of the current stream may work on these tensors through their addresses: plain, dense tensors
     (a subclass may have no storage behind its address, or a meaning of its own) of one shape on the current device."""
-    first = tensors[0]
-    return (all(type(t) in _PLAIN_TENSORS for t in tensors)
-            and first.device.type == "cuda" and first.device.index == torch.cuda.current_device()
-            and all(t.device == first.device and t.shape == first.shape and t.layout == torch.strided and t.is_contiguous()
-                    and not t.is_neg() for t in tensors))
+    device, shape = tensors[0].device, tensors[0].shape
+    for t in tensors:
+        if (type(t) not in _PLAIN_TENSORS or t.device != device or t.shape != shape or t.layout != torch.strided
+                or not t.is_contiguous() or t.is_neg()):
+            return False
+    return device.type == "cuda" and device.index == torch.cuda.current_device()
 
 
 def apply_update(p: Tensor, update: Tensor, keep: float, lr: float) -> bool:

@@ -13,7 +13,9 @@ step is a chain of this package's kernels on one stream:
 Every product is brought to the kernel's single form ``acc = Za^T Zb`` with K-contiguous operands
 by keeping each basis in both orientations as operand planes; the planes are rebuilt only when the
 basis tensor changes (refresh, initialisation, or a user writing into ``state``).  The planes are scaled fp16 pairs
-(``kernels.HalfPlanes``); with ``SOAP_TP_MIXED_CORRECTIONS=0`` they are tf32 pairs and every product is three tf32 MMAs.
+(``kernels.HalfPlanes``); where a matrix has rows or columns so small beside the others that pairs would hold fewer bits of
+them than tf32 values with bf16 corrections do, the rotation's kernels find that out on the device and run on such planes
+instead (``csrc/gemm_half.h``, ``RangeGuard``).  With ``SOAP_TP_MIXED_CORRECTIONS=0`` every product is three tf32 MMAs.
 """
 from __future__ import annotations
 
@@ -42,7 +44,7 @@ class BasisPlanes:
         self.owner = None                 # weak reference to the tensor object the planes were made from
         self.plain = None                 # operand Q   (depth = rows of Q)
         self.transposed = None            # operand Q^T (depth = cols of Q)
-        self.addresses: tuple = ()        # both as the native step takes them
+        self.addresses: tuple = ()        # both, and the basis itself, as the native calls take them
 
     def refresh(self, Q: Tensor, size: int) -> None:
         key = (Q.data_ptr(), Q._version, size)
@@ -55,9 +57,9 @@ class BasisPlanes:
             # (an address that was recycled by a tensor of another size starts over)
             make = _operand if self.half else _tf32_operand
             self.plain, self.transposed = make(size, size, Q.device), make(size, size, Q.device)
-            if isinstance(self.plain, k.HalfPlanes):
-                self.addresses = self.plain.operand() + self.transposed.operand()
         split(view, self.plain, self.transposed)
+        if isinstance(self.plain, k.HalfPlanes):
+            self.addresses = self.plain.operand() + self.transposed.operand() + (Q.data_ptr(), Q.stride(0), Q.stride(1))
         self.key = (Q.data_ptr(), Q._version, size)
         self.owner = weakref.ref(Q)
 
@@ -204,16 +206,52 @@ def gram_updates_for_bases(gradient: Tensor, state, beta: float, rows: int, cols
     gram_updates(gp, gtp, state, beta, rows, cols)
 
 
-def _step_workspace(rows: int, cols: int, device, terms: int) -> tuple:
-    """Scratch planes of an ordinary step as the native step takes them (shared by parameters of one shape)."""
-    key = ("step", rows, cols, str(device), terms)
+class _Scratch:
+    """Buffers of a rotation as the native calls take them, shared by matrices of one shape: with ``update`` those of a step's
+    way back as well, with ``averages`` the planes of its Gram products."""
+
+    def __init__(self, rows: int, cols: int, device, terms: int, update: bool, averages: bool) -> None:
+        self.wide = torch.zeros(1, dtype=torch.int32, device=device)        # the decision on the range
+        self.maxima = torch.empty(max(1, rows), dtype=torch.int32, device=device)
+        planes = [workspace_planes("X", rows, cols, device, terms=terms)]
+        if averages:
+            planes.append(workspace_planes("GT", cols, rows, device, terms=terms))
+        middle = workspace_planes("T", cols, rows, device, blocked=True)
+        mixed = [tf32_workspace(*size, device) for size in (
+            ("G", rows, cols), ("T", cols, rows), ("L", rows, rows), ("LT", rows, rows), ("R", cols, cols), ("RT", cols, cols))]
+        turned = planes[1].target() if averages else (0, 0, 64, 0, self.maxima.data_ptr())
+        addresses = (planes[0].target() + turned + middle.operand() + (self.wide.data_ptr(), int(k.SPLIT_ROUND_NEAREST))
+                     + tuple(value for each in mixed for value in each.mixed_target()))
+        self.keep = planes + [middle] + mixed                               # (addresses alone hold nothing)
+        if update:
+            update_planes, mixed_update = workspace_planes("U", rows, cols, device, blocked=True), tf32_workspace("U", rows, cols, device)
+            addresses += update_planes.operand() + mixed_update.mixed_target()
+            self.keep += [update_planes, mixed_update]
+        else:
+            addresses += (0,) * 9
+        self.native = _C.RotationScratch(addresses)
+
+
+def _scratch(rows: int, cols: int, device, terms: int, update: bool = False, averages: bool = False) -> _Scratch:
+    key = ("scratch", rows, cols, device, terms, update, averages)
     entry = _WORKSPACES.get(key)
     if entry is None:
-        xp, gtp = (workspace_planes(tag, *size, device, terms=terms) for tag, size in (("X", (rows, cols)), ("GT", (cols, rows))))
-        middle, update = (workspace_planes(tag, *size, device, blocked=True)
-                          for tag, size in (("T", (cols, rows)), ("U", (rows, cols))))
-        entry = _WORKSPACES[key] = (xp.target() + gtp.target(), middle.operand() + update.operand())
+        entry = _WORKSPACES[key] = _Scratch(rows, cols, device, terms, update, averages)
     return entry
+
+
+def rotate_matrix(source: Tensor, left: BasisPlanes, right: BasisPlanes, turned: bool, out: Tensor) -> None:
+    """``out <- Q_l^T X Q_r`` (``turned``: ``Q_l X Q_r^T``) for an fp32 matrix; ``out`` is column-major and may be ``source``."""
+    rows, cols = source.shape
+    if k.MIXED_CORRECTIONS:
+        if rows and cols:
+            k.rotate_half(_scratch(rows, cols, source.device, 2).native, k.strided_source(source) + left.addresses + right.addresses,
+                          turned, out)
+        return
+    planes = workspace_planes("X", rows, cols, source.device)
+    split(source, planes)
+    first, second = (left.transposed, right.transposed) if turned else (left.plain, right.plain)
+    rotate_planes(planes, first, second, rows, cols, source.device, tag="T", mode=k.EPI_STORE, out=out)
 
 
 _CHAIN_STREAMS: Dict[torch.device, "torch.cuda.Stream"] = {}
@@ -227,12 +265,11 @@ def _chain_stream(device) -> int:
     return stream.cuda_stream
 
 
-def _native_step(gradient: Tensor, state, step: int, rows: int, cols: int, *, beta, beta1, beta2, eps) -> Tensor:
-    """A step without a refresh, its eight launches issued by one native call."""
+def _native_step(gradient: Tensor, state, step: int, rows: int, cols: int, *, beta, beta1, beta2, eps, averages: bool) -> Tensor:
+    """An ordinary step, its eight launches issued by one native call; without ``averages`` the rotations and Adam only."""
     g = gradient.detach().reshape(rows, cols)
     if g.dtype != torch.float32 and g.dtype != torch.bfloat16:
         g = g.float()
-    half = g.dtype == torch.bfloat16
     ctx = context_for(state)
     ctx.left.refresh(state["left_basis"], rows)
     ctx.right.refresh(state["right_basis"], cols)
@@ -240,21 +277,54 @@ def _native_step(gradient: Tensor, state, step: int, rows: int, cols: int, *, be
     momentum, variance = state["momentum"], state["variance"]
     left, right = state["left_preconditioner"], state["right_preconditioner"]
     assert (left.stride(0) == 1 or rows == 1) and (right.stride(0) == 1 or cols == 1)
-    planes, scratch = _step_workspace(rows, cols, g.device, 1 if half else 2)
+    scratch = _scratch(rows, cols, g.device, 1 if g.dtype == torch.bfloat16 else 2, update=True, averages=averages)
     update = torch.empty((rows, cols), dtype=torch.float32, device=g.device)
-    _C.steady_step((g.data_ptr(), int(half), g.stride(0), g.stride(1), rows, cols, *planes, *ctx.left.addresses,
-                    *ctx.right.addresses, *scratch, momentum.data_ptr(), k._ld(momentum), variance.data_ptr(), k._ld(variance),
-                    update.data_ptr(), left.data_ptr(), k._ld(left), right.data_ptr(), k._ld(right),
-                    k.status_word(g.device).data_ptr(), k._stream(), _chain_stream(g.device)),
-                   beta, beta1, beta2, eps / math.sqrt(bias2), 1.0 / (1.0 - beta1**step), 1.0 / math.sqrt(bias2))
-    torch.autograd.graph.increment_version((momentum, variance, left, right))
-    for name, count in _STEP_LAUNCHES:
+    arguments = (k.strided_source(g) + ctx.left.addresses + ctx.right.addresses
+                 + (momentum.data_ptr(), k._ld(momentum), variance.data_ptr(), k._ld(variance), update.data_ptr(),
+                    left.data_ptr(), k._ld(left), right.data_ptr(), k._ld(right)))
+    tail = (k.status_word(g.device).data_ptr(), k._stream(), _chain_stream(g.device))
+    scalars = (beta, beta1, beta2, eps / math.sqrt(bias2), 1.0 / (1.0 - beta1**step), 1.0 / math.sqrt(bias2))
+    if TIMER.enabled:
+        for name, phase in _STEP_STAGES if averages else _STEP_STAGES[:-1]:
+            with TIMER.stage(name, g.device):
+                _C.steady_step(scratch.native, arguments + (phase,) + tail, *scalars)
+    else:
+        _C.steady_step(scratch.native, arguments + (_ALL_PHASES if averages else _ALL_PHASES - _C.STEP_AVERAGES,) + tail, *scalars)
+    torch.autograd.graph.increment_version((momentum, variance, left, right) if averages else (momentum, variance))
+    for name, count in (("largest_kernel", 1), ("half_planes_kernel", 1), ("gemm_half_kernel", 6 if averages else 4)):
         k.LAUNCH_COUNTS[name] = k.LAUNCH_COUNTS.get(name, 0) + count
-    state["step"] = step
     return update
 
 
-_STEP_LAUNCHES = (("largest_kernel", 1), ("half_planes_kernel", 1), ("gemm_half_kernel", 6))
+_STEP_STAGES = (("split_gradient", _C.STEP_PLANES), ("rotate_forward+adam", _C.STEP_FORWARD),
+                ("rotate_backward", _C.STEP_BACKWARD), ("gram", _C.STEP_AVERAGES))
+_ALL_PHASES = sum(phase for _, phase in _STEP_STAGES)
+
+
+def _tf32_step(gradient: Tensor, state, step: int, rows: int, cols: int, *, beta, beta1, beta2, eps, averages: bool) -> Tensor:
+    """The same on tf32 planes, launch by launch (``SOAP_TP_MIXED_CORRECTIONS=0``)."""
+    device = gradient.device
+    with TIMER.stage("split_gradient", device):
+        xp, gtp = gradient_planes(gradient.reshape(rows, cols), plain="X", turned="GT" if averages else None)
+    ctx = context_for(state)
+    ctx.left.refresh(state["left_basis"], rows)
+    ctx.right.refresh(state["right_basis"], cols)
+    bias2 = 1.0 - beta2**step
+    adam = dict(beta1=beta1, beta2=beta2, eps=eps / math.sqrt(bias2),
+                bias_correction1=1.0 - beta1**step, bias_correction2=bias2)
+    up = workspace_planes("U", rows, cols, device, blocked=True)
+    with TIMER.stage("rotate_forward+adam", device):
+        rotate_planes(xp, ctx.left.plain, ctx.right.plain, rows, cols, device, tag="T",
+                      mode=k.EPI_ADAM, out_planes=up, momentum=state["momentum"][:rows, :cols],
+                      variance=state["variance"][:rows, :cols], adam=adam)
+    update = torch.empty((rows, cols), dtype=torch.float32, device=device)
+    with TIMER.stage("rotate_backward", device):
+        rotate_planes(up, ctx.left.transposed, ctx.right.transposed, rows, cols, device, tag="T",
+                      mode=k.EPI_ROW_MAJOR, out=update)
+    if averages:
+        with TIMER.stage("gram", device):
+            gram_updates(xp, gtp, state, beta, rows, cols)
+    return update
 
 
 def soap_step(
@@ -286,30 +356,12 @@ def soap_step(
 
     step = int(state["step"]) + 1
     refreshing = step % interval == 0
-    if not refreshing and k.MIXED_CORRECTIONS and not TIMER.enabled and rows and cols:
-        return _native_step(gradient, state, step, rows, cols, beta=beta, beta1=beta1, beta2=beta2, eps=eps)
-    with TIMER.stage("split_gradient", device):
-        xp, gtp = gradient_planes(gradient.reshape(rows, cols), plain="X", turned=None if refreshing else "GT")
-    ctx = context_for(state)
-    ctx.left.refresh(state["left_basis"], rows)
-    ctx.right.refresh(state["right_basis"], cols)
-    bias2 = 1.0 - beta2**step
-    adam = dict(beta1=beta1, beta2=beta2, eps=eps / math.sqrt(bias2),
-                bias_correction1=1.0 - beta1**step, bias_correction2=bias2)
-    up = workspace_planes("U", rows, cols, device, blocked=True)
-    with TIMER.stage("rotate_forward+adam", device):
-        rotate_planes(xp, ctx.left.plain, ctx.right.plain, rows, cols, device, tag="T",
-                      mode=k.EPI_ADAM, out_planes=up, momentum=state["momentum"][:rows, :cols],
-                      variance=state["variance"][:rows, :cols], adam=adam)
-    update = torch.empty((rows, cols), dtype=torch.float32, device=device)
-    with TIMER.stage("rotate_backward", device):
-        rotate_planes(up, ctx.left.transposed, ctx.right.transposed, rows, cols, device, tag="T",
-                      mode=k.EPI_ROW_MAJOR, out=update)
-    with TIMER.stage("gram", device):
-        if refreshing:
+    # (an empty matrix has nothing to rotate on pairs; the other path takes it as every product does)
+    run = _native_step if k.MIXED_CORRECTIONS and rows and cols else _tf32_step
+    update = run(gradient, state, step, rows, cols, beta=beta, beta1=beta1, beta2=beta2, eps=eps, averages=not refreshing)
+    if refreshing:
+        with TIMER.stage("gram", device):
             gram_updates_for_bases(gradient.reshape(rows, cols), state, beta, rows, cols)
-        else:
-            gram_updates(xp, gtp, state, beta, rows, cols)
     if refreshing:
         with TIMER.stage("refresh", device):
             refresh(state, global_shape)
@@ -363,26 +415,23 @@ def prepare_refresh(rows: int, cols: int, device) -> None:
         qr_driver._workspace(cols, device, 1)     # the second of two concurrent factorisations
     else:
         qr_driver._workspace(rows, device, 0), qr_driver._workspace(cols, device, 1)
-    workspace_matrix("perm", rows, cols, device)
-    workspace_planes("X", rows, cols, device)
-    for tag, depth, width in (("U", rows, cols), ("T", cols, rows)):
-        workspace_planes(tag, depth, width, device, blocked=True)
+    for tag in ("perm", "space"):
+        workspace_matrix(tag, rows, cols, device)
+    if k.MIXED_CORRECTIONS and rows and cols:
+        _scratch(rows, cols, device, 2)
+    else:
+        for tag, depth, width in (("X", rows, cols), ("T", cols, rows)):
+            workspace_planes(tag, depth, width, device)
     warm_refresh_kernels(device, sizes={rows, cols})
 
 
 def rotate(matrix: Tensor, Q_left: Tensor, Q_right: Tensor, global_shape, direction: str) -> Tensor:
     rows, cols = global_shape
-    device = matrix.device
     left, right = BasisPlanes(), BasisPlanes()
     left.refresh(Q_left, rows)
     right.refresh(Q_right, cols)
     view = matrix[:rows, :cols]
-    source = workspace_planes("X", rows, cols, device)
-    split(view, source)
-    if direction == "forward":
-        rotate_planes(source, left.plain, right.plain, rows, cols, device, tag="T", mode=k.EPI_STORE, out=view)
-    else:
-        rotate_planes(source, left.transposed, right.transposed, rows, cols, device, tag="T", mode=k.EPI_STORE, out=view)
+    rotate_matrix(view, left, right, direction != "forward", view)
     return matrix
 
 
@@ -419,13 +468,10 @@ def refresh(state: MutableMapping[str, Any], global_shape) -> Tuple[Tensor, Tens
     ctx = context_for(state)
     ctx.left.refresh(state["left_basis"], rows)
     ctx.right.refresh(state["right_basis"], cols)
-    # momentum out of the old bases: Q_L M Q_R^T, kept as planes for the way back
+    # momentum out of the old bases: Q_L M Q_R^T, in fp32 so that the way back sees the range of every row and column
+    parameter_space = workspace_matrix("space", rows, cols, device)
     with TIMER.stage("refresh.momentum_out", device):
-        mp = workspace_planes("X", rows, cols, device)
-        split(momentum[:rows, :cols], mp)
-        parameter_space = workspace_planes("U", rows, cols, device, blocked=True)
-        rotate_planes(mp, ctx.left.transposed, ctx.right.transposed, rows, cols, device, tag="T",
-                      mode=k.EPI_SPLIT, out_planes=parameter_space)
+        rotate_matrix(momentum[:rows, :cols], ctx.left, ctx.right, True, parameter_space)
     with TIMER.stage("refresh.power_iteration", device):
         left_order = estimated_order(state["left_preconditioner"], state["left_basis"], state["left_work"], rows)
         right_order = estimated_order(state["right_preconditioner"], state["right_basis"], state["right_work"], cols)
@@ -443,6 +489,5 @@ def refresh(state: MutableMapping[str, Any], global_shape) -> Tuple[Tensor, Tens
     with TIMER.stage("refresh.momentum_in", device):
         ctx.left.refresh(state["left_basis"], rows)
         ctx.right.refresh(state["right_basis"], cols)
-        rotate_planes(parameter_space, ctx.left.plain, ctx.right.plain, rows, cols, device, tag="T",
-                      mode=k.EPI_STORE, out=momentum[:rows, :cols])
+        rotate_matrix(parameter_space, ctx.left, ctx.right, False, momentum[:rows, :cols])
     return left_order, right_order
