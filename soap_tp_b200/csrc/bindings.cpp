@@ -187,6 +187,8 @@ PYBIND11_MODULE(_C, m) {
         },
         "acc[m,n] = sum_k Za[k,m] Zb[k,n] from scaled fp16 planes, with fused epilogue (gemm_half.h)");
 
+  m.def("half_on_pairs", &half_on_pairs, "Whether an M x N product of fp16 pairs runs on CTA pairs by default");
+
   m.def("half_planes",
         [](uint64_t src, int source_type, int64_t s_i, int64_t s_j, int rows, int cols, uint64_t ph, uint64_t pl, int64_t pld,
            uint64_t pscale, uint64_t plargest, uint64_t th, uint64_t tl, int64_t tld, uint64_t tscale, uint64_t tlargest,

@@ -584,6 +584,19 @@ void launch(bool pairs, const HalfMaps& maps, const HalfArgs& args, int* status,
 
 }  // namespace
 
+bool half_on_pairs(int M, int N, bool symmetric) {
+  if (!gemm_cta_pairs_wanted()) return false;
+  // A pair's 256 x 256 tile takes about 1.5 times as long as a CTA's 128 x 128 one (it loads half as much per product): pairs
+  // unless single CTAs get by with so few waves that they finish earlier.  Pairs against singles, measured: 1024^3 32 and
+  // 24 us, 2048^3 50 and 69, 4096^3 333 and 410; symmetric, then drained every 128 of K, 1024 39 and 28, 2048 54 and 44, 4096 186 and
+  // 255 (drained every 64, one term: 220 and 241).
+  auto tiles_of = [&](int64_t side) {
+    const int64_t m = (M + side - 1) / side, n = (N + side - 1) / side;
+    return symmetric ? m * (m + 1) / 2 : m * n;
+  };
+  return 3 * ((tiles_of(256) + 73) / 74) <= 2 * ((tiles_of(128) + 147) / 148);
+}
+
 void gemm_half(const HalfOperand& a, const HalfOperand& b, const HalfProblem& prob, int* status, cudaStream_t stream) {
   if (prob.M <= 0 || prob.N <= 0) return;
   if (prob.K <= 0) throw std::invalid_argument("gemm_half needs K >= 1");
@@ -610,15 +623,7 @@ void gemm_half(const HalfOperand& a, const HalfOperand& b, const HalfProblem& pr
     make_mixed_maps(maps.mixed + 2, b.mixed, prob.K, prob.N);
   }
   const HalfArgs args{prob, a.scale, a.scale_stride, b.scale, a.l ? 2 : 1, b.l ? 2 : 1};
-  // A pair's 256 x 256 tile takes about 1.5 times as long as a CTA's 128 x 128 one (it loads half as much per product): pairs
-  // unless single CTAs get by with so few waves that they finish earlier.  Pairs against singles, measured: 1024^3 32 and
-  // 24 us, 2048^3 50 and 69, 4096^3 333 and 410; symmetric, then drained every 128 of K, 1024 39 and 28, 2048 54 and 44, 4096 186 and
-  // 255 (drained every 64, one term: 220 and 241).
-  auto tiles_of = [&](int64_t side) {
-    const int64_t m = (prob.M + side - 1) / side, n = (prob.N + side - 1) / side;
-    return prob.symmetric ? m * (m + 1) / 2 : m * n;
-  };
-  const bool pairs = prob.tiles ? prob.tiles == 2 : 3 * ((tiles_of(256) + 73) / 74) <= 2 * ((tiles_of(128) + 147) / 148);
+  const bool pairs = prob.tiles ? prob.tiles == 2 : half_on_pairs(prob.M, prob.N, prob.symmetric);
   switch (prob.mode) {
     case kEpiStore: launch<kEpiStore>(pairs, maps, args, status, stream); return;
     case kEpiSplit: launch<kEpiSplit>(pairs, maps, args, status, stream); return;

@@ -54,6 +54,9 @@ struct HalfProblem {
   SplitTarget mixed;
 };
 
+// Whether such a product runs on CTA pairs where it does not say.
+bool half_on_pairs(int M, int N, bool symmetric);
+
 void gemm_half(const HalfOperand& a, const HalfOperand& b, const HalfProblem& prob, int* status, cudaStream_t stream);
 
 // Where one orientation of a matrix goes as scaled fp16 planes (h == null: not wanted).  `scale` has one entry per vector,

@@ -930,6 +930,7 @@ bool g_use_pairs = true;
 }  // namespace
 
 void gemm_use_cta_pairs(bool on) { g_use_pairs = on; }
+bool gemm_cta_pairs_wanted() { return g_use_pairs; }
 
 void gemm_tf32x3(const GemmOperands& ops, const GemmProblem& prob, int* status, cudaStream_t stream) {
   if (prob.M <= 0 || prob.N <= 0) return;
