@@ -254,14 +254,18 @@ def rotate_matrix(source: Tensor, left: BasisPlanes, right: BasisPlanes, turned:
     rotate_planes(planes, first, second, rows, cols, source.device, tag="T", mode=k.EPI_STORE, out=out)
 
 
-_CHAIN_STREAMS: Dict[torch.device, "torch.cuda.Stream"] = {}
+_CHAIN_STREAMS: Dict[tuple, "torch.cuda.Stream"] = {}
 
 
-def _chain_stream(device) -> int:
-    """The high-priority stream of the rotations (forked from and joined to the step's own stream within every step)."""
-    stream = _CHAIN_STREAMS.get(device)
+def _chain_stream(device, home: int) -> int:
+    """The stream of the rotations of steps on the stream ``home`` (forked from and joined to it within every step): one of its
+    own for every caller's stream, so that callers do not wait for one another, and of that stream's priority."""
+    stream = _CHAIN_STREAMS.get((device, home))
     if stream is None:
-        stream = _CHAIN_STREAMS[device] = torch.cuda.Stream(device=device, priority=-1)
+        if len(_CHAIN_STREAMS) >= 64:          # (streams that came and went; nothing is left on theirs)
+            _CHAIN_STREAMS.clear()
+        stream = torch.cuda.Stream(device=device, priority=torch.cuda.current_stream().priority)
+        _CHAIN_STREAMS[(device, home)] = stream
     return stream.cuda_stream
 
 
@@ -282,7 +286,8 @@ def _native_step(gradient: Tensor, state, step: int, rows: int, cols: int, *, be
     arguments = (k.strided_source(g) + ctx.left.addresses + ctx.right.addresses
                  + (momentum.data_ptr(), k._ld(momentum), variance.data_ptr(), k._ld(variance), update.data_ptr(),
                     left.data_ptr(), k._ld(left), right.data_ptr(), k._ld(right)))
-    tail = (k.status_word(g.device).data_ptr(), k._stream(), _chain_stream(g.device))
+    home = k._stream()
+    tail = (k.status_word(g.device).data_ptr(), home, _chain_stream(g.device, home))
     scalars = (beta, beta1, beta2, eps / math.sqrt(bias2), 1.0 / (1.0 - beta1**step), 1.0 / math.sqrt(bias2))
     if TIMER.enabled:
         for name, phase in _STEP_STAGES if averages else _STEP_STAGES[:-1]:

@@ -4,6 +4,7 @@ import subprocess
 import sys
 
 import pytest
+import torch
 
 from soap_tp_b200.engine import kernels as k
 
@@ -30,3 +31,50 @@ def test_the_pair_switch_of_the_environment():
         out = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, SOAP_TP_GEMM_CTA_PAIRS=value), text=True,
                              capture_output=True, check=True)
         assert out.stdout.strip().endswith(expected)
+
+
+class FakeStream:
+    made = 0
+
+    def __init__(self, device=None, priority=0):
+        FakeStream.made += 1
+        self.priority, self.cuda_stream = priority, 1000 + FakeStream.made
+
+
+@pytest.fixture
+def streams(monkeypatch):
+    """Streams of the caller: (handle, priority) becomes current."""
+    from soap_tp_b200.engine import local
+
+    current = FakeStream()
+    monkeypatch.setattr(torch.cuda, "Stream", FakeStream)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: current)
+    monkeypatch.setattr(local, "_CHAIN_STREAMS", {})
+
+    def chain_of(handle, priority=0):
+        current.cuda_stream, current.priority = handle, priority
+        return local._chain_stream(torch.device("cuda", 0), handle)
+
+    return local, chain_of
+
+
+def test_every_callers_stream_has_rotations_of_its_own(streams):
+    local, chain_of = streams
+    first, second = chain_of(1), chain_of(2)
+    assert first != second and chain_of(1) == first and chain_of(2) == second
+    assert {first, second}.isdisjoint({1, 2})
+
+
+def test_rotations_have_the_callers_priority(streams):
+    local, chain_of = streams
+    for handle, priority in ((1, 0), (2, -1)):
+        handle = chain_of(handle, priority)
+        stream, = (s for s in local._CHAIN_STREAMS.values() if s.cuda_stream == handle)
+        assert stream.priority == priority
+
+
+def test_streams_that_come_and_go_are_not_kept(streams):
+    local, chain_of = streams
+    for handle in range(500):
+        chain_of(handle)
+    assert len(local._CHAIN_STREAMS) <= 64
