@@ -254,12 +254,16 @@ def rotate_matrix(source: Tensor, left: BasisPlanes, right: BasisPlanes, turned:
     rotate_planes(planes, first, second, rows, cols, source.device, tag="T", mode=k.EPI_STORE, out=out)
 
 
+# SOAP_TP_OVERLAP_GRAM=0: the Gram averages run after the rotations on the same stream instead of beside them
+OVERLAP_GRAM = os.environ.get("SOAP_TP_OVERLAP_GRAM", "1") != "0"
 _CHAIN_STREAMS: Dict[tuple, "torch.cuda.Stream"] = {}
 
 
 def _chain_stream(device, home: int) -> int:
     """The stream of the rotations of steps on the stream ``home`` (forked from and joined to it within every step): one of its
     own for every caller's stream, so that callers do not wait for one another, and of that stream's priority."""
+    if not OVERLAP_GRAM:
+        return home
     stream = _CHAIN_STREAMS.get((device, home))
     if stream is None:
         if len(_CHAIN_STREAMS) >= 64:          # (streams that came and went; nothing is left on theirs)

@@ -78,3 +78,9 @@ def test_streams_that_come_and_go_are_not_kept(streams):
     for handle in range(500):
         chain_of(handle)
     assert len(local._CHAIN_STREAMS) <= 64
+
+
+def test_the_overlap_switch_leaves_everything_on_the_callers_stream(streams, monkeypatch):
+    local, chain_of = streams
+    monkeypatch.setattr(local, "OVERLAP_GRAM", False)
+    assert chain_of(7) == 7 and not local._CHAIN_STREAMS
