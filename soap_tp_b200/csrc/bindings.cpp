@@ -203,7 +203,7 @@ PYBIND11_MODULE(_C, m) {
   py::class_<RotationScratch>(m, "RotationScratch", "Scratch planes of rotations of one shape, as addresses (see Arguments)")
       .def(py::init<const std::vector<int64_t>&>());
   // Integers: the matrix and its bases (Arguments), the moments, results and phases in the order of SteadyStep, then the status
-  // word, the stream and the stream of the rotations.
+  // word, the stream and the stream of the averages.
   m.def("steady_step", [](const RotationScratch& scratch, const std::vector<int64_t>& v, double beta, float beta1, float beta2,
                           float eps, float inv_bc1, float inv_sqrt_bc2) {
     Arguments in(v);
@@ -219,7 +219,7 @@ PYBIND11_MODULE(_C, m) {
     s.phases = static_cast<int>(in.next());
     int* status = in.pointer<int>();
     cudaStream_t stream = in.stream();
-    s.chain = in.stream();
+    s.side = in.stream();
     in.finish();
     s.beta = beta; s.beta1 = beta1; s.beta2 = beta2; s.eps = eps; s.inv_bc1 = inv_bc1; s.inv_sqrt_bc2 = inv_sqrt_bc2;
     py::gil_scoped_release release;

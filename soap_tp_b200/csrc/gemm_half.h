@@ -129,7 +129,7 @@ struct SteadyStep {
   double beta;
   float beta1, beta2, eps, inv_bc1, inv_sqrt_bc2;
   int phases;                                                // kStep*
-  cudaStream_t chain;                                        // the rotations run here, the averages on the step's own stream
+  cudaStream_t side;                                         // the averages run here, beside the rotations (or the step's own)
 };
 constexpr int kStepPlanes = 1, kStepForward = 2, kStepBackward = 4, kStepAverages = 8;
 void steady_step(const SteadyStep& s, int* status, cudaStream_t stream);

@@ -3,10 +3,11 @@
 // 182 us, issued from here 118 us.
 //
 // The four products of the rotation chain depend on one another and each ends in a wave of tiles that leaves SMs idle; the
-// Gram averages depend on the gradient only.  So the chain runs on a stream of its own, issued first, and the averages fill what
-// it leaves free.  Device time of a step on one stream and with the chain beside it: 256 x 512 103 and 74 us, 512 x 1376 154 and
-// 136 us, 1000 x 1501 182 and 178 us, 2048 x 5504 1393 and 1329 us, 4096 x 4096 1975 and 1827 us, 8192 x 8192 within the runs'
-// spread.  A higher priority for it would take 1 to 2 % more off, at the expense of whatever else the caller runs.
+// Gram averages depend on the gradient only.  So the averages run on a stream beside it and fill what the chain leaves free.
+// The chain stays on the caller's stream: its first product then overlaps the tail of the operand planes, which an event
+// between streams does not allow.  Device time of a step, everything on one stream / the chain beside / the averages beside:
+// 256 x 512 126 / 92 / 85 us, 512 x 1376 175 / 158 / 121 us, 1000 x 1501 198 / 198 / 148 us, 2048 x 5504 1388 / 1352 / 1186 us,
+// 4096 x 4096 1900 / 1863 / 1748 us, 8192 x 8192 within the runs' spread.
 #include <optional>
 #include <stdexcept>
 
@@ -90,12 +91,12 @@ void steady_step(const SteadyStep& s, int* status, cudaStream_t stream) {
   if (r.rows <= 0 || r.cols <= 0) throw std::invalid_argument("steady_step: empty matrix");
   if (s.phases & kStepPlanes) make_planes(r, stream);
   const bool averages = s.phases & kStepAverages, rotations = s.phases & (kStepForward | kStepBackward);
-  const cudaStream_t chain = averages && rotations ? s.chain : stream;
+  const cudaStream_t side = averages && rotations ? s.side : stream;
   std::optional<Fork> fork;
-  if (chain != stream) fork.emplace(stream, chain);
+  if (side != stream) fork.emplace(stream, side);
 
   if (s.phases & kStepForward) {
-    first_product(r, source_of(r), false, r.left, status, chain);           // T = X^T Q_L
+    first_product(r, source_of(r), false, r.left, status, stream);          // T = X^T Q_L
     HalfProblem adam = second_product(r);                                   // Y = T^T Q_R, Adam(Y) -> U
     adam.mode = kEpiAdam;
     adam.Ch = const_cast<uint16_t*>(s.update.h); adam.Cl = const_cast<uint16_t*>(s.update.l); adam.ldp = s.update.ld;
@@ -103,14 +104,14 @@ void steady_step(const SteadyStep& s, int* status, cudaStream_t stream) {
     adam.mixed = s.update.mixed;
     adam.mom = s.momentum; adam.ldm = s.ldm; adam.var = s.variance; adam.ldv = s.ldv;
     adam.beta1 = s.beta1; adam.beta2 = s.beta2; adam.eps = s.eps; adam.inv_bc1 = s.inv_bc1; adam.inv_sqrt_bc2 = s.inv_sqrt_bc2;
-    gemm_half(r.middle, r.right, adam, status, chain);
+    gemm_half(r.middle, r.right, adam, status, stream);
   }
   if (s.phases & kStepBackward) {
-    first_product(r, s.update, true, r.left_turned, status, chain);         // T2 = U^T Q_L^T
+    first_product(r, s.update, true, r.left_turned, status, stream);        // T2 = U^T Q_L^T
     HalfProblem out = second_product(r);                                    // T2^T Q_R^T
     out.mode = kEpiRowMajor;
     out.C = s.out; out.ldc = r.cols;
-    gemm_half(r.middle, r.right_turned, out, status, chain);
+    gemm_half(r.middle, r.right_turned, out, status, stream);
   }
   if (averages) {
     // Products of a vector of G with another one: what counts is their error against the vectors' own sizes, which the pairs
@@ -123,10 +124,10 @@ void steady_step(const SteadyStep& s, int* status, cudaStream_t stream) {
     gram.beta = static_cast<float>(s.beta);
     gram.M = gram.N = r.rows; gram.K = r.cols;
     gram.C = s.left_gram; gram.ldc = s.ld_left;
-    gemm_half(xt, xt, gram, status, stream);
+    gemm_half(xt, xt, gram, status, side);
     gram.M = gram.N = r.cols; gram.K = r.rows;
     gram.C = s.right_gram; gram.ldc = s.ld_right;
-    gemm_half(x, x, gram, status, stream);
+    gemm_half(x, x, gram, status, side);
   }
 }
 

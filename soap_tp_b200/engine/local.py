@@ -256,20 +256,20 @@ def rotate_matrix(source: Tensor, left: BasisPlanes, right: BasisPlanes, turned:
 
 # SOAP_TP_OVERLAP_GRAM=0: the Gram averages run after the rotations on the same stream instead of beside them
 OVERLAP_GRAM = os.environ.get("SOAP_TP_OVERLAP_GRAM", "1") != "0"
-_CHAIN_STREAMS: Dict[tuple, "torch.cuda.Stream"] = {}
+_SIDE_STREAMS: Dict[tuple, "torch.cuda.Stream"] = {}
 
 
-def _chain_stream(device, home: int) -> int:
-    """The stream of the rotations of steps on the stream ``home`` (forked from and joined to it within every step): one of its
+def _side_stream(device, home: int) -> int:
+    """The stream of the averages of steps on the stream ``home`` (forked from and joined to it within every step): one of its
     own for every caller's stream, so that callers do not wait for one another, and of that stream's priority."""
     if not OVERLAP_GRAM:
         return home
-    stream = _CHAIN_STREAMS.get((device, home))
+    stream = _SIDE_STREAMS.get((device, home))
     if stream is None:
-        if len(_CHAIN_STREAMS) >= 64:          # (streams that came and went; nothing is left on theirs)
-            _CHAIN_STREAMS.clear()
+        if len(_SIDE_STREAMS) >= 64:          # (streams that came and went; nothing is left on theirs)
+            _SIDE_STREAMS.clear()
         stream = torch.cuda.Stream(device=device, priority=torch.cuda.current_stream().priority)
-        _CHAIN_STREAMS[(device, home)] = stream
+        _SIDE_STREAMS[(device, home)] = stream
     return stream.cuda_stream
 
 
@@ -291,7 +291,7 @@ def _native_step(gradient: Tensor, state, step: int, rows: int, cols: int, *, be
                  + (momentum.data_ptr(), k._ld(momentum), variance.data_ptr(), k._ld(variance), update.data_ptr(),
                     left.data_ptr(), k._ld(left), right.data_ptr(), k._ld(right)))
     home = k._stream()
-    tail = (k.status_word(g.device).data_ptr(), home, _chain_stream(g.device, home))
+    tail = (k.status_word(g.device).data_ptr(), home, _side_stream(g.device, home))
     scalars = (beta, beta1, beta2, eps / math.sqrt(bias2), 1.0 / (1.0 - beta1**step), 1.0 / math.sqrt(bias2))
     if TIMER.enabled:
         for name, phase in _STEP_STAGES if averages else _STEP_STAGES[:-1]:

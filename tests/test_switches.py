@@ -49,38 +49,38 @@ def streams(monkeypatch):
     current = FakeStream()
     monkeypatch.setattr(torch.cuda, "Stream", FakeStream)
     monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: current)
-    monkeypatch.setattr(local, "_CHAIN_STREAMS", {})
+    monkeypatch.setattr(local, "_SIDE_STREAMS", {})
 
-    def chain_of(handle, priority=0):
+    def side_of(handle, priority=0):
         current.cuda_stream, current.priority = handle, priority
-        return local._chain_stream(torch.device("cuda", 0), handle)
+        return local._side_stream(torch.device("cuda", 0), handle)
 
-    return local, chain_of
+    return local, side_of
 
 
-def test_every_callers_stream_has_rotations_of_its_own(streams):
-    local, chain_of = streams
-    first, second = chain_of(1), chain_of(2)
-    assert first != second and chain_of(1) == first and chain_of(2) == second
+def test_every_callers_stream_has_averages_of_its_own(streams):
+    local, side_of = streams
+    first, second = side_of(1), side_of(2)
+    assert first != second and side_of(1) == first and side_of(2) == second
     assert {first, second}.isdisjoint({1, 2})
 
 
-def test_rotations_have_the_callers_priority(streams):
-    local, chain_of = streams
+def test_averages_have_the_callers_priority(streams):
+    local, side_of = streams
     for handle, priority in ((1, 0), (2, -1)):
-        handle = chain_of(handle, priority)
-        stream, = (s for s in local._CHAIN_STREAMS.values() if s.cuda_stream == handle)
+        handle = side_of(handle, priority)
+        stream, = (s for s in local._SIDE_STREAMS.values() if s.cuda_stream == handle)
         assert stream.priority == priority
 
 
 def test_streams_that_come_and_go_are_not_kept(streams):
-    local, chain_of = streams
+    local, side_of = streams
     for handle in range(500):
-        chain_of(handle)
-    assert len(local._CHAIN_STREAMS) <= 64
+        side_of(handle)
+    assert len(local._SIDE_STREAMS) <= 64
 
 
 def test_the_overlap_switch_leaves_everything_on_the_callers_stream(streams, monkeypatch):
-    local, chain_of = streams
+    local, side_of = streams
     monkeypatch.setattr(local, "OVERLAP_GRAM", False)
-    assert chain_of(7) == 7 and not local._CHAIN_STREAMS
+    assert side_of(7) == 7 and not local._SIDE_STREAMS
