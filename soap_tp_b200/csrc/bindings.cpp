@@ -59,19 +59,9 @@ class Arguments {
     t.hi = pointer<float>(); t.ldo = next(); t.hl = pointer<uint16_t>(); t.ld16 = next();
     return t;
   }
-  void matrix_and_bases(Rotation& r) {
-    r.source = pointer<void>(); r.source_type = static_cast<int>(next()); r.s_i = next(); r.s_j = next();
-    r.rows = static_cast<int>(next()); r.cols = static_cast<int>(next());
-    auto basis = [&](HalfOperand& plain, HalfOperand& turned, WideBasis& source, int size) {
-      plain = operand(); turned = operand();
-      source.src = pointer<float>(); source.s_i = next(); source.s_j = next(); source.size = size;
-      plain.mixed = source.plain; turned.mixed = source.turned;
-    };
-    basis(r.left, r.left_turned, r.guard.bases[0], r.rows);
-    basis(r.right, r.right_turned, r.guard.bases[1], r.cols);
-  }
+  bool done() const { return at_ == values_.size(); }
   void finish() const {
-    if (at_ != values_.size()) throw std::invalid_argument("too many integers for this call");
+    if (!done()) throw std::invalid_argument("too many integers for this call");
   }
 
  private:
@@ -84,22 +74,55 @@ class Arguments {
 struct RotationScratch {
   Rotation rotation{};       // without the matrix and its bases
   HalfOperand update{};
+  SplitTarget mixed_update{};
+  CUtensorMap source_maps[2], middle_maps[2], update_maps[2], basis_maps[4][2];      // bases: left, its transpose, right, ...
 
-  explicit RotationScratch(const std::vector<int64_t>& values) {
+  RotationScratch(int rows, int cols, const std::vector<int64_t>& values) {
     Arguments in(values);
     Rotation& r = rotation;
+    r.rows = rows; r.cols = cols;
     r.x = in.target(); r.xt = in.target();
     r.middle = in.operand();
     r.guard.wide = in.pointer<int>(); r.guard.nearest = static_cast<int>(in.next());
     r.guard.mixed = in.mixed();
-    r.middle.mixed = in.mixed();
-    for (WideBasis& basis : r.guard.bases) {
+    r.mixed_middle = in.mixed();
+    for (int side = 0; side < 2; ++side) {
+      WideBasis& basis = r.guard.bases[side];
       basis.plain = in.mixed();
       basis.turned = in.mixed();
+      basis.size = side ? cols : rows;
+      mixed_maps(basis_maps[2 * side], basis.plain, basis.size, basis.size);
+      mixed_maps(basis_maps[2 * side + 1], basis.turned, basis.size, basis.size);
     }
-    update = in.operand();
-    update.mixed = in.mixed();
+    mixed_maps(source_maps, r.guard.mixed, rows, cols);
+    mixed_maps(middle_maps, r.mixed_middle, cols, rows);
+    r.mixed_source = source_maps;
+    r.middle.mixed = middle_maps;
+    if (!in.done()) {
+      update = in.operand();
+      mixed_update = in.mixed();
+      mixed_maps(update_maps, mixed_update, rows, cols);
+      update.mixed = update_maps;
+    }
     in.finish();
+  }
+  RotationScratch(const RotationScratch&) = delete;          // (the operands point into the object)
+  RotationScratch& operator=(const RotationScratch&) = delete;
+
+  // The rotation of a matrix by its bases.
+  Rotation of(Arguments& in) const {
+    Rotation r = rotation;
+    r.source = in.pointer<void>(); r.source_type = static_cast<int>(in.next()); r.s_i = in.next(); r.s_j = in.next();
+    HalfOperand* const planes[] = {&r.left, &r.left_turned, &r.right, &r.right_turned};
+    for (int i = 0; i < 4; ++i) {
+      *planes[i] = in.operand();
+      planes[i]->mixed = basis_maps[i];
+      if (i % 2) {
+        WideBasis& basis = r.guard.bases[i / 2];
+        basis.src = in.pointer<float>(); basis.s_i = in.next(); basis.s_j = in.next();
+      }
+    }
+    return r;
   }
 };
 
@@ -201,16 +224,16 @@ PYBIND11_MODULE(_C, m) {
         "Scaled fp16 operand planes of a matrix in one or both orientations (gemm_half.h)");
 
   py::class_<RotationScratch>(m, "RotationScratch", "Scratch planes of rotations of one shape, as addresses (see Arguments)")
-      .def(py::init<const std::vector<int64_t>&>());
-  // Integers: the matrix and its bases (Arguments), the moments, results and phases in the order of SteadyStep, then the status
+      .def(py::init<int, int, const std::vector<int64_t>&>());
+  // Integers: the matrix and its bases (RotationScratch::of), the moments, results and phases in the order of SteadyStep, then the status
   // word, the stream and the stream of the averages.
   m.def("steady_step", [](const RotationScratch& scratch, const std::vector<int64_t>& v, double beta, float beta1, float beta2,
                           float eps, float inv_bc1, float inv_sqrt_bc2) {
     Arguments in(v);
     SteadyStep s{};
-    s.rotation = scratch.rotation;
+    s.rotation = scratch.of(in);
     s.update = scratch.update;
-    in.matrix_and_bases(s.rotation);
+    s.mixed_update = scratch.mixed_update;
     s.momentum = in.pointer<float>(); s.ldm = in.next();
     s.variance = in.pointer<float>(); s.ldv = in.next();
     s.out = in.pointer<float>();
@@ -232,8 +255,7 @@ PYBIND11_MODULE(_C, m) {
   // Integers: the matrix and its bases, then direction, result, its pitch, the status word and the stream.
   m.def("rotate_half", [](const RotationScratch& scratch, const std::vector<int64_t>& v) {
     Arguments in(v);
-    Rotation r = scratch.rotation;
-    in.matrix_and_bases(r);
+    const Rotation r = scratch.of(in);
     const bool turned = in.next() != 0;
     float* out = in.pointer<float>();
     const int64_t ldc = in.next();

@@ -559,11 +559,6 @@ CUtensorMap make_map(const uint16_t* base, int64_t K, int64_t rows, int64_t ld) 
   return encode_k_major(CU_TENSOR_MAP_DATA_TYPE_FLOAT16, base, K, rows, 2 * ld, kBK, 128, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
-void make_mixed_maps(CUtensorMap* to, const SplitTarget& planes, int64_t K, int64_t rows) {
-  to[0] = encode_k_major(CU_TENSOR_MAP_DATA_TYPE_FLOAT32, planes.hi, K, rows, 4 * planes.ldo, kMixedBK, 128, CU_TENSOR_MAP_SWIZZLE_128B);
-  to[1] = encode_interleaved(planes.hl, K, rows, planes.ld16, 2 * kMixedBK, 128);
-}
-
 template <int MODE>
 void launch(bool pairs, const HalfMaps& maps, const HalfArgs& args, int* status, cudaStream_t stream) {
   const HalfProblem& p = args.p;
@@ -583,6 +578,11 @@ void launch(bool pairs, const HalfMaps& maps, const HalfArgs& args, int* status,
 }
 
 }  // namespace
+
+void mixed_maps(CUtensorMap (&maps)[2], const SplitTarget& planes, int64_t K, int64_t cols) {
+  maps[0] = encode_k_major(CU_TENSOR_MAP_DATA_TYPE_FLOAT32, planes.hi, K, cols, 4 * planes.ldo, kMixedBK, 128, CU_TENSOR_MAP_SWIZZLE_128B);
+  maps[1] = encode_interleaved(planes.hl, K, cols, planes.ld16, 2 * kMixedBK, 128);
+}
 
 bool half_on_pairs(int M, int N, bool symmetric) {
   if (!gemm_cta_pairs_wanted()) return false;
@@ -608,7 +608,7 @@ void gemm_half(const HalfOperand& a, const HalfOperand& b, const HalfProblem& pr
                     (reinterpret_cast<uintptr_t>(prob.Ch) & 15) != 0 || (reinterpret_cast<uintptr_t>(prob.Cl) & 15) != 0))
     throw std::invalid_argument("gemm_half: output planes need 16-byte alignment and a pitch that is a multiple of 64");
   if (prob.wide) {
-    if (!a.mixed.hl || !b.mixed.hl) throw std::invalid_argument("gemm_half: a decided product needs both operands' mixed form");
+    if (!a.mixed || !b.mixed) throw std::invalid_argument("gemm_half: a decided product needs both operands' mixed form");
     if (to_planes && (!prob.mixed.hi || !prob.mixed.hl || prob.mixed.ldo < prob.M || prob.mixed.ld16 < bf16_plane_index(prob.M - 1) + 33 ||
                       !writes_pairs(prob.mixed)))
       throw std::invalid_argument("gemm_half: mixed output planes need 8-byte alignment and an even pitch");
@@ -619,8 +619,10 @@ void gemm_half(const HalfOperand& a, const HalfOperand& b, const HalfProblem& pr
   maps.b_h = make_map(b.h, prob.K, prob.N, b.ld);
   maps.b_l = b.l ? make_map(b.l, prob.K, prob.N, b.ld) : maps.b_h;
   if (prob.wide) {
-    make_mixed_maps(maps.mixed, a.mixed, prob.K, prob.M);
-    make_mixed_maps(maps.mixed + 2, b.mixed, prob.K, prob.N);
+    for (int i = 0; i < 2; ++i) {
+      maps.mixed[i] = a.mixed[i];
+      maps.mixed[2 + i] = b.mixed[i];
+    }
   }
   const HalfArgs args{prob, a.scale, a.scale_stride, b.scale, a.l ? 2 : 1, b.l ? 2 : 1};
   const bool pairs = prob.tiles ? prob.tiles == 2 : half_on_pairs(prob.M, prob.N, prob.symmetric);

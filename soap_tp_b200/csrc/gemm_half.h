@@ -1,6 +1,7 @@
 // Host-side interface of the fp16-pair GEMM (gemm_half.cu) and of the kernels that make its operands (half_planes.cu).
 #pragma once
 #include <cstdint>
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include "elementwise.h"
@@ -24,8 +25,12 @@ struct HalfOperand {
   int64_t ld;              // multiple of 64
   const float* scale;
   int64_t scale_stride;    // 0 for the second operand of a product, whose scales are applied after the sum over K
-  SplitTarget mixed{};     // the same operand in the mixed form, read where HalfProblem::wide says so
+  // The same operand in the mixed form, read where HalfProblem::wide says so: maps of its two planes (mixed_maps).
+  const CUtensorMap* mixed = nullptr;
 };
+// The tensor maps of K x cols mixed planes, which belong to scratch and are made once with it (a map takes the host 0.2 us, and a
+// step's products would need sixteen).
+void mixed_maps(CUtensorMap (&maps)[2], const SplitTarget& planes, int64_t K, int64_t cols);
 
 constexpr int kHalfScaleBlock = 128;
 
@@ -107,6 +112,8 @@ struct Rotation {
   HalfTarget x, xt;                                          // planes of G (depth rows) and G^T (depth cols), written
   HalfOperand left, left_turned, right, right_turned;        // planes of Q_L, Q_L^T, Q_R, Q_R^T
   HalfOperand middle;                                        // scratch planes cols x rows, scales per block
+  SplitTarget mixed_middle;                                  // the same in the mixed form
+  const CUtensorMap* mixed_source;                           // maps of guard.mixed
   RangeGuard guard;
 };
 
@@ -117,6 +124,7 @@ void rotate_half(const Rotation& r, bool turned, float* out, int64_t ldc, int* s
 struct SteadyStep {
   Rotation rotation;                                         // of the gradient
   HalfOperand update;                                        // scratch planes rows x cols, scales per block
+  SplitTarget mixed_update;
   float* momentum;
   int64_t ldm;
   float* variance;

@@ -53,13 +53,13 @@ void first_product(const Rotation& r, const HalfOperand& source, bool settled, c
   p.alpha = 1.0f;
   p.Ch = const_cast<uint16_t*>(r.middle.h); p.Cl = const_cast<uint16_t*>(r.middle.l); p.ldp = r.middle.ld;
   p.Cscale = const_cast<float*>(r.middle.scale); p.ldscale = r.middle.scale_stride;
-  p.wide = r.guard.wide; p.settled = settled; p.mixed = r.middle.mixed;
+  p.wide = r.guard.wide; p.settled = settled; p.mixed = r.mixed_middle;
   gemm_half(source, basis, p, status, stream);
 }
 
 HalfOperand source_of(const Rotation& r) {
   HalfOperand x = operand(r.x);
-  x.mixed = r.guard.mixed;
+  x.mixed = r.mixed_source;
   return x;
 }
 
@@ -101,7 +101,7 @@ void steady_step(const SteadyStep& s, int* status, cudaStream_t stream) {
     adam.mode = kEpiAdam;
     adam.Ch = const_cast<uint16_t*>(s.update.h); adam.Cl = const_cast<uint16_t*>(s.update.l); adam.ldp = s.update.ld;
     adam.Cscale = const_cast<float*>(s.update.scale); adam.ldscale = s.update.scale_stride;
-    adam.mixed = s.update.mixed;
+    adam.mixed = s.mixed_update;
     adam.mom = s.momentum; adam.ldm = s.ldm; adam.var = s.variance; adam.ldv = s.ldv;
     adam.beta1 = s.beta1; adam.beta2 = s.beta2; adam.eps = s.eps; adam.inv_bc1 = s.inv_bc1; adam.inv_sqrt_bc2 = s.inv_sqrt_bc2;
     gemm_half(r.middle, r.right, adam, status, stream);

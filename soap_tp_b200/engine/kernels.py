@@ -558,7 +558,7 @@ def adam_update(gradient: Tensor, momentum: Tensor, variance: Tensor, beta1: flo
 
 def strided_source(matrix: Tensor) -> tuple:
     """A 2-D fp32 or bf16 tensor as the native rotation takes it."""
-    return (matrix.data_ptr(), int(matrix.dtype == torch.bfloat16), matrix.stride(0), matrix.stride(1), *matrix.shape)
+    return (matrix.data_ptr(), int(matrix.dtype == torch.bfloat16), *matrix.stride())
 
 
 def rotate_half(scratch, matrix_and_bases: tuple, turned: bool, out: Tensor) -> None:

@@ -227,9 +227,7 @@ class _Scratch:
             update_planes, mixed_update = workspace_planes("U", rows, cols, device, blocked=True), tf32_workspace("U", rows, cols, device)
             addresses += update_planes.operand() + mixed_update.mixed_target()
             self.keep += [update_planes, mixed_update]
-        else:
-            addresses += (0,) * 9
-        self.native = _C.RotationScratch(addresses)
+        self.native = _C.RotationScratch(rows, cols, addresses)
 
 
 def _scratch(rows: int, cols: int, device, terms: int, update: bool = False, averages: bool = False) -> _Scratch:
