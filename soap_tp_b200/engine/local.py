@@ -45,6 +45,7 @@ class BasisPlanes:
         self.plain = None                 # operand Q   (depth = rows of Q)
         self.transposed = None            # operand Q^T (depth = cols of Q)
         self.addresses: tuple = ()        # both, and the basis itself, as the native calls take them
+        self.copy: Optional[Tensor] = None    # of a basis of another type, which the addresses mean then
 
     def refresh(self, Q: Tensor, size: int) -> None:
         key = (Q.data_ptr(), Q._version, size)
@@ -53,13 +54,16 @@ class BasisPlanes:
         if key == self.key and self.owner is not None and self.owner() is Q:
             return
         view = Q[:size, :size]
+        self.copy = None if Q.dtype == torch.float32 else view.float()
+        if self.copy is not None:
+            view = self.copy
         if self.plain is None or self.plain.depth != size or self.plain.device != Q.device:
             # (an address that was recycled by a tensor of another size starts over)
             make = _operand if self.half else _tf32_operand
             self.plain, self.transposed = make(size, size, Q.device), make(size, size, Q.device)
         split(view, self.plain, self.transposed)
         if isinstance(self.plain, k.HalfPlanes):
-            self.addresses = self.plain.operand() + self.transposed.operand() + (Q.data_ptr(), Q.stride(0), Q.stride(1))
+            self.addresses = self.plain.operand() + self.transposed.operand() + (view.data_ptr(), *view.stride())
         self.key = (Q.data_ptr(), Q._version, size)
         self.owner = weakref.ref(Q)
 

@@ -183,3 +183,24 @@ def test_the_decision(rows, cols, layout):
         local.rotate_matrix(source, left, right, False, out)
         scratch = local._scratch(rows, cols, out.device, 2)
         assert scratch.wide.tolist() == [wide]
+
+
+@pytest.mark.parametrize("dtype", [torch.float64, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("orders", [0, 9])
+def test_bases_of_other_types_are_read_as_what_they_hold(dtype, orders):
+    """Also where the rotation reads the basis itself, for its mixed form."""
+    from soap_tp_b200.engine import kernels as k
+    from soap_tp_b200.engine import local
+
+    g = torch.Generator().manual_seed(5)
+    matrix = _gradient(150, 90, orders, "even", "rows", seed=8).float()
+    bases = [torch.linalg.qr(torch.randn(n, n, generator=g))[0].to(dtype) for n in (150, 90)]
+    results = []
+    for held in (bases, [b.float() for b in bases]):
+        out = _packed(matrix)
+        local.rotate(out, held[0].cuda().T.contiguous().T, held[1].cuda().T.contiguous().T, (150, 90), "forward")
+        results.append(out)
+    k.check_status()
+    assert torch.equal(*results)
+    expected = bases[0].double().T @ matrix.double() @ bases[1].double()
+    assert float((results[0].double().cpu() - expected).norm()) <= 2e-6 * float(expected.norm())
