@@ -286,7 +286,6 @@ def _native_step(gradient: Tensor, state, step: int, rows: int, cols: int, *, be
     bias2 = 1.0 - beta2**step
     momentum, variance = state["momentum"], state["variance"]
     left, right = state["left_preconditioner"], state["right_preconditioner"]
-    assert (left.stride(0) == 1 or rows == 1) and (right.stride(0) == 1 or cols == 1)
     scratch = _scratch(rows, cols, g.device, 1 if g.dtype == torch.bfloat16 else 2, update=True, averages=averages)
     update = torch.empty((rows, cols), dtype=torch.float32, device=g.device)
     arguments = (k.strided_source(g) + ctx.left.addresses + ctx.right.addresses
@@ -338,6 +337,21 @@ def _tf32_step(gradient: Tensor, state, step: int, rows: int, cols: int, *, beta
     return update
 
 
+def _check_state(state: MutableMapping[str, Any], rows: int, cols: int) -> None:
+    """The kernels write these buffers through raw pointers: fp32, of at least their matrix's size, column-major."""
+    for name, height, width in (("momentum", rows, cols), ("variance", rows, cols), ("left_preconditioner", rows, rows),
+                                ("right_preconditioner", cols, cols)):
+        buffer = state[name]
+        if buffer.dtype is torch.float32 and buffer.shape == (height, width) and buffer.stride() == (1, height):
+            continue                      # as they are allocated
+        if buffer.dtype != torch.float32:
+            raise ValueError(f"state['{name}'] must use float32, got {buffer.dtype}.")
+        if buffer.ndim != 2 or buffer.shape[0] < height or buffer.shape[1] < width:
+            raise ValueError(f"state['{name}'] has shape {tuple(buffer.shape)}, smaller than {(height, width)}.")
+        if (buffer.stride(0) != 1 and height > 1) or (buffer.stride(1) < height and width > 1):
+            raise ValueError(f"state['{name}'] must be column-major, got strides {buffer.stride()}.")
+
+
 def soap_step(
     gradient: Tensor,
     state: MutableMapping[str, Any],
@@ -365,6 +379,7 @@ def soap_step(
         state["step"] = 0
         return torch.zeros((rows, cols), dtype=torch.float32, device=device)
 
+    _check_state(state, rows, cols)
     step = int(state["step"]) + 1
     refreshing = step % interval == 0
     # (an empty matrix has nothing to rotate on pairs; the other path takes it as every product does)
