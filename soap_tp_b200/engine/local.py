@@ -141,7 +141,7 @@ def product(a, b, **epilogue) -> None:
 def workspace_planes(tag: str, depth: int, cols: int, device, *, blocked: bool = False, terms: int = 2):
     """Scratch operand planes shared by every parameter of the same shape on ``device``.  ``blocked``: written by a
     product's epilogue; ``terms=1``: written from bf16 values."""
-    key = (tag, depth, cols, str(device), terms)
+    key = (tag, depth, cols, str(device), terms, blocked, k.MIXED_CORRECTIONS and tag not in CLASSIC_TAGS)
     planes = _WORKSPACES.get(key)
     if planes is None:
         planes = (k.Planes.empty(depth, cols, device) if tag in CLASSIC_TAGS
