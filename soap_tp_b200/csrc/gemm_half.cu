@@ -44,7 +44,7 @@ constexpr int kBK = 64;                          // one 128-byte swizzle row of 
 // squares, a rotation along a leading singular vector) all err to one side, and small products that meet a main sum are
 // truncated at its size.  Relative error of products of positive operands, drained every 64 / every 128 / mixed form: two
 // terms 2.7e-7 / 6.6e-7 / 4.6e-7 at K = 8192 and 2.1e-7 / 6.6e-7 / 4.5e-7 at K = 128, one term against two 2.1e-7 / 3.7e-7 /
-// 3.1e-7 and 1.3e-7 / 3.6e-7 / 2.7e-7.  The price: two terms 4096^3 351 us instead of 319, one term against two 293 instead of 247.
+// 3.1e-7 and 1.3e-7 / 3.6e-7 / 2.7e-7.  The price: two terms 4096^3 340 us instead of 319, one term against two 290 instead of 247.
 constexpr int kScaleBlocks = kHalfScaleBlock / kBK;      // k-blocks that share one of A's scales
 constexpr int kMixedBK = 32;                     // one 128-byte swizzle row of fp32, or of the interleaved bf16 plane
 constexpr int kMixedDrain = 2;                   // its k-blocks per promotion
@@ -587,9 +587,9 @@ void mixed_maps(CUtensorMap (&maps)[2], const SplitTarget& planes, int64_t K, in
 bool half_on_pairs(int M, int N, bool symmetric) {
   if (!gemm_cta_pairs_wanted()) return false;
   // A pair's 256 x 256 tile takes about 1.5 times as long as a CTA's 128 x 128 one (it loads half as much per product): pairs
-  // unless single CTAs get by with so few waves that they finish earlier.  Pairs against singles, measured: 1024^3 32 and
-  // 24 us, 2048^3 50 and 69, 4096^3 333 and 410; symmetric, then drained every 128 of K, 1024 39 and 28, 2048 54 and 44, 4096 186 and
-  // 255 (drained every 64, one term: 220 and 241).
+  // unless single CTAs get by with so few waves that they finish earlier.  Pairs against singles, two terms: 1024^3 29 and
+  // 22 us, 1536^3 37 and 30, 2048^3 47 and 70, 3072^3 139 and 209, 4096^3 340 and 439; symmetric, two terms and one: 1024 33 and
+  // 24, 28 and 19; 2048 50 and 41, 39 and 32; 3072 144 and 164, 100 and 113; 4096 190 and 291, 134 and 206.
   auto tiles_of = [&](int64_t side) {
     const int64_t m = (M + side - 1) / side, n = (N + side - 1) / side;
     return symmetric ? m * (m + 1) / 2 : m * n;

@@ -153,10 +153,11 @@ def round_up(value: int, multiple: int) -> int:
     return -(-value // multiple) * multiple
 
 
-# SOAP_TP_MIXED_CORRECTIONS=0 keeps every product on three tf32 MMAs per k-step.  By default the products of the
-# single-GPU step run on scaled fp16 pairs (``HalfPlanes``), those of the multi-GPU engine and of the one-sided step take their
-# two correction terms as bf16 MMAs (``Planes``, mixed form); the factorisations (QR, eigensolvers, power iteration) always use
-# the full 3xTF32 form.
+# SOAP_TP_MIXED_CORRECTIONS=0 keeps every product on three tf32 MMAs per k-step.  By default the products of an ordinary
+# single-GPU step, of rotations and of the one-sided step's average run on scaled fp16 pairs (``HalfPlanes``; rotations of
+# matrices whose range asks for it on mixed planes); those of the multi-GPU engine, of the one-sided update and of averages that
+# bases are derived from take their two correction terms as bf16 MMAs (``Planes``, mixed form); the factorisations (QR,
+# eigensolvers, power iteration) always use the full 3xTF32 form.
 MIXED_CORRECTIONS = os.environ.get("SOAP_TP_MIXED_CORRECTIONS", "1") != "0"
 
 

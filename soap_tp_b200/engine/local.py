@@ -81,9 +81,9 @@ _CONTEXTS: "OrderedDict[tuple, ParameterContext]" = OrderedDict()
 _WORKSPACES: Dict[tuple, Any] = {}
 
 
-# Operand planes of the eigenbases kept between steps (SOAP_TP_BASIS_CACHE_GB, default 40): 12 bytes per basis element
-# (two orientations, value plane + low plane), three times the bases themselves.  Beyond the limit the least recently
-# used parameters' planes are dropped and split again on use (most recently used first, see ``context_for``).
+# Operand planes of the eigenbases kept between steps (SOAP_TP_BASIS_CACHE_GB, default 40), counted as 12 bytes per basis
+# element; fp16 pairs hold 8 (two orientations of 4), tf32 planes 16.  Beyond the limit parameters' planes are dropped (the
+# most recently used first, see ``context_for``) and split again on use.
 BASIS_CACHE_BYTES = int(float(os.environ.get("SOAP_TP_BASIS_CACHE_GB", "40")) * 2**30)
 
 
@@ -202,9 +202,10 @@ def gram_updates_for_bases(gradient: Tensor, state, beta: float, rows: int, cols
     """The averages of a step that derives bases from them (the first one, and those with a refresh), on tf32 planes like
     everything else that is factored.
 
-    A factorisation decides signs by rounding (the last pivot's by its last bit), so the averages that go into one keep, bit
-    for bit, the products they have always been formed with: the same gradient and state give the same bases, not the same
-    ones up to signs."""
+    The QR panel kernels take the sign of a basis's last column from a rounding residue (``|x|^2 - x_1^2`` of a column of one
+    element), so that column and what is expressed in it would change sign with the last bits of the averages.  These keep
+    the products they have always been formed with: the same gradient and state give the same bases, not the same ones up
+    to a sign."""
     gp, gtp = tf32_workspace("G", rows, cols, gradient.device), tf32_workspace("GT", cols, rows, gradient.device)
     split(gradient.detach(), gp, gtp)
     gram_updates(gp, gtp, state, beta, rows, cols)

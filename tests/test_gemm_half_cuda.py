@@ -99,7 +99,9 @@ def test_products_match_fp64(K, M, N, tiles, terms):
 @pytest.mark.parametrize("tiles", [1, 2])
 def test_chained_products_and_adam(M, N, K, tiles):
     """Planes written by a product (one scale per 128 rows and column), used as the first operand of the next one, with
-    rows whose sizes differ by ten orders; the Adam epilogue against fp64."""
+    rows whose sizes differ by ten orders: every row of the planes to the rounding of its own size, or to 2^-39 of the largest
+    row that shares its scale (rotations whose rows ask for more take the mixed form, tests/test_range_cuda.py); the Adam
+    epilogue against fp64."""
     from soap_tp_b200.engine import kernels as k
 
     g = torch.Generator().manual_seed(M)
@@ -110,6 +112,11 @@ def test_chained_products_and_adam(M, N, K, tiles):
     k.gemm_half(_planes(a.cuda()), _planes(b.cuda()), mode=k.EPI_SPLIT, out_planes=t, tiles=tiles)
     expected_t = a.double().T @ b.double()
     assert _rel(t.dense(), expected_t) < BOUND
+    error = (t.dense().cpu() - expected_t).norm(dim=1)
+    for first in range(0, M, k.HALF_SCALE_BLOCK):
+        block = slice(first, min(M, first + k.HALF_SCALE_BLOCK))
+        floor = 2.0**-39 * expected_t[block].abs().amax(dim=0).norm()
+        assert bool((error[block] <= BOUND * expected_t[block].norm(dim=1) + floor).all())
     cp = _planes(c.cuda())
     moments = [torch.randn(M, N, generator=g), torch.rand(M, N, generator=g) + 0.1]
     m, v = (x.cuda().T.contiguous().T for x in moments)
