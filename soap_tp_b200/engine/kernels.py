@@ -146,7 +146,11 @@ def mark_written(*tensors: Optional[Tensor]) -> None:
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """Handle of the current stream of the current device (every launch asks; the stream object costs 3 us to make)."""
+    return _raw_stream(torch.cuda.current_device())
+
+
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", lambda index: torch.cuda.current_stream(index).cuda_stream)
 
 
 def round_up(value: int, multiple: int) -> int:
@@ -578,12 +582,12 @@ _PLAIN_TENSORS = (Tensor, torch.nn.Parameter)
 def _addressable(*tensors: Tensor) -> bool:
     """Whether a flat kernel of the current stream may work on these tensors through their addresses: plain, dense tensors
     (a subclass may have no storage behind its address, or a meaning of its own) of one shape on the current device."""
-    device, shape = tensors[0].device, tensors[0].shape
+    index, shape = tensors[0].get_device(), tensors[0].shape
     for t in tensors:
-        if (type(t) not in _PLAIN_TENSORS or t.device != device or t.shape != shape or t.layout != torch.strided
+        if (type(t) not in _PLAIN_TENSORS or t.get_device() != index or t.shape != shape or t.layout is not torch.strided
                 or not t.is_contiguous() or t.is_neg()):
             return False
-    return device.type == "cuda" and device.index == torch.cuda.current_device()
+    return tensors[0].is_cuda and index == torch.cuda.current_device()
 
 
 def apply_update(p: Tensor, update: Tensor, keep: float, lr: float) -> bool:

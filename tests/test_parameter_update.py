@@ -53,8 +53,13 @@ class OnDevice:
 
     dtype, shape, layout = torch.float32, torch.Size([8]), torch.strided
 
+    is_cuda = True
+
     def __init__(self, index):
-        self.device = torch.device("cuda", index)
+        self.index = index
+
+    def get_device(self):
+        return self.index
 
     def is_contiguous(self):
         return True
