@@ -1,7 +1,7 @@
 """Single-GPU (grid (1, 1)) device pipeline.
 
 With one rank the packed block-cyclic buffers ARE the dense column-major matrices, so the whole
-step is a chain of this package's kernels on one stream:
+step is a chain of this package's kernels on the caller's stream, its averages on one beside it:
 
     split G (both orientations)                                   largest_kernel, half_planes_kernel
     T   = X^T Q_L                (planes)                          gemm_half / split epilogue
