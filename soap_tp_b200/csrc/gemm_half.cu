@@ -5,10 +5,10 @@
 // and has no l), against one tf32 MMA (half the fp16 rate) and two bf16 ones of the mixed form in gemm_tf32x3.cu: 3/4 of
 // the tensor time, half the operand bytes, and a representation that is off by 2^-23 instead of 2^-20.
 //
-// Structure (192 KB of stages, one CTA per SM, 320 threads):
+// Structure (192 KB of stages, one CTA per SM, 576 threads):
 //   warp 0, one lane : TMA producer - up to four boxes of 128 rows x 64 fp16 (128-byte swizzle) per stage
 //   warp 1, one lane : MMA issuer
-//   warps 2..9       : promotion and epilogue
+//   warps 2..17      : promotion and epilogue
 // PAIR: the two CTAs of a cluster share a 256 x 256 tile (cta_group::2, each stages its own 128 rows of A and half of the
 // rows of B, no multicast); otherwise one CTA computes 128 x 128.  TMA zero-fills rows and K beyond the operands.
 //
@@ -51,9 +51,10 @@ constexpr int kMixedDrain = 2;                   // its k-blocks per promotion
 constexpr int kBoxBytes = 128 * kBK * 2;
 constexpr int kStagePool = 12 * kBoxBytes;       // 3 stages of four boxes, 4 of three, 6 of two
 constexpr int kMaxStages = 6;
-constexpr int kEpiWarps = 8;
+constexpr int kEpiWarps = 16;
 constexpr int kThreads = 64 + 32 * kEpiWarps;
-constexpr int kSmemBytes = kStagePool + 1024 + 256;
+constexpr int kScaleBytes = 256 * 4;              // B's scales of the tile's columns
+constexpr int kSmemBytes = kStagePool + kScaleBytes + 1024 + 256;
 // Between A's factor and B's the sums are kept 2^-16 below scale: B's planes are 2^14 and more above scale where B is of
 // order one, and a large A must not overflow before B's factor brings the product back into range.
 constexpr float kDown = 1.0f / 65536.0f, kUp = 65536.0f;
@@ -139,19 +140,37 @@ __device__ __forceinline__ void store_column(const HalfProblem& p, bool wide, in
   else store_half_column(p, m0, n, lane, v);
 }
 
+// One line of L2 per lane: the epilogue's loads of what it reads back would otherwise all reach memory at the end of a wave of tiles
+// (Adam, 8192^3: 3003 -> 2617 us).  Not the old result of symmetric products on pairs, whose loop is too short to hide it (one term,
+// 4096: 123 us without, 145 with; on single CTAs 1024: 29 and 26).
+template <int BN, int MODE>
+__device__ __forceinline__ void prefetch_old(const HalfProblem& p, int m0, int n0, int ew, int lane) {
+  auto columns = [&](const float* base, int64_t ld) {
+    const int row = m0 + 32 * (lane & 3);
+    for (int nl = 8 * ew + (lane >> 2); nl < BN; nl += 8 * kEpiWarps)
+      if (row < p.M && n0 + nl < p.N) asm volatile("prefetch.global.L2 [%0];" ::"l"(base + row + static_cast<int64_t>(n0 + nl) * ld));
+  };
+  if constexpr (MODE == kEpiAdam) {
+    columns(p.mom, p.ldm);
+    columns(p.var, p.ldv);
+  } else if constexpr (MODE == kEpiStore) {
+    if (BN == 128 && p.beta != 0.f) columns(p.C, p.ldc);
+  }
+}
+
 // Epilogue over the staged tile: tile[n_local * PITCH + m_local] holds sums 2^-16 below scale, without B's scales (`wide`: the
 // sums themselves).  Accesses are four bytes per lane along M, so that no alignment of the outputs is needed, with kUnroll
 // columns in flight.
 template <int BN, int MODE, int PITCH>
-__device__ __forceinline__ void half_epilogue(const HalfArgs& args, bool wide, float* tile, int m0, int n0, int ew, int lane) {
+__device__ __forceinline__ void half_epilogue(const HalfArgs& args, const float* column_scales, bool wide, float* tile, int m0, int n0,
+                                              int ew, int lane) {
   const HalfProblem& p = args.p;
-  auto column_scale = [&](int n) { return wide ? kDown : args.b_scale[n]; };      // kDown undoes kUp: a factor of one
   const int rows = min(kBM, p.M - m0), cols = min(BN, p.N - n0);
   const float alpha = p.alpha;
   if constexpr (MODE == kEpiRowMajor) {
     ColumnFactor scaled[BN / 32];
 #pragma unroll
-    for (int j = 0; j < BN / 32; ++j) scaled[j] = ColumnFactor((lane + 32 * j < cols) ? column_scale(n0 + lane + 32 * j) : 0.f);
+    for (int j = 0; j < BN / 32; ++j) scaled[j] = ColumnFactor(column_scales[lane + 32 * j]);
     for (int r = ew; r < rows; r += kEpiWarps) {
       float* dst = p.C + static_cast<int64_t>(m0 + r) * p.ldc + n0;
 #pragma unroll
@@ -162,7 +181,7 @@ __device__ __forceinline__ void half_epilogue(const HalfArgs& args, bool wide, f
     }
   } else if constexpr (MODE == kEpiSplit) {
     for (int nl = ew; nl < cols; nl += kEpiWarps) {
-      const ColumnFactor scaled(column_scale(n0 + nl));
+      const ColumnFactor scaled(column_scales[nl]);
       float v[4];
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
@@ -174,12 +193,11 @@ __device__ __forceinline__ void half_epilogue(const HalfArgs& args, bool wide, f
     }
   } else if constexpr (MODE == kEpiAdam) {
     for (int base = ew * kUnroll; base < cols; base += kEpiWarps * kUnroll) {
-      float mo[kUnroll][kRowsPerLane], va[kUnroll][kRowsPerLane], scale[kUnroll];
+      float mo[kUnroll][kRowsPerLane], va[kUnroll][kRowsPerLane];
 #pragma unroll
       for (int u = 0; u < kUnroll; ++u) {
         const int n = n0 + base + u;
         const bool here = base + u < cols;
-        scale[u] = here ? column_scale(n) : 0.f;
 #pragma unroll
         for (int i = 0; i < kRowsPerLane; ++i) {
           const int r = lane + 32 * i;
@@ -193,7 +211,7 @@ __device__ __forceinline__ void half_epilogue(const HalfArgs& args, bool wide, f
         if (base + u >= cols) break;
         const int n = n0 + base + u;
         float* column = tile + (base + u) * PITCH;
-        const ColumnFactor scaled(scale[u]);
+        const ColumnFactor scaled(column_scales[base + u]);
 #pragma unroll
         for (int i = 0; i < kRowsPerLane; ++i) {
           const int r = lane + 32 * i;
@@ -222,12 +240,11 @@ __device__ __forceinline__ void half_epilogue(const HalfArgs& args, bool wide, f
   } else {
     // kEpiStore.  Symmetric: entries on and below the diagonal, whose final values go back into the tile for the mirror.
     for (int base = ew * kUnroll; base < cols; base += kEpiWarps * kUnroll) {
-      float old[kUnroll][kRowsPerLane], scale[kUnroll];
+      float old[kUnroll][kRowsPerLane];
 #pragma unroll
       for (int u = 0; u < kUnroll; ++u) {
         const int n = n0 + base + u;
         const bool here = base + u < cols;
-        scale[u] = here ? column_scale(n) : 0.f;
 #pragma unroll
         for (int i = 0; i < kRowsPerLane; ++i) {
           const int r = lane + 32 * i;
@@ -240,7 +257,7 @@ __device__ __forceinline__ void half_epilogue(const HalfArgs& args, bool wide, f
         const int n = n0 + base + u;
         if (base + u >= cols) break;
         float* column = tile + (base + u) * PITCH;
-        const ColumnFactor scaled(scale[u]);
+        const ColumnFactor scaled(column_scales[base + u]);
 #pragma unroll
         for (int i = 0; i < kRowsPerLane; ++i) {
           const int r = lane + 32 * i;
@@ -266,13 +283,18 @@ __device__ __forceinline__ void half_epilogue(const HalfArgs& args, bool wide, f
   }
 }
 
-template <bool PAIR, typename Epilogue>
-__device__ __forceinline__ void half_kernel_body(const HalfMaps& maps, const HalfArgs& args, int* status, Epilogue epilogue) {
+template <bool PAIR>
+constexpr int kColumns = (PAIR ? 256 : 128) / (kEpiWarps / 4);      // of the tile, per epilogue thread
+
+template <bool PAIR, typename Prefetch, typename Epilogue>
+__device__ __forceinline__ void half_kernel_body(const HalfMaps& maps, const HalfArgs& args, int* status, Prefetch prefetch,
+                                                 Epilogue epilogue) {
   constexpr int BN = PAIR ? 256 : 128;
   constexpr int kCtas = PAIR ? 2 : 1;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + kStagePool);      // PAIR: used in the leader CTA only
+  float* column_scales = reinterpret_cast<float*>(smem + kStagePool);
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + kStagePool + kScaleBytes);      // PAIR: used in the leader CTA only
   uint64_t* empty_bar = full_bar + kMaxStages;      // each CTA its own: "my stage may be refilled"
   uint64_t* acc_full = empty_bar + kMaxStages;      // [2] each CTA its own: tensor core -> epilogue
   uint64_t* acc_empty = acc_full + 2;               // [2] PAIR: leader's only, epilogue warps of both CTAs -> tensor core
@@ -403,10 +425,13 @@ __device__ __forceinline__ void half_kernel_body(const HalfMaps& maps, const Hal
     bool ok = true;
     int s = 0, kb = 0;
     uint32_t parity = 0;
+    // Whether the next k-block's operands and accumulator are there is looked up while this one's products are still being issued:
+    // a wait between two k-blocks, however short, drains the tensor core's queue of a few products (350 of 1860 cycles of a k-block).
+    bool loaded = false, drained = false;
     for (int d = 0; d < loop.drains; ++d) {
       const int buf = d & 1;
       if (d >= 2) {
-        ok = mbar_wait_bounded(&acc_empty[buf], ((d >> 1) - 1) & 1, abort_flag, status, kStatusAccumWaitTimeout);
+        ok = drained || mbar_wait_bounded(&acc_empty[buf], ((d >> 1) - 1) & 1, abort_flag, status, kStatusAccumWaitTimeout);
         if (!ok) break;
         tc_fence_after_sync();
       }
@@ -415,9 +440,14 @@ __device__ __forceinline__ void half_kernel_body(const HalfMaps& maps, const Hal
 #pragma unroll
       for (int i = 0; i < (kMixed ? kMixedDrain : 1); ++i, ++kb) {
         if (kMixed && kb == loop.blocks) break;
-        ok = mbar_wait_bounded(&full_bar[s], parity, abort_flag, status, kStatusTmaWaitTimeout);
+        ok = loaded || mbar_wait_bounded(&full_bar[s], parity, abort_flag, status, kStatusTmaWaitTimeout);
         if (!ok) break;
         tc_fence_after_sync();
+        auto look_ahead = [&] {
+          const int next = s + 1 == loop.stages ? 0 : s + 1;
+          loaded = kb + 1 < loop.blocks && mbar_test(&full_bar[next], next ? parity : parity ^ 1);
+          drained = d >= 1 && d + 1 < loop.drains && mbar_test(&acc_empty[buf ^ 1], (((d + 1) >> 1) - 1) & 1);
+        };
         const uint32_t stage = smem_u32(smem + s * loop.stage_bytes);
         const uint64_t a_0 = umma_desc_kmajor<128>(stage);
         const uint64_t b_0 = umma_desc_kmajor<128>(stage + loop.b_at);
@@ -435,6 +465,7 @@ __device__ __forceinline__ void half_kernel_body(const HalfMaps& maps, const Hal
             mma16(acc, a_1 + kLb, b_1, more);                                                                          // lb * hb
             mma16(acc, a_1, b_1 + kLb, 1);                                                                             // hb * lb
           }
+          look_ahead();
           if (!main_first) {
 #pragma unroll
             for (int k = 0; k < kMixedBK / 8; ++k) mma32(acc, a_0 + k * kStep, b_0 + k * kStep, 1);
@@ -448,6 +479,7 @@ __device__ __forceinline__ void half_kernel_body(const HalfMaps& maps, const Hal
 #pragma unroll
             for (int k = 0; k < kBK / 16; ++k, more = 1) mma16(acc, a_0 + k * kStep, b_0 + kSecond + k * kStep, more);  // h * l
           }
+          look_ahead();
 #pragma unroll
           for (int k = 0; k < kBK / 16; ++k, more = 1) mma16(acc, a_0 + k * kStep, b_0 + k * kStep, more);              // h * h
         }
@@ -472,14 +504,17 @@ __device__ __forceinline__ void half_kernel_body(const HalfMaps& maps, const Hal
     // ---------------- promotion + epilogue (each CTA its own 128 rows) ----------------
     const int ew = warp - 2;
     const int quarter = warp & 3;              // TMEM lane quarter this warp may read
-    const int half = ew >> 2;                  // which half of the tile's columns
-    constexpr int kCols = BN / 2;
-    const int col0 = half * kCols;
+    constexpr int kCols = kColumns<PAIR>;      // of the tile, per thread
+    const int col0 = (ew >> 2) * kCols;
+    // What the epilogue reads is fetched while the products run: B's scales into shared memory, and what it reads back into L2.
+    for (int n = threadIdx.x - 64; n < BN; n += 32 * kEpiWarps)
+      column_scales[n] = wide || n0 + n >= prob.N ? kDown : args.b_scale[n0 + n];      // kDown undoes kUp: a factor of one
+    prefetch(m0, n0, ew, lane);
     const float* a_scale = args.a_scale + min(m0 + quarter * 32 + lane, prob.M - 1);     // this thread's row
     const uint32_t drained = PAIR ? map_to_cta(smem_u32(&acc_empty[0]), 0) : 0;
-    float sum[kCols];
+    uint64_t sum[kCols / 2];                   // pairs of neighbouring columns
 #pragma unroll
-    for (int j = 0; j < kCols; ++j) sum[j] = 0.0f;
+    for (int j = 0; j < kCols / 2; ++j) sum[j] = 0;
     const int64_t a_stride = wide ? 0 : args.a_stride;
     const int drains = (prob.K + kBK - 1) / kBK;         // of either form
     float scale = wide ? 1.0f : *a_scale * kDown;
@@ -490,13 +525,14 @@ __device__ __forceinline__ void half_kernel_body(const HalfMaps& maps, const Hal
       if (!mbar_wait_bounded(&acc_full[buf], (d >> 1) & 1, abort_flag, status, kStatusAccumWaitTimeout)) break;
       tc_fence_after_sync();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(buf * BN + col0);
+      const uint64_t scales = pack_floats(scale, scale);
 #pragma unroll
-      for (int cc = 0; cc < kCols; cc += 32) {
-        uint32_t raw[32];
-        tmem_ld_32x32(taddr + static_cast<uint32_t>(cc), raw);
+      for (int cc = 0; cc < kCols; cc += 16) {
+        uint32_t raw[16];
+        tmem_ld_32x16(taddr + static_cast<uint32_t>(cc), raw);
         tmem_ld_wait();
 #pragma unroll
-        for (int j = 0; j < 32; ++j) sum[cc + j] = fmaf(__uint_as_float(raw[j]), scale, sum[cc + j]);
+        for (int j = 0; j < 8; ++j) fma_pair(sum[cc / 2 + j], pack_pair(raw[2 * j], raw[2 * j + 1]), scales);
       }
       scale = next;
       tc_fence_before_sync();
@@ -508,7 +544,7 @@ __device__ __forceinline__ void half_kernel_body(const HalfMaps& maps, const Hal
     }
     // The stages are idle once the accumulator has been drained for the last time: the sums are staged there and the epilogue runs as a
     // compact rolled loop over the tile.
-    epilogue(reinterpret_cast<float*>(smem), wide, sum, col0, quarter * 32 + lane, abort_flag, m0, n0, ew, lane);
+    epilogue(reinterpret_cast<float*>(smem), column_scales, wide, sum, col0, quarter * 32 + lane, abort_flag, m0, n0, ew, lane);
   }
 
   tc_fence_before_sync();
@@ -530,13 +566,14 @@ static_assert(256 * (kBM + 2) * 4 <= kStagePool, "the staged tile fits where the
 template <bool PAIR, int MODE>
 __device__ __forceinline__ void half_kernel_impl(const HalfMaps& maps, const HalfArgs& args, int* status) {
   constexpr int BN = PAIR ? 256 : 128;
-  half_kernel_body<PAIR>(maps, args, status, [&](float* tile, bool wide, float (&sum)[BN / 2], int col0, int row, volatile int* abort_flag,
+  half_kernel_body<PAIR>(maps, args, status, [&](int m0, int n0, int ew, int lane) { prefetch_old<BN, MODE>(args.p, m0, n0, ew, lane); },
+                         [&](float* tile, const float* column_scales, bool wide, uint64_t (&sum)[kColumns<PAIR> / 2], int col0, int row, volatile int* abort_flag,
                                                  int m0, int n0, int ew, int lane) {
 #pragma unroll
-    for (int j = 0; j < BN / 2; ++j) tile[(col0 + j) * kPitch<MODE> + row] = sum[j];
+    for (int j = 0; j < kColumns<PAIR>; ++j) tile[(col0 + j) * kPitch<MODE> + row] = pair_element(sum[j / 2], j & 1);
     asm volatile("bar.sync 1, %0;" ::"r"(kEpiWarps * 32) : "memory");
     // read after the barrier, so that all warps of the CTA agree (the epilogue has a barrier of its own)
-    if (*abort_flag == 0 && m0 < args.p.M) half_epilogue<BN, MODE, kPitch<MODE>>(args, wide, tile, m0, n0, ew, lane);
+    if (*abort_flag == 0 && m0 < args.p.M) half_epilogue<BN, MODE, kPitch<MODE>>(args, column_scales, wide, tile, m0, n0, ew, lane);
   });
 }
 

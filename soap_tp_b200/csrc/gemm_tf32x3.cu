@@ -39,22 +39,15 @@ namespace soapb200 {
 namespace {
 
 constexpr int kBM = 128;
-#ifndef SOAP_GEMM_BK
-#define SOAP_GEMM_BK 32
-#endif
-// K extent of one pipeline stage: 32 fp32 = one 128-byte swizzle row (two 96 KB stages for 256-wide
-// tiles) or 16 fp32 = one 64-byte swizzle row (four 48 KB stages).  Both were measured at 8192^3; the
-// deeper pipeline of the 64-byte variant did not help (4.23 ms against 4.15 ms), because the kernel
-// is bound by the L2 -> shared-memory traffic of the four operand planes, not by load latency.
-constexpr int kBK = SOAP_GEMM_BK;
+// K extent of one pipeline stage of the kernels that have an SM to themselves: 32 fp32 = one 128-byte swizzle row.
+constexpr int kBK = 32;
 // Timing experiments only: SOAP_GEMM_TERMS < 3 drops correction products (wrong results, same data movement), which
 // tells how much of the kernel's time is tensor-pipe time and how much is operand traffic.
 #ifndef SOAP_GEMM_TERMS
 #define SOAP_GEMM_TERMS 3
 #endif
-static_assert(kBK == 16 || kBK == 32, "one swizzle row per k-block: 64 or 128 bytes");
 constexpr int kRowBytes = kBK * 4;
-constexpr int kEpiWarps = 8;     // two warps per TMEM lane quarter, each owning half of the tile's columns
+constexpr int kEpiWarps = 16;    // four warps per TMEM lane quarter, each owning a quarter of the tile's columns
 constexpr int kThreads = 64 + 32 * kEpiWarps;
 // The tensor core adds into its fp32 accumulator with truncation, so an accumulation that runs over
 // the whole K extent drifts linearly in K (measured 6e-5 relative at K = 8192).  The accumulator is
@@ -62,15 +55,23 @@ constexpr int kThreads = 64 + 32 * kEpiWarps;
 // running sum held in registers while the tensor core fills the other TMEM buffer.
 constexpr int kPromote = 64 / kBK;  // k-blocks (64 elements of K) accumulated inside TMEM before promotion
 
-template <int BN>
+// Tile of a single CTA: BN columns, BK of K per stage, EW epilogue warps, CTAS of them on an SM.
+template <int BN_, int BK_, int EW, int CTAS>
 struct TileConfig {
-  static constexpr int kStageBytes = 2 * (kBM + BN) * kBK * 4;
-  static constexpr int kStagesFit = (196 * 1024) / kStageBytes;
-  static constexpr int kStages = kStagesFit > 6 ? 6 : kStagesFit;
+  static constexpr int BN = BN_, BK = BK_, kRowBytes = 4 * BK, kWarps = EW, kCtasPerSm = CTAS;
+  static constexpr int kThreads = 64 + 32 * EW;
+  static constexpr int kPromote = 64 / BK;
+  static constexpr int kStageBytes = 2 * (kBM + BN) * BK * 4;
+  static constexpr int kStages = (CTAS == 1 ? 196 * 1024 : 98 * 1024) / kStageBytes;
+  static_assert(BK == 16 || BK == 32, "one swizzle row per k-block: 64 or 128 bytes");
   static constexpr int kSmemBytes = kStages * kStageBytes + 1024 /*alignment slack*/ + 256 /*barriers*/;
   static constexpr int kTmemCols = 2 * BN;  // two accumulator buffers (ping-pong)
-  static constexpr int kColsPerThread = BN / 2;
+  static constexpr int kColsPerThread = 4 * BN / EW;
+  static_assert(kTmemCols * CTAS <= 512 && BN * (kBM + 4) * 4 <= kStages * kStageBytes, "accumulators and the staged tile fit");
 };
+using WideTile = TileConfig<256, 32, kEpiWarps, 1>;
+using NarrowTile = TileConfig<128, 32, kEpiWarps, 1>;
+using CompactTile = TileConfig<128, 16, 8, 2>;
 
 struct alignas(64) GemmMaps {
   CUtensorMap a_hi, a_lo, b_hi, b_lo;     // MIXED: a_lo / b_lo describe the interleaved bf16 plane (hb | lb)
@@ -306,15 +307,15 @@ __device__ __forceinline__ bool aligned16(const void* p, int64_t pitch_floats) {
 }
 
 // Fused epilogue over the staged tile (tile[n_local * kTilePitch + m_local]).  `ew` is the index of the
-// calling warp among the kEpiWarps epilogue warps.
-template <int BN, int MODE>
+// calling warp among the EW epilogue warps.
+template <int BN, int MODE, int EW>
 __device__ __forceinline__ void run_epilogue(const GemmProblem& prob, const float* tile, int m0, int n0, int ew, int lane,
                                              int64_t c_shift) {
   const int rows = min(kBM, prob.M - m0);
   const int cols = min(BN, prob.N - n0);
   if constexpr (MODE == kEpiRowMajor) {
     // one warp per output row, lanes sweep the columns so the stores are contiguous
-    for (int r = ew; r < rows; r += kEpiWarps) {
+    for (int r = ew; r < rows; r += EW) {
       float* dst = prob.C + static_cast<int64_t>(m0 + r) * prob.ldc + n0;
       for (int n = lane; n < cols; n += 32) dst[n] = prob.alpha * tile[n * kTilePitch + r];
     }
@@ -331,7 +332,7 @@ __device__ __forceinline__ void run_epilogue(const GemmProblem& prob, const floa
   if constexpr (MODE == kEpiPush)   // plane bases are segment starts (256-byte aligned); pitches and block size decide
     vector = vector && (prob.push_nb & 3) == 0 && (prob.push_ld & 3) == 0 && (prob.push_ld16 & 3) == 0;
   if (!vector) {
-    for (int nl = ew; nl < cols; nl += kEpiWarps) {
+    for (int nl = ew; nl < cols; nl += EW) {
       const int n = n0 + nl;
       for (int r = lane; r < rows; r += 32) {
         const int m = m0 + r;
@@ -344,7 +345,7 @@ __device__ __forceinline__ void run_epilogue(const GemmProblem& prob, const floa
   constexpr int kUnroll = 4;   // columns per warp whose loads are in flight together
   const int m = m0 + 4 * lane;
   const int gm = global_row(prob, m);   // the four rows of a lane are consecutive globally too (block sizes are multiples of 4)
-  for (int base = ew * kUnroll; base < cols; base += kEpiWarps * kUnroll) {
+  for (int base = ew * kUnroll; base < cols; base += EW * kUnroll) {
     Vec4 old0[kUnroll], old1[kUnroll];
     int state[kUnroll];        // 0: skip, 1: vector, 2: element by element (diagonal band of a symmetric product)
 #pragma unroll
@@ -376,13 +377,13 @@ __device__ __forceinline__ void run_epilogue(const GemmProblem& prob, const floa
 // c' = 64 * remap[2b + (n' >= 64)] + (n' & 63) of the next arrangement.  The result is written as
 // operand planes in two orientations: (m, c') at [c' + m * ldp] (the operand of the next pair update)
 // and, for rows m < m_limit, at [m + c' * ld2] (the operand of the next Gram product).
-template <int BN>
+template <int BN, int EW>
 __device__ __forceinline__ void run_pair_update(const GemmProblem& prob, const float* tile, int m0, int ew, int lane,
                                                 int batch) {
   const int pos0 = prob.remap[2 * batch], pos1 = prob.remap[2 * batch + 1];
   const int rows = min(kBM, prob.M - m0);
   // orientation 1: one warp per result row, lanes along the result columns (runs of 32 contiguous floats)
-  for (int r = ew; r < rows; r += kEpiWarps) {
+  for (int r = ew; r < rows; r += EW) {
     if (m0 + r < prob.o1_row_start) continue;
     const int64_t row_base = static_cast<int64_t>(m0 + r) * prob.ldp;
 #pragma unroll
@@ -397,7 +398,7 @@ __device__ __forceinline__ void run_pair_update(const GemmProblem& prob, const f
   }
   // orientation 2: one warp per result column, four rows per lane
   if (prob.C2hi != nullptr && m0 < prob.m_limit && rows == kBM) {
-    for (int nl = ew; nl < 128; nl += kEpiWarps) {
+    for (int nl = ew; nl < 128; nl += EW) {
       const int dst = ((nl < 64) ? pos0 : pos1) * 64 + (nl & 63);
       const Vec4 v = load4(tile + nl * kTilePitch + 4 * lane);
       Vec4 hi, lo;
@@ -413,11 +414,23 @@ __device__ __forceinline__ void run_pair_update(const GemmProblem& prob, const f
   }
 }
 
-template <int BN, int MODE, bool MIXED>
-__global__ void __launch_bounds__(kThreads, 1)
+// Split-K (kEpiStore only): blockIdx.y owns `count` groups of 32 of K from group `first` and writes its own partial result at
+// C + blockIdx.y * split_stride; the caller sums the partials in fixed order.  The same split in every kernel, so that the
+// choice of a tile does not change a bit of the result.
+struct SplitRange {
+  int first, count;
+};
+__device__ __forceinline__ SplitRange split_range(int K) {
+  const int groups = (K + 31) / 32, per_split = (groups + gridDim.y - 1) / gridDim.y;
+  const int first = blockIdx.y * per_split;
+  return SplitRange{first, max(0, min(groups, first + per_split) - first)};
+}
+
+template <typename Cfg, int MODE, bool MIXED>
+__global__ void __launch_bounds__(Cfg::kThreads, Cfg::kCtasPerSm)
 gemm_tf32x3_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ GemmProblem prob, int* status) {
-  // (the mixed variant needs the 32-element k-block build: 128-byte fp32 rows and 64-byte bf16 rows; the host refuses otherwise)
-  using Cfg = TileConfig<BN>;
+  constexpr int BN = Cfg::BN, kBK = Cfg::BK, kRowBytes = Cfg::kRowBytes, kPromote = Cfg::kPromote;
+  static_assert(!MIXED || kBK == 32, "the interleaved bf16 plane comes in groups of 32 of K");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + Cfg::kStages * Cfg::kStageBytes);
@@ -456,7 +469,7 @@ gemm_tf32x3_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant_
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&acc_full[b], 1);
-      mbar_init(&acc_empty[b], kEpiWarps);
+      mbar_init(&acc_empty[b], Cfg::kWarps);
     }
     *abort_flag = 0;
     mbar_fence_init();
@@ -474,12 +487,8 @@ gemm_tf32x3_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant_
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
 
-  // Split-K (kEpiStore only): blockIdx.y owns k-blocks [kb_first, kb_first + k_blocks) and writes its
-  // own partial result at C + blockIdx.y * split_stride; the caller sums the partials in fixed order.
-  const int total_k_blocks = (prob.K + kBK - 1) / kBK;
-  const int per_split = (total_k_blocks + gridDim.y - 1) / gridDim.y;
-  const int kb_first = blockIdx.y * per_split;
-  const int k_blocks = max(0, min(total_k_blocks, kb_first + per_split) - kb_first);
+  const SplitRange range = split_range(prob.K);
+  const int kb_first = range.first * (32 / kBK), k_blocks = range.count * (32 / kBK);
   const int chunks = (k_blocks + kPromote - 1) / kPromote;
 
   if (warp == 0 && lane == 0) {
@@ -592,12 +601,11 @@ gemm_tf32x3_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant_
     // ---------------- promotion + epilogue ----------------
     const int ew = warp - 2;
     const int quarter = warp & 3;              // TMEM lane quarter this warp may read
-    const int half = ew >> 2;                  // which half of the tile's columns
     constexpr int kCols = Cfg::kColsPerThread;
-    const int col0 = half * kCols;
-    float sum[kCols];
+    const int col0 = (ew >> 2) * kCols;        // this warp's columns of the tile
+    uint64_t sum[kCols / 2];                   // pairs of neighbouring columns
 #pragma unroll
-    for (int j = 0; j < kCols; ++j) sum[j] = 0.0f;
+    for (int j = 0; j < kCols / 2; ++j) sum[j] = 0;
     bool ok = true;
     for (int c = 0; c < chunks && ok; ++c) {
       const int buf = c & 1;
@@ -607,12 +615,12 @@ gemm_tf32x3_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant_
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) +
                              static_cast<uint32_t>(buf * BN + col0);
 #pragma unroll
-      for (int cc = 0; cc < kCols; cc += 32) {
-        uint32_t raw[32];
-        tmem_ld_32x32(taddr + static_cast<uint32_t>(cc), raw);
+      for (int cc = 0; cc < kCols; cc += 16) {
+        uint32_t raw[16];
+        tmem_ld_32x16(taddr + static_cast<uint32_t>(cc), raw);
         tmem_ld_wait();
 #pragma unroll
-        for (int j = 0; j < 32; ++j) sum[cc + j] += __uint_as_float(raw[j]);
+        for (int j = 0; j < 8; ++j) add_pair(sum[cc / 2 + j], pack_pair(raw[2 * j], raw[2 * j + 1]));
       }
       tc_fence_before_sync();
       __syncwarp();
@@ -626,14 +634,14 @@ gemm_tf32x3_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant_
     {
       const int m_local = quarter * 32 + lane;
 #pragma unroll
-      for (int jx = 0; jx < kCols; ++jx) tile[(col0 + jx) * kTilePitch + m_local] = sum[jx];
+      for (int jx = 0; jx < kCols; ++jx) tile[(col0 + jx) * kTilePitch + m_local] = pair_element(sum[jx / 2], jx & 1);
     }
-    asm volatile("bar.sync 1, %0;" ::"r"(kEpiWarps * 32) : "memory");
+    asm volatile("bar.sync 1, %0;" ::"r"(Cfg::kWarps * 32) : "memory");
     if (ok) {
       const int64_t c_shift = ((gridDim.y > 1) ? static_cast<int64_t>(blockIdx.y) * prob.split_stride : 0) +
                               static_cast<int64_t>(blockIdx.z) * prob.c_batch_stride;
-      if constexpr (MODE == kEpiPairUpdate) run_pair_update<BN>(prob, tile, m0, ew, lane, blockIdx.z);
-      else run_epilogue<BN, MODE>(prob, tile, m0, n0, ew, lane, c_shift);
+      if constexpr (MODE == kEpiPairUpdate) run_pair_update<BN, Cfg::kWarps>(prob, tile, m0, ew, lane, blockIdx.z);
+      else run_epilogue<BN, MODE, Cfg::kWarps>(prob, tile, m0, n0, ew, lane, c_shift);
     }
   }
 
@@ -722,7 +730,9 @@ gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ 
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
 
-  const int k_blocks = (prob.K + kBK - 1) / kBK;
+  const SplitRange range = split_range(prob.K);
+  const int kb_first = range.first, k_blocks = range.count;
+  static_assert(kBK == 32, "a k-block is a group of the split");
   const int chunks = (k_blocks + kPromote - 1) / kPromote;
 
   if (warp == 0 && lane == 0) {
@@ -736,7 +746,7 @@ gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ 
       uint8_t* stage = smem + s * kPairStageBytes;
       if (cta == 0) mbar_expect_tx(&full_bar[s], 2 * kPairStageBytes);
       const uint32_t leader_bar = map_to_cta(smem_u32(&full_bar[s]), 0);
-      const int k0 = kb * kBK;
+      const int k0 = (kb_first + kb) * kBK;
       const int k2 = MIXED ? 2 * k0 : k0;        // the interleaved bf16 plane has 64 elements per 32 of K
       tma_load_2d_pair(stage, &maps.a_hi, leader_bar, k0, m0);
       tma_load_2d_pair(stage + kBM * kRowBytes, &maps.a_lo, leader_bar, k2, m0);
@@ -815,13 +825,12 @@ gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ 
     // ---------------- promotion + epilogue (each CTA its own 128 rows) ----------------
     const int ew = warp - 2;
     const int quarter = warp & 3;
-    const int half = ew >> 2;
-    constexpr int kCols = BN / 2;
-    const int col0 = half * kCols;
+    constexpr int kCols = 4 * BN / kEpiWarps;
+    const int col0 = (ew >> 2) * kCols;
     const uint32_t leader_acc_empty0 = map_to_cta(smem_u32(&acc_empty[0]), 0);
-    float sum[kCols];
+    uint64_t sum[kCols / 2];                   // pairs of neighbouring columns
 #pragma unroll
-    for (int j = 0; j < kCols; ++j) sum[j] = 0.0f;
+    for (int j = 0; j < kCols / 2; ++j) sum[j] = 0;
     bool ok = true;
     for (int c = 0; c < chunks && ok; ++c) {
       const int buf = c & 1;
@@ -831,12 +840,12 @@ gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ 
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) +
                              static_cast<uint32_t>(buf * BN + col0);
 #pragma unroll
-      for (int cc = 0; cc < kCols; cc += 32) {
-        uint32_t raw[32];
-        tmem_ld_32x32(taddr + static_cast<uint32_t>(cc), raw);
+      for (int cc = 0; cc < kCols; cc += 16) {
+        uint32_t raw[16];
+        tmem_ld_32x16(taddr + static_cast<uint32_t>(cc), raw);
         tmem_ld_wait();
 #pragma unroll
-        for (int j = 0; j < 32; ++j) sum[cc + j] += __uint_as_float(raw[j]);
+        for (int j = 0; j < 8; ++j) add_pair(sum[cc / 2 + j], pack_pair(raw[2 * j], raw[2 * j + 1]));
       }
       tc_fence_before_sync();
       __syncwarp();
@@ -846,10 +855,11 @@ gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ 
     {
       const int m_local = quarter * 32 + lane;
 #pragma unroll
-      for (int jx = 0; jx < kCols; ++jx) tile[(col0 + jx) * kTilePitch + m_local] = sum[jx];
+      for (int jx = 0; jx < kCols; ++jx) tile[(col0 + jx) * kTilePitch + m_local] = pair_element(sum[jx / 2], jx & 1);
     }
     asm volatile("bar.sync 1, %0;" ::"r"(kEpiWarps * 32) : "memory");
-    if (ok && m0 < prob.M) run_epilogue<BN, MODE>(prob, tile, m0, n0, ew, lane, 0);
+    if (ok && m0 < prob.M)
+      run_epilogue<BN, MODE, kEpiWarps>(prob, tile, m0, n0, ew, lane, static_cast<int64_t>(blockIdx.y) * prob.split_stride);
   }
 
   tc_fence_before_sync();
@@ -865,9 +875,9 @@ gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ 
 // Host side: tensor maps and launch.
 
 // K-contiguous fp32 matrix [rows][K] with row pitch ld (floats); box = one k-block x box_rows rows.
-CUtensorMap make_operand_map(const float* base, int64_t K, int64_t rows, int64_t ld, int box_rows) {
-  return encode_k_major(CU_TENSOR_MAP_DATA_TYPE_FLOAT32, base, K, rows, 4 * ld, kBK, box_rows,
-                        kRowBytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B);
+CUtensorMap make_operand_map(const float* base, int64_t K, int64_t rows, int64_t ld, int box_rows, int depth = kBK) {
+  return encode_k_major(CU_TENSOR_MAP_DATA_TYPE_FLOAT32, base, K, rows, 4 * ld, depth, box_rows,
+                        depth == 32 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B);
 }
 
 // Interleaved bf16 plane; box = hb and lb of one k-block x box_rows rows.
@@ -875,28 +885,28 @@ CUtensorMap make_bf16_map(const uint16_t* base, int64_t K, int64_t rows, int64_t
   return encode_interleaved(base, K, rows, ld, 2 * kBK, box_rows);
 }
 
-template <int BN, int MODE, bool MIXED>
+template <typename Cfg, int MODE, bool MIXED>
 void launch(const GemmOperands& ops, const GemmProblem& prob, int* status, cudaStream_t stream) {
-  using Cfg = TileConfig<BN>;
+  constexpr int BN = Cfg::BN;
   static PerDeviceOnce configured;
-  allow_dynamic_smem(reinterpret_cast<const void*>(gemm_tf32x3_kernel<BN, MODE, MIXED>), Cfg::kSmemBytes, configured, "gemm_tf32x3");
+  allow_dynamic_smem(reinterpret_cast<const void*>(gemm_tf32x3_kernel<Cfg, MODE, MIXED>), Cfg::kSmemBytes, configured, "gemm_tf32x3");
   GemmMaps maps;
   const int64_t a_k = ops.a_k_total ? ops.a_k_total : prob.K, a_rows = ops.a_rows_total ? ops.a_rows_total : prob.M;
   const int64_t b_k = ops.b_k_total ? ops.b_k_total : prob.K, b_rows = ops.b_rows_total ? ops.b_rows_total : prob.N;
-  maps.a_hi = make_operand_map(ops.a_hi, a_k, a_rows, ops.lda, kBM);
-  maps.b_hi = make_operand_map(ops.b_hi, b_k, b_rows, ops.ldb, BN);
+  maps.a_hi = make_operand_map(ops.a_hi, a_k, a_rows, ops.lda, kBM, Cfg::BK);
+  maps.b_hi = make_operand_map(ops.b_hi, b_k, b_rows, ops.ldb, BN, Cfg::BK);
   if constexpr (MIXED) {
     maps.a_lo = make_bf16_map(ops.a_hl, a_k, a_rows, ops.lda16, kBM);
     maps.b_lo = make_bf16_map(ops.b_hl, b_k, b_rows, ops.ldb16, BN);
   } else {
-    maps.a_lo = make_operand_map(ops.a_lo, a_k, a_rows, ops.lda, kBM);
-    maps.b_lo = make_operand_map(ops.b_lo, b_k, b_rows, ops.ldb, BN);
+    maps.a_lo = make_operand_map(ops.a_lo, a_k, a_rows, ops.lda, kBM, Cfg::BK);
+    maps.b_lo = make_operand_map(ops.b_lo, b_k, b_rows, ops.ldb, BN, Cfg::BK);
   }
   const int tiles_m = (prob.M + kBM - 1) / kBM;
   const int tiles_n = (prob.N + BN - 1) / BN;
   const int splits = (MODE == kEpiStore && prob.k_splits > 1) ? prob.k_splits : 1;
   dim3 grid(tiles_m * tiles_n, splits, prob.batches > 1 ? prob.batches : 1);
-  gemm_tf32x3_kernel<BN, MODE, MIXED><<<grid, kThreads, Cfg::kSmemBytes, stream>>>(maps, prob, status);
+  gemm_tf32x3_kernel<Cfg, MODE, MIXED><<<grid, Cfg::kThreads, Cfg::kSmemBytes, stream>>>(maps, prob, status);
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) throw std::runtime_error(std::string("gemm_tf32x3 launch: ") + cudaGetErrorString(err));
 }
@@ -919,7 +929,8 @@ void launch_pair(const GemmOperands& ops, const GemmProblem& prob, int* status, 
   }
   const int tiles_m = (prob.M + 2 * kBM - 1) / (2 * kBM);
   const int tiles_n = (prob.N + kPairBN - 1) / kPairBN;
-  dim3 grid(2 * tiles_m * tiles_n, 1, 1);
+  const int splits = (MODE == kEpiStore && prob.k_splits > 1) ? prob.k_splits : 1;
+  dim3 grid(2 * tiles_m * tiles_n, splits, 1);
   gemm_pair_kernel<MODE, MIXED><<<grid, kThreads, kPairSmemBytes, stream>>>(maps, prob, status);
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) throw std::runtime_error(std::string("gemm_pair launch: ") + cudaGetErrorString(err));
@@ -939,20 +950,22 @@ void gemm_tf32x3(const GemmOperands& ops, const GemmProblem& prob, int* status, 
     throw std::invalid_argument("gemm_tf32x3: the push epilogue needs a target table and a plain (unsplit, unbatched) product");
   if (prob.K <= 0) throw std::invalid_argument("gemm_tf32x3 needs K >= 1");
   // Wide tiles when there are enough of them to fill the 148 SMs; narrower tiles otherwise.
-  const int64_t wide_tiles = static_cast<int64_t>((prob.M + kBM - 1) / kBM) * ((prob.N + 255) / 256);
-  const bool wide = prob.N > 128 && wide_tiles >= 148 && !prob.force_narrow;
+  const int64_t tile_rows = (prob.M + kBM - 1) / kBM, splits = prob.mode == kEpiStore && prob.k_splits > 1 ? prob.k_splits : 1;
+  const bool wide = prob.N > 128 && tile_rows * ((prob.N + 255) / 256) * splits >= 148 && !prob.force_narrow;
+  const bool crowded = tile_rows * ((prob.N + 127) / 128) * splits * (prob.batches > 1 ? prob.batches : 1) > 148;
   const bool mixed = ops.a_hl && ops.b_hl;
-  if (mixed && kBK != 32) throw std::invalid_argument("gemm_tf32x3: mixed corrections need the 32-element k-block build");
 #define SOAP_GEMM_LAUNCH(MODE_)                                                                      \
   do {                                                                                               \
     if (mixed) {                                                                                     \
-      wide ? launch<256, MODE_, true>(ops, prob, status, stream) : launch<128, MODE_, true>(ops, prob, status, stream);   \
+      wide ? launch<WideTile, MODE_, true>(ops, prob, status, stream) : launch<NarrowTile, MODE_, true>(ops, prob, status, stream);   \
     } else {                                                                                         \
-      wide ? launch<256, MODE_, false>(ops, prob, status, stream) : launch<128, MODE_, false>(ops, prob, status, stream); \
+      if (wide) launch<WideTile, MODE_, false>(ops, prob, status, stream);                             \
+      else if (crowded) launch<CompactTile, MODE_, false>(ops, prob, status, stream);                  \
+      else launch<NarrowTile, MODE_, false>(ops, prob, status, stream);                                \
     }                                                                                                \
   } while (0)
-  // CTA pairs for large plain problems: no batching, no split-K
-  const bool pairs = g_use_pairs && wide && kBK == 32 && prob.M >= 2 * kBM && prob.batches <= 1 && prob.k_splits <= 1 &&
+  // CTA pairs for large plain problems: no batching
+  const bool pairs = g_use_pairs && wide && prob.M >= 2 * kBM && prob.batches <= 1 &&
                      prob.mode != kEpiPairUpdate;
   if (pairs) {
 #define SOAP_PAIR_LAUNCH(MODE_)                                                                                  \
@@ -989,7 +1002,7 @@ void gemm_tf32x3(const GemmOperands& ops, const GemmProblem& prob, int* status, 
       if (prob.N != 128 || prob.remap == nullptr || prob.Chi == nullptr)
         throw std::invalid_argument("gemm_tf32x3: the pair update needs N = 128, a remap table and output planes");
       if (mixed) throw std::invalid_argument("gemm_tf32x3: the pair update takes fp32 planes only");
-      launch<128, kEpiPairUpdate, false>(ops, prob, status, stream);
+      launch<CompactTile, kEpiPairUpdate, false>(ops, prob, status, stream);
       break;
     default:
       throw std::invalid_argument("gemm_tf32x3: unknown epilogue mode");

@@ -44,6 +44,19 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   return done != 0;
 }
 
+// Whether the phase is over, without waiting.
+__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
+  uint32_t done;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.b32 %0, 1, 0, p;\n\t}"
+      : "=r"(done)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return done != 0;
+}
+
 // Wait on an mbarrier phase with an iteration budget.  `abort_flag` lives in shared memory and is
 // polled so that one role's timeout releases the other roles quickly.  Returns false on give-up.
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
@@ -111,20 +124,38 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                : "memory");
 }
-// 32 lanes x 32 columns of fp32 accumulator -> 32 registers per thread (thread t = TMEM lane base+t).
-__device__ __forceinline__ void tmem_ld_32x32(uint32_t taddr, uint32_t (&r)[32]) {
+// 32 lanes x 16 columns of fp32 accumulator -> 16 registers per thread (thread t = TMEM lane base+t).
+__device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-        "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
-        "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(taddr)
       : "memory");
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+
+// Two fp32 values in one register pair, added and multiplied by one instruction, each rounded as fmaf and + round it.
+__device__ __forceinline__ uint64_t pack_pair(uint32_t low, uint32_t high) {
+  uint64_t pair;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(pair) : "r"(low), "r"(high));
+  return pair;
+}
+__device__ __forceinline__ uint64_t pack_floats(float low, float high) {
+  return pack_pair(__float_as_uint(low), __float_as_uint(high));
+}
+__device__ __forceinline__ float pair_element(uint64_t pair, int which) {
+  uint32_t low, high;
+  asm("mov.b64 {%0, %1}, %2;" : "=r"(low), "=r"(high) : "l"(pair));
+  return __uint_as_float(which ? high : low);
+}
+__device__ __forceinline__ void fma_pair(uint64_t& sum, uint64_t a, uint64_t b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(sum) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ void add_pair(uint64_t& sum, uint64_t a) {
+  asm("add.rn.f32x2 %0, %0, %1;" : "+l"(sum) : "l"(a));
+}
 
 // K-major operand tile in shared memory written by a 128-byte-swizzled TMA box whose inner extent
 // is exactly 128 bytes (32 fp32): rows are 128 B apart, 8-row groups 1024 B apart.

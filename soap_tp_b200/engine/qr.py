@@ -96,7 +96,7 @@ def _skinny_product(ws: dict, a: k.Planes, b: k.Planes, out: k.Planes, scratch: 
     ld = M
     partials = ws[scratch]
     view = partials[: ld * N].view(N, ld).T
-    k.gemm(a, b, mode=k.EPI_STORE, out=view, out_ld=ld, force_narrow=True, k_splits=splits, split_stride=ld * N)
+    k.gemm(a, b, mode=k.EPI_STORE, out=view, out_ld=ld, force_narrow=M <= 128, k_splits=splits, split_stride=ld * N)
     _C.sum_partials_to_planes(partials.data_ptr(), splits, ld * N, ld, out.hi.data_ptr(), out.lo.data_ptr(), out.ld,
                               M, N, k._stream())
     k._count("sum_partials_kernel")

@@ -328,3 +328,36 @@ def test_push_epilogue_fills_the_consumers_planes(I, J, nb, grid, K, mixed):
             planes = k.Planes(hi, None, I, len(wanted), ld, low, ld16) if mixed else k.Planes(hi, low, I, len(wanted), ld)
             got = planes.dense().cpu()                            # I x len(wanted)
             assert _rel(got, expected[:, wanted]) < (1e-5 if mixed else 2e-6), (pr, pc)
+
+
+@pytest.mark.parametrize("M,K,splits", [(128, 1000, 1), (128, 1000, 3), (100, 257, 7), (256, 1000, 5), (300, 96, 1)])
+def test_tiles_do_not_change_a_bit(M, K, splits):
+    """Few tiles have an SM each, many share them two by two, and wide ones or CTA pairs take over from there: the same values,
+    whole products and split ones (whose parts are the same groups of 32 of K for every tile)."""
+    from soap_tp_b200.engine import kernels as k
+
+    device, g = torch.device("cuda", 0), torch.Generator(device="cuda").manual_seed(M + K)
+    N = 128 * 200 + 5
+    A, B = (torch.randn(K, n, generator=g, device=device) for n in (M, N))
+    a, b = k.split_planes(A), k.split_planes(B)
+    narrow = k.Planes(b.hi[: 128 * 3], b.lo[: 128 * 3], K, 128 * 3, b.ld)
+    if splits == 1:
+        few, many, wide = (torch.zeros(n, M, device=device).T for n in (128 * 3, N, N))
+        k.gemm(a, narrow, out=few)
+        k.gemm(a, b, out=many, force_narrow=True)
+        k.gemm(a, b, out=wide)
+        assert torch.equal(few, many[:, : 128 * 3]) and torch.equal(many, wide)
+        low, high = k.Planes.empty(M, 128 * 3, device), k.Planes.empty(M, N, device)
+        old = torch.randn(M, N, generator=g, device=device)
+        k.split_planes(old[:, : 128 * 3], out=low)
+        k.split_planes(old, out=high)
+        k.gemm(a, narrow, mode=k.EPI_SPLIT, out_planes=low, alpha=-1.0, beta=1.0)
+        k.gemm(a, b, mode=k.EPI_SPLIT, out_planes=high, alpha=-1.0, beta=1.0, force_narrow=True)
+        assert torch.equal(low.hi[: 128 * 3, :M], high.hi[: 128 * 3, :M]) and torch.equal(low.lo[: 128 * 3, :M], high.lo[: 128 * 3, :M])
+        return
+    parts = [torch.full((splits, n, M), float("nan"), device=device) for n in (128 * 3, N, N)]
+    for operand, part, force in ((narrow, parts[0], True), (b, parts[1], True), (b, parts[2], False)):
+        k.gemm(a, operand, out=part[0].T, out_ld=M, k_splits=splits, split_stride=M * operand.cols, force_narrow=force)
+    assert torch.equal(parts[0], parts[1][:, : 128 * 3]) and torch.equal(parts[1], parts[2])
+    exact = A.double().T @ B.double()
+    assert float((parts[2].double().sum(dim=0).T - exact).norm() / exact.norm()) < 2e-6
