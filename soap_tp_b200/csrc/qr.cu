@@ -367,7 +367,7 @@ void qr_panel(const float* p_hi, const float* p_lo, int64_t ldp, int r, int b, f
   static PerDeviceOnce configured;
   allow_dynamic_smem(reinterpret_cast<const void*>(qr_panel_kernel), smem, configured, "qr_panel");
   PanelArgs args{p_hi, p_lo, ldp, r, b, v_hi, v_lo, ldv, vt_hi, vt_lo, ldvt, tau, t_hi, t_lo, tt_hi, tt_lo, ldt,
-                 reinterpret_cast<unsigned long long*>(exchange), epoch, status, trace, debug_skip};
+                 reinterpret_cast<unsigned long long*>(exchange), epoch, status, trace, 0, debug_skip};
   void* params[] = {&args};
   const int ctas = (r + kRows - 1) / kRows;
   // Cooperative launch: the CTAs exchange data through global memory while running, so all of them

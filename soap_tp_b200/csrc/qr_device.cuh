@@ -52,6 +52,7 @@ struct PanelArgs {
   long long* trace;              // optional diagnostics output, may be null: the pair kernel stores its number of
                                  // exchange steps; the one-column kernel stores clock64 stamps of CTA 0 at column 64
                                  // when it is compiled with SOAP_QR_TRACE
+  int aligned;                   // the pair kernel may read the panel and write V 16 bytes at a time
   int debug_skip;                // SOAP_QR_TRACE builds only: bit 0 skips the T column, bit 1 the pivot-row bookkeeping
 };
 

@@ -29,6 +29,7 @@
 #include <stdexcept>
 #include <string>
 
+#include "ptx.cuh"
 #include "qr.h"
 #include "qr_device.cuh"
 
@@ -67,10 +68,12 @@ __device__ __forceinline__ unsigned long long pack_word(float value, unsigned in
   return (static_cast<unsigned long long>(seq) << 32) | __float_as_uint(value);
 }
 
+// Where a compiler could round once or twice (the sum of two products, a square that is used twice) the operations are spelled
+// out: the sign of a basis's last column hangs on the last bits of what comes before it, and must not change with the code around.
 __device__ __forceinline__ void householder_scalars(float alpha, float normsq, float& tau, float& scale) {
   tau = 0.f;
   scale = 0.f;
-  const float tail = normsq - alpha * alpha;
+  const float tail = __fsub_rn(normsq, __fmul_rn(alpha, alpha));
   if (tail > 0.f && normsq > 0.f) {
     const float beta = -copysignf(sqrtf(normsq), alpha);
     tau = (beta - alpha) * __frcp_rn(beta);
@@ -84,12 +87,12 @@ __device__ __forceinline__ void householder_scalars(float alpha, float normsq, f
 template <int kPer>
 __global__ void __launch_bounds__(kPanelThreads, 1) qr_panel_pairs_kernel(PanelArgs a) {
   constexpr int kCtaRows = 4 * kPer;
-  constexpr int kSlice = kPer + 4;     // floats between the four slices of a pivot column in shared memory
   constexpr int kVec = kPer / 4;       // 128-bit loads per sweep and pivot column
   constexpr int kPollPairs = kPer == 64 ? 7 : 17;   // 128-bit loads a thread keeps in flight per polling round
-  __shared__ __align__(16) float xcol[2][4 * kSlice];   // pivot column c (double buffered); zero above the pivot row
-  __shared__ __align__(16) float ycol[2][4 * kSlice];   // column c + 1 as it is before H_c is applied
-  __shared__ float stats[2][8];                         // {p1_c, D1_c, p2_c, -, p1_c1, D1_c1, p2_c1, D2_c1}
+  __shared__ __align__(16) float xcol[2][kCtaRows];     // pivot column c (double buffered); zero above the pivot row
+  __shared__ __align__(16) float ycol[2][kCtaRows];     // column c + 1 as it is before H_c is applied
+  __shared__ float2 slices[4][kB];                      // dot products of the four row slices with every column
+  __shared__ float4 sums[kB];                           // {D1_j, D2_j, p1_j, p2_j}, the same in every CTA
   __shared__ float taus[kB];
   __shared__ float scol1[kB];                           // column c of S = V^T V (entries above the diagonal)
   __shared__ float scol2[kB];                           // column c + 1 of S
@@ -97,11 +100,14 @@ __global__ void __launch_bounds__(kPanelThreads, 1) qr_panel_pairs_kernel(PanelA
   __shared__ float row2_local[kB];
   __shared__ int abort_flag;
   extern __shared__ float dyn[];
-  float (*T)[kPitch] = reinterpret_cast<float (*)[kPitch]>(dyn);   // CTA 0: compact-WY factor; all: output staging
+  float (*T)[kPitch] = reinterpret_cast<float (*)[kPitch]>(dyn);   // last CTA: compact-WY factor
 
   const int t = threadIdx.x;
-  const int j = t >> 2;                  // column owned by this lane quad
-  const int q = t & 3;                   // 64-row slice within the CTA's slab
+  // A warp owns one slice of 32 columns, so that a sweep's loads of a pivot column are one address for all its lanes.  The
+  // exchange is carried out by lane quads, one per column.
+  const int j = ((t >> 7) << 5) | (t & 31);
+  const int q = (t >> 5) & 3;            // kPer-row slice within the CTA's slab
+  const int jx = t >> 2, qx = t & 3;     // column and part of its exchange
   const int row0 = blockIdx.x * kCtaRows;
   const int rows_here = min(kCtaRows, a.r - row0);
   const int ctas = gridDim.x;
@@ -113,22 +119,28 @@ __global__ void __launch_bounds__(kPanelThreads, 1) qr_panel_pairs_kernel(PanelA
   const bool has_rows = rows_here > 0;
 
   float P[kPer];
+  {
+    const int64_t off = row0 + my_first + static_cast<int64_t>(j) * a.ldp;
+    if (a.aligned && my_first + kPer <= rows_here && j < a.b) {
 #pragma unroll
-  for (int k = 0; k < kPer; ++k) {
-    const int i = my_first + k;
-    float v = 0.f;
-    if (i < rows_here && j < a.b) {
-      const int64_t off = (row0 + i) + static_cast<int64_t>(j) * a.ldp;
-      v = a.p_hi[off] + a.p_lo[off];
+      for (int k = 0; k < kPer; k += 4) {
+        const float4 h = *reinterpret_cast<const float4*>(a.p_hi + off + k), l = *reinterpret_cast<const float4*>(a.p_lo + off + k);
+        P[k] = h.x + l.x;
+        P[k + 1] = h.y + l.y;
+        P[k + 2] = h.z + l.z;
+        P[k + 3] = h.w + l.w;
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < kPer; ++k) P[k] = (my_first + k < rows_here && j < a.b) ? a.p_hi[off + k] + a.p_lo[off + k] : 0.f;
     }
-    P[k] = v;
   }
   if (t < kB) taus[t] = 0.f;
   if (t == 0) abort_flag = 0;
   if (builds_t)
     for (int idx = t; idx < kB * kPitch; idx += kPanelThreads) dyn[idx] = 0.f;
   if (j < 2) {
-    float* dst = (j == 0) ? &xcol[0][q * kSlice] : &ycol[0][q * kSlice];
+    float* dst = (j == 0) ? &xcol[0][my_first] : &ycol[0][my_first];
 #pragma unroll
     for (int k = 0; k < kPer; ++k) dst[k] = P[k];
   }
@@ -151,49 +163,48 @@ __global__ void __launch_bounds__(kPanelThreads, 1) qr_panel_pairs_kernel(PanelA
     const bool mine1 = local1 >= 0 && local1 < kPer;
     const bool mine2 = local2 >= 0 && local2 < kPer && row2_exists;
 
-    // ---- sweep 1: dot products of both pivot columns with this lane's slice of column j ----
-    float partial1 = 0.f, partial2 = 0.f;
+    // ---- sweep 1: dot products of both pivot columns with this thread's slice of column j ----
     if (has_rows) {
-      float x0 = 0.f, x1 = 0.f, x2 = 0.f, x3 = 0.f, y0 = 0.f, y1 = 0.f, y2 = 0.f, y3 = 0.f;
-      const float4* x4 = reinterpret_cast<const float4*>(&xcol[parity][q * kSlice]);
-      const float4* y4 = reinterpret_cast<const float4*>(&ycol[parity][q * kSlice]);
+      uint64_t x01 = 0, x23 = 0, y01 = 0, y23 = 0;
+      const ulonglong2* x4 = reinterpret_cast<const ulonglong2*>(&xcol[parity][my_first]);
+      const ulonglong2* y4 = reinterpret_cast<const ulonglong2*>(&ycol[parity][my_first]);
 #pragma unroll
       for (int k4 = 0; k4 < kVec; ++k4) {
-        const float4 x = x4[k4];
-        const float4 y = y4[k4];
-        x0 = fmaf(P[4 * k4 + 0], x.x, x0);
-        x1 = fmaf(P[4 * k4 + 1], x.y, x1);
-        x2 = fmaf(P[4 * k4 + 2], x.z, x2);
-        x3 = fmaf(P[4 * k4 + 3], x.w, x3);
-        y0 = fmaf(P[4 * k4 + 0], y.x, y0);
-        y1 = fmaf(P[4 * k4 + 1], y.y, y1);
-        y2 = fmaf(P[4 * k4 + 2], y.z, y2);
-        y3 = fmaf(P[4 * k4 + 3], y.w, y3);
+        const ulonglong2 x = x4[k4];
+        const ulonglong2 y = y4[k4];
+        const uint64_t low = pack_floats(P[4 * k4], P[4 * k4 + 1]), high = pack_floats(P[4 * k4 + 2], P[4 * k4 + 3]);
+        fma_pair(x01, low, x.x);
+        fma_pair(x23, high, x.y);
+        fma_pair(y01, low, y.x);
+        fma_pair(y23, high, y.y);
       }
-      partial1 = (x0 + x1) + (x2 + x3);
-      partial2 = (y0 + y1) + (y2 + y3);
+      slices[q][j] = make_float2((pair_element(x01, 0) + pair_element(x01, 1)) + (pair_element(x23, 0) + pair_element(x23, 1)),
+                                 (pair_element(y01, 0) + pair_element(y01, 1)) + (pair_element(y23, 0) + pair_element(y23, 1)));
     }
-    partial1 += __shfl_xor_sync(0xffffffffu, partial1, 1);
-    partial1 += __shfl_xor_sync(0xffffffffu, partial1, 2);
-    partial2 += __shfl_xor_sync(0xffffffffu, partial2, 1);
-    partial2 += __shfl_xor_sync(0xffffffffu, partial2, 2);   // all four lanes: this CTA's partial dots for column j
-    float row1 = 0.f, row2 = 0.f;                             // entries (c, j) and (c + 1, j), on the lanes that hold them
-    if (mine1) row1 = take_entry<kPer>(P, local1, false);
-    if (mine2) row2 = take_entry<kPer>(P, local2, false);
-    if (ctas > 1) {
-      if (q == 0) {
-        unsigned long long* mine = &slots[(static_cast<int64_t>(blockIdx.x) * kB + j) * 2];
-        asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(mine), "l"(pack_word(partial1, seq)),
-                     "l"(pack_word(partial2, seq))
-                     : "memory");
-      }
-      unsigned long long* rows = &slots[(static_cast<int64_t>(ctas) * kB + j) * 2];
-      if (mine1) ll_publish(rows, row1, seq);
-      if (mine2) ll_publish(rows + 1, row2, seq);
-    } else {
-      if (mine1) row1_local[j] = row1;
-      if (mine2) row2_local[j] = row2;
-      if (!row2_exists && q == 0) row2_local[j] = 0.f;
+    // entries (c, j) and (c + 1, j), on the warps that hold them
+    unsigned long long* rows = &slots[(static_cast<int64_t>(ctas) * kB + j) * 2];
+    if (mine1) {
+      const float entry = take_entry<kPer>(P, local1, false);
+      if (ctas > 1) ll_publish(rows, entry, seq);
+      else row1_local[j] = entry;
+    }
+    if (mine2) {
+      const float entry = take_entry<kPer>(P, local2, false);
+      if (ctas > 1) ll_publish(rows + 1, entry, seq);
+      else row2_local[j] = entry;
+    }
+    if (ctas == 1 && !row2_exists && q == 0) row2_local[j] = 0.f;
+    __syncthreads();                                                              // barrier 1
+    float partial1 = 0.f, partial2 = 0.f;                     // this CTA's dot products with column jx
+    if (qx == 0 && has_rows) {
+      partial1 = (slices[0][jx].x + slices[1][jx].x) + (slices[2][jx].x + slices[3][jx].x);
+      partial2 = (slices[0][jx].y + slices[1][jx].y) + (slices[2][jx].y + slices[3][jx].y);
+    }
+    if (qx == 0 && ctas > 1) {
+      unsigned long long* mine = &slots[(static_cast<int64_t>(blockIdx.x) * kB + jx) * 2];
+      asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(mine), "l"(pack_word(partial1, seq)),
+                   "l"(pack_word(partial2, seq))
+                   : "memory");
     }
 
     // ---- CTA 0, while the published words travel: the columns of T the previous step produced ----
@@ -205,9 +216,9 @@ __global__ void __launch_bounds__(kPanelThreads, 1) qr_panel_pairs_kernel(PanelA
       }
     }
 
-    // ---- exchange: lane q polls CTAs q, q+4, q+8, ... (index `ctas` holds the two pivot rows) ----
-    float total1 = partial1, total2 = partial2, p1 = 0.f, p2 = 0.f;
+    // ---- exchange: lane qx polls CTAs qx, qx + 4, qx + 8, ... (index `ctas` holds the two pivot rows) ----
     if (ctas > 1) {
+      float total1 = 0.f, total2 = 0.f, p1 = 0.f, p2 = 0.f;
       float part1 = 0.f, part2 = 0.f;
       bool failed = false;
       for (int base = 0; base <= ctas && !failed; base += 4 * kPollPairs) {
@@ -218,16 +229,16 @@ __global__ void __launch_bounds__(kPanelThreads, 1) qr_panel_pairs_kernel(PanelA
           pending = false;
 #pragma unroll
           for (int u = 0; u < kPollPairs; ++u) {
-            const int g = base + q + 4 * u;
+            const int g = base + qx + 4 * u;
             if (g <= ctas)
               asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];"
                            : "=l"(w1[u]), "=l"(w2[u])
-                           : "l"(&slots[(static_cast<int64_t>(g) * kB + j) * 2])
+                           : "l"(&slots[(static_cast<int64_t>(g) * kB + jx) * 2])
                            : "memory");
           }
 #pragma unroll
           for (int u = 0; u < kPollPairs; ++u) {
-            const int g = base + q + 4 * u;
+            const int g = base + qx + 4 * u;
             if (g <= ctas) {
               if (static_cast<unsigned int>(w1[u] >> 32) != seq) pending = true;
               if (static_cast<unsigned int>(w2[u] >> 32) != seq && (g < ctas || row2_exists)) pending = true;
@@ -238,7 +249,7 @@ __global__ void __launch_bounds__(kPanelThreads, 1) qr_panel_pairs_kernel(PanelA
         failed = pending;
 #pragma unroll
         for (int u = 0; u < kPollPairs; ++u) {
-          const int g = base + q + 4 * u;
+          const int g = base + qx + 4 * u;
           if (g < ctas) {
             part1 += __uint_as_float(static_cast<unsigned int>(w1[u]));
             part2 += __uint_as_float(static_cast<unsigned int>(w2[u]));
@@ -254,49 +265,40 @@ __global__ void __launch_bounds__(kPanelThreads, 1) qr_panel_pairs_kernel(PanelA
       }
       // fixed-shape reductions over the four lanes: identical on every CTA
       float o = __shfl_xor_sync(0xffffffffu, part1, 1);
-      float pair_sum = (q & 1) ? (o + part1) : (part1 + o);
+      float pair_sum = (qx & 1) ? (o + part1) : (part1 + o);
       o = __shfl_xor_sync(0xffffffffu, pair_sum, 2);
-      total1 = (q & 2) ? (o + pair_sum) : (pair_sum + o);
+      total1 = (qx & 2) ? (o + pair_sum) : (pair_sum + o);
       o = __shfl_xor_sync(0xffffffffu, part2, 1);
-      pair_sum = (q & 1) ? (o + part2) : (part2 + o);
+      pair_sum = (qx & 1) ? (o + part2) : (part2 + o);
       o = __shfl_xor_sync(0xffffffffu, pair_sum, 2);
-      total2 = (q & 2) ? (o + pair_sum) : (pair_sum + o);
+      total2 = (qx & 2) ? (o + pair_sum) : (pair_sum + o);
       p1 += __shfl_xor_sync(0xffffffffu, p1, 1);
       p1 += __shfl_xor_sync(0xffffffffu, p1, 2);              // exactly one lane held the pivot-row words
       p2 += __shfl_xor_sync(0xffffffffu, p2, 1);
       p2 += __shfl_xor_sync(0xffffffffu, p2, 2);
+      if (qx == 0) sums[jx] = make_float4(total1, total2, p1, p2);
+    } else if (qx == 0) {
+      sums[jx] = make_float4(partial1, partial2, row1_local[jx], row2_local[jx]);
     }
-    if (q == 0 && j == c) {
-      stats[parity][0] = p1;
-      stats[parity][1] = total1;
-      stats[parity][2] = p2;
-    }
-    if (q == 0 && j == c + 1) {
-      stats[parity][4] = p1;
-      stats[parity][5] = total1;
-      stats[parity][6] = p2;
-      stats[parity][7] = total2;
-    }
-    __syncthreads();                                                              // barrier 1
+    __syncthreads();                                                              // barrier 2
     if (abort_flag) break;
-    if (ctas == 1) {
-      p1 = row1_local[j];
-      p2 = row2_local[j];
-    }
 
     // ---- scalars of the step (every thread computes the same values) ----
-    const float a1 = (ctas == 1) ? row1_local[c] : stats[parity][0];
-    const float n1 = stats[parity][1];
-    const float p2c = (ctas == 1) ? row2_local[c] : stats[parity][2];
+    const float4 own = sums[j], first = sums[c];
+    const float total1 = own.x, total2 = own.y, p1 = own.z, p2 = own.w;
+    const float a1 = first.z;
+    const float n1 = first.x;
+    const float p2c = first.w;
     float t1, s1;
     householder_scalars(a1, n1, t1, s1);
     bool pair = false;
     float k = 0.f, yc = 0.f, yc1 = 0.f, t2 = 0.f, s2 = 0.f, p1c1 = 0.f, p2c1 = 0.f, d1c1 = 0.f;
     if (can_pair) {
-      p1c1 = (ctas == 1) ? row1_local[c + 1] : stats[parity][4];
-      d1c1 = stats[parity][5];
-      p2c1 = (ctas == 1) ? row2_local[c + 1] : stats[parity][6];
-      const float d2c1 = stats[parity][7];
+      const float4 second = sums[c + 1];
+      p1c1 = second.z;
+      d1c1 = second.x;
+      p2c1 = second.w;
+      const float d2c1 = second.y;
       const float w1c1 = p1c1 + s1 * (d1c1 - a1 * p1c1);       // v_c . y
       k = t1 * w1c1;
       yc = p1c1 - k;
@@ -307,7 +309,7 @@ __global__ void __launch_bounds__(kPanelThreads, 1) qr_panel_pairs_kernel(PanelA
         householder_scalars(yc1, n2, t2, s2);
       }
     }
-    // ---- this lane's column ----
+    // ---- this thread's column ----
     const float sj = (j < c) ? my_scale : 1.f;                  // finished columns are kept unscaled in the registers
     const float w1 = (p1 + s1 * (total1 - a1 * p1)) * sj;       // v_c . column_j
     float w2 = 0.f;
@@ -321,8 +323,9 @@ __global__ void __launch_bounds__(kPanelThreads, 1) qr_panel_pairs_kernel(PanelA
         const float sum_x = total1 - a1 * p1 - p2c * p2;
         w2 = (p2 + s2 * (sum_y - k * s1 * sum_x)) * sj;
       } else if (j == c) {                                      // v_c . v_{c+1}
-        const float sxy = (d1c1 - a1 * p1c1 - p2c * p2c1) - k * s1 * (n1 - a1 * a1 - p2c * p2c);
-        w2 = s1 * p2c + s1 * s2 * sxy;
+        const float tail_x = fmaf(-p2c, p2c, __fsub_rn(n1, __fmul_rn(a1, a1)));
+        const float sxy = fmaf(-__fmul_rn(k, s1), tail_x, fmaf(-p2c, p2c1, fmaf(-a1, p1c1, d1c1)));
+        w2 = fmaf(s1, p2c, __fmul_rn(__fmul_rn(s1, s2), sxy));
       }
     }
     if (j == c) my_scale = s1;
@@ -348,27 +351,36 @@ __global__ void __launch_bounds__(kPanelThreads, 1) qr_panel_pairs_kernel(PanelA
     if (j > c && has_rows) {
       float B = 0.f;
       if (pair && j > c + 1) B = t2 * w2 * s2;
-      const float A = t1 * w1 * s1 - B * k * s1;               // column c + 1 of a pair: y' = y - k s_c x (unscaled v)
-      const float4* x4 = reinterpret_cast<const float4*>(&xcol[parity][q * kSlice]);
+      const float A = fmaf(__fmul_rn(t1, w1), s1, -__fmul_rn(__fmul_rn(B, k), s1));               // column c + 1 of a pair: y' = y - k s_c x (unscaled v)
+      const ulonglong2* x4 = reinterpret_cast<const ulonglong2*>(&xcol[parity][my_first]);
+      const uint64_t minus_a = pack_floats(-A, -A), minus_b = pack_floats(-B, -B);
       if (pair) {
-        const float4* y4 = reinterpret_cast<const float4*>(&ycol[parity][q * kSlice]);
+        const ulonglong2* y4 = reinterpret_cast<const ulonglong2*>(&ycol[parity][my_first]);
 #pragma unroll
         for (int k4 = 0; k4 < kVec; ++k4) {
-          const float4 x = x4[k4];
-          const float4 y = y4[k4];
-          P[4 * k4 + 0] = fmaf(-B, y.x, fmaf(-A, x.x, P[4 * k4 + 0]));
-          P[4 * k4 + 1] = fmaf(-B, y.y, fmaf(-A, x.y, P[4 * k4 + 1]));
-          P[4 * k4 + 2] = fmaf(-B, y.z, fmaf(-A, x.z, P[4 * k4 + 2]));
-          P[4 * k4 + 3] = fmaf(-B, y.w, fmaf(-A, x.w, P[4 * k4 + 3]));
+          const ulonglong2 x = x4[k4];
+          const ulonglong2 y = y4[k4];
+          uint64_t low = pack_floats(P[4 * k4], P[4 * k4 + 1]), high = pack_floats(P[4 * k4 + 2], P[4 * k4 + 3]);
+          fma_pair(low, minus_a, x.x);
+          fma_pair(high, minus_a, x.y);
+          fma_pair(low, minus_b, y.x);
+          fma_pair(high, minus_b, y.y);
+          P[4 * k4] = pair_element(low, 0);
+          P[4 * k4 + 1] = pair_element(low, 1);
+          P[4 * k4 + 2] = pair_element(high, 0);
+          P[4 * k4 + 3] = pair_element(high, 1);
         }
       } else if (A != 0.f) {
 #pragma unroll
         for (int k4 = 0; k4 < kVec; ++k4) {
-          const float4 x = x4[k4];
-          P[4 * k4 + 0] = fmaf(-A, x.x, P[4 * k4 + 0]);
-          P[4 * k4 + 1] = fmaf(-A, x.y, P[4 * k4 + 1]);
-          P[4 * k4 + 2] = fmaf(-A, x.z, P[4 * k4 + 2]);
-          P[4 * k4 + 3] = fmaf(-A, x.w, P[4 * k4 + 3]);
+          const ulonglong2 x = x4[k4];
+          uint64_t low = pack_floats(P[4 * k4], P[4 * k4 + 1]), high = pack_floats(P[4 * k4 + 2], P[4 * k4 + 3]);
+          fma_pair(low, minus_a, x.x);
+          fma_pair(high, minus_a, x.y);
+          P[4 * k4] = pair_element(low, 0);
+          P[4 * k4 + 1] = pair_element(low, 1);
+          P[4 * k4 + 2] = pair_element(high, 0);
+          P[4 * k4 + 3] = pair_element(high, 1);
         }
       }
       // The pivot rows right of the pivots now hold R entries nobody reads again: zero them so that later
@@ -376,13 +388,13 @@ __global__ void __launch_bounds__(kPanelThreads, 1) qr_panel_pairs_kernel(PanelA
       if (mine1) take_entry<kPer>(P, local1, true);
       if (pair && mine2) take_entry<kPer>(P, local2, true);
       if (j == next || j == next + 1) {
-        float* dst = (j == next) ? &xcol[parity ^ 1][q * kSlice] : &ycol[parity ^ 1][q * kSlice];
+        float* dst = (j == next) ? &xcol[parity ^ 1][my_first] : &ycol[parity ^ 1][my_first];
         float4* d4 = reinterpret_cast<float4*>(dst);
 #pragma unroll
         for (int k4 = 0; k4 < kVec; ++k4) d4[k4] = make_float4(P[4 * k4], P[4 * k4 + 1], P[4 * k4 + 2], P[4 * k4 + 3]);
       }
     }
-    __syncthreads();                                                              // barrier 2
+    __syncthreads();                                                              // barrier 3
     built_c = c;
     built_pair = pair ? 1 : 0;
     c = next;
@@ -417,44 +429,37 @@ __global__ void __launch_bounds__(kPanelThreads, 1) qr_panel_pairs_kernel(PanelA
     __syncthreads();
   }
 
-  // ---- outputs: V (r x b) and V^T (b x r) through a shared-memory tile, 64 rows at a time ----
-  const float out_scale = (j < reflectors) ? my_scale : 0.f;
+  // ---- outputs: V (r x b) and V^T (b x r), from the registers: 16 bytes a thread along V's columns, and along the rows of V^T
+  // (lanes are neighbouring columns) 128 bytes a warp ----
+  if (j < a.b) {
+    const float out_scale = (j < reflectors) ? my_scale : 0.f;
 #pragma unroll
-  for (int k = 0; k < kPer; ++k) {
-    const int gi = row0 + my_first + k;
-    float v = 0.f;
-    if (j < reflectors) v = (gi > j) ? P[k] * out_scale : (gi == j ? 1.f : 0.f);
-    P[k] = v;
-  }
-  float (*stage)[kPitch] = T;   // 64 x 129 staging tile (T has been written out)
-  constexpr int kLanesPerTile = 64 / kPer;    // quad lanes whose slices make up one 64-row tile
-  for (int tile = 0; tile < kCtaRows / 64; ++tile) {
-    __syncthreads();
-    if (q / kLanesPerTile == tile) {
+    for (int k = 0; k < kPer; k += 4) {
+      float v[4], h[4];
 #pragma unroll
-      for (int k = 0; k < kPer; ++k) stage[(q % kLanesPerTile) * kPer + k][j] = P[k];
-    }
-    __syncthreads();
-    for (int idx = t; idx < 64 * kB; idx += kPanelThreads) {
-      const int k = idx & 63, jj = idx >> 6;             // consecutive threads -> consecutive rows (V)
-      const int i = tile * 64 + k;
-      if (i < rows_here && jj < a.b) {
-        const float v = stage[k][jj];
-        const float h = tf32_rn(v);
-        const int64_t off = (row0 + i) + static_cast<int64_t>(jj) * a.ldv;
-        a.v_hi[off] = h;
-        a.v_lo[off] = v - h;
+      for (int u = 0; u < 4; ++u) {
+        const int gi = row0 + my_first + k + u;
+        v[u] = (j < reflectors) ? ((gi > j) ? P[k + u] * out_scale : (gi == j ? 1.f : 0.f)) : 0.f;
+        h[u] = tf32_rn(v[u]);
+        v[u] -= h[u];
+        if (my_first + k + u < rows_here) {
+          const int64_t off = j + static_cast<int64_t>(gi) * a.ldvt;
+          a.vt_hi[off] = h[u];
+          a.vt_lo[off] = v[u];
+        }
       }
-    }
-    for (int idx = t; idx < 64 * kB; idx += kPanelThreads) {
-      const int jj = idx & (kB - 1), k = idx >> 7;       // consecutive threads -> consecutive columns (V^T)
-      const int i = tile * 64 + k;
-      if (i < rows_here && jj < a.b) {
-        const float v = stage[k][jj];
-        const float h = tf32_rn(v);
-        const int64_t off = jj + static_cast<int64_t>(row0 + i) * a.ldvt;
-        a.vt_hi[off] = h;
-        a.vt_lo[off] = v - h;
+      const int64_t off = row0 + my_first + k + static_cast<int64_t>(j) * a.ldv;
+      if (a.aligned && my_first + k + 4 <= rows_here) {
+        *reinterpret_cast<float4*>(a.v_hi + off) = make_float4(h[0], h[1], h[2], h[3]);
+        *reinterpret_cast<float4*>(a.v_lo + off) = make_float4(v[0], v[1], v[2], v[3]);
+      } else {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          if (my_first + k + u < rows_here) {
+            a.v_hi[off + u] = h[u];
+            a.v_lo[off + u] = v[u];
+          }
+        }
       }
     }
   }
@@ -491,8 +496,10 @@ void qr_panel_pairs(const float* p_hi, const float* p_lo, int64_t ldp, int r, in
   if (rows_per_cta != 128 && rows_per_cta != 256) throw std::invalid_argument("qr_panel_pairs: rows_per_cta is 128 or 256");
   if (rows_per_cta == 128 && r > 148 * 128) rows_per_cta = 256;   // one CTA per SM at most
   const unsigned int epoch = next_panel_epoch();
+  const bool aligned = ((reinterpret_cast<uintptr_t>(p_hi) | reinterpret_cast<uintptr_t>(p_lo) | reinterpret_cast<uintptr_t>(v_hi) |
+                         reinterpret_cast<uintptr_t>(v_lo)) & 15) == 0 && ldp % 4 == 0 && ldv % 4 == 0;
   PanelArgs args{p_hi, p_lo, ldp, r, b, v_hi, v_lo, ldv, vt_hi, vt_lo, ldvt, tau, t_hi, t_lo, tt_hi, tt_lo, ldt,
-                 reinterpret_cast<unsigned long long*>(exchange), epoch, status, steps_taken, 0};
+                 reinterpret_cast<unsigned long long*>(exchange), epoch, status, steps_taken, aligned, 0};
   if (rows_per_cta == 128) launch_pairs<32>(args, r, stream);
   else launch_pairs<64>(args, r, stream);
 }
