@@ -7,6 +7,7 @@
 #include <pybind11/pybind11.h>
 #include <pybind11/stl.h>
 
+#include <array>
 #include <cstdint>
 #include <stdexcept>
 #include <tuple>
@@ -126,6 +127,25 @@ struct RotationScratch {
   }
 };
 
+namespace {
+// An ordinary step's operands, results and scalars (beta, beta1, beta2, eps, 1 / bias 1, 1 / sqrt(bias 2)).
+SteadyStep step_of(const RotationScratch& scratch, Arguments& in, const std::array<double, 6>& scalars) {
+  SteadyStep s{};
+  s.rotation = scratch.of(in);
+  s.update = scratch.update;
+  s.mixed_update = scratch.mixed_update;
+  s.momentum = in.pointer<float>(); s.ldm = in.next();
+  s.variance = in.pointer<float>(); s.ldv = in.next();
+  s.out = in.pointer<float>();
+  s.left_gram = in.pointer<float>(); s.ld_left = in.next();
+  s.right_gram = in.pointer<float>(); s.ld_right = in.next();
+  s.beta = scalars[0];
+  s.beta1 = static_cast<float>(scalars[1]); s.beta2 = static_cast<float>(scalars[2]); s.eps = static_cast<float>(scalars[3]);
+  s.inv_bc1 = static_cast<float>(scalars[4]); s.inv_sqrt_bc2 = static_cast<float>(scalars[5]);
+  return s;
+}
+}  // namespace
+
 PYBIND11_MODULE(_C, m) {
   m.doc() = "sm_100a kernels of soap_tp_b200";
   m.def("compiled_gpu_backend", [] { return "cuda"; });
@@ -225,29 +245,34 @@ PYBIND11_MODULE(_C, m) {
 
   py::class_<RotationScratch>(m, "RotationScratch", "Scratch planes of rotations of one shape, as addresses (see Arguments)")
       .def(py::init<int, int, const std::vector<int64_t>&>());
-  // Integers: the matrix and its bases (RotationScratch::of), the moments, results and phases in the order of SteadyStep, then the status
-  // word, the stream and the stream of the averages.
-  m.def("steady_step", [](const RotationScratch& scratch, const std::vector<int64_t>& v, double beta, float beta1, float beta2,
-                          float eps, float inv_bc1, float inv_sqrt_bc2) {
+  // Integers: the matrix and its bases (RotationScratch::of), the moments and results in the order of SteadyStep; then of the call: the
+  // phases, the status word, the stream and the stream of the averages.
+  m.def("steady_step", [](const RotationScratch& scratch, const std::vector<int64_t>& v, const std::array<double, 6>& scalars, int phases,
+                          uint64_t status, uint64_t stream, uint64_t side) {
     Arguments in(v);
-    SteadyStep s{};
-    s.rotation = scratch.of(in);
-    s.update = scratch.update;
-    s.mixed_update = scratch.mixed_update;
-    s.momentum = in.pointer<float>(); s.ldm = in.next();
-    s.variance = in.pointer<float>(); s.ldv = in.next();
-    s.out = in.pointer<float>();
-    s.left_gram = in.pointer<float>(); s.ld_left = in.next();
-    s.right_gram = in.pointer<float>(); s.ld_right = in.next();
-    s.phases = static_cast<int>(in.next());
-    int* status = in.pointer<int>();
-    cudaStream_t stream = in.stream();
-    s.side = in.stream();
+    SteadyStep s = step_of(scratch, in, scalars);
     in.finish();
-    s.beta = beta; s.beta1 = beta1; s.beta2 = beta2; s.eps = eps; s.inv_bc1 = inv_bc1; s.inv_sqrt_bc2 = inv_sqrt_bc2;
+    s.phases = phases;
+    s.side = stream_of(side);
     py::gil_scoped_release release;
-    steady_step(s, status, stream);
+    steady_step(s, ptr<int>(status), stream_of(stream));
   }, "The launches of one ordinary single-GPU step, or some of its phases (gemm_half.h, SteadyStep)");
+  m.def("steady_step_shares", &steady_step_shares, "Whether steps of such matrices can share launches");
+  m.attr("STEP_GROUP") = kHalfGroup;
+  m.def("steady_steps", [](const std::vector<std::tuple<const RotationScratch*, std::vector<int64_t>, std::array<double, 6>>>& steps,
+                           uint64_t status, uint64_t stream, uint64_t side) {
+    std::vector<SteadyStep> all;
+    for (const auto& [scratch, v, scalars] : steps) {
+      if (!scratch) throw std::invalid_argument("steady_steps: no scratch");
+      Arguments in(v);
+      all.push_back(step_of(*scratch, in, scalars));
+      in.finish();
+      all.back().phases = kStepPlanes | kStepForward | kStepBackward | kStepAverages;
+      all.back().side = stream_of(side);
+    }
+    py::gil_scoped_release release;
+    steady_steps(all.data(), static_cast<int>(all.size()), ptr<int>(status), stream_of(stream));
+  }, "Ordinary steps of several small parameters in shared launches");
   m.attr("STEP_PLANES") = kStepPlanes;
   m.attr("STEP_FORWARD") = kStepForward;
   m.attr("STEP_BACKWARD") = kStepBackward;
@@ -302,8 +327,11 @@ PYBIND11_MODULE(_C, m) {
                        stream_of(stream));
         });
 
-  m.def("apply_update", [](uint64_t p, int type, uint64_t update, int64_t n, float keep, float lr, uint64_t stream) {
-    apply_update(ptr<void>(p), type, ptr<const float>(update), n, keep, lr, stream_of(stream));
+  // (parameter, update, elements) each
+  m.def("apply_updates", [](const std::vector<std::tuple<uint64_t, uint64_t, int64_t>>& all, int type, float keep, float lr, uint64_t stream) {
+    std::vector<UpdateJob> jobs;
+    for (const auto& [p, update, n] : all) jobs.push_back(UpdateJob{ptr<void>(p), ptr<const float>(update), n});
+    apply_updates(jobs.data(), static_cast<int>(jobs.size()), type, keep, lr, stream_of(stream));
   });
   m.def("adamw_update", [](uint64_t p, int type, uint64_t gradient, uint64_t mo, uint64_t v, int64_t n, float beta1_rest,
                            float beta2, float beta2_rest, float bias1, float bias2, float eps, float keep, float lr,

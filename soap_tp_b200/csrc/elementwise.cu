@@ -1,5 +1,6 @@
 // Memory-bound kernels of the SOAP pipeline: fused Adam, the 3xTF32 operand split (optionally
 // transposing), column dot products for the eigenvalue estimates, and index-mapped gathers.
+#include <algorithm>
 #include <stdexcept>
 #include <string>
 #include <type_traits>
@@ -81,15 +82,27 @@ __device__ __forceinline__ T updated(T p, float update, float keep, float lr) {
   return round_to<T>(fmaf(-lr, to_float(round_to<T>(update)), to_float(kept)));
 }
 
-// 16 bytes of update per thread and step where everything is aligned (`quads`); the rest one by one.
-template <typename T>
-__global__ void __launch_bounds__(256) apply_update_kernel(T* __restrict__ p, const float* __restrict__ update, int64_t n,
-                                                          int64_t quads, float keep, float lr) {
+// Several parameters in one launch, so that those of small matrices do not each wait for the one before.
+constexpr int kUpdateGroup = 16;
+template <int N>
+struct UpdateGroup {
+  UpdateJob jobs[N];
+  int64_t quads[N];              // leading elements that are aligned to be taken four at a time, in fours
+  GroupBlocks<N> blocks;
+};
+
+// 16 bytes of update per thread and step where everything is aligned; the rest one by one.
+template <typename T, int N>
+__global__ void __launch_bounds__(256) apply_updates_kernel(const __grid_constant__ UpdateGroup<N> group, float keep, float lr) {
   struct alignas(4 * sizeof(T)) Four {
     T x[4];
   };
-  const int64_t first = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
+  const int member = group.blocks.member(blockIdx.x), block = blockIdx.x - group.blocks.first(member);
+  T* __restrict__ p = static_cast<T*>(group.jobs[member].p);
+  const float* __restrict__ update = group.jobs[member].update;
+  const int64_t n = group.jobs[member].n, quads = group.quads[member];
+  const int64_t first = block * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+  const int64_t stride = static_cast<int64_t>(group.blocks.count(member)) * blockDim.x;
   for (int64_t i = first; i < quads; i += stride) {
     Four mine = reinterpret_cast<Four*>(p)[i];
     const float4 u = reinterpret_cast<const float4*>(update)[i];
@@ -248,17 +261,49 @@ void adam_update(const float* g, int64_t ldg, float* m, int64_t ldm, float* v, i
   check_launch("adam_kernel");
 }
 
-void apply_update(void* p, int type, const float* update, int64_t n, float keep, float lr, cudaStream_t stream) {
-  if (n <= 0) return;
-  auto go = [&](auto* typed) {
-    const bool aligned = reinterpret_cast<uintptr_t>(typed) % (4 * sizeof(*typed)) == 0 && (reinterpret_cast<uintptr_t>(update) & 15) == 0;
-    const int64_t quads = aligned ? n / 4 : 0;
-    apply_update_kernel<<<grid_for(aligned ? (n + 3) / 4 : n, 256), 256, 0, stream>>>(typed, update, n, quads, keep, lr);
-    check_launch("apply_update_kernel");
+namespace {
+template <typename T, int N>
+void launch_updates(const UpdateJob* jobs, int count, float keep, float lr, cudaStream_t stream) {
+  UpdateGroup<N> group;
+  for (int i = 0; i < count; ++i) {
+    const UpdateJob& job = jobs[i];
+    const bool aligned = reinterpret_cast<uintptr_t>(job.p) % (4 * sizeof(T)) == 0 && (reinterpret_cast<uintptr_t>(job.update) & 15) == 0;
+    group.jobs[i] = job;
+    group.quads[i] = aligned ? job.n / 4 : 0;
+    group.blocks.add(grid_for(aligned ? (job.n + 3) / 4 : job.n, 256));
+  }
+  apply_updates_kernel<T, N><<<group.blocks.total(), 256, 0, stream>>>(group, keep, lr);
+  check_launch("apply_updates_kernel");
+}
+}  // namespace
+
+void apply_updates(const UpdateJob* jobs, int count, int type, float keep, float lr, cudaStream_t stream) {
+  if (type != 0 && type != 1) throw std::invalid_argument("apply_updates: unknown parameter type");
+  auto go = [&](auto* typed, const UpdateJob* some, int n) {
+    using T = std::remove_pointer_t<decltype(typed)>;
+    if (n == 1) launch_updates<T, 1>(some, n, keep, lr, stream);
+    else launch_updates<T, kUpdateGroup>(some, n, keep, lr, stream);
   };
-  if (type == 0) go(static_cast<float*>(p));
-  else if (type == 1) go(static_cast<__nv_bfloat16*>(p));
-  else throw std::invalid_argument("apply_update: unknown parameter type");
+  const int64_t width = type == 0 ? sizeof(float) : sizeof(__nv_bfloat16);
+  auto overlap = [&](const UpdateJob& a, const UpdateJob& b) {
+    const auto x = reinterpret_cast<uintptr_t>(a.p), y = reinterpret_cast<uintptr_t>(b.p);
+    return x < y + width * b.n && y < x + width * a.n;
+  };
+  UpdateJob some[kUpdateGroup];
+  int n = 0;
+  auto flush = [&] {
+    if (n == 0) return;
+    if (type == 0) go(static_cast<float*>(nullptr), some, n);
+    else go(static_cast<__nv_bfloat16*>(nullptr), some, n);
+    n = 0;
+  };
+  for (int i = 0; i < count; ++i) {
+    if (jobs[i].n <= 0) continue;
+    // parameters that share memory are updated one after the other
+    if (n == kUpdateGroup || std::any_of(some, some + n, [&](const UpdateJob& other) { return overlap(other, jobs[i]); })) flush();
+    some[n++] = jobs[i];
+  }
+  flush();
 }
 
 void adamw_update(void* p, int type, const void* gradient, float* m, float* v, int64_t n, float beta1_rest, float beta2,

@@ -27,10 +27,15 @@ void split_planes(const void* src, int source_type, int64_t s_i, int64_t s_j, in
                   const SplitTarget& turned, float scale, int nearest, cudaStream_t stream);
 
 // Parameter updates in one pass, contiguous arrays of n elements; parameter (and `gradient`) type 0: fp32, 1: bf16.
-//   apply_update:  p <- p * keep (rounded to p's type; skipped for keep == 1), then p <- p - lr * update, the update rounded
+//   apply_updates: p <- p * keep (rounded to p's type; skipped for keep == 1), then p <- p - lr * update, the update rounded
 //                  to p's type first -- value for value what p.mul_(keep); p.add_(update.to(p.dtype), alpha=-lr) computes.
 //   adamw_update:  m <- m + (1 - b1)(g - m), v <- b2 v + (1 - b2) g^2, then the same with (m / bias1) / (sqrt(v / bias2) + eps).
-void apply_update(void* p, int type, const float* update, int64_t n, float keep, float lr, cudaStream_t stream);
+struct UpdateJob {
+  void* p;
+  const float* update;
+  int64_t n;
+};
+void apply_updates(const UpdateJob* jobs, int count, int type, float keep, float lr, cudaStream_t stream);
 void adamw_update(void* p, int type, const void* gradient, float* m, float* v, int64_t n, float beta1_rest, float beta2,
                   float beta2_rest, float bias1, float bias2, float eps, float keep, float lr, cudaStream_t stream);
 

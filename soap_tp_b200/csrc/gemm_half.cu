@@ -287,7 +287,7 @@ template <bool PAIR>
 constexpr int kColumns = (PAIR ? 256 : 128) / (kEpiWarps / 4);      // of the tile, per epilogue thread
 
 template <bool PAIR, typename Prefetch, typename Epilogue>
-__device__ __forceinline__ void half_kernel_body(const HalfMaps& maps, const HalfArgs& args, int* status, Prefetch prefetch,
+__device__ __forceinline__ void half_kernel_body(const HalfMaps& maps, const HalfArgs& args, int block, int* status, Prefetch prefetch,
                                                  Epilogue epilogue) {
   constexpr int BN = PAIR ? 256 : 128;
   constexpr int kCtas = PAIR ? 2 : 1;
@@ -311,7 +311,7 @@ __device__ __forceinline__ void half_kernel_body(const HalfMaps& maps, const Hal
   constexpr int kGroup = PAIR ? 8 : 16;
   const int tiles_m = (prob.M + kTileM - 1) / kTileM;
   const int tiles_n = (prob.N + BN - 1) / BN;
-  const int index = PAIR ? blockIdx.x >> 1 : blockIdx.x;
+  const int index = PAIR ? block >> 1 : block;
   const int per_group = kGroup * tiles_n;
   const int first_m = index / per_group * kGroup;
   const int rows_in_group = min(kGroup, tiles_m - first_m);
@@ -564,9 +564,9 @@ constexpr int kPitch = (MODE == kEpiSplit || MODE == kEpiAdam) ? kBM + 2 : kBM +
 static_assert(256 * (kBM + 2) * 4 <= kStagePool, "the staged tile fits where the stages were");
 
 template <bool PAIR, int MODE>
-__device__ __forceinline__ void half_kernel_impl(const HalfMaps& maps, const HalfArgs& args, int* status) {
+__device__ __forceinline__ void half_kernel_impl(const HalfMaps& maps, const HalfArgs& args, int block, int* status) {
   constexpr int BN = PAIR ? 256 : 128;
-  half_kernel_body<PAIR>(maps, args, status, [&](int m0, int n0, int ew, int lane) { prefetch_old<BN, MODE>(args.p, m0, n0, ew, lane); },
+  half_kernel_body<PAIR>(maps, args, block, status, [&](int m0, int n0, int ew, int lane) { prefetch_old<BN, MODE>(args.p, m0, n0, ew, lane); },
                          [&](float* tile, const float* column_scales, bool wide, uint64_t (&sum)[kColumns<PAIR> / 2], int col0, int row, volatile int* abort_flag,
                                                  int m0, int n0, int ew, int lane) {
 #pragma unroll
@@ -580,13 +580,22 @@ __device__ __forceinline__ void half_kernel_impl(const HalfMaps& maps, const Hal
 template <int MODE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 half_pair_kernel(const __grid_constant__ HalfMaps maps, const __grid_constant__ HalfArgs args, int* status) {
-  half_kernel_impl<true, MODE>(maps, args, status);
+  half_kernel_impl<true, MODE>(maps, args, blockIdx.x, status);
 }
 
-template <int MODE>
+// N products of single CTAs in one launch, one after another in the grid.
+template <int N>
+struct HalfGroup {
+  HalfMaps maps[N];
+  HalfArgs args[N];
+  GroupBlocks<N> blocks;
+};
+
+template <int MODE, int N>
 __global__ void __launch_bounds__(kThreads, 1)
-half_single_kernel(const __grid_constant__ HalfMaps maps, const __grid_constant__ HalfArgs args, int* status) {
-  half_kernel_impl<false, MODE>(maps, args, status);
+half_single_kernel(const __grid_constant__ HalfGroup<N> group, int* status) {
+  const int member = group.blocks.member(blockIdx.x);
+  half_kernel_impl<false, MODE>(group.maps[member], group.args[member], blockIdx.x - group.blocks.first(member), status);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -596,22 +605,45 @@ CUtensorMap make_map(const uint16_t* base, int64_t K, int64_t rows, int64_t ld) 
   return encode_k_major(CU_TENSOR_MAP_DATA_TYPE_FLOAT16, base, K, rows, 2 * ld, kBK, 128, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
+int single_tiles(const HalfProblem& p) { return ((p.M + kBM - 1) / kBM) * ((p.N + 127) / 128); }
+
+template <int MODE, int N>
+cudaError_t launch_singles(const HalfMaps* maps, const HalfArgs* args, int count, int* status, cudaStream_t stream) {
+  static PerDeviceOnce configured;
+  allow_dynamic_smem(reinterpret_cast<const void*>(half_single_kernel<MODE, N>), kSmemBytes, configured, "gemm_half");
+  HalfGroup<N> group;
+  for (int i = 0; i < count; ++i) {
+    group.maps[i] = maps[i];
+    group.args[i] = args[i];
+    group.blocks.add(single_tiles(args[i].p));
+  }
+  return launch_dependent(half_single_kernel<MODE, N>, dim3(group.blocks.total()), dim3(kThreads), kSmemBytes, stream, group, status);
+}
+
 template <int MODE>
-void launch(bool pairs, const HalfMaps& maps, const HalfArgs& args, int* status, cudaStream_t stream) {
-  const HalfProblem& p = args.p;
+void launch(bool pairs, const HalfMaps* maps, const HalfArgs* args, int count, int* status, cudaStream_t stream) {
   cudaError_t err;
   if (pairs) {
     static PerDeviceOnce configured;
     allow_dynamic_smem(reinterpret_cast<const void*>(half_pair_kernel<MODE>), kSmemBytes, configured, "gemm_half");
+    const HalfProblem& p = args->p;
     const int tiles = ((p.M + 2 * kBM - 1) / (2 * kBM)) * ((p.N + 255) / 256);
-    err = launch_dependent(half_pair_kernel<MODE>, dim3(2 * tiles), dim3(kThreads), kSmemBytes, stream, maps, args, status);
+    err = launch_dependent(half_pair_kernel<MODE>, dim3(2 * tiles), dim3(kThreads), kSmemBytes, stream, *maps, *args, status);
   } else {
-    static PerDeviceOnce configured;
-    allow_dynamic_smem(reinterpret_cast<const void*>(half_single_kernel<MODE>), kSmemBytes, configured, "gemm_half");
-    const int tiles = ((p.M + kBM - 1) / kBM) * ((p.N + 127) / 128);
-    err = launch_dependent(half_single_kernel<MODE>, dim3(tiles), dim3(kThreads), kSmemBytes, stream, maps, args, status);
+    err = count == 1 ? launch_singles<MODE, 1>(maps, args, count, status, stream)
+                     : launch_singles<MODE, kHalfGroup>(maps, args, count, status, stream);
   }
   if (err != cudaSuccess) throw std::runtime_error(std::string("gemm_half launch: ") + cudaGetErrorString(err));
+}
+
+void launch_mode(bool pairs, const HalfMaps* maps, const HalfArgs* args, int count, int* status, cudaStream_t stream) {
+  switch (args->p.mode) {
+    case kEpiStore: launch<kEpiStore>(pairs, maps, args, count, status, stream); return;
+    case kEpiSplit: launch<kEpiSplit>(pairs, maps, args, count, status, stream); return;
+    case kEpiAdam: launch<kEpiAdam>(pairs, maps, args, count, status, stream); return;
+    case kEpiRowMajor: launch<kEpiRowMajor>(pairs, maps, args, count, status, stream); return;
+    default: throw std::invalid_argument("gemm_half: unknown epilogue mode");
+  }
 }
 
 }  // namespace
@@ -634,8 +666,9 @@ bool half_on_pairs(int M, int N, bool symmetric) {
   return 3 * ((tiles_of(256) + 73) / 74) <= 2 * ((tiles_of(128) + 147) / 148);
 }
 
-void gemm_half(const HalfOperand& a, const HalfOperand& b, const HalfProblem& prob, int* status, cudaStream_t stream) {
-  if (prob.M <= 0 || prob.N <= 0) return;
+namespace {
+// Checks a product and fills what its kernel reads.
+void prepare(const HalfOperand& a, const HalfOperand& b, const HalfProblem& prob, HalfMaps& maps, HalfArgs& args) {
   if (prob.K <= 0) throw std::invalid_argument("gemm_half needs K >= 1");
   if (b.scale_stride != 0) throw std::invalid_argument("gemm_half: the second operand has one scale per column");
   if (prob.symmetric && (prob.mode != kEpiStore || prob.M != prob.N))
@@ -650,7 +683,6 @@ void gemm_half(const HalfOperand& a, const HalfOperand& b, const HalfProblem& pr
                       !writes_pairs(prob.mixed)))
       throw std::invalid_argument("gemm_half: mixed output planes need 8-byte alignment and an even pitch");
   }
-  HalfMaps maps;
   maps.a_h = make_map(a.h, prob.K, prob.M, a.ld);
   maps.a_l = a.l ? make_map(a.l, prob.K, prob.M, a.ld) : maps.a_h;
   maps.b_h = make_map(b.h, prob.K, prob.N, b.ld);
@@ -661,15 +693,29 @@ void gemm_half(const HalfOperand& a, const HalfOperand& b, const HalfProblem& pr
       maps.mixed[2 + i] = b.mixed[i];
     }
   }
-  const HalfArgs args{prob, a.scale, a.scale_stride, b.scale, a.l ? 2 : 1, b.l ? 2 : 1};
+  args = HalfArgs{prob, a.scale, a.scale_stride, b.scale, a.l ? 2 : 1, b.l ? 2 : 1};
+}
+}  // namespace
+
+void gemm_half(const HalfOperand& a, const HalfOperand& b, const HalfProblem& prob, int* status, cudaStream_t stream) {
+  if (prob.M <= 0 || prob.N <= 0) return;
+  HalfMaps maps;
+  HalfArgs args;
+  prepare(a, b, prob, maps, args);
   const bool pairs = prob.tiles ? prob.tiles == 2 : half_on_pairs(prob.M, prob.N, prob.symmetric);
-  switch (prob.mode) {
-    case kEpiStore: launch<kEpiStore>(pairs, maps, args, status, stream); return;
-    case kEpiSplit: launch<kEpiSplit>(pairs, maps, args, status, stream); return;
-    case kEpiAdam: launch<kEpiAdam>(pairs, maps, args, status, stream); return;
-    case kEpiRowMajor: launch<kEpiRowMajor>(pairs, maps, args, status, stream); return;
-    default: throw std::invalid_argument("gemm_half: unknown epilogue mode");
+  launch_mode(pairs, &maps, &args, 1, status, stream);
+}
+
+void gemm_half_group(const HalfJob* jobs, int count, int* status, cudaStream_t stream) {
+  if (count < 1 || count > kHalfGroup) throw std::invalid_argument("gemm_half: too many products for one launch");
+  HalfMaps maps[kHalfGroup];
+  HalfArgs args[kHalfGroup];
+  for (int i = 0; i < count; ++i) {
+    if (jobs[i].problem.M <= 0 || jobs[i].problem.N <= 0 || jobs[i].problem.mode != jobs[0].problem.mode)
+      throw std::invalid_argument("gemm_half: products of one launch are not empty and end in the same epilogue");
+    prepare(jobs[i].a, jobs[i].b, jobs[i].problem, maps[i], args[i]);
   }
+  launch_mode(false, maps, args, count, status, stream);
 }
 
 }  // namespace soapb200

@@ -64,6 +64,14 @@ bool half_on_pairs(int M, int N, bool symmetric);
 
 void gemm_half(const HalfOperand& a, const HalfOperand& b, const HalfProblem& prob, int* status, cudaStream_t stream);
 
+// Up to kHalfGroup products with the same epilogue in one launch of single CTAs.
+constexpr int kHalfGroup = 8;
+struct HalfJob {
+  HalfOperand a, b;
+  HalfProblem problem;
+};
+void gemm_half_group(const HalfJob* jobs, int count, int* status, cudaStream_t stream);
+
 // Where one orientation of a matrix goes as scaled fp16 planes (h == null: not wanted).  `scale` has one entry per vector,
 // `largest` is scratch of the same length (needed without planes too where a RangeGuard looks at it).
 struct HalfTarget {
@@ -102,6 +110,16 @@ struct RangeGuard {
 // i < rows, j < cols; source_type 0: fp32, 1: bf16.
 void half_planes(const void* src, int source_type, int64_t s_i, int64_t s_j, int rows, int cols, const HalfTarget& plain,
                  const HalfTarget& turned, const RangeGuard& guard, cudaStream_t stream);
+// The same for up to kHalfGroup matrices in the same launches; all with a decision on the range.
+struct PlanesJob {
+  const void* src;
+  int source_type;
+  int64_t s_i, s_j;
+  int rows, cols;
+  HalfTarget plain, turned;
+  RangeGuard guard;
+};
+void half_planes_group(const PlanesJob* jobs, int count, cudaStream_t stream);
 
 // A matrix to be rotated by two bases (steady_step.cpp).
 struct Rotation {
@@ -141,6 +159,10 @@ struct SteadyStep {
 };
 constexpr int kStepPlanes = 1, kStepForward = 2, kStepBackward = 4, kStepAverages = 8;
 void steady_step(const SteadyStep& s, int* status, cudaStream_t stream);
+// Whether every product of such a step runs on single CTAs, so that several small parameters can share its launches; and the
+// steps of up to kHalfGroup such parameters (all phases; scratch of their own each).
+bool steady_step_shares(int rows, int cols);
+void steady_steps(const SteadyStep* steps, int count, int* status, cudaStream_t stream);
 
 // Scale of a vector or block from the bit pattern of its largest magnitude (clamped so that both factors are normal):
 // x * multiplier is what the planes hold, `inverse` undoes it.  Infinities and NaN pass through with a factor of one.

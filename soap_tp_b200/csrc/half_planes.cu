@@ -10,6 +10,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include <algorithm>
 #include <stdexcept>
 #include <string>
 #include <type_traits>
@@ -26,22 +27,58 @@ using namespace sweep;
 
 __device__ __forceinline__ uint32_t magnitude(float x) { return __float_as_uint(x) & 0x7fffffffu; }
 
+// Scratch of the largest magnitudes back to zero.  A kernel, so that the chain of dependent launches goes through it; a memset
+// of each array would stand between two of them.
+template <int N>
+struct ClearGroup {
+  uint32_t* words[2 * N];
+  int counts[2 * N];
+};
+template <int N>
+__global__ void __launch_bounds__(kThreads) clear_kernel(const __grid_constant__ ClearGroup<N> group) {
+  wait_for_predecessor();
+  let_successor_start();
+  uint32_t* words = group.words[blockIdx.y];
+  for (int i = blockIdx.x * kThreads + threadIdx.x; i < group.counts[blockIdx.y]; i += gridDim.x * kThreads) words[i] = 0;
+}
+
+// A matrix as the two passes over it see it.
+struct Source {
+  const void* src;
+  int64_t s_fast, s_slow;
+  int n_fast, n_slow, tiles_fast;
+  bool pairs;
+};
+struct LargestJob {
+  Source from;
+  int strip;
+  uint32_t *of_fast, *of_slow;
+};
+template <int N>
+struct LargestGroup {
+  LargestJob jobs[N];
+  GroupBlocks<N> blocks;
+};
+
 // Largest magnitude (as a bit pattern, which orders like the value) along the fast and the slow axis.  A CTA walks
 // `strip` tiles along the slow axis and keeps the maxima of its fast-axis elements in registers meanwhile.
-template <typename T>
-__global__ void __launch_bounds__(kThreads) largest_kernel(const T* __restrict__ src, int64_t s_fast, int64_t s_slow, int n_fast,
-                                                           int n_slow, int strip, bool pairs, uint32_t* __restrict__ of_fast,
-                                                           uint32_t* __restrict__ of_slow) {
+template <typename T, int N>
+__global__ void __launch_bounds__(kThreads) largest_kernel(const __grid_constant__ LargestGroup<N> group) {
   __shared__ uint32_t fast_max[8][kTile];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int fast0 = blockIdx.x * kTile;
+  const int member = group.blocks.member(blockIdx.x), block = blockIdx.x - group.blocks.first(member);
+  const LargestJob& job = group.jobs[member];
+  const T* src = static_cast<const T*>(job.from.src);
+  const int n_fast = job.from.n_fast, n_slow = job.from.n_slow, strip = job.strip;
+  uint32_t *of_fast = job.of_fast, *of_slow = job.of_slow;
+  const int fast0 = block % job.from.tiles_fast * kTile, strip0 = block / job.from.tiles_fast * strip;
   wait_for_predecessor();
   let_successor_start();
   uint32_t mine0 = 0, mine1 = 0;
   for (int t = 0; t < strip; ++t) {
-    const int slow0 = (blockIdx.y * strip + t) * kTile;
+    const int slow0 = (strip0 + t) * kTile;
     if (slow0 >= n_slow) break;
-    sweep_tile(src, s_fast, s_slow, fast0, slow0, n_fast, n_slow, pairs, [&](int, int slow, float x0, float x1) {
+    sweep_tile(src, job.from.s_fast, job.from.s_slow, fast0, slow0, n_fast, n_slow, job.from.pairs, [&](int, int slow, float x0, float x1) {
       const uint32_t a = magnitude(x0), b = magnitude(x1);
       mine0 = max(mine0, a);
       mine1 = max(mine1, b);
@@ -156,24 +193,37 @@ __device__ __noinline__ void help(const MixedWork& work, float (*tile)[kTile + 1
 // `along`: depth runs along the source's fast axis; `across`: depth runs along its slow axis.  The first rows of CTAs are there
 // for the decision and the mixed form (DECIDED); eight CTAs per SM, so that their registers do not cost the others occupancy (with the 48 that
 // they ask for the planes of 4096^2 fp32 took 65 us instead of 59).
-template <typename T, bool DECIDED>
-__global__ void __launch_bounds__(kThreads, DECIDED ? 8 : 1) half_planes_kernel(const T* __restrict__ src, int64_t s_fast, int64_t s_slow,
-                                                               int n_fast, int n_slow, bool pairs, const HalfTarget along,
-                                                               const HalfTarget across, const __grid_constant__ Work<DECIDED> work) {
+template <bool DECIDED>
+struct PlaneJob {
+  Source from;
+  HalfTarget along, across;
+  Work<DECIDED> work;
+};
+template <bool DECIDED, int N>
+struct PlaneGroup {
+  PlaneJob<DECIDED> jobs[N];
+  GroupBlocks<N> blocks;
+};
+template <typename T, bool DECIDED, int N>
+__global__ void __launch_bounds__(kThreads, DECIDED ? 8 : 1) half_planes_kernel(const __grid_constant__ PlaneGroup<DECIDED, N> group) {
   __shared__ float tile[kTile][kTile + 1];           // [slow][fast]
   __shared__ float up_along[kTile], up_across[kTile];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int member = group.blocks.member(blockIdx.x), block = blockIdx.x - group.blocks.first(member);
+  const PlaneJob<DECIDED>& job = group.jobs[member];
+  const int n_fast = job.from.n_fast, n_slow = job.from.n_slow;
+  const HalfTarget along = job.along, across = job.across;
   wait_for_predecessor();
   let_successor_start();
-  int tile_row = blockIdx.y;
+  int tile_row = block / job.from.tiles_fast;
   if constexpr (DECIDED) {
-    tile_row -= work.rows;
+    tile_row -= job.work.rows;
     if (tile_row < 0) {
-      help<T>(work, tile, blockIdx.y * gridDim.x + blockIdx.x, work.rows * gridDim.x);
+      help<T>(job.work, tile, block, job.work.rows * job.from.tiles_fast);
       return;
     }
   }
-  const int fast0 = blockIdx.x * kTile, slow0 = tile_row * kTile;
+  const int fast0 = block % job.from.tiles_fast * kTile, slow0 = tile_row * kTile;
   if (threadIdx.x < kTile) {
     const int slow = slow0 + threadIdx.x;
     if (along.h && slow < n_slow) {
@@ -189,10 +239,11 @@ __global__ void __launch_bounds__(kThreads, DECIDED ? 8 : 1) half_planes_kernel(
       if (slow0 == 0) across.scale[fast] = s.inverse;
     }
   }
-  sweep_tile(src, s_fast, s_slow, fast0, slow0, n_fast, n_slow, pairs, [&](int fast, int slow, float x0, float x1) {
-    tile[slow][fast] = x0;
-    tile[slow][fast + 1] = x1;
-  });
+  sweep_tile(static_cast<const T*>(job.from.src), job.from.s_fast, job.from.s_slow, fast0, slow0, n_fast, n_slow, job.from.pairs,
+             [&](int fast, int slow, float x0, float x1) {
+               tile[slow][fast] = x0;
+               tile[slow][fast + 1] = x1;
+             });
   __syncthreads();
   // pitches are multiples of 64, so the second half of a pair that ends the depth lands in the padding
   if (along.h && fast0 + 2 * lane < n_fast) {
@@ -228,33 +279,84 @@ MixedJob basis_job(const WideBasis& b) {
                                                      : mixed_job(b.src, b.s_j, b.s_i, b.size, b.size, b.turned, b.plain);
 }
 
+// One matrix with its axes told apart.
+struct Oriented {
+  Source from;
+  HalfTarget along, across;
+  SplitTarget mixed_along, mixed_across;
+  const RangeGuard* guard;
+  int tiles_slow() const { return (from.n_slow + kTile - 1) / kTile; }
+  int helper_rows() const { return guard->wide ? (148 + from.tiles_fast - 1) / from.tiles_fast : 0; }
+};
+
+void check_job(const PlanesJob& job) {
+  for (const HalfTarget* t : {&job.plain, &job.turned}) {
+    if (t->h && (!t->largest || t->ld % 64 != 0 || t->ld < (t == &job.plain ? job.rows : job.cols) ||
+                 (reinterpret_cast<uintptr_t>(t->h) & 15) != 0 || (reinterpret_cast<uintptr_t>(t->l) & 15) != 0))
+      throw std::invalid_argument("half_planes: planes need 16-byte alignment and a pitch that is a multiple of 64");
+    if (job.guard.wide && !t->largest)
+      throw std::invalid_argument("half_planes: a decision on the range needs the maxima of both orientations");
+  }
+  if (job.source_type != 0 && job.source_type != 1) throw std::invalid_argument("half_planes: unknown source type");
+}
+
 template <typename T>
-void launch(const T* src, int64_t s_fast, int64_t s_slow, int n_fast, int n_slow, const HalfTarget& along,
-            const HalfTarget& across, const SplitTarget& mixed_along, const SplitTarget& mixed_across, const RangeGuard& guard,
-            cudaStream_t stream) {
-  const bool pairs = reads_pairs(src, s_fast, s_slow, n_slow);
-  if (along.largest) check(cudaMemsetAsync(along.largest, 0, sizeof(uint32_t) * n_slow, stream), "half_planes");
-  if (across.largest) check(cudaMemsetAsync(across.largest, 0, sizeof(uint32_t) * n_fast, stream), "half_planes");
-  const int tiles_fast = (n_fast + kTile - 1) / kTile, tiles_slow = (n_slow + kTile - 1) / kTile;
-  // enough CTAs for every SM several times over before a CTA takes more than one tile
-  int strip = static_cast<int>(static_cast<int64_t>(tiles_fast) * tiles_slow / (148 * 8));
-  strip = strip < 1 ? 1 : (strip > 16 ? 16 : strip);
-  const int helper_rows = guard.wide ? (148 + tiles_fast - 1) / tiles_fast : 0;
-  const dim3 strips(tiles_fast, (tiles_slow + strip - 1) / strip), tiles(tiles_fast, tiles_slow + helper_rows);
-  if (strips.y > 65535 || tiles.y > 65535) throw std::invalid_argument("half_planes: matrix too long");
-  check(launch_dependent(largest_kernel<T>, strips, dim3(kThreads), 0, stream, src, s_fast, s_slow, n_fast, n_slow, strip, pairs,
-                         across.largest, along.largest),
-        "largest_kernel");
-  auto convert = [&](auto kernel, const auto& work) {
-    check(launch_dependent(kernel, tiles, dim3(kThreads), 0, stream, src, s_fast, s_slow, n_fast, n_slow, pairs, along, across, work),
-          "half_planes_kernel");
-  };
-  if (guard.wide)
-    convert(half_planes_kernel<T, true>,
-            MixedWork{guard.wide, {along.largest, across.largest}, {n_slow, n_fast}, guard.nearest, helper_rows, mixed_job(src, s_fast, s_slow, n_fast, n_slow, mixed_along, mixed_across),
-                      {basis_job(guard.bases[0]), basis_job(guard.bases[1])}});
-  else
-    convert(half_planes_kernel<T, false>, NoWork{});
+Oriented oriented(const PlanesJob& job) {
+  const bool rows_fast = fast_is_first(job.s_i, job.s_j, job.rows, job.cols);
+  Oriented o{};
+  o.from.src = job.src;
+  o.from.s_fast = rows_fast ? job.s_i : job.s_j;
+  o.from.s_slow = rows_fast ? job.s_j : job.s_i;
+  o.from.n_fast = rows_fast ? job.rows : job.cols;
+  o.from.n_slow = rows_fast ? job.cols : job.rows;
+  o.from.tiles_fast = (o.from.n_fast + kTile - 1) / kTile;
+  o.from.pairs = reads_pairs(static_cast<const T*>(job.src), o.from.s_fast, o.from.s_slow, o.from.n_slow);
+  o.along = rows_fast ? job.plain : job.turned;
+  o.across = rows_fast ? job.turned : job.plain;
+  (rows_fast ? o.mixed_along : o.mixed_across) = job.guard.mixed;
+  o.guard = &job.guard;
+  if (o.tiles_slow() + o.helper_rows() > 65535) throw std::invalid_argument("half_planes: matrix too long");
+  return o;
+}
+
+template <typename T, bool DECIDED, int N>
+void launch(const Oriented* jobs, int count, cudaStream_t stream) {
+  ClearGroup<N> clear{};
+  LargestGroup<N> largest;
+  PlaneGroup<DECIDED, N> planes;
+  int longest = 1;
+  for (int i = 0; i < count; ++i) {
+    const Oriented& o = jobs[i];
+    const Source& from = o.from;
+    const int tiles = from.tiles_fast * o.tiles_slow();
+    clear.words[2 * i] = o.along.largest;
+    clear.counts[2 * i] = o.along.largest ? from.n_slow : 0;
+    clear.words[2 * i + 1] = o.across.largest;
+    clear.counts[2 * i + 1] = o.across.largest ? from.n_fast : 0;
+    longest = std::max({longest, from.n_slow, from.n_fast});
+    // enough CTAs for every SM several times over before a CTA takes more than one tile
+    const int strip = std::clamp(tiles / (148 * 8), 1, 16);
+    largest.jobs[i] = LargestJob{from, strip, o.across.largest, o.along.largest};
+    largest.blocks.add(from.tiles_fast * ((o.tiles_slow() + strip - 1) / strip));
+    PlaneJob<DECIDED>& job = planes.jobs[i];
+    job.from = from;
+    job.along = o.along;
+    job.across = o.across;
+    if constexpr (DECIDED) {
+      const RangeGuard& guard = *o.guard;
+      job.work = MixedWork{guard.wide, {o.along.largest, o.across.largest}, {from.n_slow, from.n_fast}, guard.nearest, o.helper_rows(),
+                           mixed_job(static_cast<const T*>(from.src), from.s_fast, from.s_slow, from.n_fast, from.n_slow, o.mixed_along,
+                                     o.mixed_across),
+                           {basis_job(guard.bases[0]), basis_job(guard.bases[1])}};
+    }
+    planes.blocks.add(tiles + o.helper_rows() * from.tiles_fast);
+  }
+  const dim3 block(kThreads);
+  check(launch_dependent(clear_kernel<N>, dim3(std::min(8, (longest + kThreads - 1) / kThreads), 2 * count), block, 0, stream, clear),
+        "clear_kernel");
+  check(launch_dependent(largest_kernel<T, N>, dim3(largest.blocks.total()), block, 0, stream, largest), "largest_kernel");
+  check(launch_dependent(half_planes_kernel<T, DECIDED, N>, dim3(planes.blocks.total()), block, 0, stream, planes),
+        "half_planes_kernel");
 }
 
 }  // namespace
@@ -262,21 +364,31 @@ void launch(const T* src, int64_t s_fast, int64_t s_slow, int n_fast, int n_slow
 void half_planes(const void* src, int source_type, int64_t s_i, int64_t s_j, int rows, int cols, const HalfTarget& plain,
                  const HalfTarget& turned, const RangeGuard& guard, cudaStream_t stream) {
   if (rows <= 0 || cols <= 0 || (!plain.h && !turned.h)) return;
-  for (const HalfTarget* t : {&plain, &turned}) {
-    if (t->h && (!t->largest || t->ld % 64 != 0 || t->ld < (t == &plain ? rows : cols) ||
-                 (reinterpret_cast<uintptr_t>(t->h) & 15) != 0 || (reinterpret_cast<uintptr_t>(t->l) & 15) != 0))
-      throw std::invalid_argument("half_planes: planes need 16-byte alignment and a pitch that is a multiple of 64");
-    if (guard.wide && !t->largest)
-      throw std::invalid_argument("half_planes: a decision on the range needs the maxima of both orientations");
-  }
-  const bool rows_fast = fast_is_first(s_i, s_j, rows, cols);
+  const PlanesJob job{src, source_type, s_i, s_j, rows, cols, plain, turned, guard};
+  check_job(job);
   auto go = [&](auto* typed) {
-    if (rows_fast) launch(typed, s_i, s_j, rows, cols, plain, turned, guard.mixed, SplitTarget{}, guard, stream);
-    else launch(typed, s_j, s_i, cols, rows, turned, plain, SplitTarget{}, guard.mixed, guard, stream);
+    using T = std::remove_pointer_t<decltype(typed)>;
+    const Oriented o = oriented<T>(job);
+    if (guard.wide) launch<T, true, 1>(&o, 1, stream);
+    else launch<T, false, 1>(&o, 1, stream);
   };
-  if (source_type == 0) go(static_cast<const float*>(src));
-  else if (source_type == 1) go(static_cast<const __nv_bfloat16*>(src));
-  else throw std::invalid_argument("half_planes: unknown source type");
+  if (source_type == 0) go(static_cast<float*>(nullptr));
+  else go(static_cast<__nv_bfloat16*>(nullptr));
+}
+
+void half_planes_group(const PlanesJob* jobs, int count, cudaStream_t stream) {
+  if (count < 1 || count > kHalfGroup) throw std::invalid_argument("half_planes: too many matrices for one launch");
+  Oriented of_floats[kHalfGroup], of_halves[kHalfGroup];
+  int floats = 0, halves = 0;
+  for (int i = 0; i < count; ++i) {
+    check_job(jobs[i]);
+    if (jobs[i].rows <= 0 || jobs[i].cols <= 0 || !jobs[i].guard.wide)
+      throw std::invalid_argument("half_planes: matrices of one launch are not empty and have a decision on their range");
+    if (jobs[i].source_type == 0) of_floats[floats++] = oriented<float>(jobs[i]);
+    else of_halves[halves++] = oriented<__nv_bfloat16>(jobs[i]);
+  }
+  if (floats) launch<float, true, kHalfGroup>(of_floats, floats, stream);
+  if (halves) launch<__nv_bfloat16, true, kHalfGroup>(of_halves, halves, stream);
 }
 
 }  // namespace soapb200

@@ -43,6 +43,32 @@ class ScopedEvent {
   cudaEvent_t event_ = nullptr;
 };
 
+// The blocks of up to N problems that share a launch, one problem's after another's.
+template <int N>
+class GroupBlocks {
+ public:
+  void add(int blocks) {
+    ends_[count_] = (count_ ? ends_[count_ - 1] : 0) + blocks;
+    ++count_;
+  }
+  int total() const { return ends_[count_ - 1]; }
+#ifdef __CUDACC__
+  __device__ __forceinline__ int member(int block) const {
+    int i = 0;
+    if constexpr (N > 1) {
+      while (i + 1 < count_ && block >= ends_[i]) ++i;
+    }
+    return i;
+  }
+  __device__ __forceinline__ int first(int member) const { return N > 1 && member ? ends_[member - 1] : 0; }
+  __device__ __forceinline__ int count(int member) const { return ends_[member] - first(member); }
+#endif
+
+ private:
+  int ends_[N];
+  int count_ = 0;
+};
+
 // Launch that may begin before the kernel ahead of it in the stream has ended (programmatic dependent launch): what a kernel
 // does before `wait_for_predecessor` -- barriers, TMEM, descriptor prefetch -- overlaps the tail of the one before, and the
 // gap between two launches closes (a step of eight dependent launches: 118 -> 106 us at 256 x 512, 193 -> 181 us at

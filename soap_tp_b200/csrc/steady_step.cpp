@@ -45,8 +45,7 @@ class Fork {
 
 namespace {
 // T = X^T Q (cols x rows), or U^T Q (the same shape): the first product of a rotation.
-void first_product(const Rotation& r, const HalfOperand& source, bool settled, const HalfOperand& basis, int* status,
-                   cudaStream_t stream) {
+HalfJob first_product(const Rotation& r, const HalfOperand& source, bool settled, const HalfOperand& basis) {
   HalfProblem p{};
   p.M = r.cols; p.N = r.rows; p.K = r.rows;
   p.mode = kEpiSplit;
@@ -54,7 +53,7 @@ void first_product(const Rotation& r, const HalfOperand& source, bool settled, c
   p.Ch = const_cast<uint16_t*>(r.middle.h); p.Cl = const_cast<uint16_t*>(r.middle.l); p.ldp = r.middle.ld;
   p.Cscale = const_cast<float*>(r.middle.scale); p.ldscale = r.middle.scale_stride;
   p.wide = r.guard.wide; p.settled = settled; p.mixed = r.mixed_middle;
-  gemm_half(source, basis, p, status, stream);
+  return HalfJob{source, basis, p};
 }
 
 HalfOperand source_of(const Rotation& r) {
@@ -71,15 +70,81 @@ HalfProblem second_product(const Rotation& r) {
   return p;
 }
 
-void make_planes(const Rotation& r, cudaStream_t stream) {
-  half_planes(r.source, r.source_type, r.s_i, r.s_j, r.rows, r.cols, r.x, r.xt, r.guard, stream);
+PlanesJob planes_of(const Rotation& r) {
+  return PlanesJob{r.source, r.source_type, r.s_i, r.s_j, r.rows, r.cols, r.x, r.xt, r.guard};
+}
+
+// The products of a step.
+HalfJob rotated(const SteadyStep& s) {                                      // T = X^T Q_L
+  const Rotation& r = s.rotation;
+  return first_product(r, source_of(r), false, r.left);
+}
+HalfJob adam(const SteadyStep& s) {                                         // Y = T^T Q_R, Adam(Y) -> U
+  const Rotation& r = s.rotation;
+  HalfProblem p = second_product(r);
+  p.mode = kEpiAdam;
+  p.Ch = const_cast<uint16_t*>(s.update.h); p.Cl = const_cast<uint16_t*>(s.update.l); p.ldp = s.update.ld;
+  p.Cscale = const_cast<float*>(s.update.scale); p.ldscale = s.update.scale_stride;
+  p.mixed = s.mixed_update;
+  p.mom = s.momentum; p.ldm = s.ldm; p.var = s.variance; p.ldv = s.ldv;
+  p.beta1 = s.beta1; p.beta2 = s.beta2; p.eps = s.eps; p.inv_bc1 = s.inv_bc1; p.inv_sqrt_bc2 = s.inv_sqrt_bc2;
+  return HalfJob{r.middle, r.right, p};
+}
+HalfJob turned_back(const SteadyStep& s) {                                  // T2 = U^T Q_L^T
+  return first_product(s.rotation, s.update, true, s.rotation.left_turned);
+}
+HalfJob result(const SteadyStep& s) {                                       // T2^T Q_R^T
+  const Rotation& r = s.rotation;
+  HalfProblem p = second_product(r);
+  p.mode = kEpiRowMajor;
+  p.C = s.out; p.ldc = r.cols;
+  return HalfJob{r.middle, r.right_turned, p};
+}
+// L = beta L + (1 - beta) G G^T, R likewise.  Products of a vector of G with another one: what counts is their error against the
+// vectors' own sizes, which the pairs keep in every range (2^-23 of an element, 2^-39 of its vector's largest).
+HalfJob average(const SteadyStep& s, bool left) {
+  const Rotation& r = s.rotation;
+  const HalfOperand x = operand(left ? r.xt : r.x);
+  HalfProblem p{};
+  p.mode = kEpiStore;
+  p.symmetric = 1;
+  p.alpha = static_cast<float>(1.0 - s.beta);
+  p.beta = static_cast<float>(s.beta);
+  p.M = p.N = left ? r.rows : r.cols;
+  p.K = left ? r.cols : r.rows;
+  p.C = left ? s.left_gram : s.right_gram;
+  p.ldc = left ? s.ld_left : s.ld_right;
+  return HalfJob{x, x, p};
+}
+
+// The phases of one step, or of several that share their launches.
+template <typename Planes, typename Launch>
+void issue(const SteadyStep& s, cudaStream_t stream, Planes planes, Launch launch) {
+  if (s.phases & kStepPlanes) planes();
+  const bool averages = s.phases & kStepAverages, rotations = s.phases & (kStepForward | kStepBackward);
+  const cudaStream_t side = averages && rotations ? s.side : stream;
+  std::optional<Fork> fork;
+  if (side != stream) fork.emplace(stream, side);
+  if (s.phases & kStepForward) {
+    launch(rotated, stream);
+    launch(adam, stream);
+  }
+  if (s.phases & kStepBackward) {
+    launch(turned_back, stream);
+    launch(result, stream);
+  }
+  if (averages) {
+    launch([](const SteadyStep& one) { return average(one, true); }, side);
+    launch([](const SteadyStep& one) { return average(one, false); }, side);
+  }
 }
 }  // namespace
 
 void rotate_half(const Rotation& r, bool turned, float* out, int64_t ldc, int* status, cudaStream_t stream) {
   if (r.rows <= 0 || r.cols <= 0) return;
-  make_planes(r, stream);
-  first_product(r, source_of(r), false, turned ? r.left_turned : r.left, status, stream);
+  half_planes(r.source, r.source_type, r.s_i, r.s_j, r.rows, r.cols, r.x, r.xt, r.guard, stream);
+  const HalfJob first = first_product(r, source_of(r), false, turned ? r.left_turned : r.left);
+  gemm_half(first.a, first.b, first.problem, status, stream);
   HalfProblem store = second_product(r);
   store.mode = kEpiStore;
   store.C = out; store.ldc = ldc;
@@ -89,46 +154,36 @@ void rotate_half(const Rotation& r, bool turned, float* out, int64_t ldc, int* s
 void steady_step(const SteadyStep& s, int* status, cudaStream_t stream) {
   const Rotation& r = s.rotation;
   if (r.rows <= 0 || r.cols <= 0) throw std::invalid_argument("steady_step: empty matrix");
-  if (s.phases & kStepPlanes) make_planes(r, stream);
-  const bool averages = s.phases & kStepAverages, rotations = s.phases & (kStepForward | kStepBackward);
-  const cudaStream_t side = averages && rotations ? s.side : stream;
-  std::optional<Fork> fork;
-  if (side != stream) fork.emplace(stream, side);
+  issue(s, stream, [&] { half_planes(r.source, r.source_type, r.s_i, r.s_j, r.rows, r.cols, r.x, r.xt, r.guard, stream); },
+        [&](auto product, cudaStream_t on) {
+          const HalfJob job = product(s);
+          gemm_half(job.a, job.b, job.problem, status, on);
+        });
+}
 
-  if (s.phases & kStepForward) {
-    first_product(r, source_of(r), false, r.left, status, stream);          // T = X^T Q_L
-    HalfProblem adam = second_product(r);                                   // Y = T^T Q_R, Adam(Y) -> U
-    adam.mode = kEpiAdam;
-    adam.Ch = const_cast<uint16_t*>(s.update.h); adam.Cl = const_cast<uint16_t*>(s.update.l); adam.ldp = s.update.ld;
-    adam.Cscale = const_cast<float*>(s.update.scale); adam.ldscale = s.update.scale_stride;
-    adam.mixed = s.mixed_update;
-    adam.mom = s.momentum; adam.ldm = s.ldm; adam.var = s.variance; adam.ldv = s.ldv;
-    adam.beta1 = s.beta1; adam.beta2 = s.beta2; adam.eps = s.eps; adam.inv_bc1 = s.inv_bc1; adam.inv_sqrt_bc2 = s.inv_sqrt_bc2;
-    gemm_half(r.middle, r.right, adam, status, stream);
+bool steady_step_shares(int rows, int cols) {
+  return rows > 0 && cols > 0 && !half_on_pairs(cols, rows, false) && !half_on_pairs(rows, cols, false) &&
+         !half_on_pairs(rows, rows, true) && !half_on_pairs(cols, cols, true);
+}
+
+void steady_steps(const SteadyStep* steps, int count, int* status, cudaStream_t stream) {
+  if (count < 1 || count > kHalfGroup) throw std::invalid_argument("steady_steps: too many steps for shared launches");
+  for (int i = 0; i < count; ++i) {
+    if (steps[i].rotation.rows <= 0 || steps[i].rotation.cols <= 0) throw std::invalid_argument("steady_steps: empty matrix");
+    if (steps[i].phases != steps[0].phases || steps[i].side != steps[0].side)
+      throw std::invalid_argument("steady_steps: steps that share launches have the same phases and streams");
   }
-  if (s.phases & kStepBackward) {
-    first_product(r, s.update, true, r.left_turned, status, stream);        // T2 = U^T Q_L^T
-    HalfProblem out = second_product(r);                                    // T2^T Q_R^T
-    out.mode = kEpiRowMajor;
-    out.C = s.out; out.ldc = r.cols;
-    gemm_half(r.middle, r.right_turned, out, status, stream);
-  }
-  if (averages) {
-    // Products of a vector of G with another one: what counts is their error against the vectors' own sizes, which the pairs
-    // keep in every range (2^-23 of an element, 2^-39 of its vector's largest).
-    const HalfOperand x = operand(r.x), xt = operand(r.xt);
-    HalfProblem gram{};              // L = beta L + (1 - beta) G G^T, R likewise
-    gram.mode = kEpiStore;
-    gram.symmetric = 1;
-    gram.alpha = static_cast<float>(1.0 - s.beta);
-    gram.beta = static_cast<float>(s.beta);
-    gram.M = gram.N = r.rows; gram.K = r.cols;
-    gram.C = s.left_gram; gram.ldc = s.ld_left;
-    gemm_half(xt, xt, gram, status, side);
-    gram.M = gram.N = r.cols; gram.K = r.rows;
-    gram.C = s.right_gram; gram.ldc = s.ld_right;
-    gemm_half(x, x, gram, status, side);
-  }
+  issue(steps[0], stream,
+        [&] {
+          PlanesJob jobs[kHalfGroup];
+          for (int i = 0; i < count; ++i) jobs[i] = planes_of(steps[i].rotation);
+          half_planes_group(jobs, count, stream);
+        },
+        [&](auto product, cudaStream_t on) {
+          HalfJob jobs[kHalfGroup];
+          for (int i = 0; i < count; ++i) jobs[i] = product(steps[i]);
+          gemm_half_group(jobs, count, status, on);
+        });
 }
 
 }  // namespace soapb200

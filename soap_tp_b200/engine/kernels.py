@@ -335,6 +335,7 @@ def half_planes(source: Tensor, plain: Optional[HalfPlanes] = None, turned: Opti
     _C.half_planes(source.data_ptr(), int(source.dtype == torch.bfloat16), source.stride(0), source.stride(1), rows, cols,
                    *(plain.target() if plain is not None else _NO_TARGET),
                    *(turned.target() if turned is not None else _NO_TARGET), _stream())
+    _count("clear_kernel")
     _count("largest_kernel")
     _count("half_planes_kernel")
 
@@ -571,7 +572,7 @@ def rotate_half(scratch, matrix_and_bases: tuple, turned: bool, out: Tensor) -> 
     assert out.stride(0) == 1 or out.shape[0] == 1
     _C.rotate_half(scratch, matrix_and_bases + (int(turned), out.data_ptr(), _ld(out), status_word(out.device).data_ptr(), _stream()))
     mark_written(out)
-    for name in ("largest_kernel", "half_planes_kernel", "gemm_half_kernel", "gemm_half_kernel"):
+    for name in ("clear_kernel", "largest_kernel", "half_planes_kernel", "gemm_half_kernel", "gemm_half_kernel"):
         _count(name)
 
 
@@ -590,16 +591,27 @@ def _addressable(*tensors: Tensor) -> bool:
     return tensors[0].is_cuda and index == torch.cuda.current_device()
 
 
+def apply_updates(pairs, keep: float, lr: float) -> list:
+    """``p.mul_(keep); p.add_(update.to(p.dtype), alpha=-lr)`` for several ``(p, update)`` in one pass each and as few launches as
+    there are parameter types, value for value; returns the pairs that the kernel does not take (nothing is done to them)."""
+    jobs: Dict[int, list] = {}
+    left = []
+    for p, update in pairs:
+        kind = _PARAMETER_TYPES.get(p.dtype)
+        if kind is None or update.dtype != torch.float32 or not _addressable(p, update):
+            left.append((p, update))
+        else:
+            jobs.setdefault(kind, []).append((p, (p.data_ptr(), update.data_ptr(), p.numel())))
+    for kind, some in jobs.items():
+        _C.apply_updates([job for _, job in some], kind, keep, lr, _stream())
+        mark_written(*(p for p, _ in some))
+        _count("apply_updates_kernel")
+    return left
+
+
 def apply_update(p: Tensor, update: Tensor, keep: float, lr: float) -> bool:
-    """``p.mul_(keep); p.add_(update.to(p.dtype), alpha=-lr)`` in one pass, value for value; ``False`` (and nothing done) for
-    tensors that the kernel does not take."""
-    kind = _PARAMETER_TYPES.get(p.dtype)
-    if kind is None or update.dtype != torch.float32 or not _addressable(p, update):
-        return False
-    _C.apply_update(p.data_ptr(), kind, update.data_ptr(), p.numel(), keep, lr, _stream())
-    mark_written(p)
-    _count("apply_update_kernel")
-    return True
+    """The same for one; ``False`` (and nothing done) for tensors that the kernel does not take."""
+    return not apply_updates([(p, update)], keep, lr)
 
 
 def adamw_update(p: Tensor, gradient: Tensor, exp_avg: Tensor, exp_avg_sq: Tensor, beta1: float, beta2: float, bias1: float,

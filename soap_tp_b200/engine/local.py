@@ -138,10 +138,10 @@ def product(a, b, **epilogue) -> None:
     (k.gemm_half if isinstance(a, k.HalfPlanes) else k.gemm)(a, b, **epilogue)
 
 
-def workspace_planes(tag: str, depth: int, cols: int, device, *, blocked: bool = False, terms: int = 2):
+def workspace_planes(tag: str, depth: int, cols: int, device, *, blocked: bool = False, terms: int = 2, slot: int = 0):
     """Scratch operand planes shared by every parameter of the same shape on ``device``.  ``blocked``: written by a
-    product's epilogue; ``terms=1``: written from bf16 values."""
-    key = (tag, depth, cols, str(device), terms, blocked, k.MIXED_CORRECTIONS and tag not in CLASSIC_TAGS)
+    product's epilogue; ``terms=1``: written from bf16 values; ``slot``: one more set, for steps that share launches."""
+    key = (tag, depth, cols, str(device), terms, blocked, k.MIXED_CORRECTIONS and tag not in CLASSIC_TAGS, slot)
     planes = _WORKSPACES.get(key)
     if planes is None:
         planes = (k.Planes.empty(depth, cols, device) if tag in CLASSIC_TAGS
@@ -177,9 +177,9 @@ def gradient_planes(gradient: Tensor, *, plain: Optional[str] = None, turned: Op
     return xp, gtp
 
 
-def tf32_workspace(tag: str, depth: int, cols: int, device) -> k.Planes:
+def tf32_workspace(tag: str, depth: int, cols: int, device, slot: int = 0) -> k.Planes:
     """Scratch planes of the tf32 form with bf16 corrections (``kernels.Planes``, mixed)."""
-    key = ("tf32", tag, depth, cols, str(device))
+    key = ("tf32", tag, depth, cols, str(device), slot)
     planes = _WORKSPACES.get(key)
     if planes is None:
         planes = _WORKSPACES[key] = _tf32_operand(depth, cols, device)
@@ -215,31 +215,32 @@ class _Scratch:
     """Buffers of a rotation as the native calls take them, shared by matrices of one shape: with ``update`` those of a step's
     way back as well, with ``averages`` the planes of its Gram products."""
 
-    def __init__(self, rows: int, cols: int, device, terms: int, update: bool, averages: bool) -> None:
+    def __init__(self, rows: int, cols: int, device, terms: int, update: bool, averages: bool, slot: int) -> None:
         self.wide = torch.zeros(1, dtype=torch.int32, device=device)        # the decision on the range
         self.maxima = torch.empty(max(1, rows), dtype=torch.int32, device=device)
-        planes = [workspace_planes("X", rows, cols, device, terms=terms)]
+        planes = [workspace_planes("X", rows, cols, device, terms=terms, slot=slot)]
         if averages:
-            planes.append(workspace_planes("GT", cols, rows, device, terms=terms))
-        middle = workspace_planes("T", cols, rows, device, blocked=True)
-        mixed = [tf32_workspace(*size, device) for size in (
+            planes.append(workspace_planes("GT", cols, rows, device, terms=terms, slot=slot))
+        middle = workspace_planes("T", cols, rows, device, blocked=True, slot=slot)
+        mixed = [tf32_workspace(*size, device, slot) for size in (
             ("G", rows, cols), ("T", cols, rows), ("L", rows, rows), ("LT", rows, rows), ("R", cols, cols), ("RT", cols, cols))]
         turned = planes[1].target() if averages else (0, 0, 64, 0, self.maxima.data_ptr())
         addresses = (planes[0].target() + turned + middle.operand() + (self.wide.data_ptr(), int(k.SPLIT_ROUND_NEAREST))
                      + tuple(value for each in mixed for value in each.mixed_target()))
         self.keep = planes + [middle] + mixed                               # (addresses alone hold nothing)
         if update:
-            update_planes, mixed_update = workspace_planes("U", rows, cols, device, blocked=True), tf32_workspace("U", rows, cols, device)
+            update_planes = workspace_planes("U", rows, cols, device, blocked=True, slot=slot)
+            mixed_update = tf32_workspace("U", rows, cols, device, slot)
             addresses += update_planes.operand() + mixed_update.mixed_target()
             self.keep += [update_planes, mixed_update]
         self.native = _C.RotationScratch(rows, cols, addresses)
 
 
-def _scratch(rows: int, cols: int, device, terms: int, update: bool = False, averages: bool = False) -> _Scratch:
-    key = ("scratch", rows, cols, device, terms, update, averages)
+def _scratch(rows: int, cols: int, device, terms: int, update: bool = False, averages: bool = False, slot: int = 0) -> _Scratch:
+    key = ("scratch", rows, cols, device, terms, update, averages, slot)
     entry = _WORKSPACES.get(key)
     if entry is None:
-        entry = _WORKSPACES[key] = _Scratch(rows, cols, device, terms, update, averages)
+        entry = _WORKSPACES[key] = _Scratch(rows, cols, device, terms, update, averages, slot)
     return entry
 
 
@@ -276,8 +277,9 @@ def _side_stream(device, home: int) -> int:
     return stream.cuda_stream
 
 
-def _native_step(gradient: Tensor, state, step: int, rows: int, cols: int, *, beta, beta1, beta2, eps, averages: bool) -> Tensor:
-    """An ordinary step, its eight launches issued by one native call; without ``averages`` the rotations and Adam only."""
+def _native_arguments(gradient: Tensor, state, step: int, rows: int, cols: int, averages: bool, slot: int, *, beta, beta1, beta2,
+                      eps) -> tuple:
+    """An ordinary step as the native call takes it: scratch, addresses and scalars; then the tensor of its result."""
     g = gradient.detach().reshape(rows, cols)
     if g.dtype != torch.float32 and g.dtype != torch.bfloat16:
         g = g.float()
@@ -287,24 +289,72 @@ def _native_step(gradient: Tensor, state, step: int, rows: int, cols: int, *, be
     bias2 = 1.0 - beta2**step
     momentum, variance = state["momentum"], state["variance"]
     left, right = state["left_preconditioner"], state["right_preconditioner"]
-    scratch = _scratch(rows, cols, g.device, 1 if g.dtype == torch.bfloat16 else 2, update=True, averages=averages)
+    scratch = _scratch(rows, cols, g.device, 1 if g.dtype == torch.bfloat16 else 2, update=True, averages=averages, slot=slot)
     update = torch.empty((rows, cols), dtype=torch.float32, device=g.device)
     arguments = (k.strided_source(g) + ctx.left.addresses + ctx.right.addresses
                  + (momentum.data_ptr(), k._ld(momentum), variance.data_ptr(), k._ld(variance), update.data_ptr(),
                     left.data_ptr(), k._ld(left), right.data_ptr(), k._ld(right)))
-    home = k._stream()
-    tail = (k.status_word(g.device).data_ptr(), home, _side_stream(g.device, home))
     scalars = (beta, beta1, beta2, eps / math.sqrt(bias2), 1.0 / (1.0 - beta1**step), 1.0 / math.sqrt(bias2))
+    # (the gradient and the planes of the bases are held until the launches are issued)
+    return (scratch.native, arguments, scalars), update, (g, ctx)
+
+
+def _count_launches(averages: bool) -> None:
+    for name, count in (("clear_kernel", 1), ("largest_kernel", 1), ("half_planes_kernel", 1), ("gemm_half_kernel", 6 if averages else 4)):
+        k.LAUNCH_COUNTS[name] = k.LAUNCH_COUNTS.get(name, 0) + count
+
+
+_WRITTEN = ("momentum", "variance", "left_preconditioner", "right_preconditioner")
+
+
+def _native_step(gradient: Tensor, state, step: int, rows: int, cols: int, *, beta, beta1, beta2, eps, averages: bool) -> Tensor:
+    """An ordinary step, its launches issued by one native call; without ``averages`` the rotations and Adam only."""
+    call, update, held = _native_arguments(gradient, state, step, rows, cols, averages, 0, beta=beta, beta1=beta1, beta2=beta2, eps=eps)
+    home = k._stream()
+    tail = (k.status_word(update.device).data_ptr(), home, _side_stream(update.device, home))
     if TIMER.enabled:
         for name, phase in _STEP_STAGES if averages else _STEP_STAGES[:-1]:
-            with TIMER.stage(name, g.device):
-                _C.steady_step(scratch.native, arguments + (phase,) + tail, *scalars)
+            with TIMER.stage(name, update.device):
+                _C.steady_step(*call, phase, *tail)
     else:
-        _C.steady_step(scratch.native, arguments + (_ALL_PHASES if averages else _ALL_PHASES - _C.STEP_AVERAGES,) + tail, *scalars)
-    torch.autograd.graph.increment_version((momentum, variance, left, right) if averages else (momentum, variance))
-    for name, count in (("largest_kernel", 1), ("half_planes_kernel", 1), ("gemm_half_kernel", 6 if averages else 4)):
-        k.LAUNCH_COUNTS[name] = k.LAUNCH_COUNTS.get(name, 0) + count
+        _C.steady_step(*call, _ALL_PHASES if averages else _ALL_PHASES - _C.STEP_AVERAGES, *tail)
+    torch.autograd.graph.increment_version([state[name] for name in (_WRITTEN if averages else _WRITTEN[:2])])
+    _count_launches(averages)
     return update
+
+
+def shares_launches(state, rows: int, cols: int, interval: int) -> bool:
+    """Whether the next step of this parameter is an ordinary one whose launches it can share with other small parameters'."""
+    return (k.MIXED_CORRECTIONS and not TIMER.enabled and "left_basis" in state and (int(state["step"]) + 1) % interval != 0
+            and _C.steady_step_shares(rows, cols))
+
+
+def shared_steps(parameters, *, beta: float, beta1: float, beta2: float, eps: float) -> list:
+    """Ordinary steps of several small parameters, ``(gradient, state, rows, cols)`` each, on one device; their updates.
+
+    A product of a small matrix leaves most of the GPU idle and ends in latencies (fill, drain, epilogue, launch) that are as
+    long as its work; eight of them in one launch take about as long as one."""
+    for _, state, rows, cols in parameters:
+        _check_state(state, rows, cols)
+    updates = []
+    for first in range(0, len(parameters), _C.STEP_GROUP):
+        some = parameters[first:first + _C.STEP_GROUP]
+        calls, held, used = [], [], {}
+        for gradient, state, rows, cols in some:
+            # parameters of one shape that run together have scratch of their own each
+            slot = used[(rows, cols)] = used.get((rows, cols), -1) + 1
+            call, update, holds = _native_arguments(gradient, state, int(state["step"]) + 1, rows, cols, True, slot, beta=beta,
+                                                    beta1=beta1, beta2=beta2, eps=eps)
+            calls.append(call)
+            held.append(holds)
+            updates.append(update)
+        device, home = updates[-1].device, k._stream()
+        _C.steady_steps(calls, k.status_word(device).data_ptr(), home, _side_stream(device, home))
+        torch.autograd.graph.increment_version([state[name] for _, state, _, _ in some for name in _WRITTEN])
+        for _, state, _, _ in some:
+            state["step"] = int(state["step"]) + 1
+        _count_launches(True)
+    return updates
 
 
 _STEP_STAGES = (("split_gradient", _C.STEP_PLANES), ("rotate_forward+adam", _C.STEP_FORWARD),

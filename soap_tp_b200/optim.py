@@ -32,19 +32,21 @@ import torch.distributed as dist
 from torch import Tensor
 
 from .layout import allocate_2d_block_cyclic, most_square_grid
+from .ops.basis import BASIS_IMPLEMENTATIONS
+from .profiling import profile_enabled
 from .step import soap_step, state_shapes
 
 
-def _apply(p: Tensor, update: Tensor, lr: float, weight_decay: float) -> None:
-    """Decoupled weight decay, then the update."""
-    if p.is_cuda:
+def _apply(pairs, lr: float, weight_decay: float) -> None:
+    """Decoupled weight decay, then the update, of several ``(p, update)``."""
+    if pairs and pairs[0][0].is_cuda:
         from .engine import kernels
 
-        if kernels.apply_update(p, update, 1.0 - lr * weight_decay, lr):
-            return
-    if weight_decay != 0.0:
-        p.mul_(1.0 - lr * weight_decay)
-    p.add_(update.to(p.dtype), alpha=-lr)
+        pairs = kernels.apply_updates(pairs, 1.0 - lr * weight_decay, lr)
+    for p, update in pairs:
+        if weight_decay != 0.0:
+            p.mul_(1.0 - lr * weight_decay)
+        p.add_(update.to(p.dtype), alpha=-lr)
 
 
 class SoapTP(torch.optim.Optimizer):
@@ -117,6 +119,7 @@ class SoapTP(torch.optim.Optimizer):
         world, rank = dist.get_world_size(), dist.get_rank()
         for group in self.param_groups:
             lr, wd = group["lr"], group["weight_decay"]
+            together = []        # small matrices on an ordinary step
             for p in group["params"]:
                 if p.grad is None:
                     continue
@@ -137,7 +140,10 @@ class SoapTP(torch.optim.Optimizer):
                         interval=group["precondition_frequency"], implementation=group["basis_implementation"])
                     if not rows_sharded:
                         update = update.T
-                    _apply(p, update, lr, wd)
+                    _apply([(p, update)], lr, wd)
+                    continue
+                if world == 1 and self._shares_launches(p, state, plan, group):
+                    together.append((p, (gradient, state, *plan["global_shape"])))
                     continue
                 if plan["replicated"] and world > 1:
                     gradient = gradient.chunk(world, dim=plan["shard_dim"])[rank].contiguous()
@@ -152,8 +158,28 @@ class SoapTP(torch.optim.Optimizer):
                     parts = [torch.empty_like(update) for _ in range(world)]
                     dist.all_gather(parts, update.contiguous())
                     update = torch.cat(parts, dim=plan["shard_dim"])
-                _apply(p, update, lr, wd)
+                _apply([(p, update)], lr, wd)
+            if together:
+                from .engine import kernels, local
+
+                updates = local.shared_steps([arguments for _, arguments in together], beta=group["shampoo_beta"],
+                                             beta1=group["betas"][0], beta2=group["betas"][1], eps=group["eps"])
+                _apply([(p, update.view(p.grad.shape)) for (p, _), update in zip(together, updates)], lr, wd)
+                kernels.poll_status(together[0][0].device)
         return loss
+
+    @staticmethod
+    def _shares_launches(p: Tensor, state: dict, plan: dict, group: dict) -> bool:
+        """Whether ``p`` takes its step together with the group's other small matrices, in the same launches; what is refused, or
+        traced, is left to ``soap_step``."""
+        if (not p.is_cuda or p.get_device() != torch.cuda.current_device() or p.grad.get_device() != p.get_device()
+                or group["basis_implementation"] not in BASIS_IMPLEMENTATIONS or "left_basis" not in state
+                or profile_enabled(int(state["step"]) + 1)):
+            return False
+        from .engine import local
+
+        rows, cols = plan["global_shape"]
+        return p.grad.numel() == rows * cols and local.shares_launches(state, rows, cols, group["precondition_frequency"])
 
     def _adamw(self, p: Tensor, group: dict) -> None:
         state = self.state[p]

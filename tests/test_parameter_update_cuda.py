@@ -72,3 +72,22 @@ def test_adamw_average_is_lerp_for_every_beta(beta1):
     assert torch.equal(m, expected)
     if beta1 == 0.0:
         assert torch.equal(m, grad)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("count", [2, 16, 17])
+def test_apply_several_at_once(dtype, count):
+    """More parameters than a launch takes, aligned and not, empty ones, and two that share memory (one after the other)."""
+    from soap_tp_b200.engine import kernels as k
+
+    g = torch.Generator().manual_seed(count)
+    flat = torch.randn(40000, generator=g).to(dtype).cuda()
+    sizes = [0, 1, 5, 512, 1025, 3000][:count] + [777] * max(0, count - 6)
+    starts = [sum(sizes[:i]) for i in range(count)]
+    parameters = [flat[a:a + n] for a, n in zip(starts, sizes)] + [flat[100:900]]
+    pairs = [(p, torch.randn(p.numel(), generator=g).cuda()) for p in parameters]
+    expected = flat.clone()
+    for (a, n), (_, update) in zip(list(zip(starts, sizes)) + [(100, 800)], pairs):
+        expected[a:a + n].mul_(0.99).add_(update.to(dtype), alpha=-3e-3)
+    assert k.apply_updates(pairs, 0.99, 3e-3) == []
+    assert torch.equal(flat, expected)
