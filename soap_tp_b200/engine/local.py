@@ -35,6 +35,9 @@ from . import factor
 _C = k._C
 
 
+_NO_OPERAND = (0, 0, 64, 0, 0)        # of an orientation that the native call does not use
+
+
 class BasisPlanes:
     """Both orientations of one orthogonal basis as operand planes, tied to a tensor version."""
 
@@ -46,6 +49,20 @@ class BasisPlanes:
         self.transposed = None            # operand Q^T (depth = cols of Q)
         self.addresses: tuple = ()        # both, and the basis itself, as the native calls take them
         self.copy: Optional[Tensor] = None    # of a basis of another type, which the addresses mean then
+
+    def once(self, Q: Tensor, size: int, turned: bool) -> "BasisPlanes":
+        """The planes of one orientation only, for one use."""
+        view = Q[:size, :size]
+        self.copy = None if Q.dtype == torch.float32 else view.float()
+        if self.copy is not None:
+            view = self.copy
+        planes = (_operand if self.half else _tf32_operand)(size, size, Q.device)
+        self.plain, self.transposed = (None, planes) if turned else (planes, None)
+        split(view, self.plain, self.transposed)
+        if isinstance(planes, k.HalfPlanes):
+            here = planes.operand()
+            self.addresses = (_NO_OPERAND + here if turned else here + _NO_OPERAND) + (view.data_ptr(), *view.stride())
+        return self
 
     def refresh(self, Q: Tensor, size: int) -> None:
         key = (Q.data_ptr(), Q._version, size)
@@ -504,11 +521,10 @@ def prepare_refresh(rows: int, cols: int, device) -> None:
 
 def rotate(matrix: Tensor, Q_left: Tensor, Q_right: Tensor, global_shape, direction: str) -> Tensor:
     rows, cols = global_shape
-    left, right = BasisPlanes(), BasisPlanes()
-    left.refresh(Q_left, rows)
-    right.refresh(Q_right, cols)
+    turned = direction != "forward"
+    left, right = BasisPlanes().once(Q_left, rows, turned), BasisPlanes().once(Q_right, cols, turned)
     view = matrix[:rows, :cols]
-    rotate_matrix(view, left, right, direction != "forward", view)
+    rotate_matrix(view, left, right, turned, view)
     return matrix
 
 
