@@ -460,7 +460,10 @@ gemm_tf32x3_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant_
   const int m0 = tile_m * kBM;
   const int n0 = tile_n * BN;
   // Symmetric products: tiles strictly above the diagonal are produced by mirroring.
-  if (prob.symmetric && global_col(prob, n0) > global_row(prob, min(m0 + kBM, prob.M) - 1)) return;
+  if (prob.symmetric && global_col(prob, n0) > global_row(prob, min(m0 + kBM, prob.M) - 1)) {
+    wait_for_predecessor();      // (no part of this grid ends before its predecessor has)
+    return;
+  }
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < Cfg::kStages; ++s) {
@@ -486,6 +489,8 @@ gemm_tf32x3_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant_
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  wait_for_predecessor();
+  let_successor_start();
 
   const SplitRange range = split_range(prob.K);
   const int kb_first = range.first * (32 / kBK), k_blocks = range.count * (32 / kBK);
@@ -702,7 +707,10 @@ gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ 
   const int n0 = tile_n * BN;
   const int b_row0 = n0 + static_cast<int>(cta) * (BN / 2);  // this CTA's half of the B tile
   // Symmetric products: pair tiles strictly above the diagonal are produced by mirroring (same decision in both CTAs).
-  if (prob.symmetric && global_col(prob, n0) > global_row(prob, min(pair_m0 + 2 * kBM, prob.M) - 1)) return;
+  if (prob.symmetric && global_col(prob, n0) > global_row(prob, min(pair_m0 + 2 * kBM, prob.M) - 1)) {
+    wait_for_predecessor();
+    return;
+  }
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kPairStages; ++s) {
@@ -729,6 +737,8 @@ gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ 
   cluster_sync_all();                 // both CTAs' barriers exist before anything arrives on them remotely
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  wait_for_predecessor();
+  let_successor_start();
 
   const SplitRange range = split_range(prob.K);
   const int kb_first = range.first, k_blocks = range.count;
@@ -906,8 +916,8 @@ void launch(const GemmOperands& ops, const GemmProblem& prob, int* status, cudaS
   const int tiles_n = (prob.N + BN - 1) / BN;
   const int splits = (MODE == kEpiStore && prob.k_splits > 1) ? prob.k_splits : 1;
   dim3 grid(tiles_m * tiles_n, splits, prob.batches > 1 ? prob.batches : 1);
-  gemm_tf32x3_kernel<Cfg, MODE, MIXED><<<grid, Cfg::kThreads, Cfg::kSmemBytes, stream>>>(maps, prob, status);
-  cudaError_t err = cudaGetLastError();
+  const cudaError_t err =
+      launch_dependent(gemm_tf32x3_kernel<Cfg, MODE, MIXED>, grid, dim3(Cfg::kThreads), Cfg::kSmemBytes, stream, maps, prob, status);
   if (err != cudaSuccess) throw std::runtime_error(std::string("gemm_tf32x3 launch: ") + cudaGetErrorString(err));
 }
 
@@ -931,8 +941,8 @@ void launch_pair(const GemmOperands& ops, const GemmProblem& prob, int* status, 
   const int tiles_n = (prob.N + kPairBN - 1) / kPairBN;
   const int splits = (MODE == kEpiStore && prob.k_splits > 1) ? prob.k_splits : 1;
   dim3 grid(2 * tiles_m * tiles_n, splits, 1);
-  gemm_pair_kernel<MODE, MIXED><<<grid, kThreads, kPairSmemBytes, stream>>>(maps, prob, status);
-  cudaError_t err = cudaGetLastError();
+  const cudaError_t err =
+      launch_dependent(gemm_pair_kernel<MODE, MIXED>, grid, dim3(kThreads), kPairSmemBytes, stream, maps, prob, status);
   if (err != cudaSuccess) throw std::runtime_error(std::string("gemm_pair launch: ") + cudaGetErrorString(err));
 }
 

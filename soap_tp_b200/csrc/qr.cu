@@ -302,15 +302,29 @@ __global__ void __launch_bounds__(kPanelThreads, 1) qr_panel_kernel(PanelArgs a)
   }
 }
 
-__global__ void sum_partials_kernel(const float* __restrict__ partials, int splits, int64_t stride, int64_t ld, float* hi,
-                                    float* lo, int64_t ldp, int rows, int cols) {
-  const int64_t total = static_cast<int64_t>(rows) * cols;
-  for (int64_t idx = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; idx < total;
-       idx += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int i = static_cast<int>(idx % rows);
-    const int64_t c = idx / rows;
+// Bound by latency (128 x r results from L2): the loads of four parts are in flight together, and the index is divided in 32 bits
+// where it fits.  The parts are added in their order.
+template <typename Index>
+__global__ void sum_partials_kernel(const float* partials, int splits, int64_t stride, int64_t ld, float* hi, float* lo, int64_t ldp,
+                                    int rows, int cols) {
+  wait_for_predecessor();
+  let_successor_start();
+  const Index total = static_cast<Index>(rows) * static_cast<Index>(cols);
+  for (Index idx = blockIdx.x * static_cast<Index>(blockDim.x) + threadIdx.x; idx < total;
+       idx += static_cast<Index>(gridDim.x) * blockDim.x) {
+    const int64_t c = idx / static_cast<Index>(rows);
+    const int i = static_cast<int>(idx - static_cast<Index>(c) * rows);
+    const float* from = partials + i + c * ld;
     float acc = 0.f;
-    for (int s = 0; s < splits; ++s) acc += partials[s * stride + i + c * ld];
+    int s = 0;
+    for (; s + 4 <= splits; s += 4) {
+      const float x0 = from[s * stride], x1 = from[(s + 1) * stride], x2 = from[(s + 2) * stride], x3 = from[(s + 3) * stride];
+      acc += x0;
+      acc += x1;
+      acc += x2;
+      acc += x3;
+    }
+    for (; s < splits; ++s) acc += from[s * stride];
     const float h = tf32_rn(acc);
     hi[i + c * ldp] = h;
     lo[i + c * ldp] = acc - h;
@@ -380,9 +394,11 @@ void qr_panel(const float* p_hi, const float* p_lo, int64_t ldp, int r, int b, f
 void sum_partials_to_planes(const float* partials, int splits, int64_t stride, int64_t ld, float* hi, float* lo,
                             int64_t ldp, int rows, int cols, cudaStream_t stream) {
   if (rows <= 0 || cols <= 0) return;
-  sum_partials_kernel<<<grid_for(static_cast<int64_t>(rows) * cols), 256, 0, stream>>>(partials, splits, stride, ld, hi, lo,
-                                                                                   ldp, rows, cols);
-  check_launch("sum_partials_kernel");
+  const int64_t total = static_cast<int64_t>(rows) * cols;
+  auto* kernel = total < (int64_t{1} << 31) ? sum_partials_kernel<uint32_t> : sum_partials_kernel<int64_t>;
+  const cudaError_t err = launch_dependent(kernel, dim3(grid_for(total)), dim3(256), 0, stream, partials, splits, stride, ld, hi, lo, ldp,
+                                           rows, cols);
+  if (err != cudaSuccess) throw std::runtime_error(std::string("sum_partials_kernel: ") + cudaGetErrorString(err));
 }
 
 void identity_planes(float* hi, float* lo, int64_t ldp, int rows, int cols, cudaStream_t stream, int first_col) {
