@@ -10,6 +10,7 @@
 #include <array>
 #include <cstdint>
 #include <stdexcept>
+#include <string>
 #include <tuple>
 #include <vector>
 
@@ -71,19 +72,53 @@ class Arguments {
 };
 }  // namespace
 
+// The planes of a basis in both orientations (one of them may be absent), handed over once with the basis itself.
+struct BasisOperands {
+  HalfOperand plain{}, turned{};
+  const float* src;
+  int64_t s_i, s_j;
+  CUtensorMap maps[2][2];
+
+  BasisOperands(int size, const std::vector<int64_t>& values) {
+    Arguments in(values);
+    int i = 0;
+    for (HalfOperand* o : {&plain, &turned}) {
+      *o = in.operand();
+      if (o->h) {
+        half_maps(maps[i], o->h, o->l, o->ld, size, size);
+        o->maps = maps[i];
+      }
+      ++i;
+    }
+    src = in.pointer<float>(); s_i = in.next(); s_j = in.next();
+    in.finish();
+  }
+  BasisOperands(const BasisOperands&) = delete;              // (the operands point into the object)
+  BasisOperands& operator=(const BasisOperands&) = delete;
+};
+
 // The scratch of rotations of one shape, handed over once: planes, the decision on the range, and the mixed form of everything.
 struct RotationScratch {
   Rotation rotation{};       // without the matrix and its bases
   HalfOperand update{};
   SplitTarget mixed_update{};
-  CUtensorMap source_maps[2], middle_maps[2], update_maps[2], basis_maps[4][2];      // bases: left, its transpose, right, ...
+  CUtensorMap source_maps[2], middle_maps[2], update_maps[2], basis_maps[4][2];      // mixed; bases: left, its transpose, right, ...
+  CUtensorMap x_maps[2], xt_maps[2], half_middle_maps[2], half_update_maps[2];       // fp16 pairs
 
   RotationScratch(int rows, int cols, const std::vector<int64_t>& values) {
     Arguments in(values);
     Rotation& r = rotation;
     r.rows = rows; r.cols = cols;
     r.x = in.target(); r.xt = in.target();
+    half_maps(x_maps, r.x.h, r.x.l, r.x.ld, rows, cols);
+    r.x_maps = x_maps;
+    if (r.xt.h) {
+      half_maps(xt_maps, r.xt.h, r.xt.l, r.xt.ld, cols, rows);
+      r.xt_maps = xt_maps;
+    }
     r.middle = in.operand();
+    half_maps(half_middle_maps, r.middle.h, r.middle.l, r.middle.ld, cols, rows);
+    r.middle.maps = half_middle_maps;
     r.guard.wide = in.pointer<int>(); r.guard.nearest = static_cast<int>(in.next());
     r.guard.mixed = in.mixed();
     r.mixed_middle = in.mixed();
@@ -104,6 +139,8 @@ struct RotationScratch {
       mixed_update = in.mixed();
       mixed_maps(update_maps, mixed_update, rows, cols);
       update.mixed = update_maps;
+      half_maps(half_update_maps, update.h, update.l, update.ld, rows, cols);
+      update.maps = half_update_maps;
     }
     in.finish();
   }
@@ -111,17 +148,16 @@ struct RotationScratch {
   RotationScratch& operator=(const RotationScratch&) = delete;
 
   // The rotation of a matrix by its bases.
-  Rotation of(Arguments& in) const {
+  Rotation of(Arguments& in, const BasisOperands& left, const BasisOperands& right) const {
     Rotation r = rotation;
     r.source = in.pointer<void>(); r.source_type = static_cast<int>(in.next()); r.s_i = in.next(); r.s_j = in.next();
+    r.left = left.plain; r.left_turned = left.turned; r.right = right.plain; r.right_turned = right.turned;
     HalfOperand* const planes[] = {&r.left, &r.left_turned, &r.right, &r.right_turned};
-    for (int i = 0; i < 4; ++i) {
-      *planes[i] = in.operand();
-      planes[i]->mixed = basis_maps[i];
-      if (i % 2) {
-        WideBasis& basis = r.guard.bases[i / 2];
-        basis.src = in.pointer<float>(); basis.s_i = in.next(); basis.s_j = in.next();
-      }
+    for (int i = 0; i < 4; ++i) planes[i]->mixed = basis_maps[i];
+    for (int side = 0; side < 2; ++side) {
+      const BasisOperands& from = side ? right : left;
+      WideBasis& basis = r.guard.bases[side];
+      basis.src = from.src; basis.s_i = from.s_i; basis.s_j = from.s_j;
     }
     return r;
   }
@@ -129,9 +165,10 @@ struct RotationScratch {
 
 namespace {
 // An ordinary step's operands, results and scalars (beta, beta1, beta2, eps, 1 / bias 1, 1 / sqrt(bias 2)).
-SteadyStep step_of(const RotationScratch& scratch, Arguments& in, const std::array<double, 6>& scalars) {
+SteadyStep step_of(const RotationScratch& scratch, const BasisOperands& left, const BasisOperands& right, Arguments& in,
+                   const std::array<double, 6>& scalars) {
   SteadyStep s{};
-  s.rotation = scratch.of(in);
+  s.rotation = scratch.of(in, left, right);
   s.update = scratch.update;
   s.mixed_update = scratch.mixed_update;
   s.momentum = in.pointer<float>(); s.ldm = in.next();
@@ -245,12 +282,36 @@ PYBIND11_MODULE(_C, m) {
 
   py::class_<RotationScratch>(m, "RotationScratch", "Scratch planes of rotations of one shape, as addresses (see Arguments)")
       .def(py::init<int, int, const std::vector<int64_t>&>());
-  // Integers: the matrix and its bases (RotationScratch::of), the moments and results in the order of SteadyStep; then of the call: the
-  // phases, the status word, the stream and the stream of the averages.
-  m.def("steady_step", [](const RotationScratch& scratch, const std::vector<int64_t>& v, const std::array<double, 6>& scalars, int phases,
-                          uint64_t status, uint64_t stream, uint64_t side) {
+  py::class_<BasisOperands>(m, "BasisOperands", "Planes of a basis in both orientations, and the basis, as addresses")
+      .def(py::init<int, const std::vector<int64_t>&>());
+  // A plain product of classic planes.  Integers: hi, lo, pitch of both operands; M, N, K, mode, symmetric, force_narrow; result, its
+  // pitch; hi, lo, pitch of the result's planes; splits and the distance of their results; the status word and the stream.
+  m.def("gemm_planes", [](const std::vector<int64_t>& v, float alpha, float beta) {
     Arguments in(v);
-    SteadyStep s = step_of(scratch, in, scalars);
+    GemmOperands ops{};
+    ops.a_hi = in.pointer<const float>(); ops.a_lo = in.pointer<const float>(); ops.lda = in.next();
+    ops.b_hi = in.pointer<const float>(); ops.b_lo = in.pointer<const float>(); ops.ldb = in.next();
+    GemmProblem prob{};
+    prob.M = static_cast<int>(in.next()); prob.N = static_cast<int>(in.next()); prob.K = static_cast<int>(in.next());
+    prob.mode = static_cast<int>(in.next()); prob.symmetric = static_cast<int>(in.next()); prob.force_narrow = static_cast<int>(in.next());
+    prob.C = in.pointer<float>(); prob.ldc = in.next();
+    prob.Chi = in.pointer<float>(); prob.Clo = in.pointer<float>(); prob.ldp = in.next();
+    prob.k_splits = static_cast<int>(in.next()); prob.split_stride = in.next();
+    prob.alpha = alpha; prob.beta = beta;
+    int* status = in.pointer<int>();
+    cudaStream_t stream = in.stream();
+    in.finish();
+    py::gil_scoped_release release;
+    gemm_tf32x3(ops, prob, status, stream);
+  });
+
+  // Integers: the matrix (RotationScratch::of), the moments and results in the order of SteadyStep; then of the call: the phases, the
+  // status word, the stream and the stream of the averages.
+  m.def("steady_step", [](const RotationScratch& scratch, const BasisOperands& left, const BasisOperands& right,
+                          const std::vector<int64_t>& v, const std::array<double, 6>& scalars, int phases, uint64_t status, uint64_t stream,
+                          uint64_t side) {
+    Arguments in(v);
+    SteadyStep s = step_of(scratch, left, right, in, scalars);
     in.finish();
     s.phases = phases;
     s.side = stream_of(side);
@@ -259,13 +320,14 @@ PYBIND11_MODULE(_C, m) {
   }, "The launches of one ordinary single-GPU step, or some of its phases (gemm_half.h, SteadyStep)");
   m.def("steady_step_shares", &steady_step_shares, "Whether steps of such matrices can share launches");
   m.attr("STEP_GROUP") = kHalfGroup;
-  m.def("steady_steps", [](const std::vector<std::tuple<const RotationScratch*, std::vector<int64_t>, std::array<double, 6>>>& steps,
+  m.def("steady_steps", [](const std::vector<std::tuple<const RotationScratch*, const BasisOperands*, const BasisOperands*,
+                                                        std::vector<int64_t>, std::array<double, 6>>>& steps,
                            uint64_t status, uint64_t stream, uint64_t side) {
     std::vector<SteadyStep> all;
-    for (const auto& [scratch, v, scalars] : steps) {
-      if (!scratch) throw std::invalid_argument("steady_steps: no scratch");
+    for (const auto& [scratch, left, right, v, scalars] : steps) {
+      if (!scratch || !left || !right) throw std::invalid_argument("steady_steps: no scratch or bases");
       Arguments in(v);
-      all.push_back(step_of(*scratch, in, scalars));
+      all.push_back(step_of(*scratch, *left, *right, in, scalars));
       in.finish();
       all.back().phases = kStepPlanes | kStepForward | kStepBackward | kStepAverages;
       all.back().side = stream_of(side);
@@ -277,10 +339,10 @@ PYBIND11_MODULE(_C, m) {
   m.attr("STEP_FORWARD") = kStepForward;
   m.attr("STEP_BACKWARD") = kStepBackward;
   m.attr("STEP_AVERAGES") = kStepAverages;
-  // Integers: the matrix and its bases, then direction, result, its pitch, the status word and the stream.
-  m.def("rotate_half", [](const RotationScratch& scratch, const std::vector<int64_t>& v) {
+  // Integers: the matrix, then direction, result, its pitch, the status word and the stream.
+  m.def("rotate_half", [](const RotationScratch& scratch, const BasisOperands& left, const BasisOperands& right, const std::vector<int64_t>& v) {
     Arguments in(v);
-    const Rotation r = scratch.of(in);
+    const Rotation r = scratch.of(in, left, right);
     const bool turned = in.next() != 0;
     float* out = in.pointer<float>();
     const int64_t ldc = in.next();
@@ -290,6 +352,11 @@ PYBIND11_MODULE(_C, m) {
     py::gil_scoped_release release;
     rotate_half(r, turned, out, ldc, status, stream);
   }, "A matrix rotated by two bases on scaled fp16 planes, or on their mixed form where its range asks for it (gemm_half.h)");
+
+  m.def("read_status", [](uint64_t word, uint64_t pinned, uint64_t stream) {
+    const cudaError_t err = cudaMemcpyAsync(ptr<void>(pinned), ptr<const void>(word), sizeof(int), cudaMemcpyDeviceToHost, stream_of(stream));
+    if (err != cudaSuccess) throw std::runtime_error(std::string("read_status: ") + cudaGetErrorString(err));
+  }, "Copies a device's status word into pinned host memory");
 
   m.def("gemm_simt",
         [](uint64_t A, int64_t a_sk, int64_t a_sm, uint64_t B, int64_t b_sk, int64_t b_sn, uint64_t C, int64_t c_sm,

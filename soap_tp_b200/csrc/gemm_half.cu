@@ -648,6 +648,11 @@ void launch_mode(bool pairs, const HalfMaps* maps, const HalfArgs* args, int cou
 
 }  // namespace
 
+void half_maps(CUtensorMap (&maps)[2], const uint16_t* h, const uint16_t* l, int64_t ld, int64_t K, int64_t cols) {
+  maps[0] = make_map(h, K, cols, ld);
+  maps[1] = l ? make_map(l, K, cols, ld) : maps[0];
+}
+
 void mixed_maps(CUtensorMap (&maps)[2], const SplitTarget& planes, int64_t K, int64_t cols) {
   maps[0] = encode_k_major(CU_TENSOR_MAP_DATA_TYPE_FLOAT32, planes.hi, K, cols, 4 * planes.ldo, kMixedBK, 128, CU_TENSOR_MAP_SWIZZLE_128B);
   maps[1] = encode_interleaved(planes.hl, K, cols, planes.ld16, 2 * kMixedBK, 128);
@@ -683,10 +688,13 @@ void prepare(const HalfOperand& a, const HalfOperand& b, const HalfProblem& prob
                       !writes_pairs(prob.mixed)))
       throw std::invalid_argument("gemm_half: mixed output planes need 8-byte alignment and an even pitch");
   }
-  maps.a_h = make_map(a.h, prob.K, prob.M, a.ld);
-  maps.a_l = a.l ? make_map(a.l, prob.K, prob.M, a.ld) : maps.a_h;
-  maps.b_h = make_map(b.h, prob.K, prob.N, b.ld);
-  maps.b_l = b.l ? make_map(b.l, prob.K, prob.N, b.ld) : maps.b_h;
+  CUtensorMap made[2];
+  if (!a.maps) half_maps(made, a.h, a.l, a.ld, prob.K, prob.M);
+  maps.a_h = a.maps ? a.maps[0] : made[0];
+  maps.a_l = a.maps ? a.maps[1] : made[1];
+  if (!b.maps) half_maps(made, b.h, b.l, b.ld, prob.K, prob.N);
+  maps.b_h = b.maps ? b.maps[0] : made[0];
+  maps.b_l = b.maps ? b.maps[1] : made[1];
   if (prob.wide) {
     for (int i = 0; i < 2; ++i) {
       maps.mixed[i] = a.mixed[i];

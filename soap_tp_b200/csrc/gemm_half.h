@@ -27,9 +27,12 @@ struct HalfOperand {
   int64_t scale_stride;    // 0 for the second operand of a product, whose scales are applied after the sum over K
   // The same operand in the mixed form, read where HalfProblem::wide says so: maps of its two planes (mixed_maps).
   const CUtensorMap* mixed = nullptr;
+  // Maps of h and l where they were made with the planes (half_maps); null: made for the product.
+  const CUtensorMap* maps = nullptr;
 };
-// The tensor maps of K x cols mixed planes, which belong to scratch and are made once with it (a map takes the host 0.2 us, and a
-// step's products would need sixteen).
+// The tensor maps of K x cols planes, fp16 pairs and mixed, which belong to scratch or to a basis's planes and are made once with
+// them (a map takes the host 0.2 us, and a step's products need forty).
+void half_maps(CUtensorMap (&maps)[2], const uint16_t* h, const uint16_t* l, int64_t ld, int64_t K, int64_t cols);
 void mixed_maps(CUtensorMap (&maps)[2], const SplitTarget& planes, int64_t K, int64_t cols);
 
 constexpr int kHalfScaleBlock = 128;
@@ -132,6 +135,7 @@ struct Rotation {
   HalfOperand middle;                                        // scratch planes cols x rows, scales per block
   SplitTarget mixed_middle;                                  // the same in the mixed form
   const CUtensorMap* mixed_source;                           // maps of guard.mixed
+  const CUtensorMap *x_maps, *xt_maps;                       // of x and xt
   RangeGuard guard;
 };
 

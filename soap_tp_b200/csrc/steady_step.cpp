@@ -18,7 +18,7 @@
 namespace soapb200 {
 
 namespace {
-HalfOperand operand(const HalfTarget& t) { return HalfOperand{t.h, t.l, t.ld, t.scale, 0}; }
+HalfOperand operand(const HalfTarget& t, const CUtensorMap* maps) { return HalfOperand{t.h, t.l, t.ld, t.scale, 0, nullptr, maps}; }
 
 // A second stream that is forked from `home` and joined to it again when the scope ends, by whatever way.
 class Fork {
@@ -57,7 +57,7 @@ HalfJob first_product(const Rotation& r, const HalfOperand& source, bool settled
 }
 
 HalfOperand source_of(const Rotation& r) {
-  HalfOperand x = operand(r.x);
+  HalfOperand x = operand(r.x, r.x_maps);
   x.mixed = r.mixed_source;
   return x;
 }
@@ -104,7 +104,7 @@ HalfJob result(const SteadyStep& s) {                                       // T
 // vectors' own sizes, which the pairs keep in every range (2^-23 of an element, 2^-39 of its vector's largest).
 HalfJob average(const SteadyStep& s, bool left) {
   const Rotation& r = s.rotation;
-  const HalfOperand x = operand(left ? r.xt : r.x);
+  const HalfOperand x = left ? operand(r.xt, r.xt_maps) : operand(r.x, r.x_maps);
   HalfProblem p{};
   p.mode = kEpiStore;
   p.symmetric = 1;

@@ -116,9 +116,11 @@ class _StatusMonitor:
                 word.zero_()
                 self.pending = [False, False]
                 _raise_for(self.index, code)
-        self.words[self.turn].copy_(word[:1], non_blocking=True)
         if self.events is not None:
+            _C.read_status(word.data_ptr(), self.words[self.turn].data_ptr(), _stream())
             self.events[self.turn].record()
+        else:
+            self.words[self.turn].copy_(word[:1])
         self.pending[self.turn] = True
         self.turn = previous
 
@@ -198,6 +200,7 @@ class Planes:
     # windows handed out by `sub` (a launch-heavy driver asks for the same few thousand windows at every refresh, and
     # slicing tensors is what its launching thread would otherwise spend its time on)
     _windows: Dict[tuple, "Planes"] = field(default_factory=dict, repr=False, compare=False)
+    _pointers: Optional[tuple] = field(default=None, repr=False, compare=False)
 
     @property
     def mixed(self) -> bool:
@@ -236,6 +239,12 @@ class Planes:
         if len(self._windows) < 65536:
             self._windows[key] = window
         return window
+
+    def pointers(self) -> tuple:
+        """hi, lo and pitch of classic planes for the native calls (windows are kept, so that this is looked up once for each)."""
+        if self._pointers is None:
+            self._pointers = (self.hi.data_ptr(), self.lo.data_ptr(), self.ld)
+        return self._pointers
 
     def low_pointers(self) -> dict:
         """Pointer arguments of the low part for the native calls."""
@@ -449,6 +458,21 @@ def gemm(
         M, N, K = batch["M"], batch["N"], batch["K"]   # per batch item; a and b describe the whole buffers
     if M == 0 or N == 0:
         return
+    if batch is None and lower_of_grid is None and (mode == EPI_SPLIT or mode == EPI_STORE) and a.hl is None and b.hl is None and (
+            out_planes is None or out_planes.hl is None):
+        c_ptr = ldc = 0
+        if out is not None:
+            assert out.stride(0) == 1 or out.shape[0] == 1
+            c_ptr, ldc = out.data_ptr(), out_ld if out_ld is not None else _ld(out)
+        target = (0, 0, 0)
+        if out_planes is not None:
+            assert out_planes.depth == M and out_planes.cols == N
+            target = out_planes.pointers()
+        _C.gemm_planes((*a.pointers(), *b.pointers(), M, N, K, mode, int(symmetric), int(force_narrow), c_ptr, ldc, *target, k_splits,
+                        split_stride, status_word(a.device).data_ptr(), _stream()), alpha, beta)
+        mark_written(out)
+        _count("gemm_tf32x3_kernel")
+        return
     c_ptr, ldc = 0, 0
     if out is not None:
         c_ptr = out.data_ptr()
@@ -567,10 +591,10 @@ def strided_source(matrix: Tensor) -> tuple:
     return (matrix.data_ptr(), int(matrix.dtype == torch.bfloat16), *matrix.stride())
 
 
-def rotate_half(scratch, matrix_and_bases: tuple, turned: bool, out: Tensor) -> None:
+def rotate_half(scratch, left, right, matrix: Tensor, turned: bool, out: Tensor) -> None:
     """``out <- Q_L^T G Q_R`` (``turned``: ``Q_L G Q_R^T``), ``out`` column-major."""
     assert out.stride(0) == 1 or out.shape[0] == 1
-    _C.rotate_half(scratch, matrix_and_bases + (int(turned), out.data_ptr(), _ld(out), status_word(out.device).data_ptr(), _stream()))
+    _C.rotate_half(scratch, left, right, strided_source(matrix) + (int(turned), out.data_ptr(), _ld(out), status_word(out.device).data_ptr(), _stream()))
     mark_written(out)
     for name in ("clear_kernel", "largest_kernel", "half_planes_kernel", "gemm_half_kernel", "gemm_half_kernel"):
         _count(name)

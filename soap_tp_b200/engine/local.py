@@ -47,8 +47,8 @@ class BasisPlanes:
         self.owner = None                 # weak reference to the tensor object the planes were made from
         self.plain = None                 # operand Q   (depth = rows of Q)
         self.transposed = None            # operand Q^T (depth = cols of Q)
-        self.addresses: tuple = ()        # both, and the basis itself, as the native calls take them
-        self.copy: Optional[Tensor] = None    # of a basis of another type, which the addresses mean then
+        self.native = None                # both, and the basis itself, as the native calls take them
+        self.copy: Optional[Tensor] = None    # of a basis of another type, which they mean then
 
     def once(self, Q: Tensor, size: int, turned: bool) -> "BasisPlanes":
         """The planes of one orientation only, for one use."""
@@ -61,7 +61,7 @@ class BasisPlanes:
         split(view, self.plain, self.transposed)
         if isinstance(planes, k.HalfPlanes):
             here = planes.operand()
-            self.addresses = (_NO_OPERAND + here if turned else here + _NO_OPERAND) + (view.data_ptr(), *view.stride())
+            self.native = _C.BasisOperands(size, (_NO_OPERAND + here if turned else here + _NO_OPERAND) + (view.data_ptr(), *view.stride()))
         return self
 
     def refresh(self, Q: Tensor, size: int) -> None:
@@ -80,7 +80,7 @@ class BasisPlanes:
             self.plain, self.transposed = make(size, size, Q.device), make(size, size, Q.device)
         split(view, self.plain, self.transposed)
         if isinstance(self.plain, k.HalfPlanes):
-            self.addresses = self.plain.operand() + self.transposed.operand() + (view.data_ptr(), *view.stride())
+            self.native = _C.BasisOperands(size, self.plain.operand() + self.transposed.operand() + (view.data_ptr(), *view.stride()))
         self.key = (Q.data_ptr(), Q._version, size)
         self.owner = weakref.ref(Q)
 
@@ -115,6 +115,7 @@ def context_for(state: MutableMapping[str, Any]) -> ParameterContext:
         _CONTEXTS[key] = ctx
     else:
         _CONTEXTS.move_to_end(key)
+        return ctx                     # (nothing was added)
     total = sum(c.bytes for c in _CONTEXTS.values())
     if total > BASIS_CACHE_BYTES or len(_CONTEXTS) > 4096:
         # contexts of tensors that no longer exist go first; then the MOST recently used ones: an optimizer walks
@@ -266,8 +267,7 @@ def rotate_matrix(source: Tensor, left: BasisPlanes, right: BasisPlanes, turned:
     rows, cols = source.shape
     if k.MIXED_CORRECTIONS:
         if rows and cols:
-            k.rotate_half(_scratch(rows, cols, source.device, 2).native, k.strided_source(source) + left.addresses + right.addresses,
-                          turned, out)
+            k.rotate_half(_scratch(rows, cols, source.device, 2).native, left.native, right.native, source, turned, out)
         return
     planes = workspace_planes("X", rows, cols, source.device)
     split(source, planes)
@@ -296,7 +296,7 @@ def _side_stream(device, home: int) -> int:
 
 def _native_arguments(gradient: Tensor, state, step: int, rows: int, cols: int, averages: bool, slot: int, *, beta, beta1, beta2,
                       eps) -> tuple:
-    """An ordinary step as the native call takes it: scratch, addresses and scalars; then the tensor of its result."""
+    """An ordinary step as the native call takes it: scratch, bases, addresses and scalars; then the tensor of its result."""
     g = gradient.detach().reshape(rows, cols)
     if g.dtype != torch.float32 and g.dtype != torch.bfloat16:
         g = g.float()
@@ -308,12 +308,12 @@ def _native_arguments(gradient: Tensor, state, step: int, rows: int, cols: int, 
     left, right = state["left_preconditioner"], state["right_preconditioner"]
     scratch = _scratch(rows, cols, g.device, 1 if g.dtype == torch.bfloat16 else 2, update=True, averages=averages, slot=slot)
     update = torch.empty((rows, cols), dtype=torch.float32, device=g.device)
-    arguments = (k.strided_source(g) + ctx.left.addresses + ctx.right.addresses
+    arguments = (k.strided_source(g)
                  + (momentum.data_ptr(), k._ld(momentum), variance.data_ptr(), k._ld(variance), update.data_ptr(),
                     left.data_ptr(), k._ld(left), right.data_ptr(), k._ld(right)))
     scalars = (beta, beta1, beta2, eps / math.sqrt(bias2), 1.0 / (1.0 - beta1**step), 1.0 / math.sqrt(bias2))
     # (the gradient and the planes of the bases are held until the launches are issued)
-    return (scratch.native, arguments, scalars), update, (g, ctx)
+    return (scratch.native, ctx.left.native, ctx.right.native, arguments, scalars), update, (g, ctx)
 
 
 def _count_launches(averages: bool) -> None:
