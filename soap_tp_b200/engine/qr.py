@@ -122,34 +122,39 @@ _PANEL_STREAMS: Dict[tuple, "torch.cuda.Stream"] = {}
 def _panel_stream(device, slot: int) -> "torch.cuda.Stream":
     key = (str(device), slot)
     if key not in _PANEL_STREAMS:
-        _PANEL_STREAMS[key] = torch.cuda.Stream(device=device, priority=-1)
+        _PANEL_STREAMS[key] = torch.cuda.Stream(device=device, priority=-2)
     return _PANEL_STREAMS[key]
 
 
-def householder_qr_pair(jobs) -> None:
+def householder_qr_pair(jobs, beside=None) -> None:
     """Factor several independent matrices at the same time.
 
     ``jobs`` is a list of ``(matrix, Q, column_order)``.  Each factorisation is issued panel by panel on
     its own stream, alternating between the jobs, so that the latency-bound panel kernel of one
     factorisation (a few dozen thread blocks) runs while the tensor-core updates of the other keep the
     remaining SMs busy.  The calling stream waits for all of them.
+
+    ``beside``: called once the first panels are issued; what it gives the calling stream runs beside the factorisations, whose
+    streams go first.  It may read the old ``Q``, which is not written before that, and nothing that the factorisations write.
     """
     if len(jobs) == 1:
+        if beside is not None:
+            beside()
         householder_qr(*jobs[0])
         return
     device = jobs[0][0].device
     main = torch.cuda.current_stream(device)
-    ready = torch.cuda.Event()
+    ready, readers = torch.cuda.Event(), torch.cuda.Event()
     ready.record(main)
     streams, steps = [], []
     for slot, (matrix, Q, order) in enumerate(jobs):
         key = (str(device), slot)
         if key not in _SIDE_STREAMS:
-            _SIDE_STREAMS[key] = torch.cuda.Stream(device=device)
+            _SIDE_STREAMS[key] = torch.cuda.Stream(device=device, priority=-1)
         stream = _SIDE_STREAMS[key]
         stream.wait_event(ready)
         streams.append(stream)
-        steps.append(_factorisation_steps(matrix, Q, order, slot))
+        steps.append(_factorisation_steps(matrix, Q, order, slot, readers=readers if beside is not None else None))
     alive = list(range(len(jobs)))
     while alive:
         for slot in list(alive):
@@ -158,6 +163,10 @@ def householder_qr_pair(jobs) -> None:
                     next(steps[slot])
                 except StopIteration:
                     alive.remove(slot)
+        if beside is not None:
+            beside()
+            readers.record(main)
+            beside = None
     for stream in streams:
         done = torch.cuda.Event()
         done.record(stream)
@@ -212,14 +221,15 @@ def _pair_reflector(ws: dict, V: k.Planes, a: int, n: int, suffix: str = "", bac
 
 
 def _factorisation_steps(matrix: Optional[Tensor], Q: Optional[Tensor], column_order: Optional[Tensor], slot: int,
-                         forward_q: bool = False, publisher=None, size: Optional[int] = None, device=None):
+                         forward_q: bool = False, publisher=None, size: Optional[int] = None, device=None, readers=None):
     """The blocked factorisation as a generator: yields after the launches of every panel.
 
     With a ``publisher`` (``engine/dist_qr.py``) this rank only runs the panel chain and the trailing updates:
     the reflectors ``V`` and the products ``Z_p = T_p V_p^T`` are written into the publisher's buffers, which
     other ranks can read, ``publisher.announce(p)`` is called on the main stream once panel ``p``'s are complete,
     and the explicit ``Q`` is accumulated elsewhere.  ``matrix=None``: the workspace planes ``C`` already hold
-    the (column-permuted) input.
+    the (column-permuted) input.  ``readers``: an event after which ``Q`` may be overwritten (recorded by the time the last
+    panel is issued).
     """
     n = matrix.shape[0] if matrix is not None else int(size)
     device = matrix.device if matrix is not None else device
@@ -399,6 +409,8 @@ def _factorisation_steps(matrix: Optional[Tensor], Q: Optional[Tensor], column_o
         if p % 2 == 1 and paired(p - 1):
             continue                                     # applied together with panel p - 1
         block = Qp.sub(j0, j0, r, r)
+        if p == 0 and readers is not None:
+            main.wait_event(readers)
         if paired(p):
             v2, z2 = _pair_reflector(ws, V, p, n, backward=True)
             w2 = ws["W2"].sub(0, 0, 2 * PANEL, r)
