@@ -199,13 +199,13 @@ PYBIND11_MODULE(_C, m) {
          uint64_t remap, uint64_t C2hi, uint64_t C2lo, int64_t ld2, int m_limit, int o1_row_start, int tri_nb,
          int tri_pr, int tri_Pr, int tri_pc, int tri_Pc, int tri_m0, int tri_n0, uint64_t a_hl, int64_t lda16,
          uint64_t b_hl, int64_t ldb16, uint64_t Chl, int64_t ldp16, uint64_t push_table, int64_t push_ld,
-         int64_t push_ld16, int push_nb, int push_Pr, int push_Pc, int push_pr, int push_pc, int push_mixed) {
+         int64_t push_ld16, int push_nb, int push_Pr, int push_Pc, int push_pr, int push_pc, int push_mixed, int b_exact) {
         GemmOperands ops{};
         ops.a_hi = ptr<const float>(a_hi); ops.a_lo = ptr<const float>(a_lo); ops.lda = lda;
         ops.b_hi = ptr<const float>(b_hi); ops.b_lo = ptr<const float>(b_lo); ops.ldb = ldb;
         GemmProblem prob{};
         prob.M = M; prob.N = N; prob.K = K;
-        prob.mode = mode; prob.symmetric = symmetric; prob.force_narrow = force_narrow;
+        prob.mode = mode; prob.symmetric = symmetric; prob.force_narrow = force_narrow; prob.b_exact = b_exact;
         prob.alpha = alpha; prob.beta = beta;
         prob.C = ptr<float>(C); prob.ldc = ldc;
         prob.Chi = ptr<float>(Chi); prob.Clo = ptr<float>(Clo); prob.ldp = ldp;
@@ -243,7 +243,7 @@ PYBIND11_MODULE(_C, m) {
       py::arg("a_hl") = 0, py::arg("lda16") = 0, py::arg("b_hl") = 0, py::arg("ldb16") = 0, py::arg("Chl") = 0,
       py::arg("ldp16") = 0, py::arg("push_table") = 0, py::arg("push_ld") = 0, py::arg("push_ld16") = 0,
       py::arg("push_nb") = 1, py::arg("push_Pr") = 1, py::arg("push_Pc") = 1, py::arg("push_pr") = 0,
-      py::arg("push_pc") = 0, py::arg("push_mixed") = 0,
+      py::arg("push_pc") = 0, py::arg("push_mixed") = 0, py::arg("b_exact") = 0,
       "3xTF32 tcgen05 GEMM acc[m,n] = sum_k Za[k,m] Zb[k,n] with fused epilogue");
 
   m.def("gemm_use_cta_pairs", [](bool on) { gemm_use_cta_pairs(on); },

@@ -50,6 +50,7 @@ struct GemmProblem {
   int tri_nb, tri_pr, tri_Pr, tri_pc, tri_Pc;   // symmetric == 2: block size and grid coordinates of this rank
   int tri_m0, tri_n0;                           // symmetric == 2: local row / column index of output element (0, 0)
   int force_narrow;  // use 128-wide tiles regardless of the problem size
+  int b_exact;       // mixed operands: B's values are tf32 (it comes from bf16 values), so its remainders are zero and not multiplied
   int k_splits;      // kEpiStore: split K over this many CTAs per tile, partial s written at C + s*split_stride
   int64_t split_stride;
   float alpha, beta;

@@ -567,7 +567,7 @@ gemm_tf32x3_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant_
             const uint64_t adv = static_cast<uint64_t>(k * 32 >> 4);
             umma_f16_ss(tmem_acc, a_hl + kLb + adv, b_hl + adv, idesc16, first ? 0u : 1u);      // lo * hi
             first = 0;
-            umma_f16_ss(tmem_acc, a_hl + adv, b_hl + kLb + adv, idesc16, 1);                    // hi * lo
+            if (!prob.b_exact) umma_f16_ss(tmem_acc, a_hl + adv, b_hl + kLb + adv, idesc16, 1);  // hi * lo
           }
           if (!tf32_first) {
 #pragma unroll
@@ -808,7 +808,7 @@ gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ 
             const uint64_t adv = static_cast<uint64_t>(k * 32 >> 4);
             umma_f16_ss_pair(tmem_acc, a_2 + kLb + adv, b_2 + adv, idesc16, first ? 0u : 1u);     // lo * hi
             first = 0;
-            umma_f16_ss_pair(tmem_acc, a_2 + adv, b_2 + kLb + adv, idesc16, 1);                   // hi * lo
+            if (!prob.b_exact) umma_f16_ss_pair(tmem_acc, a_2 + adv, b_2 + kLb + adv, idesc16, 1);  // hi * lo
           }
           if (!tf32_first) {
 #pragma unroll

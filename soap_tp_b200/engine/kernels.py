@@ -443,6 +443,7 @@ def gemm(
     batch: Optional[dict] = None,
     lower_of_grid: Optional[tuple] = None,
     push: Optional[dict] = None,
+    second_exact: bool = False,
 ) -> None:
     """``acc[m, n] = sum_k a[k, m] * b[k, n]`` then the fused epilogue (see ``csrc/gemm.h``).
 
@@ -450,6 +451,7 @@ def gemm(
     ``EPI_SPLIT``/``EPI_ADAM``) or a row-major ``M x N`` tensor for ``EPI_ROW_MAJOR``.  ``EPI_PUSH`` writes no
     local output: ``push`` = ``dict(table, ld, ld16, nb, Pr, Pc, pr, pc, mixed)`` names the operand planes of the
     consuming ranks (``csrc/gemm.h``, ``kEpiPush``), which the epilogue fills through peer pointers.
+    ``second_exact``: ``b`` comes from bf16 values; a product of mixed planes then leaves out the terms that are zero.
     """
     if batch is None:
         assert a.depth == b.depth, (a.depth, b.depth)
@@ -487,7 +489,7 @@ def gemm(
     chi = clo = ldp = 0
     mixed_arguments = {}
     if a.mixed:
-        mixed_arguments.update(a_hl=a.hl.data_ptr(), lda16=a.ld16, b_hl=b.hl.data_ptr(), ldb16=b.ld16)
+        mixed_arguments.update(a_hl=a.hl.data_ptr(), lda16=a.ld16, b_hl=b.hl.data_ptr(), ldb16=b.ld16, b_exact=int(second_exact))
     if out_planes is not None:
         assert batch is not None or (out_planes.depth == M and out_planes.cols == N)
         low = out_planes.low_pointers()

@@ -77,7 +77,8 @@ def step(gradient: Tensor, state: MutableMapping[str, Any], *, beta: float, beta
                 bias_correction2=bias2)
     ut = local.tf32_workspace("os_UT", h, rows, device)
     # Y^T = Q^T G^T with Adam in the epilogue: momentum, variance and U^T are h x rows_local, column-major
-    k.gemm(basis.plain, gtp, mode=k.EPI_ADAM, out_planes=ut, momentum=state["momentum"], variance=state["variance"], adam=adam)
+    k.gemm(basis.plain, gtp, mode=k.EPI_ADAM, out_planes=ut, momentum=state["momentum"], variance=state["variance"], adam=adam,
+           second_exact=gradient.dtype == torch.bfloat16)
     update = torch.empty((rows, h), dtype=torch.float32, device=device)
     k.gemm(basis.transposed, ut, out=update.T)                          # (U Q^T)^T = Q U^T, i.e. the row-major update
     refreshing = count % interval == 0

@@ -361,3 +361,27 @@ def test_tiles_do_not_change_a_bit(M, K, splits):
     assert torch.equal(parts[0], parts[1][:, : 128 * 3]) and torch.equal(parts[1], parts[2])
     exact = A.double().T @ B.double()
     assert float((parts[2].double().sum(dim=0).T - exact).norm() / exact.norm()) < 2e-6
+
+
+@pytest.mark.parametrize("M,N,K", [(7, 9, 5), (130, 70, 33), (300, 257, 129), (2048, 3000, 520)])
+def test_terms_of_exact_operands_left_out(M, N, K):
+    """A second operand from bf16 values has remainders of zero: leaving their products out does not change a bit."""
+    from soap_tp_b200.engine import kernels as k
+
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    A, B = torch.randn(K, M, generator=g, device="cuda"), torch.randn(K, N, generator=g, device="cuda").bfloat16()
+    B[::3] *= 2.0**-100
+    a, b = k.split_planes(A, mixed=True), k.Planes.empty(K, N, A.device, mixed=True)
+    k.split_planes_both(B, b, None)
+    assert not bool(b.halves()[1].any())
+    adam = dict(beta1=0.9, beta2=0.95, eps=1e-8, bias_correction1=0.5, bias_correction2=0.25)
+    results = []
+    for exact in (False, True):
+        out = torch.zeros(N, M, device="cuda").T
+        k.gemm(a, b, out=out, second_exact=exact)
+        momentum, variance = (torch.full((N, M), value, device="cuda").T for value in (0.1, 0.2))
+        planes = k.Planes.empty(M, N, A.device, mixed=True)
+        k.gemm(a, b, mode=k.EPI_ADAM, out_planes=planes, momentum=momentum, variance=variance, adam=adam, second_exact=exact)
+        results.append((out, momentum, variance, planes.hi[:N, :M]))
+    for x, y in zip(*results):
+        assert torch.equal(x, y)
