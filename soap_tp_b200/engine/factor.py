@@ -19,15 +19,16 @@ def householder_qr(matrix: Tensor, Q: Tensor, column_order: Optional[Tensor] = N
     return qr.householder_qr(matrix, Q, column_order)
 
 
-def householder_qr_pair(jobs, beside=None) -> None:
+def householder_qr_pair(jobs, beside=None, starts=None) -> None:
     """Several independent QR factorisations issued concurrently; ``jobs``: ``(matrix, Q, column_order)``.  ``beside``: issues
-    what runs on the calling stream meanwhile (``qr.householder_qr_pair``)."""
+    what runs on the calling stream meanwhile; ``starts``: an event per job from which on it may begin
+    (``qr.householder_qr_pair``)."""
     from ..ops.basis import count_qr_call
     from . import qr
 
     for _ in jobs:
         count_qr_call()
-    qr.householder_qr_pair(jobs, beside)
+    qr.householder_qr_pair(jobs, beside, starts)
 
 
 def symmetric_eigenbasis(P: Tensor, Q: Tensor, work: Tensor, values: Tensor, implementation: str) -> Tensor:

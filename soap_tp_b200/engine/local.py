@@ -211,12 +211,14 @@ def rotate_planes(source, first, second, rows: int, cols: int, device, *, tag: s
     product(middle, second, **final)
 
 
-def gram_updates(xp, gtp, state, beta: float, rows: int, cols: int) -> None:
+def gram_updates(xp, gtp, state, beta: float, rows: int, cols: int, between=None) -> None:
     product(gtp, gtp, out=state["left_preconditioner"][:rows, :rows], alpha=1.0 - beta, beta=beta, symmetric=True)
+    if between is not None:
+        between()
     product(xp, xp, out=state["right_preconditioner"][:cols, :cols], alpha=1.0 - beta, beta=beta, symmetric=True)
 
 
-def gram_updates_for_bases(gradient: Tensor, state, beta: float, rows: int, cols: int) -> None:
+def gram_updates_for_bases(gradient: Tensor, state, beta: float, rows: int, cols: int, between=None) -> None:
     """The averages of a step that derives bases from them (the first one, and those with a refresh), on tf32 planes like
     everything else that is factored.
 
@@ -226,7 +228,7 @@ def gram_updates_for_bases(gradient: Tensor, state, beta: float, rows: int, cols
     to a sign."""
     gp, gtp = tf32_workspace("G", rows, cols, gradient.device), tf32_workspace("GT", cols, rows, gradient.device)
     split(gradient.detach(), gp, gtp)
-    gram_updates(gp, gtp, state, beta, rows, cols)
+    gram_updates(gp, gtp, state, beta, rows, cols, between)
 
 
 class _Scratch:
@@ -457,9 +459,22 @@ def soap_step(
         update = run(gradient, state, step, rows, cols, averages=True, **scalars)
     else:
         # The averages first: the update does not depend on them, and runs beside the factorisations of the refresh, which leave most
-        # of the GPU idle (chains of panels).
+        # of the GPU idle (chains of panels).  The left side's power iteration comes before the right side's average, so that its
+        # factorisation starts earlier.
+        orders = []
+
+        def iterate(side: str, size: int) -> None:
+            with TIMER.stage("refresh.power_iteration", device):
+                order = estimated_order(state[f"{side}_preconditioner"], state[f"{side}_basis"], state[f"{side}_work"], size)
+            orders.append((order, torch.cuda.Event()))
+            orders[-1][1].record()
+
         with TIMER.stage("gram", device):
-            gram_updates_for_bases(gradient.reshape(rows, cols), state, beta, rows, cols)
+            gram_updates_for_bases(gradient.reshape(rows, cols), state, beta, rows, cols,
+                                   None if TIMER.enabled else lambda: iterate("left", rows))
+        if TIMER.enabled:
+            iterate("left", rows)
+        iterate("right", cols)
         update = None
 
         def issue_update() -> None:
@@ -469,7 +484,7 @@ def soap_step(
         if TIMER.enabled:
             issue_update()                # (by itself, so that each stage's time is its own)
         with TIMER.stage("refresh", device):
-            refresh(state, global_shape, (lambda: None) if TIMER.enabled else issue_update)
+            refresh(state, global_shape, orders, (lambda: None) if TIMER.enabled else issue_update)
     state["step"] = step
     return update
 
@@ -564,9 +579,10 @@ def permute(matrix: Tensor, global_shape, row_order: Tensor, column_order: Tenso
     return matrix
 
 
-def refresh(state: MutableMapping[str, Any], global_shape, issue_update) -> Tuple[Tensor, Tensor]:
-    """Power iteration + QR on both sides with momentum transport and variance permutation; ``issue_update`` issues the step's own
-    update, which the momentum and variance come from.
+def refresh(state: MutableMapping[str, Any], global_shape, orders, issue_update) -> Tuple[Tensor, Tensor]:
+    """QR of the power iteration's results on both sides (``orders``: the order of the columns and the event of both, per side) with
+    momentum transport and variance permutation; ``issue_update`` issues the step's own update, which the momentum and variance
+    come from.
 
     Neither it nor the momentum's way out of the old bases depends on the factorisations: at 8192 x 8192 16 of 86 ms that were
     spent before them run beside them now (a GPU-wide product delays a panel by what is left of its tiles, so 3.5 ms are gained;
@@ -574,9 +590,7 @@ def refresh(state: MutableMapping[str, Any], global_shape, issue_update) -> Tupl
     rows, cols = global_shape
     momentum, variance = state["momentum"], state["variance"]
     device = momentum.device
-    with TIMER.stage("refresh.power_iteration", device):
-        left_order = estimated_order(state["left_preconditioner"], state["left_basis"], state["left_work"], rows)
-        right_order = estimated_order(state["right_preconditioner"], state["right_basis"], state["right_work"], cols)
+    (left_order, left_start), (right_order, right_start) = orders
     # momentum out of the old bases: Q_L M Q_R^T, in fp32 so that the way back sees the range of every row and column
     parameter_space = workspace_matrix("space", rows, cols, device)
     ctx = context_for(state)
@@ -602,7 +616,7 @@ def refresh(state: MutableMapping[str, Any], global_shape, issue_update) -> Tupl
             factor.householder_qr_pair([
                 (state["left_work"][:rows, :rows], state["left_basis"][:rows, :rows], left_order),
                 (state["right_work"][:cols, :cols], state["right_basis"][:cols, :cols], right_order)],
-                None if TIMER.enabled else beside)
+                None if TIMER.enabled else beside, (left_start, right_start))
     with TIMER.stage("refresh.momentum_in", device):
         ctx.left.refresh(state["left_basis"], rows)
         ctx.right.refresh(state["right_basis"], cols)
