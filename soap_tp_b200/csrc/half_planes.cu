@@ -2,7 +2,9 @@
 //
 // Bound by memory: the source is read twice (once for the largest magnitude of every row and column, once to convert it)
 // and each wanted plane written once.  64 x 64 tiles, turned in shared memory, so that reads run along the source's unit
-// stride and writes along each plane's, whichever way the source lies.
+// stride and writes along each plane's, whichever way the source lies; 16 bytes a thread, the reads where the source is aligned to
+// that (the planes always are).  Two elements a thread kept too few bytes in flight for 16-bit sources
+// (32064 x 2048 bf16: 110 us for the largest magnitudes, 121 us for one term of planes, 131 MB read each).
 //
 // With a RangeGuard the second pass also decides whether fp16 pairs hold the matrix and, where they do not, writes the mixed
 // form of the matrix and of its bases.  That takes no launch of its own: there is about one CTA per SM more, which looks at the
@@ -47,7 +49,7 @@ struct Source {
   const void* src;
   int64_t s_fast, s_slow;
   int n_fast, n_slow, tiles_fast;
-  bool pairs;
+  bool pairs, chunks;      // may be read two elements, 16 bytes at a time
 };
 struct LargestJob {
   Source from;
@@ -64,7 +66,7 @@ struct LargestGroup {
 // `strip` tiles along the slow axis and keeps the maxima of its fast-axis elements in registers meanwhile.
 template <typename T, int N>
 __global__ void __launch_bounds__(kThreads) largest_kernel(const __grid_constant__ LargestGroup<N> group) {
-  __shared__ uint32_t fast_max[8][kTile];
+  __shared__ uint32_t fast_max[kChunkRows<T>][kTile];      // (of the 8 warps where the source is read by pairs)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int member = group.blocks.member(blockIdx.x), block = blockIdx.x - group.blocks.first(member);
   const LargestJob& job = group.jobs[member];
@@ -74,6 +76,40 @@ __global__ void __launch_bounds__(kThreads) largest_kernel(const __grid_constant
   const int fast0 = block % job.from.tiles_fast * kTile, strip0 = block / job.from.tiles_fast * strip;
   wait_for_predecessor();
   let_successor_start();
+  if (job.from.chunks) {
+    constexpr int kAcross = kChunksPerRow<T>;      // threads that share a row
+    const int row = threadIdx.x / kAcross, offset = threadIdx.x % kAcross * kChunk<T>;
+    uint32_t mine[kChunk<T>] = {};
+    for (int t = 0; t < strip; ++t) {
+      const int slow0 = (strip0 + t) * kTile;
+      if (slow0 >= n_slow) break;
+      sweep_tile_chunks(src, job.from.s_slow, fast0, slow0, n_fast, n_slow, [&](int, int slow, const float (&x)[kChunk<T>]) {
+        uint32_t most = 0;
+#pragma unroll
+        for (int e = 0; e < kChunk<T>; ++e) {
+          const uint32_t a = magnitude(x[e]);
+          mine[e] = max(mine[e], a);
+          most = max(most, a);
+        }
+        if (of_slow) {
+#pragma unroll
+          for (int lanes = 1; lanes < kAcross; lanes *= 2) most = max(most, __shfl_xor_sync(0xffffffffu, most, lanes));
+          if (threadIdx.x % kAcross == 0 && slow0 + slow < n_slow) atomicMax(of_slow + slow0 + slow, most);
+        }
+      });
+    }
+    if (!of_fast) return;
+#pragma unroll
+    for (int e = 0; e < kChunk<T>; ++e) fast_max[row][offset + e] = mine[e];
+    __syncthreads();
+    if (threadIdx.x < kTile && fast0 + threadIdx.x < n_fast) {
+      uint32_t most = 0;
+#pragma unroll
+      for (int r = 0; r < kChunkRows<T>; ++r) most = max(most, fast_max[r][threadIdx.x]);
+      atomicMax(of_fast + fast0 + threadIdx.x, most);
+    }
+    return;
+  }
   uint32_t mine0 = 0, mine1 = 0;
   for (int t = 0; t < strip; ++t) {
     const int slow0 = (strip0 + t) * kTile;
@@ -100,13 +136,21 @@ __global__ void __launch_bounds__(kThreads) largest_kernel(const __grid_constant
   }
 }
 
-__device__ __forceinline__ void write_pair(const HalfTarget& to, int64_t at, float x0, float x1) {
-  const __half2 h = __floats2half2_rn(x0, x1);
-  *reinterpret_cast<__half2*>(to.h + at) = h;
-  if (to.l) {
-    const float2 back = __half22float2(h);
-    *reinterpret_cast<__half2*>(to.l + at) = __floats2half2_rn(x0 - back.x, x1 - back.y);
+// Eight elements along the depth of a plane, 16-byte aligned: `x(e)` the e-th.
+template <typename Element>
+__device__ __forceinline__ void write_eight(const HalfTarget& to, int64_t at, Element x) {
+  uint32_t h[4], l[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float x0 = x(2 * i), x1 = x(2 * i + 1);
+    const __half2 high = __floats2half2_rn(x0, x1);
+    const float2 back = __half22float2(high);
+    const __half2 low = __floats2half2_rn(x0 - back.x, x1 - back.y);
+    h[i] = *reinterpret_cast<const uint32_t*>(&high);
+    l[i] = *reinterpret_cast<const uint32_t*>(&low);
   }
+  *reinterpret_cast<uint4*>(to.h + at) = make_uint4(h[0], h[1], h[2], h[3]);
+  if (to.l) *reinterpret_cast<uint4*>(to.l + at) = make_uint4(l[0], l[1], l[2], l[3]);
 }
 
 // What the second pass writes beside the planes where fp16 pairs do not hold the matrix: the mixed form of it and its bases.
@@ -208,7 +252,6 @@ template <typename T, bool DECIDED, int N>
 __global__ void __launch_bounds__(kThreads, DECIDED ? 8 : 1) half_planes_kernel(const __grid_constant__ PlaneGroup<DECIDED, N> group) {
   __shared__ float tile[kTile][kTile + 1];           // [slow][fast]
   __shared__ float up_along[kTile], up_across[kTile];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int member = group.blocks.member(blockIdx.x), block = blockIdx.x - group.blocks.first(member);
   const PlaneJob<DECIDED>& job = group.jobs[member];
   const int n_fast = job.from.n_fast, n_slow = job.from.n_slow;
@@ -239,22 +282,29 @@ __global__ void __launch_bounds__(kThreads, DECIDED ? 8 : 1) half_planes_kernel(
       if (slow0 == 0) across.scale[fast] = s.inverse;
     }
   }
-  sweep_tile(static_cast<const T*>(job.from.src), job.from.s_fast, job.from.s_slow, fast0, slow0, n_fast, n_slow, job.from.pairs,
-             [&](int fast, int slow, float x0, float x1) {
-               tile[slow][fast] = x0;
-               tile[slow][fast + 1] = x1;
-             });
-  __syncthreads();
-  // pitches are multiples of 64, so the second half of a pair that ends the depth lands in the padding
-  if (along.h && fast0 + 2 * lane < n_fast) {
-    for (int s = warp; s < kTile && slow0 + s < n_slow; s += 8)
-      write_pair(along, fast0 + 2 * lane + (slow0 + s) * along.ld, tile[s][2 * lane] * up_along[s],
-                 tile[s][2 * lane + 1] * up_along[s]);
+  const T* src = static_cast<const T*>(job.from.src);
+  if (job.from.chunks) {
+    sweep_tile_chunks(src, job.from.s_slow, fast0, slow0, n_fast, n_slow, [&](int fast, int slow, const float (&x)[kChunk<T>]) {
+#pragma unroll
+      for (int e = 0; e < kChunk<T>; ++e) tile[slow][fast + e] = x[e];
+    });
+  } else {
+    sweep_tile(src, job.from.s_fast, job.from.s_slow, fast0, slow0, n_fast, n_slow, job.from.pairs,
+               [&](int fast, int slow, float x0, float x1) {
+                 tile[slow][fast] = x0;
+                 tile[slow][fast + 1] = x1;
+               });
   }
-  if (across.h && slow0 + 2 * lane < n_slow) {
-    for (int f = warp; f < kTile && fast0 + f < n_fast; f += 8)
-      write_pair(across, slow0 + 2 * lane + (fast0 + f) * across.ld, tile[2 * lane][f] * up_across[f],
-                 tile[2 * lane + 1][f] * up_across[f]);
+  __syncthreads();
+  // pitches are multiples of 64, so what of eight elements lies past the depth lands in the padding
+  const int eight = threadIdx.x % 8 * 8;
+  if (along.h && fast0 + eight < n_fast) {
+    for (int s = threadIdx.x / 8; s < kTile && slow0 + s < n_slow; s += kThreads / 8)
+      write_eight(along, fast0 + eight + (slow0 + s) * along.ld, [&](int e) { return tile[s][eight + e] * up_along[s]; });
+  }
+  if (across.h && slow0 + eight < n_slow) {
+    for (int f = threadIdx.x / 8; f < kTile && fast0 + f < n_fast; f += kThreads / 8)
+      write_eight(across, slow0 + eight + (fast0 + f) * across.ld, [&](int e) { return tile[eight + e][f] * up_across[f]; });
   }
 }
 
@@ -310,6 +360,7 @@ Oriented oriented(const PlanesJob& job) {
   o.from.n_fast = rows_fast ? job.rows : job.cols;
   o.from.n_slow = rows_fast ? job.cols : job.rows;
   o.from.tiles_fast = (o.from.n_fast + kTile - 1) / kTile;
+  o.from.chunks = reads_chunks(static_cast<const T*>(job.src), o.from.s_fast, o.from.s_slow, o.from.n_slow);
   o.from.pairs = reads_pairs(static_cast<const T*>(job.src), o.from.s_fast, o.from.s_slow, o.from.n_slow);
   o.along = rows_fast ? job.plain : job.turned;
   o.across = rows_fast ? job.turned : job.plain;

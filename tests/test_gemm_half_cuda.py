@@ -282,3 +282,29 @@ def test_operands_near_the_limits_of_fp32(sizes, mode):
     # entries of a product that fall below the smallest normal number round there
     assert bool((scaled[0] - expected).abs().max() <= 2.0**-148)
     assert _rel(scaled[0], expected.cpu()) < 1e-6
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 1), (3, 7), (64, 61), (65, 130), (130, 333), (257, 1500)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("turned", [False, True])
+def test_sources_read_sixteen_bytes_at_a_time(rows, cols, dtype, turned):
+    """A ragged matrix in a buffer whose pitch is aligned is read by 16 bytes, its last elements one by one, and nothing past it:
+    the same planes as from a copy that is read element by element."""
+    from soap_tp_b200.engine import kernels as k
+
+    g = torch.Generator().manual_seed(rows * cols)
+    height, width = (cols, rows) if turned else (rows, cols)
+    buffer = torch.full((height, -(-width // 16) * 16), float("nan"), dtype=dtype, device="cuda")
+    buffer[:, :width] = torch.randn(height, width, generator=g).to(dtype).cuda()
+    apart = torch.full((height, 2 * width + 1), float("nan"), dtype=dtype, device="cuda")
+    apart[:, 1::2] = buffer[:, :width]
+    planes = []
+    for source in (buffer[:, :width], apart[:, 1::2]):
+        source = source.T if turned else source
+        terms = 1 if dtype == torch.bfloat16 else 2
+        both = k.HalfPlanes.empty(rows, cols, source.device, terms=terms), k.HalfPlanes.empty(cols, rows, source.device, terms=terms)
+        k.half_planes(source, *both)
+        planes.append(both)
+    for a, b in zip(*planes):
+        assert torch.equal(a.dense(), b.dense()) and bool(torch.isfinite(a.dense()).all())
+        assert torch.equal(a.scale, b.scale)
