@@ -319,6 +319,7 @@ PYBIND11_MODULE(_C, m) {
     steady_step(s, ptr<int>(status), stream_of(stream));
   }, "The launches of one ordinary single-GPU step, or some of its phases (gemm_half.h, SteadyStep)");
   m.def("steady_step_shares", &steady_step_shares, "Whether steps of such matrices can share launches");
+  m.def("averages_share", &averages_share, "Whether both averages of a step run in one launch");
   m.attr("STEP_GROUP") = kHalfGroup;
   m.def("steady_steps", [](const std::vector<std::tuple<const RotationScratch*, const BasisOperands*, const BasisOperands*,
                                                         std::vector<int64_t>, std::array<double, 6>>>& steps,

@@ -16,6 +16,13 @@
 // a register-resident sum (round-to-nearest), multiplied by the scale of A's block of 128 on the way; B's scales are per
 // column and applied once, in the epilogue.  Within a k-block the small products come first.
 //
+// What bounds a pair's tile of 256 x 256 (cycles, K = 4096, two-term operands): 98k of products at the tensor core's rate, some 5k over that
+// between k-blocks, 8k from the start to the first full accumulator (barriers, TMEM, first loads), 5k to 10k of epilogue, and Adam's
+// 20k and more where all tiles of a wave reach memory at once.  4096^3 331 -> 315 us, 8192^3 2334 -> 2251 (1.47 PFLOP/s: the power cap), Adam
+// 8192^3 3003 -> 2617, 256 x 512 x 256 on single CTAs 15 -> 10 us, by draining with sixteen warps instead of eight (two columns per addition),
+// looking ahead while products are issued, and fetching the epilogue's inputs meanwhile.  Accumulators of 128 columns, four in TMEM,
+// hide the hand-over entirely but cost more than they hide on pairs (M 256 x N 128 products: 4096^3 391 us).
+//
 // Where the device word `wide` is set (RangeGuard: rows or columns that fp16 pairs do not hold) the same kernel runs the
 // mixed form: four boxes of the same size, 32 of K each, tf32 and bf16 MMAs in gemm_tf32x3.cu's order, two k-blocks per drain,
 // and bit for bit its results.  One launch serves both, so that nobody waits for the decision on the host.
@@ -583,7 +590,8 @@ half_pair_kernel(const __grid_constant__ HalfMaps maps, const __grid_constant__ 
   half_kernel_impl<true, MODE>(maps, args, blockIdx.x, status);
 }
 
-// N products of single CTAs in one launch, one after another in the grid.
+// N products of single CTAs in one launch, one after another in the grid.  (With N = 1 the search for the problem is compiled away; the
+// parameters of eight take 11 KB, which a launch of one does not pay for.)
 template <int N>
 struct HalfGroup {
   HalfMaps maps[N];

@@ -166,6 +166,8 @@ void steady_step(const SteadyStep& s, int* status, cudaStream_t stream);
 // Whether every product of such a step runs on single CTAs, so that several small parameters can share its launches; and the
 // steps of up to kHalfGroup such parameters (all phases; scratch of their own each).
 bool steady_step_shares(int rows, int cols);
+// Whether both averages of a step run on single CTAs, and so in one launch.
+bool averages_share(int rows, int cols);
 void steady_steps(const SteadyStep* steps, int count, int* status, cudaStream_t stream);
 
 // Scale of a vector or block from the bit pattern of its largest magnitude (clamped so that both factors are normal):

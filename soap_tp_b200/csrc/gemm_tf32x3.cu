@@ -69,6 +69,11 @@ struct TileConfig {
   static constexpr int kColsPerThread = 4 * BN / EW;
   static_assert(kTmemCols * CTAS <= 512 && BN * (kBM + 4) * 4 <= kStages * kStageBytes, "accumulators and the staged tile fit");
 };
+// Up to 148 tiles of 128 x 128 have an SM to themselves: three stages of 64 KB and sixteen epilogue warps (1024 x 1024 x 256 read-modify-write
+// 15.8 us; 21.5 with the compact tile, whose stages hold half as much).  More of them run two to an SM, so that one's loads and products
+// run under the other's epilogue: 8192 x 8192 x 128 284 us, one to an SM 370.  256 columns, on CTA pairs where nothing is batched, from
+// 148 of those tiles on (split products count each part): as fast for updates of K = 256 (8192: 336 and 345 us) and ahead wherever K is
+// long enough for operand traffic to count (8192^3 3.75 ms; 256 x 8192 x 8192 in five parts 186 us, 222 with compact tiles).
 using WideTile = TileConfig<256, 32, kEpiWarps, 1>;
 using NarrowTile = TileConfig<128, 32, kEpiWarps, 1>;
 using CompactTile = TileConfig<128, 16, 8, 2>;
@@ -959,7 +964,7 @@ void gemm_tf32x3(const GemmOperands& ops, const GemmProblem& prob, int* status, 
                                 prob.k_splits > 1 || prob.batches > 1 || prob.symmetric))
     throw std::invalid_argument("gemm_tf32x3: the push epilogue needs a target table and a plain (unsplit, unbatched) product");
   if (prob.K <= 0) throw std::invalid_argument("gemm_tf32x3 needs K >= 1");
-  // Wide tiles when there are enough of them to fill the 148 SMs; narrower tiles otherwise.
+  // Wide tiles when there are enough of them to fill the 148 SMs; narrower tiles otherwise (figures at the tiles' definition).
   const int64_t tile_rows = (prob.M + kBM - 1) / kBM, splits = prob.mode == kEpiStore && prob.k_splits > 1 ? prob.k_splits : 1;
   const bool wide = prob.N > 128 && tile_rows * ((prob.N + 255) / 256) * splits >= 148 && !prob.force_narrow;
   const bool crowded = tile_rows * ((prob.N + 127) / 128) * splits * (prob.batches > 1 ? prob.batches : 1) > 148;

@@ -22,6 +22,12 @@
 // graded and duplicated inputs keep the orthogonality of Q at the one-column kernel's level (the NumPy
 // restatement in utils/panel_pairs_reference.py shows 1e-3 without a guard, 2e-5 with a guard of 0.05).
 //
+// Bound by a chain of 64 steps of some 6900 cycles (5 CTAs; 9700 with 33): the exchange through L2 1800 (4300), sweep 1 1200,
+// pivot entries and publishing 1100, scalars and coefficients 1000, sweep 2 1200.  A warp owns one slice of 32 columns: a 16-byte
+// load of a pivot column is then one address for all lanes, 1.55 cycles of shared memory instead of the 2.2 that four slices in a
+// warp took (sweep 1 was 2130 cycles).  Panels of 1024 / 3000 / 8192 rows 324 / 329 / 411 us with four slices a warp, element-wise
+// loads and outputs staged through shared memory; 263 / 285 / 364 us now.
+//
 // Register tiling, exchange words ({value, sequence} in 64 bits, bounded polls), T construction by
 // CTA 0 in the shadow of the exchange and the output stage are those of qr.cu.
 #include <cuda_runtime.h>

@@ -8,6 +8,7 @@
 // between streams does not allow.  Device time of a step, everything on one stream / the chain beside / the averages beside:
 // 256 x 512 126 / 92 / 85 us, 512 x 1376 175 / 158 / 121 us, 1000 x 1501 198 / 198 / 148 us, 2048 x 5504 1388 / 1352 / 1186 us,
 // 4096 x 4096 1900 / 1863 / 1748 us, 8192 x 8192 within the runs' spread.
+#include <algorithm>
 #include <optional>
 #include <stdexcept>
 
@@ -118,8 +119,8 @@ HalfJob average(const SteadyStep& s, bool left) {
 }
 
 // The phases of one step, or of several that share their launches.
-template <typename Planes, typename Launch>
-void issue(const SteadyStep& s, cudaStream_t stream, Planes planes, Launch launch) {
+template <typename Planes, typename Launch, typename Averages>
+void issue(const SteadyStep& s, cudaStream_t stream, Planes planes, Launch launch, Averages launch_averages) {
   if (s.phases & kStepPlanes) planes();
   const bool averages = s.phases & kStepAverages, rotations = s.phases & (kStepForward | kStepBackward);
   const cudaStream_t side = averages && rotations ? s.side : stream;
@@ -133,10 +134,7 @@ void issue(const SteadyStep& s, cudaStream_t stream, Planes planes, Launch launc
     launch(turned_back, stream);
     launch(result, stream);
   }
-  if (averages) {
-    launch([](const SteadyStep& one) { return average(one, true); }, side);
-    launch([](const SteadyStep& one) { return average(one, false); }, side);
-  }
+  if (averages) launch_averages(side);
 }
 }  // namespace
 
@@ -158,12 +156,21 @@ void steady_step(const SteadyStep& s, int* status, cudaStream_t stream) {
         [&](auto product, cudaStream_t on) {
           const HalfJob job = product(s);
           gemm_half(job.a, job.b, job.problem, status, on);
+        },
+        [&](cudaStream_t side) {
+          const HalfJob both[2] = {average(s, true), average(s, false)};
+          if (averages_share(r.rows, r.cols)) {
+            gemm_half_group(both, 2, status, side);
+          } else {
+            for (const HalfJob& job : both) gemm_half(job.a, job.b, job.problem, status, side);
+          }
         });
 }
 
+bool averages_share(int rows, int cols) { return !half_on_pairs(rows, rows, true) && !half_on_pairs(cols, cols, true); }
+
 bool steady_step_shares(int rows, int cols) {
-  return rows > 0 && cols > 0 && !half_on_pairs(cols, rows, false) && !half_on_pairs(rows, cols, false) &&
-         !half_on_pairs(rows, rows, true) && !half_on_pairs(cols, cols, true);
+  return rows > 0 && cols > 0 && !half_on_pairs(cols, rows, false) && !half_on_pairs(rows, cols, false) && averages_share(rows, cols);
 }
 
 void steady_steps(const SteadyStep* steps, int count, int* status, cudaStream_t stream) {
@@ -183,6 +190,11 @@ void steady_steps(const SteadyStep* steps, int count, int* status, cudaStream_t 
           HalfJob jobs[kHalfGroup];
           for (int i = 0; i < count; ++i) jobs[i] = product(steps[i]);
           gemm_half_group(jobs, count, status, on);
+        },
+        [&](cudaStream_t side) {
+          HalfJob jobs[2 * kHalfGroup];
+          for (int i = 0; i < 2 * count; ++i) jobs[i] = average(steps[i / 2], i % 2 == 0);
+          for (int i = 0; i < 2 * count; i += kHalfGroup) gemm_half_group(jobs + i, std::min(kHalfGroup, 2 * count - i), status, side);
         });
 }
 

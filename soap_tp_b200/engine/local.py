@@ -299,9 +299,9 @@ def _side_stream(device, home: int) -> int:
 def _native_arguments(gradient: Tensor, state, step: int, rows: int, cols: int, averages: bool, slot: int, *, beta, beta1, beta2,
                       eps) -> tuple:
     """An ordinary step as the native call takes it: scratch, bases, addresses and scalars; then the tensor of its result."""
-    g = gradient.detach().reshape(rows, cols)
+    g = gradient if gradient.shape == (rows, cols) else gradient.detach().reshape(rows, cols)
     if g.dtype != torch.float32 and g.dtype != torch.bfloat16:
-        g = g.float()
+        g = g.detach().float()
     ctx = context_for(state)
     ctx.left.refresh(state["left_basis"], rows)
     ctx.right.refresh(state["right_basis"], cols)
@@ -318,8 +318,10 @@ def _native_arguments(gradient: Tensor, state, step: int, rows: int, cols: int, 
     return (scratch.native, ctx.left.native, ctx.right.native, arguments, scalars), update, (g, ctx)
 
 
-def _count_launches(averages: bool) -> None:
-    for name, count in (("clear_kernel", 1), ("largest_kernel", 1), ("half_planes_kernel", 1), ("gemm_half_kernel", 6 if averages else 4)):
+def _count_launches(averages: int, planes: int = 1) -> None:
+    """Of one step, or of several that share launches; ``averages``, ``planes``: the launches of their averages and of their planes."""
+    for name, count in (("clear_kernel", planes), ("largest_kernel", planes), ("half_planes_kernel", planes),
+                        ("gemm_half_kernel", 4 + averages)):
         k.LAUNCH_COUNTS[name] = k.LAUNCH_COUNTS.get(name, 0) + count
 
 
@@ -338,7 +340,7 @@ def _native_step(gradient: Tensor, state, step: int, rows: int, cols: int, *, be
     else:
         _C.steady_step(*call, _ALL_PHASES if averages else _ALL_PHASES - _C.STEP_AVERAGES, *tail)
     torch.autograd.graph.increment_version([state[name] for name in (_WRITTEN if averages else _WRITTEN[:2])])
-    _count_launches(averages)
+    _count_launches((1 if _C.averages_share(rows, cols) else 2) if averages else 0)
     return update
 
 
@@ -352,7 +354,8 @@ def shared_steps(parameters, *, beta: float, beta1: float, beta2: float, eps: fl
     """Ordinary steps of several small parameters, ``(gradient, state, rows, cols)`` each, on one device; their updates.
 
     A product of a small matrix leaves most of the GPU idle and ends in latencies (fill, drain, epilogue, launch) that are as
-    long as its work; eight of them in one launch take about as long as one."""
+    long as its work; eight of them in one launch take about as long as one (seven matrices of a decoder layer of hidden size 512:
+    921 us one after another, 405 together)."""
     for _, state, rows, cols in parameters:
         _check_state(state, rows, cols)
     updates = []
@@ -372,7 +375,7 @@ def shared_steps(parameters, *, beta: float, beta1: float, beta2: float, eps: fl
         torch.autograd.graph.increment_version([state[name] for _, state, _, _ in some for name in _WRITTEN])
         for _, state, _, _ in some:
             state["step"] = int(state["step"]) + 1
-        _count_launches(True)
+        _count_launches(-(-2 * len(some) // _C.STEP_GROUP), len({g.dtype for g, _ in held}))
     return updates
 
 

@@ -80,11 +80,12 @@ class SoapTP(torch.optim.Optimizer):
             raise ValueError(f"process_grid_shape={self.grid} does not match world_size={world}.")
 
     # ---- classification -------------------------------------------------------------------------
-    def _plan(self, p: Tensor, group: dict) -> Optional[dict]:
+    def _plan(self, p: Tensor, group: dict, world: Optional[int] = None) -> Optional[dict]:
         """How ``p`` is preconditioned: ``None`` (AdamW) or the ``soap_step`` layout arguments."""
         if p.ndim != 2:
             return None
-        world = dist.get_world_size() if dist.is_initialized() else 1
+        if world is None:
+            world = dist.get_world_size() if dist.is_initialized() else 1
         shard_dim = getattr(p, "tp_shard_dim", None)
         if shard_dim is not None:
             global_shape = tuple(getattr(p, "tp_global_shape"))
@@ -123,7 +124,7 @@ class SoapTP(torch.optim.Optimizer):
             for p in group["params"]:
                 if p.grad is None:
                     continue
-                plan = self._plan(p, group)
+                plan = self._plan(p, group, world)
                 if plan is None:
                     self._adamw(p, group)
                     continue
