@@ -399,8 +399,8 @@ PYBIND11_MODULE(_C, m) {
   m.def("apply_updates", [](const std::vector<std::tuple<uint64_t, uint64_t, int64_t>>& all, int type, float keep, float lr, uint64_t stream) {
     std::vector<UpdateJob> jobs;
     for (const auto& [p, update, n] : all) jobs.push_back(UpdateJob{ptr<void>(p), ptr<const float>(update), n});
-    apply_updates(jobs.data(), static_cast<int>(jobs.size()), type, keep, lr, stream_of(stream));
-  });
+    return apply_updates(jobs.data(), static_cast<int>(jobs.size()), type, keep, lr, stream_of(stream));
+  }, "Returns the launches that it took");
   m.def("adamw_update", [](uint64_t p, int type, uint64_t gradient, uint64_t mo, uint64_t v, int64_t n, float beta1_rest,
                            float beta2, float beta2_rest, float bias1, float bias2, float eps, float keep, float lr,
                            uint64_t stream) {

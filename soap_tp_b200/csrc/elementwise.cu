@@ -277,7 +277,7 @@ void launch_updates(const UpdateJob* jobs, int count, float keep, float lr, cuda
 }
 }  // namespace
 
-void apply_updates(const UpdateJob* jobs, int count, int type, float keep, float lr, cudaStream_t stream) {
+int apply_updates(const UpdateJob* jobs, int count, int type, float keep, float lr, cudaStream_t stream) {
   if (type != 0 && type != 1) throw std::invalid_argument("apply_updates: unknown parameter type");
   auto go = [&](auto* typed, const UpdateJob* some, int n) {
     using T = std::remove_pointer_t<decltype(typed)>;
@@ -290,9 +290,10 @@ void apply_updates(const UpdateJob* jobs, int count, int type, float keep, float
     return x < y + width * b.n && y < x + width * a.n;
   };
   UpdateJob some[kUpdateGroup];
-  int n = 0;
+  int n = 0, launches = 0;
   auto flush = [&] {
     if (n == 0) return;
+    ++launches;
     if (type == 0) go(static_cast<float*>(nullptr), some, n);
     else go(static_cast<__nv_bfloat16*>(nullptr), some, n);
     n = 0;
@@ -304,6 +305,7 @@ void apply_updates(const UpdateJob* jobs, int count, int type, float keep, float
     some[n++] = jobs[i];
   }
   flush();
+  return launches;
 }
 
 void adamw_update(void* p, int type, const void* gradient, float* m, float* v, int64_t n, float beta1_rest, float beta2,

@@ -35,7 +35,7 @@ struct UpdateJob {
   const float* update;
   int64_t n;
 };
-void apply_updates(const UpdateJob* jobs, int count, int type, float keep, float lr, cudaStream_t stream);
+int apply_updates(const UpdateJob* jobs, int count, int type, float keep, float lr, cudaStream_t stream);
 void adamw_update(void* p, int type, const void* gradient, float* m, float* v, int64_t n, float beta1_rest, float beta2,
                   float beta2_rest, float bias1, float bias2, float eps, float keep, float lr, cudaStream_t stream);
 

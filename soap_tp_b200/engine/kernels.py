@@ -629,9 +629,9 @@ def apply_updates(pairs, keep: float, lr: float) -> list:
         else:
             jobs.setdefault(kind, []).append((p, (p.data_ptr(), update.data_ptr(), p.numel())))
     for kind, some in jobs.items():
-        _C.apply_updates([job for _, job in some], kind, keep, lr, _stream())
+        launches = _C.apply_updates([job for _, job in some], kind, keep, lr, _stream())
         mark_written(*(p for p, _ in some))
-        _count("apply_updates_kernel")
+        LAUNCH_COUNTS["apply_updates_kernel"] = LAUNCH_COUNTS.get("apply_updates_kernel", 0) + launches
     return left
 
 
