@@ -90,7 +90,33 @@ __device__ __forceinline__ void householder_scalars(float alpha, float normsq, f
 // kPer rows of one column per thread: 64 (256-row CTAs, fewest SMs) or 32 (128-row CTAs: the sweeps are bound
 // by shared-memory load latency, and with half the registers taken by the slab every load of a sweep can be in
 // flight at once).
-template <int kPer>
+// kCluster: up to eight CTAs (1792 rows) are one cluster and write their sums into each other's shared memory instead of polling words
+// in global memory; the same values are added in the same order.  Panels of 300 / 1024 / 1792 rows 257 / 262 / 279 us by polling,
+// 214 / 229 / 243 as a cluster.  (Eight is the largest cluster that every GPU takes, and one that finds its SMs free in one of the chip's
+// groups beside other kernels.)
+constexpr int kClusterCtas = 8;
+template <bool kCluster>
+struct Inbox {};
+template <>
+struct Inbox<true> {
+  float2 dots[2][kClusterCtas][kB];    // {D1_j, D2_j} of every CTA, by step parity
+  float rows[2][2][kB];                // the two pivot rows
+  uint64_t arrived[2];                 // all of a step's bytes
+};
+
+// A value into the shared memory of CTA `rank` of the cluster, its bytes credited to a barrier there.
+__device__ __forceinline__ void send(const float* to, float value, const uint64_t* bar, int rank) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(map_to_cta(smem_u32(to), rank)),
+               "r"(__float_as_uint(value)), "r"(map_to_cta(smem_u32(bar), rank))
+               : "memory");
+}
+__device__ __forceinline__ void send(const float2* to, float x, float y, const uint64_t* bar, int rank) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];" ::"r"(map_to_cta(smem_u32(to), rank)),
+               "r"(__float_as_uint(x)), "r"(__float_as_uint(y)), "r"(map_to_cta(smem_u32(bar), rank))
+               : "memory");
+}
+
+template <int kPer, bool kCluster>
 __global__ void __launch_bounds__(kPanelThreads, 1) qr_panel_pairs_kernel(PanelArgs a) {
   constexpr int kCtaRows = 4 * kPer;
   constexpr int kVec = kPer / 4;       // 128-bit loads per sweep and pivot column
@@ -105,6 +131,7 @@ __global__ void __launch_bounds__(kPanelThreads, 1) qr_panel_pairs_kernel(PanelA
   __shared__ float row1_local[kB];                      // single-CTA launches: rows c and c + 1 without the exchange
   __shared__ float row2_local[kB];
   __shared__ int abort_flag;
+  __shared__ Inbox<kCluster> inbox;
   extern __shared__ float dyn[];
   float (*T)[kPitch] = reinterpret_cast<float (*)[kPitch]>(dyn);   // last CTA: compact-WY factor
 
@@ -143,6 +170,13 @@ __global__ void __launch_bounds__(kPanelThreads, 1) qr_panel_pairs_kernel(PanelA
   }
   if (t < kB) taus[t] = 0.f;
   if (t == 0) abort_flag = 0;
+  if constexpr (kCluster) {
+    if (t == 0) {
+      mbar_init(&inbox.arrived[0], 1);
+      mbar_init(&inbox.arrived[1], 1);
+      mbar_fence_init();
+    }
+  }
   if (builds_t)
     for (int idx = t; idx < kB * kPitch; idx += kPanelThreads) dyn[idx] = 0.f;
   if (j < 2) {
@@ -151,6 +185,7 @@ __global__ void __launch_bounds__(kPanelThreads, 1) qr_panel_pairs_kernel(PanelA
     for (int k = 0; k < kPer; ++k) dst[k] = P[k];
   }
   __syncthreads();
+  if constexpr (kCluster) cluster_sync_all();      // the barriers exist before anything arrives on them
 
   const int reflectors = min(a.b, a.r);
   const unsigned int seq_base = a.epoch * 256u;
@@ -168,6 +203,11 @@ __global__ void __launch_bounds__(kPanelThreads, 1) qr_panel_pairs_kernel(PanelA
     const int local1 = c - row0 - my_first, local2 = c + 1 - row0 - my_first;
     const bool mine1 = local1 >= 0 && local1 < kPer;
     const bool mine2 = local2 >= 0 && local2 < kPer && row2_exists;
+
+    if constexpr (kCluster) {
+      // (a step's bytes cannot arrive before the step before has ended here: its senders wait for this CTA's)
+      if (t == 0) mbar_expect_tx(&inbox.arrived[parity], static_cast<uint32_t>(kB * (8 * ctas + (row2_exists ? 8 : 4))));
+    }
 
     // ---- sweep 1: dot products of both pivot columns with this thread's slice of column j ----
     if (has_rows) {
@@ -191,22 +231,35 @@ __global__ void __launch_bounds__(kPanelThreads, 1) qr_panel_pairs_kernel(PanelA
     unsigned long long* rows = &slots[(static_cast<int64_t>(ctas) * kB + j) * 2];
     if (mine1) {
       const float entry = take_entry<kPer>(P, local1, false);
-      if (ctas > 1) ll_publish(rows, entry, seq);
-      else row1_local[j] = entry;
+      if constexpr (kCluster) {
+        for (int g = 0; g < ctas; ++g) send(&inbox.rows[parity][0][j], entry, &inbox.arrived[parity], g);
+      } else if (ctas > 1) {
+        ll_publish(rows, entry, seq);
+      } else {
+        row1_local[j] = entry;
+      }
     }
     if (mine2) {
       const float entry = take_entry<kPer>(P, local2, false);
-      if (ctas > 1) ll_publish(rows + 1, entry, seq);
-      else row2_local[j] = entry;
+      if constexpr (kCluster) {
+        for (int g = 0; g < ctas; ++g) send(&inbox.rows[parity][1][j], entry, &inbox.arrived[parity], g);
+      } else if (ctas > 1) {
+        ll_publish(rows + 1, entry, seq);
+      } else {
+        row2_local[j] = entry;
+      }
     }
     if (ctas == 1 && !row2_exists && q == 0) row2_local[j] = 0.f;
     __syncthreads();                                                              // barrier 1
     float partial1 = 0.f, partial2 = 0.f;                     // this CTA's dot products with column jx
-    if (qx == 0 && has_rows) {
+    if ((kCluster || qx == 0) && has_rows) {
       partial1 = (slices[0][jx].x + slices[1][jx].x) + (slices[2][jx].x + slices[3][jx].x);
       partial2 = (slices[0][jx].y + slices[1][jx].y) + (slices[2][jx].y + slices[3][jx].y);
     }
-    if (qx == 0 && ctas > 1) {
+    if constexpr (kCluster) {
+      for (int g = qx; g < ctas; g += 4)
+        send(&inbox.dots[parity][blockIdx.x][jx], partial1, partial2, &inbox.arrived[parity], g);
+    } else if (qx == 0 && ctas > 1) {
       unsigned long long* mine = &slots[(static_cast<int64_t>(blockIdx.x) * kB + jx) * 2];
       asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(mine), "l"(pack_word(partial1, seq)),
                    "l"(pack_word(partial2, seq))
@@ -223,11 +276,23 @@ __global__ void __launch_bounds__(kPanelThreads, 1) qr_panel_pairs_kernel(PanelA
     }
 
     // ---- exchange: lane qx polls CTAs qx, qx + 4, qx + 8, ... (index `ctas` holds the two pivot rows) ----
-    if (ctas > 1) {
+    if (kCluster || ctas > 1) {
       float total1 = 0.f, total2 = 0.f, p1 = 0.f, p2 = 0.f;
       float part1 = 0.f, part2 = 0.f;
       bool failed = false;
-      for (int base = 0; base <= ctas && !failed; base += 4 * kPollPairs) {
+      if constexpr (kCluster) {
+        failed = !mbar_wait_bounded(&inbox.arrived[parity], (step >> 1) & 1, &abort_flag, nullptr, 0);
+        for (int g = qx; g < ctas; g += 4) {
+          const float2 dots = inbox.dots[parity][g][jx];
+          part1 += dots.x;
+          part2 += dots.y;
+        }
+        if (qx == 0) {
+          p1 = inbox.rows[parity][0][jx];
+          p2 = row2_exists ? inbox.rows[parity][1][jx] : 0.f;
+        }
+      }
+      for (int base = 0; !kCluster && base <= ctas && !failed; base += 4 * kPollPairs) {
         unsigned long long w1[kPollPairs], w2[kPollPairs];
         bool pending = true;
         unsigned int polls = 0;
@@ -469,6 +534,7 @@ __global__ void __launch_bounds__(kPanelThreads, 1) qr_panel_pairs_kernel(PanelA
       }
     }
   }
+  if constexpr (kCluster) cluster_sync_all();      // nobody leaves while another CTA may still write into its shared memory
 }
 
 }  // namespace
@@ -478,15 +544,34 @@ namespace {
 template <int kPer>
 void launch_pairs(PanelArgs args, int r, cudaStream_t stream) {
   const size_t smem = static_cast<size_t>(kB) * kPitch * sizeof(float);
-  static PerDeviceOnce configured;
-  allow_dynamic_smem(reinterpret_cast<const void*>(qr_panel_pairs_kernel<kPer>), smem, configured, "qr_panel_pairs");
-  void* params[] = {&args};
   int ctas = (r + 4 * kPer - 1) / (4 * kPer);
   if (ctas > 1 && ctas < 148) ++ctas;   // the rowless CTA that builds T (see the kernel)
-  // Cooperative launch: the CTAs exchange data through global memory while running, so all of them
-  // must be resident at the same time; the runtime refuses the launch otherwise.
-  cudaError_t err = cudaLaunchCooperativeKernel(reinterpret_cast<void*>(qr_panel_pairs_kernel<kPer>), dim3(ctas),
-                                                dim3(kPanelThreads), params, smem, stream);
+  cudaError_t err;
+  if (ctas > 1 && ctas <= kClusterCtas) {
+    // a cluster's CTAs are resident together by definition
+    static PerDeviceOnce configured;
+    allow_dynamic_smem(reinterpret_cast<const void*>(qr_panel_pairs_kernel<kPer, true>), smem, configured, "qr_panel_pairs");
+    cudaLaunchAttribute cluster{};
+    cluster.id = cudaLaunchAttributeClusterDimension;
+    cluster.val.clusterDim.x = static_cast<unsigned>(ctas);
+    cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
+    cudaLaunchConfig_t config{};
+    config.gridDim = dim3(ctas);
+    config.blockDim = dim3(kPanelThreads);
+    config.dynamicSmemBytes = smem;
+    config.stream = stream;
+    config.attrs = &cluster;
+    config.numAttrs = 1;
+    err = cudaLaunchKernelEx(&config, qr_panel_pairs_kernel<kPer, true>, args);
+  } else {
+    static PerDeviceOnce configured;
+    allow_dynamic_smem(reinterpret_cast<const void*>(qr_panel_pairs_kernel<kPer, false>), smem, configured, "qr_panel_pairs");
+    void* params[] = {&args};
+    // Cooperative launch: the CTAs exchange data through global memory while running, so all of them
+    // must be resident at the same time; the runtime refuses the launch otherwise.
+    err = cudaLaunchCooperativeKernel(reinterpret_cast<void*>(qr_panel_pairs_kernel<kPer, false>), dim3(ctas), dim3(kPanelThreads),
+                                      params, smem, stream);
+  }
   if (err != cudaSuccess) throw std::runtime_error(std::string("qr_panel_pairs launch: ") + cudaGetErrorString(err));
 }
 
