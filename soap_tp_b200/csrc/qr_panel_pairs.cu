@@ -32,6 +32,7 @@
 // CTA 0 in the shadow of the exchange and the output stage are those of qr.cu.
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <stdexcept>
 #include <string>
 
@@ -90,11 +91,12 @@ __device__ __forceinline__ void householder_scalars(float alpha, float normsq, f
 // kPer rows of one column per thread: 64 (256-row CTAs, fewest SMs) or 32 (128-row CTAs: the sweeps are bound
 // by shared-memory load latency, and with half the registers taken by the slab every load of a sweep can be in
 // flight at once).
-// kCluster: up to eight CTAs (1792 rows) are one cluster and write their sums into each other's shared memory instead of polling words
-// in global memory; the same values are added in the same order.  Panels of 300 / 1024 / 1792 rows 257 / 262 / 279 us by polling,
-// 214 / 229 / 243 as a cluster.  (Eight is the largest cluster that every GPU takes, and one that finds its SMs free in one of the chip's
-// groups beside other kernels.)
-constexpr int kClusterCtas = 8;
+// kCluster: up to sixteen CTAs (3840 rows), or eight where the device takes no larger cluster, are one cluster and write their sums into
+// each other's shared memory instead of polling words in global memory; the same values are added in the same order.  Panels of
+// 300 / 1024 / 2048 / 3000 rows 257 / 262 / 275 / 288 us by polling, 214 / 229 / 244 / 277 as a cluster.  Finding sixteen free SMs in one
+// of the chip's groups beside other kernels does not cost what that gives: refresh 3000 x 2000 9.82 ms by polling, 9.34 with
+// clusters of up to eight, 8.99 of up to sixteen (8192 x 8192 75 to 77 ms with any).
+constexpr int kClusterCtas = 16, kPortableClusterCtas = 8;
 template <bool kCluster>
 struct Inbox {};
 template <>
@@ -541,28 +543,53 @@ __global__ void __launch_bounds__(kPanelThreads, 1) qr_panel_pairs_kernel(PanelA
 
 namespace {
 
-template <int kPer>
-void launch_pairs(PanelArgs args, int r, cudaStream_t stream) {
-  const size_t smem = static_cast<size_t>(kB) * kPitch * sizeof(float);
-  int ctas = (r + 4 * kPer - 1) / (4 * kPer);
-  if (ctas > 1 && ctas < 148) ++ctas;   // the rowless CTA that builds T (see the kernel)
-  cudaError_t err;
-  if (ctas > 1 && ctas <= kClusterCtas) {
-    // a cluster's CTAs are resident together by definition
-    static PerDeviceOnce configured;
-    allow_dynamic_smem(reinterpret_cast<const void*>(qr_panel_pairs_kernel<kPer, true>), smem, configured, "qr_panel_pairs");
-    cudaLaunchAttribute cluster{};
+struct ClusterLaunch {
+  cudaLaunchAttribute cluster{};
+  cudaLaunchConfig_t config{};
+  ClusterLaunch(int ctas, size_t smem, cudaStream_t stream) {
     cluster.id = cudaLaunchAttributeClusterDimension;
     cluster.val.clusterDim.x = static_cast<unsigned>(ctas);
     cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
-    cudaLaunchConfig_t config{};
     config.gridDim = dim3(ctas);
     config.blockDim = dim3(kPanelThreads);
     config.dynamicSmemBytes = smem;
     config.stream = stream;
     config.attrs = &cluster;
     config.numAttrs = 1;
-    err = cudaLaunchKernelEx(&config, qr_panel_pairs_kernel<kPer, true>, args);
+  }
+  ClusterLaunch(const ClusterLaunch&) = delete;      // (the configuration points into the object)
+};
+
+// CTAs of the largest cluster that this device takes of the kernel, which is made ready for it; looked up once for each device.
+template <int kPer>
+int largest_cluster(size_t smem) {
+  constexpr int kDevices = 64;
+  static std::atomic<int> known[kDevices] = {};
+  int device = 0;
+  if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= kDevices) return 0;
+  if (const int largest = known[device].load()) return largest;
+  auto* kernel = qr_panel_pairs_kernel<kPer, true>;
+  PerDeviceOnce once;
+  allow_dynamic_smem(reinterpret_cast<const void*>(kernel), smem, once, "qr_panel_pairs");
+  int clusters = 0;
+  ClusterLaunch launch(kClusterCtas, smem, nullptr);
+  const bool large = cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel), cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                     cudaOccupancyMaxActiveClusters(&clusters, kernel, &launch.config) == cudaSuccess && clusters > 0;
+  if (!large) cudaGetLastError();      // (a refusal is not this launch's error)
+  known[device] = large ? kClusterCtas : kPortableClusterCtas;
+  return known[device];
+}
+
+template <int kPer>
+void launch_pairs(PanelArgs args, int r, cudaStream_t stream) {
+  const size_t smem = static_cast<size_t>(kB) * kPitch * sizeof(float);
+  int ctas = (r + 4 * kPer - 1) / (4 * kPer);
+  if (ctas > 1 && ctas < 148) ++ctas;   // the rowless CTA that builds T (see the kernel)
+  cudaError_t err;
+  if (ctas > 1 && ctas <= largest_cluster<kPer>(smem)) {
+    // a cluster's CTAs are resident together by definition
+    ClusterLaunch launch(ctas, smem, stream);
+    err = cudaLaunchKernelEx(&launch.config, qr_panel_pairs_kernel<kPer, true>, args);
   } else {
     static PerDeviceOnce configured;
     allow_dynamic_smem(reinterpret_cast<const void*>(qr_panel_pairs_kernel<kPer, false>), smem, configured, "qr_panel_pairs");

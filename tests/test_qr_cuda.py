@@ -103,3 +103,37 @@ def test_panel_kernels_agree(rows):
         for a, b in zip(reference, other):
             assert float((a - b).abs().max()) < 2e-4 * max(1.0, float(a.abs().max()))
         assert torch.allclose(other[0], other[3].T, atol=1e-6)       # V and V^T outputs are the same matrix
+
+
+@pytest.mark.parametrize("rows", [2, 129, 256, 257, 1920, 1921, 3840, 3841])
+@pytest.mark.parametrize("width", [1, 2, 77, 128])
+def test_panels_at_the_edges_of_a_cluster(rows, width):
+    """From one thread block to the largest cluster of them and one past it, for both heights of a block, with panels of every
+    width: the reflectors of the one-column kernel up to rounding (the bound of the test above)."""
+    from soap_tp_b200.engine import kernels as k
+
+    device = torch.device("cuda", 0)
+    generator = torch.Generator(device=device).manual_seed(rows + width)
+    source = k.split_planes(torch.randn(rows, width, generator=generator, device=device))
+    exchange = torch.zeros(8 * 160 * 128 + 8 * 128, device=device)
+    results = []
+    for variant in ("one", 256, 128):
+        v, vt = k.Planes.empty(rows, width, device), k.Planes.empty(width, rows, device)
+        T, Tt = k.Planes.empty(width, 128, device), k.Planes.empty(width, 128, device)
+        tau = torch.zeros(256, device=device)
+        arguments = (*source.pointers(), rows, width, *v.pointers(), *vt.pointers(), tau.data_ptr(), T.hi.data_ptr(), T.lo.data_ptr(),
+                     Tt.hi.data_ptr(), Tt.lo.data_ptr(), T.ld, exchange.data_ptr(), k.status_word(device).data_ptr(), k._stream())
+        if variant == "one":
+            k._C.qr_panel(*arguments)
+        else:
+            k._C.qr_panel_pairs(*arguments, variant)
+        torch.cuda.synchronize()
+        k.check_status()
+        results.append((v.dense(), tau[: min(rows, width)], T.dense()[:, :width], Tt.dense()[:, :width].T, vt.dense().T))
+    reference = results[0]
+    last = min(rows, width) - 1 if rows <= width else None      # of a single element: its reflector hangs on rounding
+    for other in results[1:]:
+        for a, b in zip(reference, other):
+            if last is not None:
+                a, b = (x[..., :last] for x in (a, b))
+            assert a.numel() == 0 or float((a - b).abs().max()) < 2e-4 * max(1.0, float(a.abs().max()))
