@@ -669,9 +669,9 @@ void mixed_maps(CUtensorMap (&maps)[2], const SplitTarget& planes, int64_t K, in
 bool half_on_pairs(int M, int N, bool symmetric) {
   if (!gemm_cta_pairs_wanted()) return false;
   // A pair's 256 x 256 tile takes about 1.5 times as long as a CTA's 128 x 128 one (it loads half as much per product): pairs
-  // unless single CTAs get by with so few waves that they finish earlier.  Pairs against singles, two terms: 1024^3 29 and
-  // 22 us, 1536^3 37 and 30, 2048^3 47 and 70, 3072^3 139 and 209, 4096^3 340 and 439; symmetric, two terms and one: 1024 33 and
-  // 24, 28 and 19; 2048 50 and 41, 39 and 32; 3072 144 and 164, 100 and 113; 4096 190 and 291, 134 and 206.
+  // unless single CTAs get by with so few waves that they finish earlier.  Pairs against singles, two terms: 1024^3 27 and
+  // 20 us, 1536^3 34 and 27, 1792^3 40 and 58, 2048^3 44 and 64, 3072^3 132 and 178, 4096^3 319 and 409; symmetric, two terms and one: 1024
+  // 30 and 22, 26 and 17; 2048 46 and 39, 37 and 29; 3072 130 and 140, 96 and 97; 4096 196 and 267, 143 and 191.
   auto tiles_of = [&](int64_t side) {
     const int64_t m = (M + side - 1) / side, n = (N + side - 1) / side;
     return symmetric ? m * (m + 1) / 2 : m * n;
