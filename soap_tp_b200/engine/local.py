@@ -233,17 +233,20 @@ def gram_updates_for_bases(gradient: Tensor, state, beta: float, rows: int, cols
 
 class _Scratch:
     """Buffers of a rotation as the native calls take them, shared by matrices of one shape: with ``update`` those of a step's
-    way back as well, with ``averages`` the planes of its Gram products."""
+    way back as well, with ``averages`` the planes of its Gram products.  ``slots``: which set of them, of the mixed form of the
+    left basis, and of the right one's (steps that share launches, ``shared_steps``)."""
 
-    def __init__(self, rows: int, cols: int, device, terms: int, update: bool, averages: bool, slot: int) -> None:
+    def __init__(self, rows: int, cols: int, device, terms: int, update: bool, averages: bool, slots: tuple) -> None:
+        slot, left, right = slots
         self.wide = torch.zeros(1, dtype=torch.int32, device=device)        # the decision on the range
         self.maxima = torch.empty(max(1, rows), dtype=torch.int32, device=device)
         planes = [workspace_planes("X", rows, cols, device, terms=terms, slot=slot)]
         if averages:
             planes.append(workspace_planes("GT", cols, rows, device, terms=terms, slot=slot))
         middle = workspace_planes("T", cols, rows, device, blocked=True, slot=slot)
-        mixed = [tf32_workspace(*size, device, slot) for size in (
-            ("G", rows, cols), ("T", cols, rows), ("L", rows, rows), ("LT", rows, rows), ("R", cols, cols), ("RT", cols, cols))]
+        mixed = [tf32_workspace(tag, depth, width, device, which) for tag, depth, width, which in (
+            ("G", rows, cols, slot), ("T", cols, rows, slot), ("L", rows, rows, left), ("LT", rows, rows, left),
+            ("R", cols, cols, right), ("RT", cols, cols, right))]
         turned = planes[1].target() if averages else (0, 0, 64, 0, self.maxima.data_ptr())
         addresses = (planes[0].target() + turned + middle.operand() + (self.wide.data_ptr(), int(k.SPLIT_ROUND_NEAREST))
                      + tuple(value for each in mixed for value in each.mixed_target()))
@@ -256,11 +259,14 @@ class _Scratch:
         self.native = _C.RotationScratch(rows, cols, addresses)
 
 
-def _scratch(rows: int, cols: int, device, terms: int, update: bool = False, averages: bool = False, slot: int = 0) -> _Scratch:
-    key = ("scratch", rows, cols, device, terms, update, averages, slot)
+_FIRST = (0, 0, 0)
+
+
+def _scratch(rows: int, cols: int, device, terms: int, update: bool = False, averages: bool = False, slots: tuple = _FIRST) -> _Scratch:
+    key = ("scratch", rows, cols, device, terms, update, averages, slots)
     entry = _WORKSPACES.get(key)
     if entry is None:
-        entry = _WORKSPACES[key] = _Scratch(rows, cols, device, terms, update, averages, slot)
+        entry = _WORKSPACES[key] = _Scratch(rows, cols, device, terms, update, averages, slots)
     return entry
 
 
@@ -296,7 +302,7 @@ def _side_stream(device, home: int) -> int:
     return stream.cuda_stream
 
 
-def _native_arguments(gradient: Tensor, state, step: int, rows: int, cols: int, averages: bool, slot: int, *, beta, beta1, beta2,
+def _native_arguments(gradient: Tensor, state, step: int, rows: int, cols: int, averages: bool, slots: tuple, *, beta, beta1, beta2,
                       eps) -> tuple:
     """An ordinary step as the native call takes it: scratch, bases, addresses and scalars; then the tensor of its result."""
     g = gradient if gradient.shape == (rows, cols) else gradient.detach().reshape(rows, cols)
@@ -308,7 +314,7 @@ def _native_arguments(gradient: Tensor, state, step: int, rows: int, cols: int, 
     bias2 = 1.0 - beta2**step
     momentum, variance = state["momentum"], state["variance"]
     left, right = state["left_preconditioner"], state["right_preconditioner"]
-    scratch = _scratch(rows, cols, g.device, 1 if g.dtype == torch.bfloat16 else 2, update=True, averages=averages, slot=slot)
+    scratch = _scratch(rows, cols, g.device, 1 if g.dtype == torch.bfloat16 else 2, update=True, averages=averages, slots=slots)
     update = torch.empty((rows, cols), dtype=torch.float32, device=g.device)
     arguments = (k.strided_source(g)
                  + (momentum.data_ptr(), k._ld(momentum), variance.data_ptr(), k._ld(variance), update.data_ptr(),
@@ -330,7 +336,7 @@ _WRITTEN = ("momentum", "variance", "left_preconditioner", "right_preconditioner
 
 def _native_step(gradient: Tensor, state, step: int, rows: int, cols: int, *, beta, beta1, beta2, eps, averages: bool) -> Tensor:
     """An ordinary step, its launches issued by one native call; without ``averages`` the rotations and Adam only."""
-    call, update, held = _native_arguments(gradient, state, step, rows, cols, averages, 0, beta=beta, beta1=beta1, beta2=beta2, eps=eps)
+    call, update, held = _native_arguments(gradient, state, step, rows, cols, averages, _FIRST, beta=beta, beta1=beta1, beta2=beta2, eps=eps)
     home = k._stream()
     tail = (k.status_word(update.device).data_ptr(), home, _side_stream(update.device, home))
     if TIMER.enabled:
@@ -363,9 +369,13 @@ def shared_steps(parameters, *, beta: float, beta1: float, beta2: float, eps: fl
         some = parameters[first:first + _C.STEP_GROUP]
         calls, held, used = [], [], {}
         for gradient, state, rows, cols in some:
-            # parameters of one shape that run together have scratch of their own each
-            slot = used[(rows, cols)] = used.get((rows, cols), -1) + 1
-            call, update, holds = _native_arguments(gradient, state, int(state["step"]) + 1, rows, cols, True, slot, beta=beta,
+            # What runs together has scratch of its own each: parameters of one shape, and the mixed form of bases of one size
+            # whatever the other side (workspaces of different tags or sizes are different ones).
+            keys = ((rows, cols), ("left", rows), ("right", cols))
+            for key in keys:
+                used[key] = used.get(key, -1) + 1
+            slots = tuple(used[key] for key in keys)
+            call, update, holds = _native_arguments(gradient, state, int(state["step"]) + 1, rows, cols, True, slots, beta=beta,
                                                     beta1=beta1, beta2=beta2, eps=eps)
             calls.append(call)
             held.append(holds)

@@ -1,0 +1,70 @@
+"""What the optimizer hands to the native calls when small parameters share launches, with these calls recorded instead of made."""
+import pytest
+import torch
+
+from soap_tp_b200.engine import kernels as k
+from soap_tp_b200.engine import local
+
+SCALARS = dict(beta=0.95, beta1=0.9, beta2=0.95, eps=1e-8)
+
+
+class Handle:
+    """Stands for a native object."""
+
+    def __init__(self, *arguments):
+        pass
+
+
+@pytest.fixture
+def groups(monkeypatch):
+    """The steps of every shared launch, as `steady_steps` receives them."""
+    made = []
+    monkeypatch.setattr(local, "_WORKSPACES", {})
+    monkeypatch.setattr(local, "_CONTEXTS", type(local._CONTEXTS)())
+    for name in ("RotationScratch", "BasisOperands"):
+        monkeypatch.setattr(k._C, name, Handle)
+    monkeypatch.setattr(k._C, "half_planes", lambda *arguments: None)
+    monkeypatch.setattr(k._C, "steady_steps", lambda calls, *tail: made.append(calls))
+    monkeypatch.setattr(k, "MIXED_CORRECTIONS", True)
+    monkeypatch.setattr(k, "_stream", lambda: 0)
+    monkeypatch.setattr(k, "status_word", lambda device: torch.zeros(4, dtype=torch.int32))
+    monkeypatch.setattr(local, "_side_stream", lambda device, home: home)
+    return made
+
+
+def _state(rows, cols):
+    packed = lambda m, n: torch.zeros(n, m).T
+    return dict(left_preconditioner=packed(rows, rows), right_preconditioner=packed(cols, cols), left_basis=packed(rows, rows),
+                right_basis=packed(cols, cols), left_work=packed(rows, rows), right_work=packed(cols, cols),
+                momentum=packed(rows, cols), variance=packed(rows, cols), step=4)
+
+
+def _tensors(holder):
+    if torch.is_tensor(holder):
+        return [holder]
+    if isinstance(holder, (list, tuple)):
+        return [tensor for each in holder for tensor in _tensors(each)]
+    if isinstance(holder, (k.Planes, k.HalfPlanes, local._Scratch)):
+        return [tensor for each in vars(holder).values() for tensor in _tensors(each)]
+    return []
+
+
+@pytest.mark.parametrize("shapes", [
+    [(64, 64), (160, 64), (64, 160), (64, 64), (160, 64), (64, 160), (160, 160), (64, 32)],
+    [(48, 32), (32, 48)] * 4,
+    [(16, 8 * i) for i in range(1, 9)],
+    [(8 * i, 16) for i in range(1, 9)],
+    [(24, 24)] * 8,
+])
+@pytest.mark.parametrize("dtypes", [(torch.float32,), (torch.float32, torch.bfloat16)])
+def test_steps_that_share_launches_write_no_scratch_of_each_other(groups, shapes, dtypes):
+    """A decoder layer's matrices have sides in common, and all of them may take the mixed form, which writes their bases too."""
+    parameters = [(torch.zeros(shape, dtype=dtypes[i % len(dtypes)]), _state(*shape), *shape) for i, shape in enumerate(shapes)]
+    local.shared_steps(parameters, **SCALARS)
+    by_handle = {id(entry.native): entry for entry in local._WORKSPACES.values() if isinstance(entry, local._Scratch)}
+    group, = groups
+    storages = [{tensor.untyped_storage().data_ptr() for tensor in _tensors(by_handle[id(call[0])])} for call in group]
+    assert len(storages) == len(shapes) and all(len(mine) > 10 for mine in storages)
+    for i, mine in enumerate(storages):
+        for theirs in storages[:i]:
+            assert mine.isdisjoint(theirs)

@@ -114,3 +114,50 @@ def test_optimizer_steps_small_matrices_together():
         assert mine.keys() == its.keys()
         for name in mine:
             assert torch.equal(mine[name], its[name]) if torch.is_tensor(mine[name]) else mine[name] == its[name], name
+
+
+def _assert_shared_equals_alone(shapes, gradients):
+    """Two steps of every parameter, together and one after another; returns the scratch of the shared ones."""
+    from soap_tp_b200.engine import kernels as k
+    from soap_tp_b200.engine import local
+
+    scalars = dict(beta=0.95, beta1=0.9, beta2=0.95, eps=1e-8)
+    results = []
+    for together in (False, True):
+        local.release_workspaces()
+        states = [_state(*shape, 3 + i) for i, shape in enumerate(shapes)]
+        updates = []
+        for turn in range(2):
+            grads = [gradients(i, turn) for i in range(len(shapes))]
+            if together:
+                updates += local.shared_steps([(grad, state, *shape) for grad, state, shape in zip(grads, states, shapes)], **scalars)
+            else:
+                updates += [local.soap_step(grad, state, global_shape=shape, interval=1000, implementation="householder",
+                                            initializing=False, **scalars) for grad, state, shape in zip(grads, states, shapes)]
+        torch.cuda.synchronize()
+        results.append(updates + [state[name] for state in states for name in local._WRITTEN])
+    k.check_status()
+    for a, b in zip(*results):
+        assert torch.equal(a.nan_to_num(nan=123.0), b.nan_to_num(nan=123.0))
+    return [entry for entry in local._WORKSPACES.values() if isinstance(entry, local._Scratch)]
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("spread", ["graded", "zero row", "zero column"])
+def test_steps_in_the_mixed_form_that_have_sides_in_common(dtype, spread):
+    """Every one of them converts its own bases, also where another one of the same size is converted in the same launch."""
+    shapes = [(64, 64), (160, 64), (64, 160), (64, 64), (160, 64), (192, 192), (64, 192), (192, 64)]
+
+    def gradient(i, turn):
+        rows, cols = shapes[i]
+        grad = torch.randn(rows, cols, generator=torch.Generator().manual_seed(20 * turn + i))
+        if spread == "graded":
+            grad *= torch.logspace(0, -6, rows)[:, None]
+        elif spread == "zero row":
+            grad[rows // 2] = 0.0
+        else:
+            grad[:, cols // 3] = 0.0
+        return grad.to(dtype).cuda()
+
+    scratches = _assert_shared_equals_alone(shapes, gradient)
+    assert len(scratches) == len(shapes) and all(int(scratch.wide) == 1 for scratch in scratches)
