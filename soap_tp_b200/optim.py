@@ -37,6 +37,9 @@ from .profiling import profile_enabled
 from .step import soap_step, state_shapes
 
 
+SHARED_STEPS = 8        # small matrices whose steps share launches (as many as one launch takes)
+
+
 def _apply(pairs, lr: float, weight_decay: float) -> None:
     """Decoupled weight decay, then the update, of several ``(p, update)``."""
     if pairs and pairs[0][0].is_cuda:
@@ -120,7 +123,7 @@ class SoapTP(torch.optim.Optimizer):
         world, rank = dist.get_world_size(), dist.get_rank()
         for group in self.param_groups:
             lr, wd = group["lr"], group["weight_decay"]
-            together = []        # small matrices on an ordinary step
+            together, polled = [], None        # small matrices on an ordinary step
             for p in group["params"]:
                 if p.grad is None:
                     continue
@@ -145,6 +148,9 @@ class SoapTP(torch.optim.Optimizer):
                     continue
                 if world == 1 and self._shares_launches(p, state, plan, group):
                     together.append((p, (gradient, state, *plan["global_shape"])))
+                    polled = p.device
+                    if len(together) == SHARED_STEPS:
+                        self._step_together(together, group)
                     continue
                 if plan["replicated"] and world > 1:
                     gradient = gradient.chunk(world, dim=plan["shard_dim"])[rank].contiguous()
@@ -161,13 +167,23 @@ class SoapTP(torch.optim.Optimizer):
                     update = torch.cat(parts, dim=plan["shard_dim"])
                 _apply([(p, update)], lr, wd)
             if together:
-                from .engine import kernels, local
+                self._step_together(together, group)
+            if polled is not None:
+                from .engine import kernels
 
-                updates = local.shared_steps([arguments for _, arguments in together], beta=group["shampoo_beta"],
-                                             beta1=group["betas"][0], beta2=group["betas"][1], eps=group["eps"])
-                _apply([(p, update.view(p.grad.shape)) for (p, _), update in zip(together, updates)], lr, wd)
-                kernels.poll_status(together[0][0].device)
+                kernels.poll_status(polled)
         return loss
+
+    @staticmethod
+    def _step_together(together: list, group: dict) -> None:
+        """Takes the steps in ``together``, applies their updates and empties it.  As many as share launches at a time: no more
+        updates are held than that, and a step whose launches fail leaves none behind whose state has moved on without it."""
+        from .engine import local
+
+        updates = local.shared_steps([arguments for _, arguments in together], beta=group["shampoo_beta"],
+                                     beta1=group["betas"][0], beta2=group["betas"][1], eps=group["eps"])
+        _apply([(p, update.view(p.grad.shape)) for (p, _), update in zip(together, updates)], group["lr"], group["weight_decay"])
+        together.clear()
 
     @staticmethod
     def _shares_launches(p: Tensor, state: dict, plan: dict, group: dict) -> bool:

@@ -68,3 +68,61 @@ def test_steps_that_share_launches_write_no_scratch_of_each_other(groups, shapes
     for i, mine in enumerate(storages):
         for theirs in storages[:i]:
             assert mine.isdisjoint(theirs)
+
+
+@pytest.fixture
+def optimizer(groups, monkeypatch):
+    """Makes an optimizer whose small matrices share launches, and records which of them are updated."""
+    import torch.distributed as dist
+
+    from soap_tp_b200 import optim
+
+    if not dist.is_initialized():
+        dist.init_process_group("gloo", store=dist.HashStore(), rank=0, world_size=1)
+    applied = []
+    monkeypatch.setattr(optim, "_apply", lambda pairs, lr, decay: applied.extend(p for p, _ in pairs))
+    monkeypatch.setattr(optim.SoapTP, "_shares_launches", staticmethod(
+        lambda p, state, plan, group: local.shares_launches(state, *plan["global_shape"], group["precondition_frequency"])))
+    monkeypatch.setattr(k, "poll_status", lambda device: None)
+
+    def make(parameters, **options):
+        made = optim.SoapTP(parameters, **options)
+        for p in parameters:
+            p.grad = torch.zeros_like(p)
+            made.state[p] = _state(*p.shape)
+        return made
+
+    yield make, applied
+    dist.destroy_process_group()
+
+
+@pytest.mark.parametrize("count,fails", [(20, 1), (20, 2), (9, 1), (20, None)])
+def test_updates_are_applied_launch_by_launch(groups, optimizer, monkeypatch, count, fails):
+    """No more of them wait than a launch takes, and where a later launch fails every state that has advanced was applied."""
+    make, applied = optimizer
+    parameters = [torch.nn.Parameter(torch.zeros(16, 24)) for _ in range(count)]
+    soap = make(parameters, precondition_frequency=1000)
+    waiting = []
+
+    def launch(calls, *tail):
+        if len(waiting) == fails:
+            raise torch.OutOfMemoryError("out of memory")
+        waiting.append(sum(len(group) for group in groups) + len(calls) - len(applied))
+        groups.append(calls)
+
+    monkeypatch.setattr(k._C, "steady_steps", launch)
+    if fails is None:
+        soap.step()
+        assert len(applied) == count
+    else:
+        with pytest.raises(torch.OutOfMemoryError):
+            soap.step()
+    assert max(waiting) <= k._C.STEP_GROUP
+    for p in parameters:
+        assert (soap.state[p]["step"] == 5) == any(p is other for other in applied)
+
+
+def test_as_many_steps_are_collected_as_one_launch_takes():
+    from soap_tp_b200 import optim
+
+    assert optim.SHARED_STEPS == k._C.STEP_GROUP
