@@ -146,6 +146,8 @@ class SoapTP(torch.optim.Optimizer):
                         update = update.T
                     _apply([(p, update)], lr, wd)
                     continue
+                if any(p is other for other, _ in together):
+                    self._step_together(together, group)      # (a group may hold a parameter twice: one step after the other)
                 if world == 1 and self._shares_launches(p, state, plan, group):
                     together.append((p, (gradient, state, *plan["global_shape"])))
                     polled = p.device

@@ -126,3 +126,25 @@ def test_as_many_steps_are_collected_as_one_launch_takes():
     from soap_tp_b200 import optim
 
     assert optim.SHARED_STEPS == k._C.STEP_GROUP
+
+
+def test_a_parameter_that_a_group_holds_twice(groups, optimizer, monkeypatch):
+    """It takes one step after the other: never two in one launch, and the second one is a refresh where its count says so."""
+    from soap_tp_b200 import optim
+
+    make, applied = optimizer
+    p, q = (torch.nn.Parameter(torch.zeros(16, 24)) for _ in range(2))
+    refreshed = []
+
+    def refresh(gradient, state, **options):
+        refreshed.append(int(state["step"]) + 1)
+        state["step"] += 1
+        return torch.zeros(16, 24)
+
+    monkeypatch.setattr(optim, "soap_step", refresh)
+    with pytest.warns(UserWarning, match="duplicate"):
+        soap = make([p, q, p, q, p], precondition_frequency=7)
+    soap.step()
+    assert [len(calls) for calls in groups] == [2, 2] and refreshed == [7]
+    assert soap.state[p]["step"] == 7 and soap.state[q]["step"] == 6
+    assert len(applied) == 5
