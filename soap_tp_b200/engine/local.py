@@ -352,7 +352,7 @@ def _native_step(gradient: Tensor, state, step: int, rows: int, cols: int, *, be
 
 def shares_launches(state, rows: int, cols: int, interval: int) -> bool:
     """Whether the next step of this parameter is an ordinary one whose launches it can share with other small parameters'."""
-    return (k.MIXED_CORRECTIONS and not TIMER.enabled and "left_basis" in state and (int(state["step"]) + 1) % interval != 0
+    return (k.MIXED_CORRECTIONS and not TIMER.enabled and "left_basis" in state and interval > 0 and (int(state["step"]) + 1) % interval != 0
             and _C.steady_step_shares(rows, cols))
 
 

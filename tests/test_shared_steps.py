@@ -148,3 +148,14 @@ def test_a_parameter_that_a_group_holds_twice(groups, optimizer, monkeypatch):
     assert [len(calls) for calls in groups] == [2, 2] and refreshed == [7]
     assert soap.state[p]["step"] == 7 and soap.state[q]["step"] == 6
     assert len(applied) == 5
+
+
+@pytest.mark.parametrize("interval", [0, -1, -7])
+def test_an_interval_that_is_refused_stays_refused(groups, optimizer, interval):
+    make, applied = optimizer
+    p = torch.nn.Parameter(torch.zeros(16, 24))
+    soap = make([p], precondition_frequency=5)
+    soap.param_groups[0]["precondition_frequency"] = interval
+    with pytest.raises(ValueError, match="must be positive"):
+        soap.step()
+    assert groups == [] and applied == [] and soap.state[p]["step"] == 4
