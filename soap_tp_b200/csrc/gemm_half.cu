@@ -666,8 +666,7 @@ void mixed_maps(CUtensorMap (&maps)[2], const SplitTarget& planes, int64_t K, in
   maps[1] = encode_interleaved(planes.hl, K, cols, planes.ld16, 2 * kMixedBK, 128);
 }
 
-bool half_on_pairs(int M, int N, bool symmetric) {
-  if (!gemm_cta_pairs_wanted()) return false;
+bool half_fills_pairs(int M, int N, bool symmetric) {
   // A pair's 256 x 256 tile takes about 1.5 times as long as a CTA's 128 x 128 one (it loads half as much per product): pairs
   // unless single CTAs get by with so few waves that they finish earlier.  Pairs against singles, two terms: 1024^3 27 and
   // 20 us, 1536^3 34 and 27, 1792^3 40 and 58, 2048^3 44 and 64, 3072^3 132 and 178, 4096^3 319 and 409; symmetric, two terms and one: 1024
@@ -678,6 +677,8 @@ bool half_on_pairs(int M, int N, bool symmetric) {
   };
   return 3 * ((tiles_of(256) + 73) / 74) <= 2 * ((tiles_of(128) + 147) / 148);
 }
+
+bool half_on_pairs(int M, int N, bool symmetric) { return gemm_cta_pairs_wanted() && half_fills_pairs(M, N, symmetric); }
 
 namespace {
 // Checks a product and fills what its kernel reads.

@@ -62,7 +62,8 @@ struct HalfProblem {
   SplitTarget mixed;
 };
 
-// Whether such a product runs on CTA pairs where it does not say.
+// Whether such a product is large enough for CTA pairs, and whether it runs on them where it does not say (the pair switch may be off).
+bool half_fills_pairs(int M, int N, bool symmetric);
 bool half_on_pairs(int M, int N, bool symmetric);
 
 void gemm_half(const HalfOperand& a, const HalfOperand& b, const HalfProblem& prob, int* status, cudaStream_t stream);
@@ -163,8 +164,8 @@ struct SteadyStep {
 };
 constexpr int kStepPlanes = 1, kStepForward = 2, kStepBackward = 4, kStepAverages = 8;
 void steady_step(const SteadyStep& s, int* status, cudaStream_t stream);
-// Whether every product of such a step runs on single CTAs, so that several small parameters can share its launches; and the
-// steps of up to kHalfGroup such parameters (all phases; scratch of their own each).
+// Whether no product of such a step is large enough for CTA pairs, whether they are in use or not, so that several small parameters
+// can share its launches; and the steps of up to kHalfGroup such parameters (all phases; scratch of their own each).
 bool steady_step_shares(int rows, int cols);
 // Whether both averages of a step run on single CTAs, and so in one launch.
 bool averages_share(int rows, int cols);

@@ -171,7 +171,8 @@ void steady_step(const SteadyStep& s, int* status, cudaStream_t stream) {
 bool averages_share(int rows, int cols) { return !half_on_pairs(rows, rows, true) && !half_on_pairs(cols, cols, true); }
 
 bool steady_step_shares(int rows, int cols) {
-  return rows > 0 && cols > 0 && !half_on_pairs(cols, rows, false) && !half_on_pairs(rows, cols, false) && averages_share(rows, cols);
+  return rows > 0 && cols > 0 && !half_fills_pairs(cols, rows, false) && !half_fills_pairs(rows, cols, false) &&
+         !half_fills_pairs(rows, rows, true) && !half_fills_pairs(cols, cols, true);
 }
 
 void steady_steps(const SteadyStep* steps, int count, int* status, cudaStream_t stream) {

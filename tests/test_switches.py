@@ -25,6 +25,15 @@ def test_products_of_fp16_pairs_honour_the_pair_switch(size, restored):
     assert not k._C.half_on_pairs(*size)
 
 
+@pytest.mark.parametrize("shape,small", [((512, 1376), True), ((1, 1), True), ((128, 2048), True), ((2048, 2048), False),
+                                         ((8192, 8192), False), ((128, 14336), False), ((14336, 64), False)])
+@pytest.mark.parametrize("pairs", [True, False])
+def test_which_steps_share_launches_does_not_hang_on_the_pair_switch(shape, small, pairs, restored):
+    """Each step of a shared launch has scratch of its own, which large matrices cannot afford."""
+    k.use_cta_pairs(pairs)
+    assert k._C.steady_step_shares(*shape) is small
+
+
 def test_the_pair_switch_of_the_environment():
     code = "from soap_tp_b200.engine import kernels as k; print(k._C.half_on_pairs(8192, 8192, False))"
     for value, expected in (("0", "False"), ("1", "True")):
