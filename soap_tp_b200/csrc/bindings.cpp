@@ -84,7 +84,7 @@ struct BasisOperands {
     int i = 0;
     for (HalfOperand* o : {&plain, &turned}) {
       *o = in.operand();
-      if (o->h) {
+      if (o->h && size > 0) {      // (nothing reads the planes of an empty basis, and there is no map of them)
         half_maps(maps[i], o->h, o->l, o->ld, size, size);
         o->maps = maps[i];
       }

@@ -47,3 +47,27 @@ def test_row_sharded_gram_updates_validate_their_arguments():
 
     with pytest.raises(ValueError):
         gram_1d.update_left_preconditioner_from_col_shards(torch.zeros(4, 2), None, 0.5)   # no process group
+
+
+@pytest.mark.parametrize("turned", [False, True])
+def test_the_basis_of_an_empty_side_is_taken(turned):
+    """There is no tensor map of it (and none is asked for: making one needs a driver)."""
+    from soap_tp_b200.engine import kernels as k
+    from soap_tp_b200.engine import local
+
+    basis = torch.zeros(1, 1)[:0, :0]
+    planes = k.HalfPlanes.empty(0, 0, basis.device)
+    here = planes.operand()
+    k._C.BasisOperands(0, (local._NO_OPERAND + here if turned else here + local._NO_OPERAND) + (basis.data_ptr(), *basis.stride()))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(0, 5), (5, 0), (0, 0)])
+@pytest.mark.parametrize("direction", ["forward", "backward"])
+def test_the_rotation_of_an_empty_matrix_does_nothing(shape, direction):
+    from soap_tp_b200.engine import local
+
+    packed = lambda m, n: torch.ones(max(1, n), max(1, m), device="cuda").T
+    matrix = packed(*shape)
+    assert local.rotate(matrix, packed(shape[0], shape[0]), packed(shape[1], shape[1]), shape, direction) is matrix
+    assert bool((matrix == 1).all())
