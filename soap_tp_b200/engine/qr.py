@@ -134,7 +134,7 @@ def householder_qr_pair(jobs, beside=None, starts=None) -> None:
     ``jobs`` is a list of ``(matrix, Q, column_order)``.  Each factorisation is issued panel by panel on
     its own stream, alternating between the jobs, so that the latency-bound panel kernel of one
     factorisation (a few dozen thread blocks) runs while the tensor-core updates of the other keep the
-    remaining SMs busy.  The calling stream waits for all of them.
+    remaining SMs busy.  The calling stream waits for all of them, also where issuing them fails half-way.
 
     ``starts``: one event per job, recorded on the calling stream where its matrix and order were complete (by default, now).
     ``beside``: called once the first panels are issued; what it gives the calling stream runs beside the factorisations, whose
@@ -159,21 +159,27 @@ def householder_qr_pair(jobs, beside=None, starts=None) -> None:
         streams.append(stream)
         steps.append(_factorisation_steps(matrix, Q, order, slot, readers=readers if beside is not None else None))
     alive = list(range(len(jobs)))
-    while alive:
-        for slot in list(alive):
-            with torch.cuda.stream(streams[slot]):
-                try:
-                    next(steps[slot])
-                except StopIteration:
-                    alive.remove(slot)
-        if beside is not None:
-            beside()
-            readers.record(main)
-            beside = None
-    for stream in streams:
-        done = torch.cuda.Event()
-        done.record(stream)
-        main.wait_event(done)
+    try:
+        while alive:
+            for slot in list(alive):
+                with torch.cuda.stream(streams[slot]):
+                    try:
+                        next(steps[slot])
+                    except StopIteration:
+                        alive.remove(slot)
+            if beside is not None:
+                beside()
+                readers.record(main)
+                beside = None
+    except BaseException:
+        # what has been issued reads tensors that the caller now lets go of (the orders of the columns), and writes scratch
+        streams += [stream for key, stream in _PANEL_STREAMS.items() if key[0] == str(device)]
+        raise
+    finally:
+        for stream in streams:
+            done = torch.cuda.Event()
+            done.record(stream)
+            main.wait_event(done)
 
 
 def _q_stream(device, slot: int) -> "torch.cuda.Stream":
