@@ -81,7 +81,8 @@ def check_status(device: Optional[torch.device] = None) -> None:
         code = int(word[0].item())
         if code != 0:
             word.zero_()
-            _MONITORS.pop(index, None)
+            if index in _MONITORS:
+                _MONITORS.pop(index).finish()
             _raise_for(index, code)
 
 
@@ -123,6 +124,12 @@ class _StatusMonitor:
             self.words[self.turn].copy_(word[:1])
         self.pending[self.turn] = True
         self.turn = previous
+
+    def finish(self) -> None:
+        """Waits for the copy in flight, on whatever stream: its pinned memory goes back to an allocator that does not know of it."""
+        for event, pending in zip(self.events or (), self.pending):
+            if pending:
+                event.synchronize()
 
 
 _MONITORS: Dict[int, _StatusMonitor] = {}

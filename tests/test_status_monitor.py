@@ -112,3 +112,30 @@ def test_windows_of_operand_planes_are_cached_views():
     hi[2, 4] = -1.0                                   # a window is a view: it sees what is written to the parent
     assert float(window.hi[0, 0]) == -1.0
     assert window.dense().shape == (4, 3)
+
+
+def test_a_monitor_is_dropped_after_its_copy_has_landed(monkeypatch):
+    """The copy may be on another stream than the one that ``check_status`` synchronises."""
+    class Event:
+        def __init__(self):
+            self.recorded = self.waited = False
+
+        def record(self):
+            self.recorded = True
+
+        def synchronize(self):
+            self.waited = True
+
+    word = torch.zeros(4, dtype=torch.int32)
+    monitor = kernels._StatusMonitor(0, on_device=False)
+    monitor.events = [Event(), Event()]
+    monkeypatch.setattr(kernels, "_STATUS", {0: word})
+    monkeypatch.setattr(kernels, "_MONITORS", {0: monitor})
+    monkeypatch.setattr(kernels, "_stream", lambda: 0)
+    monkeypatch.setattr(kernels._C, "read_status", lambda *arguments: None)
+    monitor.poll(word)
+    word[0] = 1
+    with pytest.raises(kernels.SoapKernelError):
+        kernels.check_status()
+    assert kernels._MONITORS == {}
+    assert [event.waited for event in monitor.events] == [event.recorded for event in monitor.events] == [True, False]
