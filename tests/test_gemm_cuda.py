@@ -385,3 +385,43 @@ def test_terms_of_exact_operands_left_out(M, N, K):
         results.append((out, momentum, variance, planes.hi[:N, :M]))
     for x, y in zip(*results):
         assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("M", [256, 300])
+@pytest.mark.parametrize("K,splits", [(160, 4), (32, 3), (257, 7)])
+def test_parts_of_a_split_that_are_empty(M, K, splits):
+    """Zeros on CTA pairs as on single CTAs."""
+    from soap_tp_b200.engine import kernels as k
+
+    device, g = torch.device("cuda", 0), torch.Generator(device="cuda").manual_seed(M + K)
+    N = 128 * 200 + 5
+    a, b = (k.split_planes(torch.randn(K, n, generator=g, device=device)) for n in (M, N))
+    single, pairs = (torch.full((splits, N, M), float("nan"), device=device) for _ in range(2))
+    for part, force in ((single, True), (pairs, False)):
+        k.gemm(a, b, out=part[0].T, out_ld=M, k_splits=splits, split_stride=M * N, force_narrow=force)
+    assert torch.equal(single, pairs)
+    groups = -(-K // 32)
+    per_part = -(-groups // splits)
+    empty = -(-groups // per_part)
+    assert empty < splits and not bool(pairs[empty:].any()) and bool(pairs[empty - 1].any())
+
+
+@pytest.mark.parametrize("value", [float("inf"), -float("inf"), float("nan")])
+def test_what_is_not_finite_stays_so_without_the_terms_of_exact_operands(value):
+    """The remainder of an infinity is not a zero.  Without it a column that meets one is an infinity or NaN still, and no other
+    column changes."""
+    from soap_tp_b200.engine import kernels as k
+
+    g = torch.Generator(device="cuda").manual_seed(0)
+    A, B = torch.randn(200, 300, generator=g, device="cuda"), torch.randn(200, 140, generator=g, device="cuda").bfloat16()
+    B[17, 5] = value
+    a, b = k.split_planes(A, mixed=True), k.Planes.empty(200, 140, A.device, mixed=True)
+    k.split_planes_both(B, b, None)
+    results = []
+    for exact in (False, True):
+        out = torch.zeros(140, 300, device="cuda").T
+        k.gemm(a, b, out=out, second_exact=exact)
+        results.append(out)
+    for out in results:
+        assert not bool(out[:, 5].isfinite().any()) and bool(out[:, :5].isfinite().all()) and bool(out[:, 6:].isfinite().all())
+    assert torch.equal(results[0][:, :5], results[1][:, :5]) and torch.equal(results[0][:, 6:], results[1][:, 6:])

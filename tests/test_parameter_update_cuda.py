@@ -91,3 +91,24 @@ def test_apply_several_at_once(dtype, count):
         expected[a:a + n].mul_(0.99).add_(update.to(dtype), alpha=-3e-3)
     assert k.apply_updates(pairs, 0.99, 3e-3) == []
     assert torch.equal(flat, expected)
+
+
+def test_what_a_shared_update_does_not_take_comes_back_untouched():
+    """Parameters of both types and tensors that the kernel does not take, mixed: exactly these are returned."""
+    from soap_tp_b200.engine import kernels as k
+
+    g = torch.Generator().manual_seed(2)
+    values = lambda *shape: torch.randn(*shape, generator=g).cuda()
+    taken = [(values(*shape).to(dtype), values(*shape)) for shape in ((7, 5), (33,), (64, 130)) for dtype in (torch.float32, torch.bfloat16)]
+    refused = [(values(4, 6).double(), values(4, 6)), (values(4, 6), values(6, 4).T), (values(4, 6)[:, ::2], values(4, 3)),
+               (values(4, 6), values(4, 6).bfloat16())]
+    pairs = [pair for four in zip(refused, taken) for pair in four] + taken[len(refused):]
+    before = [p.clone() for p, _ in refused]
+    expected = []
+    for p, update in taken:
+        expected.append(p.clone())
+        expected[-1].mul_(0.99).add_(update.to(p.dtype), alpha=-0.1)
+    left = k.apply_updates(pairs, 0.99, 0.1)
+    assert [id(p) for p, _ in left] == [id(p) for p, _ in refused]
+    assert all(torch.equal(p, old) for (p, _), old in zip(refused, before))
+    assert all(torch.equal(p, new) for (p, _), new in zip(taken, expected))

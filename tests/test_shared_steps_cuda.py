@@ -161,3 +161,19 @@ def test_steps_in_the_mixed_form_that_have_sides_in_common(dtype, spread):
 
     scratches = _assert_shared_equals_alone(shapes, gradient)
     assert len(scratches) == len(shapes) and all(int(scratch.wide) == 1 for scratch in scratches)
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_a_gradient_that_is_not_finite_among_others(value, dtype):
+    """Its own step is what it would be alone, and so are the others'."""
+    shapes = [(64, 64), (160, 64), (130, 70), (64, 160)]
+
+    def gradient(i, turn):
+        grad = torch.randn(*shapes[i], generator=torch.Generator().manual_seed(20 * turn + i))
+        if i == 1:
+            grad[3, 4] = value
+        return grad.to(dtype).cuda()
+
+    scratches = _assert_shared_equals_alone(shapes, gradient)
+    assert sorted(int(scratch.wide) for scratch in scratches) == [0, 0, 0, 1]
