@@ -19,10 +19,11 @@ instead (``csrc/gemm_half.h``, ``RangeGuard``).  With ``SOAP_TP_MIXED_CORRECTION
 """
 from __future__ import annotations
 
+import functools
 import math
 import os
 import weakref
-from collections import OrderedDict
+from collections import Counter, OrderedDict
 from typing import Any, Dict, MutableMapping, Optional, Tuple
 
 import torch
@@ -356,6 +357,18 @@ def shares_launches(state, rows: int, cols: int, interval: int) -> bool:
             and _C.steady_step_shares(rows, cols))
 
 
+@functools.lru_cache(maxsize=1024)
+def _scratch_numbers(shapes: tuple) -> tuple:
+    """Which sets of scratch matrices of these shapes take that run together (``_Scratch``, ``slots``): each has its own, those of one
+    shape, and of the mixed form of bases of one size whatever the other side (workspaces of other tags or sizes are others)."""
+    whole, lefts, rights, numbers = Counter(), Counter(), Counter(), []
+    for rows, cols in shapes:
+        numbers.append((whole[rows, cols], lefts[rows], rights[cols]))
+        for count, key in ((whole, (rows, cols)), (lefts, rows), (rights, cols)):
+            count[key] += 1
+    return tuple(numbers)
+
+
 def shared_steps(parameters, *, beta: float, beta1: float, beta2: float, eps: float) -> list:
     """Ordinary steps of several small parameters, ``(gradient, state, rows, cols)`` each, on one device; their updates.
 
@@ -367,14 +380,9 @@ def shared_steps(parameters, *, beta: float, beta1: float, beta2: float, eps: fl
     updates = []
     for first in range(0, len(parameters), _C.STEP_GROUP):
         some = parameters[first:first + _C.STEP_GROUP]
-        calls, held, used = [], [], {}
-        for gradient, state, rows, cols in some:
-            # What runs together has scratch of its own each: parameters of one shape, and the mixed form of bases of one size
-            # whatever the other side (workspaces of different tags or sizes are different ones).
-            keys = ((rows, cols), ("left", rows), ("right", cols))
-            for key in keys:
-                used[key] = used.get(key, -1) + 1
-            slots = tuple(used[key] for key in keys)
+        calls, held = [], []
+        numbers = _scratch_numbers(tuple([(rows, cols) for _, _, rows, cols in some]))
+        for (gradient, state, rows, cols), slots in zip(some, numbers):
             call, update, holds = _native_arguments(gradient, state, int(state["step"]) + 1, rows, cols, True, slots, beta=beta,
                                                     beta1=beta1, beta2=beta2, eps=eps)
             calls.append(call)

@@ -123,7 +123,7 @@ class SoapTP(torch.optim.Optimizer):
         world, rank = dist.get_world_size(), dist.get_rank()
         for group in self.param_groups:
             lr, wd = group["lr"], group["weight_decay"]
-            together, polled = [], None        # small matrices on an ordinary step
+            together, polled = {}, None        # small matrices on an ordinary step, by their identities
             for p in group["params"]:
                 if p.grad is None:
                     continue
@@ -146,11 +146,11 @@ class SoapTP(torch.optim.Optimizer):
                         update = update.T
                     _apply([(p, update)], lr, wd)
                     continue
-                if any(p is other for other, _ in together):
+                if id(p) in together:
                     self._step_together(together, group)      # (a group may hold a parameter twice: one step after the other)
                 if world == 1 and self._shares_launches(p, state, plan, group):
-                    together.append((p, (gradient, state, *plan["global_shape"])))
-                    polled = p.device
+                    together[id(p)] = (p, (gradient, state, *plan["global_shape"]))
+                    polled = p
                     if len(together) == SHARED_STEPS:
                         self._step_together(together, group)
                     continue
@@ -173,18 +173,18 @@ class SoapTP(torch.optim.Optimizer):
             if polled is not None:
                 from .engine import kernels
 
-                kernels.poll_status(polled)
+                kernels.poll_status(polled.device)
         return loss
 
     @staticmethod
-    def _step_together(together: list, group: dict) -> None:
+    def _step_together(together: dict, group: dict) -> None:
         """Takes the steps in ``together``, applies their updates and empties it.  As many as share launches at a time: no more
         updates are held than that, and a step whose launches fail leaves none behind whose state has moved on without it."""
         from .engine import local
 
-        updates = local.shared_steps([arguments for _, arguments in together], beta=group["shampoo_beta"],
+        updates = local.shared_steps([arguments for _, arguments in together.values()], beta=group["shampoo_beta"],
                                      beta1=group["betas"][0], beta2=group["betas"][1], eps=group["eps"])
-        _apply([(p, update.view(p.grad.shape)) for (p, _), update in zip(together, updates)], group["lr"], group["weight_decay"])
+        _apply([(p, update.view(p.grad.shape)) for (p, _), update in zip(together.values(), updates)], group["lr"], group["weight_decay"])
         together.clear()
 
     @staticmethod
