@@ -22,14 +22,14 @@
 // graded and duplicated inputs keep the orthogonality of Q at the one-column kernel's level (the NumPy
 // restatement in utils/panel_pairs_reference.py shows 1e-3 without a guard, 2e-5 with a guard of 0.05).
 //
-// Bound by a chain of 64 steps of some 6900 cycles (5 CTAs; 9700 with 33): the exchange through L2 1800 (4300), sweep 1 1200,
-// pivot entries and publishing 1100, scalars and coefficients 1000, sweep 2 1200.  A warp owns one slice of 32 columns: a 16-byte
+// Bound by a chain of 64 steps of some 6900 cycles (5 CTAs that exchange through L2; 9700 with 33): the exchange 1800 (4300), sweep 1
+// 1200, pivot entries and publishing 1100, scalars and coefficients 1000, sweep 2 1200.  A warp owns one slice of 32 columns: a 16-byte
 // load of a pivot column is then one address for all lanes, 1.55 cycles of shared memory instead of the 2.2 that four slices in a
-// warp took (sweep 1 was 2130 cycles).  Panels of 1024 / 3000 / 8192 rows 324 / 329 / 411 us with four slices a warp, element-wise
-// loads and outputs staged through shared memory; 263 / 285 / 364 us now.
+// warp took (sweep 1 was 2130 cycles).  Panels of 1024 / 3000 / 8192 rows, exchanging through L2: 324 / 329 / 411 us with four slices
+// a warp, element-wise loads and outputs staged through shared memory; 263 / 285 / 364 us so.  (As a cluster, see kCluster: 230 / 280.)
 //
-// Register tiling, exchange words ({value, sequence} in 64 bits, bounded polls), T construction by
-// CTA 0 in the shadow of the exchange and the output stage are those of qr.cu.
+// Exchange words ({value, sequence} in 64 bits, bounded polls) are those of qr.cu.  T is built in the shadow of the exchange by the last
+// CTA, which has no rows of its own where a launch has more than one and room for one more.
 #include <cuda_runtime.h>
 
 #include <atomic>
@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(kPanelThreads, 1) qr_panel_pairs_kernel(PanelA
   const unsigned int seq_base = a.epoch * 256u;
   float my_scale = 1.f;                  // 1 / (alpha - beta) of this lane's column once it has been a pivot
   int c = 0, step = 0;
-  int built_c = -1, built_pair = 0;      // columns of T that CTA 0 still owes from the previous step
+  int built_c = -1, built_pair = 0;      // columns of T that the last CTA still owes from the previous step
 
   while (c < reflectors) {
     const int parity = step & 1;
@@ -207,7 +207,8 @@ __global__ void __launch_bounds__(kPanelThreads, 1) qr_panel_pairs_kernel(PanelA
     const bool mine2 = local2 >= 0 && local2 < kPer && row2_exists;
 
     if constexpr (kCluster) {
-      // (a step's bytes cannot arrive before the step before has ended here: its senders wait for this CTA's)
+      // Bytes of this step may be here already: a sender needs this CTA's sums of the step before, not its end.  The phase stays open all
+      // the same until this arrival, and the buffer of this parity was read before this CTA sent those sums.
       if (t == 0) mbar_expect_tx(&inbox.arrived[parity], static_cast<uint32_t>(kB * (8 * ctas + (row2_exists ? 8 : 4))));
     }
 
@@ -268,7 +269,7 @@ __global__ void __launch_bounds__(kPanelThreads, 1) qr_panel_pairs_kernel(PanelA
                    : "memory");
     }
 
-    // ---- CTA 0, while the published words travel: the columns of T the previous step produced ----
+    // ---- the last CTA, while the published words travel: the columns of T the previous step produced ----
     if (builds_t && built_c >= 0) {
       t_column(T, scol1, taus, built_c, t);
       if (built_pair) {
@@ -476,7 +477,7 @@ __global__ void __launch_bounds__(kPanelThreads, 1) qr_panel_pairs_kernel(PanelA
 
   if (a.trace && blockIdx.x == 0 && t == 0) a.trace[0] = step;   // diagnostics: exchange steps taken
 
-  // ---- CTA 0: the columns of T of the last step, then T and T^T as operand planes ----
+  // ---- the last CTA: the columns of T of the last step, then T and T^T as operand planes ----
   if (builds_t && !abort_flag) {
     if (built_c >= 0) {
       t_column(T, scol1, taus, built_c, t);

@@ -7,8 +7,9 @@
 // The chain stays on the caller's stream: its first product then overlaps the tail of the operand planes, which an event
 // between streams does not allow.  Device time of a step, everything on one stream / the chain beside / the averages beside:
 // 256 x 512 126 / 92 / 85 us, 512 x 1376 175 / 158 / 121 us, 1000 x 1501 198 / 198 / 148 us, 2048 x 5504 1388 / 1352 / 1186 us,
-// 4096 x 4096 1900 / 1863 / 1748 us, 8192 x 8192 within the runs' spread.  (As measured when they were moved; the averages beside, since then:
-// 256 x 512 59 us, 1000 x 1501 122, 2048 x 5504 1042, 4096 x 4096 1493.)
+// 4096 x 4096 1900 / 1863 / 1748 us, 8192 x 8192 within the runs' spread.  (As measured when they were moved.  Since then, steps one after
+// another that the host has issued far ahead, everything on one stream / the averages beside: 512 x 1376 127 / 102 us, 1000 x 1501 bf16
+// 155 / 132, 2048 x 5504 bf16 1172 / 1059, 4096 x 4096 bf16 1644 / 1557.)
 #include <algorithm>
 #include <optional>
 #include <stdexcept>

@@ -175,8 +175,8 @@ MIXED_CORRECTIONS = os.environ.get("SOAP_TP_MIXED_CORRECTIONS", "1") != "0"
 
 
 def use_cta_pairs(on: bool) -> None:
-    """Large plain products (tf32 planes: at least 148 tiles of 128 x 256, no batching, no split-K; fp16 pairs: where they need
-    fewer waves that way) run on CTA pairs (``cta_group::2``: 256 x 256 tiles, each CTA staging half of the B tile) unless
+    """Large plain products (tf32 planes: at least 148 tiles of 128 x 256, each part of a split counted, no batching; fp16
+    pairs: where they need fewer waves that way) run on CTA pairs (``cta_group::2``: 256 x 256 tiles, each CTA staging half of the B tile) unless
     switched off here or with ``SOAP_TP_GEMM_CTA_PAIRS=0``."""
     _C.gemm_use_cta_pairs(bool(on))
 

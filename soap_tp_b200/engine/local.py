@@ -514,10 +514,11 @@ _WARMED: Dict[Any, bool] = {}
 
 
 def warm_refresh_kernels(device, sizes=()) -> None:
-    """Launch every kernel variant a refresh uses once, on a tiny problem.
+    """Launch the kernels of a refresh once, on a tiny problem.
 
     CUDA loads a kernel's code the first time it is launched; without this the first refresh of a
-    training run pays tens of milliseconds of module loading in the middle of a step.  The eigenvalue-order sort
+    training run pays tens of milliseconds of module loading in the middle of a step.  (The tiles that products take at larger
+    sizes are not among them: launching those here as well did not shorten a first refresh.)  The eigenvalue-order sort
     sizes its shared memory by length, so it is warmed at the real ``sizes``.
     """
     for size in sizes:

@@ -92,7 +92,7 @@ def _splits(tiles: int, k_blocks: int) -> int:
 
 
 def _skinny_product(ws: dict, a: k.Planes, b: k.Planes, out: k.Planes, scratch: str = "partials") -> None:
-    """``out <- a^T b`` for a narrow ``a`` (at most 128 columns): split-K partials + ordered sum."""
+    """``out <- a^T b`` for a narrow ``a`` (at most 256 columns): split-K partials + ordered sum."""
     M, N, K = a.cols, b.cols, a.depth
     splits = _splits(-(-N // 128), -(-K // 32))
     ld = M
@@ -284,7 +284,9 @@ def _factorisation_steps(matrix: Optional[Tensor], Q: Optional[Tensor], column_o
                      T.lo.data_ptr(), Tt.hi.data_ptr(), Tt.lo.data_ptr(), T.ld, ws["exchange"].data_ptr(),
                      status_pointer, side.cuda_stream)
         if PAIR_STEPS:
-            # 256-row CTAs: measured faster than (2048 rows and up) or within 2 % of (1024 rows) 128-row CTAs
+            # 256-row CTAs.  128-row ones are faster where all of them exchange as a cluster (1024 rows: 230 us against 189, 1536: 238
+            # and 223, 256: 278 and 168) and slower from there on (2048: 244 and 331, 3000: 283 and 357, 8192: 363 and 513), but add in
+            # another order; 256 rows everywhere were chosen when both exchanged through L2 (1024 rows: within 2 %).
             _C.qr_panel_pairs(*arguments, 256)
         else:
             _C.qr_panel(*arguments)
@@ -422,7 +424,8 @@ def _factorisation_steps(matrix: Optional[Tensor], Q: Optional[Tensor], column_o
         return
     # explicit Q = H_0 H_1 ... applied to the identity, last panel first.  The pairs' reflectors (seven small products, some 70 us
     # whatever the size) are made on a stream of their own, up to two pairs ahead of their use: refresh 3000 x 2000 10.27 -> 9.81 ms,
-    # 8192 x 8192 79.1 -> 76.3.  Not for a few pairs, where the host is as long over its launches as the device: 1024 x 1024 3.13 -> 3.22.
+    # 8192 x 8192 79.1 -> 76.3.  Not for a few pairs, where the host is as long over its launches as the device: 1024 x 1024 (4 pairs)
+    # 3.25 -> 3.63 ms in refreshes that follow one another, 2048 x 2048 (8) 6.22 -> 6.51, 2560 x 2560 (10) 8.41 -> 8.48.
     pairs = [p for p in reversed(range(len(panels))) if paired(p)]
     reflectors: Dict[int, tuple] = {}
     used: Dict[int, "torch.cuda.Event"] = {}
