@@ -25,6 +25,7 @@ on; ``load_state_dict()`` checks it and restores fp32 column-major buffers bit-e
 """
 from __future__ import annotations
 
+import functools
 from typing import Any, Dict, Iterable, Optional, Tuple
 
 import torch
@@ -40,12 +41,19 @@ from .step import soap_step, state_shapes
 SHARED_STEPS = 8        # small matrices whose steps share launches (as many as one launch takes)
 
 
+@functools.cache
+def _engine() -> tuple:
+    """The modules of the device engine, whose library a program on the CPU does without.  (Kept, since an import statement takes
+    half a microsecond however often it has run, and a step asked for them twice a parameter.)"""
+    from .engine import kernels, local
+
+    return kernels, local
+
+
 def _apply(pairs, lr: float, weight_decay: float) -> None:
     """Decoupled weight decay, then the update, of several ``(p, update)``."""
     if pairs and pairs[0][0].is_cuda:
-        from .engine import kernels
-
-        pairs = kernels.apply_updates(pairs, 1.0 - lr * weight_decay, lr)
+        pairs = _engine()[0].apply_updates(pairs, 1.0 - lr * weight_decay, lr)
     for p, update in pairs:
         if weight_decay != 0.0:
             p.mul_(1.0 - lr * weight_decay)
@@ -171,19 +179,15 @@ class SoapTP(torch.optim.Optimizer):
             if together:
                 self._step_together(together, group)
             if polled is not None:
-                from .engine import kernels
-
-                kernels.poll_status(polled.device)
+                _engine()[0].poll_status(polled.device)
         return loss
 
     @staticmethod
     def _step_together(together: dict, group: dict) -> None:
         """Takes the steps in ``together``, applies their updates and empties it.  As many as share launches at a time: no more
         updates are held than that, and a step whose launches fail leaves none behind whose state has moved on without it."""
-        from .engine import local
-
-        updates = local.shared_steps([arguments for _, arguments in together.values()], beta=group["shampoo_beta"],
-                                     beta1=group["betas"][0], beta2=group["betas"][1], eps=group["eps"])
+        updates = _engine()[1].shared_steps([arguments for _, arguments in together.values()], beta=group["shampoo_beta"],
+                                            beta1=group["betas"][0], beta2=group["betas"][1], eps=group["eps"])
         _apply([(p, update.view(p.grad.shape)) for (p, _), update in zip(together.values(), updates)], group["lr"], group["weight_decay"])
         together.clear()
 
@@ -195,10 +199,8 @@ class SoapTP(torch.optim.Optimizer):
                 or group["basis_implementation"] not in BASIS_IMPLEMENTATIONS or "left_basis" not in state
                 or profile_enabled(int(state["step"]) + 1)):
             return False
-        from .engine import local
-
         rows, cols = plan["global_shape"]
-        return p.grad.numel() == rows * cols and local.shares_launches(state, rows, cols, group["precondition_frequency"])
+        return p.grad.numel() == rows * cols and _engine()[1].shares_launches(state, rows, cols, group["precondition_frequency"])
 
     def _adamw(self, p: Tensor, group: dict) -> None:
         state = self.state[p]
@@ -209,11 +211,9 @@ class SoapTP(torch.optim.Optimizer):
         state["step"] += 1
         beta1, beta2 = group["adamw_betas"]
         if p.is_cuda:
-            from .engine import kernels
-
-            if kernels.adamw_update(p, p.grad, state["exp_avg"], state["exp_avg_sq"], beta1, beta2, 1.0 - beta1 ** state["step"],
-                                    1.0 - beta2 ** state["step"], group["eps"], 1.0 - group["lr"] * group["weight_decay"],
-                                    group["lr"]):
+            if _engine()[0].adamw_update(p, p.grad, state["exp_avg"], state["exp_avg_sq"], beta1, beta2, 1.0 - beta1 ** state["step"],
+                                         1.0 - beta2 ** state["step"], group["eps"], 1.0 - group["lr"] * group["weight_decay"],
+                                         group["lr"]):
                 return
         grad = p.grad.float()
         state["exp_avg"].lerp_(grad, 1.0 - beta1)
