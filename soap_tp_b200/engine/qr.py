@@ -424,8 +424,10 @@ def _factorisation_steps(matrix: Optional[Tensor], Q: Optional[Tensor], column_o
         return
     # explicit Q = H_0 H_1 ... applied to the identity, last panel first.  The pairs' reflectors (seven small products, some 70 us
     # whatever the size) are made on a stream of their own, up to two pairs ahead of their use: refresh 3000 x 2000 10.27 -> 9.81 ms,
-    # 8192 x 8192 79.1 -> 76.3.  Not for a few pairs, where the host is as long over its launches as the device: 1024 x 1024 (4 pairs)
-    # 3.25 -> 3.63 ms in refreshes that follow one another, 2048 x 2048 (8) 6.22 -> 6.51, 2560 x 2560 (10) 8.41 -> 8.48.
+    # 8192 x 8192 79.1 -> 76.3; issued far ahead of the device 2560 x 2560 (10 pairs) 8.34 -> 8.13, 2048 x 2048 (8) 6.13 -> 5.94, 1024 x 1024
+    # (4) 2.87 -> 2.78.  It costs the host, though, which is as long over a small refresh as the device: where one follows another 1024 takes
+    # 3.63 ms instead of 3.25, 1792 (7) 5.70 for 5.32, 2048 6.51 for 6.22, 2560 8.48 for 8.41.  So from 8 pairs on, where it gives most of
+    # what it costs there.
     pairs = [p for p in reversed(range(len(panels))) if paired(p)]
     reflectors: Dict[int, tuple] = {}
     used: Dict[int, "torch.cuda.Event"] = {}
